@@ -232,3 +232,122 @@ def tolerance(case):
     if case["dtype"] == "tf32":
         return {"rel": 1e-4, "max": 5e-4}
     return {"rel": 7e-3, "max": 1.6e-2}
+
+
+# ---- what run() computes, in 64 bits and without the kernels --------------------------------------------------------
+
+E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0)
+
+
+def wrap(u):
+    """A 64-bit constant as the signed number that torch's wrapping int64 arithmetic takes."""
+    return u - (1 << 64) if u >> 63 else u
+
+
+def mix64(z):
+    """splitmix64's finaliser."""
+    z = z + wrap(0x9E3779B97F4A7C15)
+    z = (z ^ ((z >> 30) & ((1 << 34) - 1))) * wrap(0xBF58476D1CE4E5B9)
+    z = (z ^ ((z >> 27) & ((1 << 37) - 1))) * wrap(0x94D049BB133111EB)
+    return z ^ ((z >> 31) & ((1 << 33) - 1))
+
+
+def fma(a, b, c):
+    return (a.double() * b.double() + c).float()
+
+
+def log_f32(x):
+    """The generator's logarithm, one float32 operation after the other: x = m * 2^e, ln m = 2 atanh((m - 1) / (m + 1))."""
+    m, e = torch.frexp(x)
+    m, e = m * 2, e - 1
+    high = m > 1.41421354
+    m, e = torch.where(high, m * 0.5, m), torch.where(high, e + 1, e)
+    t = (m - 1) / (m + 1)
+    s = t * t
+    p = torch.full_like(t, 1 / 11)
+    for c in (1 / 9, 1 / 7, 1 / 5, 1 / 3, 1.0):
+        p = fma(p, s, float(np.float32(c)))
+    return fma(e.float(), torch.full_like(t, math.log(2)), (2 * t * p).double())
+
+
+def cos_2pi_f32(u):
+    q = u * 4
+    k = q.to(torch.int32)
+    th = (q - k) * 1.57079637
+    s = th * th
+    c, n = torch.full_like(s, -1 / math.factorial(14)), torch.full_like(s, -1 / math.factorial(15))
+    for i in range(6, -1, -1):
+        sign = -1.0 if i & 1 else 1.0
+        c = fma(c, s, float(np.float32(sign / math.factorial(2 * i))))
+        n = fma(n, s, float(np.float32(sign / math.factorial(2 * i + 1))))
+    n = n * th
+    return torch.where(k == 0, c, torch.where(k == 1, -n, torch.where(k == 2, -c, n)))
+
+
+def normals(n, seed, wide=False):
+    """clpk_fill_f32's N(0, 0.02): as the float32 values that it is defined by, or (wide) as the deviate itself in 64 bits."""
+    base = int(mix64(torch.tensor(seed, dtype=torch.int64)))
+    out = torch.empty(n, dtype=torch.float64 if wide else torch.float32, device="cuda")
+    for at in range(0, n, 1 << 25):
+        h = mix64(torch.arange(at, min(n, at + (1 << 25)), dtype=torch.int64, device="cuda") + base)
+        u1, u2 = (((h >> 41) & 0x7FFFFF) + 1).double() / 2 ** 23, (h & 0xFFFFFF).double() / 2 ** 24
+        if wide:
+            v = 0.02 * torch.sqrt(-2 * torch.log(u1)) * torch.cos(2 * math.pi * u2)
+        else:
+            v = fma(torch.sqrt(-2 * log_f32(u1.float())) * cos_2pi_f32(u2.float()), torch.full_like(u1.float(), 0.02), 0.0)
+        out[at:at + v.numel()] = v
+    return out
+
+
+def e2m1(x):
+    """Nearest e2m1 value, ties to the even code: a tie goes up where the code below it is odd."""
+    codes = torch.tensor(E2M1, device=x.device)
+    code = torch.zeros(x.shape, dtype=torch.int64, device=x.device)
+    for i in range(7):
+        edge = (E2M1[i] + E2M1[i + 1]) / 2
+        code += (x.abs() >= edge) if i & 1 else (x.abs() > edge)
+    return codes[code].copysign(x)
+
+
+def operand_f64(dtype, rows, cols, seed):
+    """(the operand's decoded values in float64, its tensor scale)"""
+    f = normals(rows * cols, seed)
+    if dtype in ("f32", "f64"):
+        return f.double().view(rows, cols), 1.0
+    if dtype == "tf32":
+        b = f.view(torch.int32)
+        b = (b + 0xFFF + ((b >> 13) & 1)) & ~0x1FFF
+        return b.view(torch.float32).double().view(rows, cols), 1.0
+    plain = {"bf16": torch.bfloat16, "f16": torch.float16, "e4m3": torch.float8_e4m3fn, "e5m2": torch.float8_e5m2}
+    if dtype in plain:
+        return f.to(plain[dtype]).double().view(rows, cols), 1.0
+    blocks = f.view(-1, SCALE_BLOCK[dtype])
+    if dtype == "mxf4":
+        scale = 1.0
+        s = torch.ldexp(torch.ones_like(blocks[:, :1]), torch.frexp(blocks.abs().amax(1, keepdim=True))[1] - 3)
+    else:
+        scale = float(np.float32(f.abs().max().item()) / np.float32(6.0 * 448.0))
+        blocks = blocks / torch.tensor(scale, dtype=torch.float32, device=f.device)
+        s = (blocks.abs().amax(1, keepdim=True) / torch.tensor(6.0, device=f.device)).clamp(max=448.0).to(torch.float8_e4m3fn).float()
+    q = torch.where(s > 0, e2m1(blocks / s), torch.zeros_like(blocks))
+    return (q.double() * s.double()).view(rows, cols), scale
+
+
+def exact(case, seed):
+    """The floating results in 64 bits: products of the operands as they are quantised, and the deviates behind the generated
+    floats.  Whole-number products, bytes, and the streams' copies and sums have none."""
+    if case["path"] == "operands" and case["dtype"] != "i8":
+        out = {"f32": normals(case["rows"] * case["cols"], seed, wide=True)}
+        if case["dtype"] != "f32":
+            out["packed"] = None
+        if case["dtype"] in SCALE_BLOCK:
+            out.update(scales=None, tensor_scale=None)
+        return out
+    if case["path"] != "gemm" or case["dtype"] == "i8":
+        return None
+    dtype, m, n, k = case["dtype"], case["m"], case["n"], case["k"]
+    a, scale_a = operand_f64(dtype, m, k, 2 * seed)
+    b, scale_b = operand_f64("e4m3" if dtype == "e5m2" else dtype, n, k, 2 * seed + 1)
+    c = a @ b.T
+    c *= float(np.float32(np.float32(scale_a) * np.float32(scale_b)))
+    return {"c": c, "status": None}
