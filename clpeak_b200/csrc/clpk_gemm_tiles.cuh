@@ -1,0 +1,371 @@
+// The dense GEMM for shapes that do not fill the chip with 512 x 256 tiles (included by gemm.cu).
+//
+// Same pieces as gemm_kernel -- CTA pairs, TMA ring, elected-lane issue, bounded waits -- with the split of the work
+// left to the launch:
+//  * Tile 256 x TN per CTA pair, TN = 32 ... 256 in steps of 32, one M = 256 row block (CTA r holds its 128 rows).
+//  * K over 1, 2 or 4 pairs of one cluster.  Every pair accumulates its own K range in tensor memory; then the pairs
+//    exchange partial sums through distributed shared memory (each owns every splits-th 32-column chunk of the tile),
+//    add them in pair order -- the same order whoever owns the chunk -- and store what they own.  Nothing goes through
+//    global memory and no workspace is needed.
+//  * Unsplit tiles are walked persistently with two accumulators, so a tile's epilogue overlaps the next main loop.
+//
+// What bounds it: a K block (128 bytes of K) costs the issuing warps about 0.12 us whatever the tile -- barrier wait,
+// four instructions, commit -- against 0.17 us of tensor pipe at TN = 256, so narrow tiles are issue-bound and their
+// width is chosen for parallelism; wide ones come within 10 % of the operand traffic's floor.  Below 2 us per K range
+// the launch is the time: 3.5 us from one launch to the next.  Device time, operands in L2, 512 x 256 tiles -> this
+// kernel: bf16 512 x 256 x 512 10.2 -> 4.4 us, e4m3 1024 x 1024 x 2048 15.0 -> 6.4, bf16 2048^3 25.1 -> 15.3, e4m3
+// 128 x 8192 x 8192 42.4 -> 18.6, bf16 64 x 64 x 16384 147 -> 13.3.  Tried: four K blocks per stage (slower from
+// TN = 64 on), asking the next stage's barrier ahead of the instructions (no effect), clusters of 16 for eight splits
+// (10 % for single tiles of K > 8000, slower elsewhere).
+#pragma once
+
+constexpr int kTilesMaxStages = 16;
+constexpr uint32_t kTilesChunk = 32;                               // columns of C per tcgen05.ld and per TMA store box
+constexpr uint32_t kTilesM = 256;
+constexpr uint32_t kTilesSmemMax = 227 * 1024;
+
+struct TilesSmem {
+    uint64_t full[kTilesMaxStages];
+    uint64_t empty[kTilesMaxStages];
+    uint64_t tmem_full[2];
+    uint64_t tmem_empty[2];
+    uint32_t tmem_base;
+};
+
+struct TilesParams {
+    uint32_t tiles_m, tiles_n, group;
+    uint32_t k_blocks;                  // of 128 bytes
+    uint32_t tn, splits, stages;
+    uint32_t kps;                       // K blocks per stage: 1 or 2
+    uint32_t tmem_cols;                 // power of two: one accumulator, or two when a cluster has several tiles
+    float alpha;
+    uint32_t *status;
+    unsigned long long *clock;
+};
+
+// bytes of one K block in a CTA: its 128 rows of A and its half of the tile's rows of B
+__host__ __device__ constexpr uint32_t tiles_block_bytes(uint32_t tn) { return kHalfTileBytes + tn / 2 * kRowBytesK; }
+
+// 32 columns of one row per lane -> the warp's staging box (32 rows x 64 bytes of bf16 in the 64-byte swizzle, or
+// x 128 bytes of fp32 / int32 in the 128-byte swizzle) -> one TMA store that clips what lies beyond C.
+template <int DT>
+__device__ __forceinline__ void tiles_store_chunk(uint32_t (&r)[32], float alpha, uint8_t *boxes, uint32_t &n_stored,
+                                                  const CUtensorMap *tmap_c, uint32_t col, uint32_t row, int lane)
+{
+    if constexpr (OutBytes<DT>::value == 2) {
+        // two 2 KiB boxes in turn: the one filled now was handed to TMA two stores ago
+        uint8_t *box = boxes + (n_stored & 1) * 2048;
+        if (lane == 0)
+            bulk_wait_read<1>();
+        __syncwarp();
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
+            w[i] = *reinterpret_cast<uint32_t *>(&v);
+        }
+        uint8_t *my_row = box + lane * 64;
+        const uint32_t sw = (uint32_t)(lane >> 1) & 3;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++)
+            *reinterpret_cast<uint4 *>(my_row + ((j ^ sw) << 4)) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            tma_store_2d(tmap_c, box, (int32_t)col, (int32_t)row);
+            bulk_commit();
+        }
+    } else {
+        if constexpr (DT == CLPK_DT_TF32) {
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+                r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+        }
+        store_staged_box(r, boxes, tmap_c, col, row, lane);
+    }
+    n_stored++;
+}
+
+// Partial sums of a 32-column chunk in the owner's shared memory: [8 groups of 4 columns][128 rows][4 words], so that
+// a warp's 32 rows are 512 consecutive bytes per group on both sides.
+constexpr uint32_t kTilesChunkBytes = kTilesChunk * 128 * 4;
+
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, uint32_t cta)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(cta));
+    return a;
+}
+
+template <int DT>
+__global__ void __launch_bounds__(kGemmThreads)
+    gemm_tiles_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                      const __grid_constant__ CUtensorMap tmap_c, TilesParams p)
+{
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const uint32_t block_bytes = tiles_block_bytes(p.tn), stage_bytes = p.kps * block_bytes;
+    uint8_t *staging = smem + (size_t)p.stages * stage_bytes;
+    TilesSmem *sh = reinterpret_cast<TilesSmem *>(staging + kEpilogueWarps * kStagingBytes);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank(), r = rank & 1, leader = rank & ~1u, split = rank >> 1;
+    const uint32_t cluster_id = blockIdx.x / (2 * p.splits), n_clusters = gridDim.x / (2 * p.splits);
+    const uint32_t n_tiles = p.tiles_m * p.tiles_n;
+    const uint32_t kb0 = split * p.k_blocks / p.splits, kb1 = (split + 1) * p.k_blocks / p.splits;
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < p.stages; s++) {
+            mbar_init(&sh->full[s], 1);
+            mbar_init(&sh->empty[s], 1);
+        }
+        for (int acc = 0; acc < 2; acc++) {
+            mbar_init(&sh->tmem_full[acc], 1);
+            mbar_init(&sh->tmem_empty[acc], 2 * kEpilogueWarps);
+        }
+        mbar_fence_init();
+        tma_prefetch_desc(&tmap_a);
+        tma_prefetch_desc(&tmap_b);
+        tma_prefetch_desc(&tmap_c);
+    }
+    if (warp == 1)
+        tmem_alloc<2>(&sh->tmem_base, p.tmem_cols);
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after_sync();
+    const uint32_t tmem = sh->tmem_base;
+    griddep_wait();                        // see join_previous_launch
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *p.status = 0u;
+    griddep_launch_dependents();
+    const unsigned long long clk0 = clock64(), ns0 = globaltimer_ns();
+
+    const uint32_t q = (uint32_t)(warp & 3), half = (uint32_t)(warp - 2) >> 2;     // epilogue warps
+    const uint32_t n_chunks = p.tn / kTilesChunk;
+    uint8_t *boxes = staging + (size_t)(warp - 2) * kStagingBytes;
+    uint32_t n_stored = 0;
+
+    if (warp == 0) {
+        // ---------------- TMA producer ----------------
+        uint32_t full0;
+        full0 = cluster_addr(&sh->full[0], leader);
+        uint32_t s = 0, parity = 1;                            // parity of the empty barrier's previous phase
+        bool ok = true;
+        for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters) {
+            uint32_t mb, nb;
+            dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
+            const int32_t row_a = (int32_t)(mb * kTilesM + r * 128), row_b = (int32_t)(nb * p.tn + r * (p.tn / 2));
+            for (uint32_t kb = kb0; kb < kb1; kb += p.kps) {
+                if (!warp_wait(&sh->empty[s], parity)) {       // a fresh barrier's preceding phase counts as complete
+                    if (lane == 0)
+                        atomicCAS(p.status, 0u, 0x221u);
+                    ok = false;
+                    break;
+                }
+                uint8_t *st = smem + (size_t)s * stage_bytes;
+                const int32_t x = (int32_t)(kb * kRowBytesK);
+                const uint32_t nk = kb1 - kb < p.kps ? kb1 - kb : p.kps;
+                if (elect_one()) {
+                    if (r == 0)
+                        mbar_expect_tx(&sh->full[s], nk * 2 * block_bytes);
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; h++)
+                        if (h < nk) {
+                            uint8_t *blk = st + h * block_bytes;
+                            tma_load_pair_at(blk, &tmap_a, x + h * kRowBytesK, row_a, full0 + 8 * s);
+                            tma_load_pair_at(blk + kHalfTileBytes, &tmap_b, x + h * kRowBytesK, row_b, full0 + 8 * s);
+                        }
+                }
+                __syncwarp();
+                if (++s == p.stages) {
+                    s = 0;
+                    parity ^= 1;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer (the pair's leader) ----------------
+        if (r == 0) {
+            constexpr uint32_t kAFmt = DT == CLPK_DT_BF16 ? kFmtBF16 : DT == CLPK_DT_F16 ? kFmtF16 : DT == CLPK_DT_TF32 ? kFmtTF32
+                                     : DT == CLPK_DT_I8 ? kFmtS8 : DT == CLPK_DT_E5M2 ? kFmtE5M2 : kFmtE4M3;
+            constexpr uint32_t kBFmt = DT == CLPK_DT_E5M2 ? kFmtE4M3 : kAFmt;
+            const uint32_t idesc = make_idesc(256, p.tn, kAFmt, kBFmt, DT == CLPK_DT_I8 ? kAccS32 : kAccF32);
+            const uint16_t pair_mask = (uint16_t)(3u << leader);
+            uint32_t s = 0, parity = 0, tcount = 0;
+            bool ok = true;
+            for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters, tcount++) {
+                const uint32_t acc = tcount & 1, use = tcount >> 1;
+                if (use > 0 && !warp_wait(&sh->tmem_empty[acc], (use - 1) & 1)) {
+                    if (lane == 0)
+                        atomicCAS(p.status, 0u, 0x222u);
+                    break;
+                }
+                tc_fence_after_sync();
+                const uint32_t d = tmem + acc * p.tn;
+                for (uint32_t kb = kb0; kb < kb1; kb += p.kps) {
+                    if (!warp_wait(&sh->full[s], parity)) {
+                        if (lane == 0)
+                            atomicCAS(p.status, 0u, 0x223u);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    const uint32_t base = smem_u32(smem + (size_t)s * stage_bytes);
+                    const uint32_t nk = kb1 - kb < p.kps ? kb1 - kb : p.kps;
+                    const uint32_t s_now = s;
+                    if (++s == p.stages) {
+                        s = 0;
+                        parity ^= 1;
+                    }
+                    if (elect_one()) {
+#pragma unroll
+                        for (uint32_t h = 0; h < 2; h++) {
+                            if (h >= nk)
+                                break;
+                            const uint32_t blk = base + h * block_bytes;
+                            const uint64_t ad = make_smem_desc(blk, 16, 1024, kSwizzle128B);
+                            const uint64_t bd = make_smem_desc(blk + kHalfTileBytes, 16, 1024, kSwizzle128B);
+#pragma unroll
+                            for (uint32_t kk = 0; kk < 4; kk++) {
+                                const uint32_t accumulate = (kb != kb0 || h != 0 || kk != 0) ? 1u : 0u;
+                                if constexpr (DT == CLPK_DT_E4M3 || DT == CLPK_DT_E5M2)
+                                    mma2_f8f6f4_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                                else if constexpr (DT == CLPK_DT_TF32)
+                                    mma2_tf32_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                                else if constexpr (DT == CLPK_DT_I8)
+                                    mma2_i8_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                                else
+                                    mma2_f16_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                            }
+                        }
+                        tc_commit_pair(&sh->empty[s_now], pair_mask);
+                    }
+                    __syncwarp();
+                }
+                if (ok && elect_one())
+                    tc_commit_pair(&sh->tmem_full[acc], pair_mask);
+                __syncwarp();
+            }
+        }
+    } else if (p.splits == 1) {
+        // ---------------- epilogue, K not split: the two warps of a lane quarter take every other chunk ----------------
+        uint32_t tcount = 0;
+        for (uint32_t tile = cluster_id; tile < n_tiles; tile += n_clusters, tcount++) {
+            uint32_t mb, nb;
+            dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
+            const uint32_t acc = tcount & 1, use = tcount >> 1;
+            if (!warp_wait(&sh->tmem_full[acc], use & 1)) {
+                if (lane == 0)
+                    atomicCAS(p.status, 0u, 0x224u);
+                break;
+            }
+            tc_fence_after_sync();
+            const uint32_t taddr = tmem + acc * p.tn + ((q * 32) << 16);
+            const uint32_t row = mb * kTilesM + r * 128 + q * 32;
+            auto release = [&]() {
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive_cluster_relaxed(&sh->tmem_empty[acc], leader);
+            };
+            if (half >= n_chunks)
+                release();
+            for (uint32_t c = half; c < n_chunks; c += 4) {
+                // two chunks in flight
+                const bool two = c + 2 < n_chunks;
+                uint32_t v0[32], v1[32];
+                tmem_ld_32x32b_x32(taddr + c * kTilesChunk, v0);
+                if (two)
+                    tmem_ld_32x32b_x32(taddr + (c + 2) * kTilesChunk, v1);
+                tmem_ld_wait();
+                if (c + 4 >= n_chunks)
+                    release();
+                tiles_store_chunk<DT>(v0, p.alpha, boxes, n_stored, &tmap_c, nb * p.tn + c * kTilesChunk, row, lane);
+                if (two)
+                    tiles_store_chunk<DT>(v1, p.alpha, boxes, n_stored, &tmap_c, nb * p.tn + (c + 2) * kTilesChunk, row, lane);
+            }
+        }
+    } else if (!warp_wait(&sh->tmem_full[0], 0)) {
+        if (lane == 0)
+            atomicCAS(p.status, 0u, 0x225u);
+    }
+
+    if (p.splits > 1) {
+        // ---------------- K split over the cluster's pairs (one tile per cluster) ----------------
+        // Every pair's instructions have retired, so the stages of the ring are free to take partial sums: slot
+        // (src, j) of CTA (owner, r) holds pair src's sums of the owner's j-th chunk, src counted without the owner.
+        tc_fence_before_sync();
+        __syncwarp();
+        cluster_sync();
+        tc_fence_after_sync();
+        const uint32_t slots = (n_chunks + p.splits - 1) / p.splits;
+        const uint32_t taddr = tmem + ((q * 32) << 16), my_row = q * 32 + lane;
+        if (warp >= 2) {
+            for (uint32_t c = half; c < n_chunks; c += 2) {
+                const uint32_t owner = c % p.splits;
+                if (owner == split)
+                    continue;
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(taddr + c * kTilesChunk, v);
+                tmem_ld_wait();
+                const uint32_t src = split < owner ? split : split - 1;
+                const uint32_t dst = cluster_addr(smem + (size_t)(src * slots + c / p.splits) * kTilesChunkBytes + my_row * 16, owner * 2 + r);
+#pragma unroll
+                for (uint32_t g = 0; g < 8; g++)
+                    st_cluster_v4(dst + g * 2048, v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+            }
+        }
+        __syncwarp();
+        cluster_sync();
+        if (warp >= 2) {
+            uint32_t mb, nb;
+            dense_tile_coords(cluster_id, p.tiles_m, p.tiles_n, p.group, mb, nb);
+            const uint32_t row = mb * kTilesM + r * 128 + q * 32;
+            for (uint32_t j = half; split + j * p.splits < n_chunks; j += 2) {
+                const uint32_t c = split + j * p.splits;
+                uint32_t own[32], sum[32];
+                tmem_ld_32x32b_x32(taddr + c * kTilesChunk, own);
+                tmem_ld_wait();
+                for (uint32_t src = 0; src < p.splits; src++) {
+                    const uint8_t *slot = smem + (size_t)((src < split ? src : src - 1) * slots + j) * kTilesChunkBytes + my_row * 16;
+#pragma unroll
+                    for (uint32_t g = 0; g < 8; g++) {
+                        uint4 v = make_uint4(own[4 * g], own[4 * g + 1], own[4 * g + 2], own[4 * g + 3]);
+                        if (src != split)
+                            v = *reinterpret_cast<const uint4 *>(slot + g * 2048);
+                        const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (uint32_t t = 0; t < 4; t++) {
+                            if (src == 0)
+                                sum[4 * g + t] = e[t];
+                            else if constexpr (DT == CLPK_DT_I8)
+                                sum[4 * g + t] += e[t];
+                            else
+                                sum[4 * g + t] = __float_as_uint(__uint_as_float(sum[4 * g + t]) + __uint_as_float(e[t]));
+                        }
+                    }
+                }
+                tiles_store_chunk<DT>(sum, p.alpha, boxes, n_stored, &tmap_c, nb * p.tn + c * kTilesChunk, row, lane);
+            }
+        }
+    }
+    // the staging boxes must have been read before this CTA's shared memory goes away
+    if (warp >= 2 && lane == 0)
+        bulk_wait_read<0>();
+
+    tc_fence_before_sync();
+    __syncthreads();
+    cluster_sync();
+    if (blockIdx.x == 0 && threadIdx.x == 0 && p.clock) {
+        p.clock[0] = clock64() - clk0;
+        p.clock[1] = globaltimer_ns() - ns0;
+    }
+    if (warp == 1)
+        tmem_dealloc<2>(tmem, p.tmem_cols);
+}

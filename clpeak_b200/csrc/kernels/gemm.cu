@@ -592,6 +592,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads)
         tmem_dealloc<2>(tmem, 512);
 }
 
+#include "../clpk_gemm_tiles.cuh"
+
 
 // ---------------------------------------------------------------------------------
 // NVFP4 GEMM: e2m1 operands, one ue4m3 scale per 16 elements along K
@@ -979,8 +981,9 @@ static int make_operand_map(CUtensorMap *map, const void *base, uint64_t rows, u
 }
 
 
-// C [m][n] row-major for the epilogue's stores: box = 32 rows x 128 bytes, 128-byte swizzle.
-static int make_output_map(CUtensorMap *map, void *base, uint64_t m, uint64_t n, int dtype)
+// C [m][n] row-major for the epilogue's stores: box = 32 rows x 128 bytes, 128-byte swizzle; `chunk_box`: 32 rows x
+// 32 columns, which are 64 bytes (64-byte swizzle) of a 16-bit output.
+static int make_output_map(CUtensorMap *map, void *base, uint64_t m, uint64_t n, int dtype, bool chunk_box = false)
 {
     EncodeTiledFn enc;
     int rc = get_encode_fn(&enc);
@@ -992,10 +995,10 @@ static int make_output_map(CUtensorMap *map, void *base, uint64_t m, uint64_t n,
     const uint32_t elem = wide ? 4 : 2;
     const cuuint64_t dims[2] = {n, m};
     const cuuint64_t strides[1] = {n * elem};
-    const cuuint32_t box[2] = {128 / elem, 32};
+    const cuuint32_t box[2] = {chunk_box ? kTilesChunk : 128 / elem, 32};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(map, type, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     chunk_box && elem == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_error("cuTensorMapEncodeTiled (output) failed with CUresult %d", (int)r);
         return CLPK_ERR_CUDA;
@@ -1099,6 +1102,104 @@ static int launch_persistent(Kernel kernel, const char *what, int threads, size_
     const cudaError_t e = cudaLaunchKernelEx(&plain, kernel, maps..., p);
     if (e != cudaSuccess)
         return cuda_fail(e, what);
+    return CLPK_OK;
+}
+
+// How gemm_tiles_kernel splits a problem; tn = 0: leave it to gemm_kernel.
+struct TilesPlan {
+    uint32_t tn, splits;
+};
+
+// The plan is the cheapest by a cost estimate in microseconds, fitted to 2500 timed launches of both kernels: 120
+// shapes with M and N from 64 to 14000, K from 256 to 16000 in all six dense types, every tile width and split
+// (residual 13 %; the chosen plan is 1 % slower than the fastest one in the geometric mean, 19 % at worst).
+//   gemm_kernel        3.6 + waves * (0.57 per 128-byte K block of a 512 x 256 tile + 2.9), and 9.3 for the cooperative
+//                      launch and its memsets when there are more than two waves
+//   gemm_tiles_kernel  3.9 + waves * (K blocks * (0.118 to issue a block + 0.175 TN / 256 for its instructions + the bytes
+//                      all SMs fetch for it at 54 TB/s) + 1.1 TN / 256 of epilogue) and, split, 1 + the exchange
+// Splits of 2 and 4 are clusters of 4 and 8 CTAs, of which the chip holds 33 and 15 at a time.  From the fifth wave of
+// 512 x 256 tiles on that kernel's smaller operand traffic wins at every K (16384 x 16384 x 256: 140 against 142 us).
+static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks)
+{
+    const uint32_t pairs = (uint32_t)num_sms() / 2;
+    auto ceil_div = [](uint32_t a, uint32_t b) { return (a - 1) / b + 1; };
+    const uint64_t big_tiles = (uint64_t)ceil_div(m, kDenseTileM) * ceil_div(n, kTileMN);
+    TilesPlan plan = {0, 1};
+    if (pairs == 0 || big_tiles > 4ull * pairs)
+        return plan;
+    const uint32_t big_waves = ceil_div((uint32_t)big_tiles, pairs);
+    float best = 0.97f * (3.6f + (big_waves > 2 ? 9.3f : 0.0f) + big_waves * (k_blocks * 0.57f + 2.9f));
+    for (uint32_t splits = 1; splits <= 4; splits *= 2) {
+        const uint32_t resident = splits == 1 ? pairs : splits == 2 ? pairs * 33 / 74 : pairs * 15 / 74;
+        if (resident == 0 || k_blocks < splits)
+            break;
+        for (uint32_t tn = 32; tn <= kTileMN; tn += 32) {
+            const uint64_t tiles = (uint64_t)ceil_div(m, kTilesM) * ceil_div(n, tn);
+            const float waves = (float)((tiles - 1) / resident + 1), wide = (float)tn / 256.0f;
+            const float fetched = (float)(tiles < resident ? tiles : resident) * splits * ((m < kTilesM ? m : kTilesM) + (n < tn ? n : tn)) * kRowBytesK;
+            float t = 3.9f + waves * (ceil_div(k_blocks, splits) * (0.118f + 0.175f * wide + fetched / 53.8e6f) + 1.14f * wide);
+            if (splits > 1)
+                t += waves * (1.0f + 4.3f * wide * (splits - 1) / splits);
+            if (t < best) {
+                best = t;
+                plan = {tn, splits};
+            }
+        }
+    }
+    return plan;
+}
+
+template <int DT>
+static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64_t row_bytes, uint32_t k_blocks, TilesPlan plan, cudaStream_t s)
+{
+    CUtensorMap tb, tc;
+    int rc = make_operand_map(&tb, a->d_b, a->n, row_bytes, plan.tn / 2);
+    if (rc != CLPK_OK)
+        return rc;
+    rc = make_output_map(&tc, a->d_c, a->m, a->n, DT, true);
+    if (rc != CLPK_OK)
+        return rc;
+    TilesParams p;
+    p.tiles_m = (a->m + kTilesM - 1) / kTilesM;
+    p.tiles_n = (a->n + plan.tn - 1) / plan.tn;
+    p.group = tuning(CLPK_TUNE_GEMM_GROUP) > 0 ? (uint32_t)tuning(CLPK_TUNE_GEMM_GROUP) : 8;
+    p.k_blocks = k_blocks;
+    p.tn = plan.tn;
+    p.splits = plan.splits;
+    p.alpha = a->alpha;
+    p.status = a->d_status;
+    const uint32_t n_tiles = p.tiles_m * p.tiles_n, pairs = (uint32_t)num_sms() / 2;
+    const uint32_t clusters = plan.splits > 1 ? n_tiles : (n_tiles < pairs ? n_tiles : pairs);
+    const size_t fixed = kEpilogueWarps * kStagingBytes + sizeof(TilesSmem) + 1024;
+    // two K blocks per stage halve the hand-overs (0.195 -> 0.137 us per block at TN = 32), but from TN = 160 on leave
+    // too few stages (2048^3 bf16 at TN = 192: 19.3 -> 20.7 us)
+    p.kps = plan.tn <= 128 ? 2 : 1;
+    p.stages = (uint32_t)((kTilesSmemMax - fixed) / (p.kps * tiles_block_bytes(plan.tn)));
+    if (p.stages > kTilesMaxStages)
+        p.stages = kTilesMaxStages;
+    p.tmem_cols = 32;
+    while (p.tmem_cols < (n_tiles > clusters ? 2 : 1) * plan.tn)
+        p.tmem_cols *= 2;
+    CLPK_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&p.clock), g_gemm_clock));
+    const size_t smem = p.stages * p.kps * tiles_block_bytes(plan.tn) + fixed;
+    CLPK_CUDA(cudaFuncSetAttribute(gemm_tiles_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTilesSmemMax));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(clusters * 2 * plan.splits);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * plan.splits;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = tuning(CLPK_TUNE_GEMM_NO_PDL) == 1 ? 0 : 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    g_last_aligned = 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tiles_kernel<DT>, ta, tb, tc, p);
+    if (e != cudaSuccess)
+        return cuda_fail(e, "gemm_tiles");
     return CLPK_OK;
 }
 
@@ -1308,6 +1409,16 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
                                       BlockScaled<true, 256>::smem_bytes, s, p, n_tiles, ta, tb, tsa, tsb, tc)
                   : launch_persistent(gemm_block_scaled_kernel<false, 256>, "gemm_nvf4", kNvGemmThreads,
                                       BlockScaled<false, 256>::smem_bytes, s, p, n_tiles, ta, tb, tsa, tsb, tc);
+    }
+    if (const TilesPlan plan = plan_tiles(a->m, a->n, p.k_blocks); plan.tn) {
+        switch (a->dtype) {
+        case CLPK_DT_BF16: return launch_tiles<CLPK_DT_BF16>(a, ta, row_bytes, p.k_blocks, plan, s);
+        case CLPK_DT_F16:  return launch_tiles<CLPK_DT_F16>(a, ta, row_bytes, p.k_blocks, plan, s);
+        case CLPK_DT_TF32: return launch_tiles<CLPK_DT_TF32>(a, ta, row_bytes, p.k_blocks, plan, s);
+        case CLPK_DT_I8:   return launch_tiles<CLPK_DT_I8>(a, ta, row_bytes, p.k_blocks, plan, s);
+        case CLPK_DT_E5M2: return launch_tiles<CLPK_DT_E5M2>(a, ta, row_bytes, p.k_blocks, plan, s);
+        default:           return launch_tiles<CLPK_DT_E4M3>(a, ta, row_bytes, p.k_blocks, plan, s);
+        }
     }
     CUtensorMap tc;
     rc = make_output_map(&tc, a->d_c, a->m, a->n, a->dtype);

@@ -1,0 +1,58 @@
+"""GEMM shapes that do not fill the chip with 512 x 256 tiles: narrower tiles, K split over the CTA pairs of a cluster,
+several tiles per pair.  Every element of C against the fp64 product of the same operands."""
+import ctypes as C
+
+import pytest
+
+from clpeak_b200 import native as N
+from tests.gpu_util import dev_empty, stream_ptr, sync
+from tests.test_gpu_gemm import WIDE_OUT, make_gemm_operands
+
+pytestmark = pytest.mark.gpu
+
+
+def as_f64(cuda, dtype, q, rows, k):
+    view = {N.DT_BF16: cuda.bfloat16, N.DT_F16: cuda.float16, N.DT_E4M3: cuda.float8_e4m3fn, N.DT_E5M2: cuda.float8_e5m2,
+            N.DT_TF32: cuda.float32, N.DT_I8: cuda.int8}[dtype]
+    return q.view(view).double().view(rows, k)
+
+
+def run_into(K, cuda, dtype, m, n, k, d_a, d_b, alpha, pad=4096):
+    canary = 0x7FC00000 if dtype in WIDE_OUT else 0x7FC0
+    c = cuda.full((m * n + pad,), canary, dtype=cuda.int32 if dtype in WIDE_OUT else cuda.int16, device="cuda")
+    status = dev_empty(1, cuda.int32)
+    args = N.GemmArgs(dtype=dtype, m=m, n=n, k=k, d_a=d_a.data_ptr(), d_b=d_b.data_ptr(), d_c=c.data_ptr(), alpha=alpha,
+                      d_status=status.data_ptr())
+    K.clpk_gemm(C.byref(args), stream_ptr())
+    sync()
+    assert int(status.item()) == 0, "a device-side wait timed out"
+    assert bool((c[m * n:] == canary).all()), "the kernel wrote beyond C"
+    assert not bool((c[:m * n] == canary).any()), "some of C was never written"
+    return c[:m * n]
+
+
+# (m, n, bytes of K): one K block and less; a ragged last block in each stage position; K split in two and four with
+# ranges of unequal length; tile widths from 32 to 256 with ragged last tiles; several tiles per CTA pair
+@pytest.mark.parametrize("m,n,k_bytes", [
+    (1, 8, 16), (64, 64, 128), (129, 40, 144), (256, 96, 400), (300, 304, 4816), (64, 64, 32768), (200, 208, 9008),
+    (512, 256, 1024), (1000, 1016, 528), (1288, 544, 12448), (2072, 3488, 928), (1024, 1024, 2048), (700, 904, 6000),
+    (64, 11984, 1872), (8192, 3000, 1024), (16384, 72, 256), (120, 2008, 3232)])
+@pytest.mark.parametrize("dtype", [N.DT_I8, N.DT_BF16, N.DT_F16, N.DT_E4M3, N.DT_E5M2, N.DT_TF32])
+def test_every_element(K, cuda, dtype, m, n, k_bytes):
+    k = k_bytes // (4 if dtype == N.DT_TF32 else 2 if dtype in (N.DT_BF16, N.DT_F16) else 1)
+    d_a, d_b = make_gemm_operands(K, cuda, dtype, m, n, k)
+    alpha = 1.0 if dtype == N.DT_I8 else 0.75
+    c = run_into(K, cuda, dtype, m, n, k, d_a, d_b, alpha)
+    fa, fb = as_f64(cuda, dtype, d_a, m, k), as_f64(cuda, N.DT_E4M3 if dtype == N.DT_E5M2 else dtype, d_b, n, k)
+    want = fa @ fb.T
+    if dtype == N.DT_I8:
+        assert bool((c.view(m, n) == want.to(cuda.int32)).all())           # |sums| < 2^24: exact in both
+    else:
+        got = c.view(cuda.float32 if dtype == N.DT_TF32 else cuda.bfloat16).double().view(m, n)
+        want *= alpha
+        # K roundings of the accumulator (truncating adder: one ulp each), one of alpha, one of the bf16 result
+        tol = (k + 1) * 2.0 ** -23 * alpha * (fa.abs() @ fb.abs().T) + (0.0 if dtype == N.DT_TF32 else 2.0 ** -8) * want.abs() + 1e-30
+        worst = float(((got - want).abs() / tol).max())
+        assert worst <= 1.0, f"worst error over all of C is {worst:.3g}x the stated tolerance"
+    again = run_into(K, cuda, dtype, m, n, k, d_a, d_b, alpha)
+    assert bool((again == c).all()), "partial sums are added in a fixed order: the same bits every time"
