@@ -1,136 +1,396 @@
-// Seeded operand generation, format conversion and block-scaled FP4
-// quantisation.  These are set-up kernels: they run outside every timed
-// region, so they are written for determinism, not speed.
+// Seeded operand generation, format conversion and block-scaled FP4 quantisation.
+//
+// Eight consecutive elements per thread and step, moved with the widest access their type and alignment allow; what is
+// left over at the end, and everything when a pointer is not aligned for that, goes one element at a time.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
 
+#include <math.h>
+
 #include "../clpk_internal.h"
-#include "../clpk_rng.h"
+#include "../clpk_rng_fast.cuh"
 #include "../clpk_formats.h"
 
 namespace clpk {
 
-__global__ void fill_f32_kernel(float *dst, uint64_t n, uint64_t seed, int dist, float mean,
-                                float stdv)
+constexpr int kFillThreads = 256;
+
+struct __align__(32) Float8 {
+    float v[8];
+};
+
+// 32 bytes, 32-byte aligned: one 256-bit access
+__device__ __forceinline__ Float8 ld_float8(const float *p)
 {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        float v;
-        if (dist == CLPK_DIST_UNIFORM01)
-            v = clpk_uniform01(seed, i);
-        else if (dist == CLPK_DIST_UNIFORM_PM1)
-            v = clpk_uniform_pm1(seed, i);
-        else
-            v = __fmaf_rn(stdv, clpk_normal01(seed, i), mean);
-        dst[i] = v;
+    unsigned long long w[4];
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]) : "l"(p));
+    Float8 r;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        r.v[2 * i] = lo_of(w[i]);
+        r.v[2 * i + 1] = hi_of(w[i]);
+    }
+    return r;
+}
+
+__device__ __forceinline__ void st_float8(float *p, f32x2 a, f32x2 b, f32x2 c, f32x2 d)
+{
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
+}
+
+// Bound by arithmetic: a normal deviate is 63 issued instructions, which keep the issue slots, the integer and the FMA
+// pipe each 70 % busy; a uniform one the two 64-bit multiplications of its random word.  8192 x 8192: normal 246 ->
+// 162 us, uniform 89 -> 66 (the stores alone would take 41).
+template <int DIST>
+__global__ void __launch_bounds__(kFillThreads) fill_f32_kernel(float *dst, uint64_t n8, uint64_t n, uint64_t mixed_seed, float mean, float stdv)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    // the 2 P values from element i on
+    auto values = [&](uint64_t i, auto &out) {
+        constexpr int P = sizeof(out) / sizeof(f32x2);
+        uint64_t h[2 * P];
+#pragma unroll
+        for (int j = 0; j < 2 * P; j++)
+            h[j] = rand64_at(mixed_seed, i + j);
+        if constexpr (DIST == CLPK_DIST_NORMAL)
+            normal01<P>(h, out);
+#pragma unroll
+        for (int j = 0; j < P; j++) {
+            const f32x2 u = pk((float)(uint32_t)(h[2 * j] >> 40), (float)(uint32_t)(h[2 * j + 1] >> 40));
+            if constexpr (DIST == CLPK_DIST_NORMAL)
+                out[j] = fma2(pk(stdv), out[j], pk(mean));
+            else if constexpr (DIST == CLPK_DIST_UNIFORM01)
+                out[j] = mul2(u, pk(5.9604644775390625e-08f));
+            else
+                out[j] = add2(mul2(u, pk(1.1920928955078125e-07f)), pk(-1.0f));
+        }
+    };
+    for (uint64_t g = first; g < n8; g += stride) {
+        f32x2 v[4];
+        values(8 * g, v);
+        st_float8(dst + 8 * g, v[0], v[1], v[2], v[3]);
+    }
+    for (uint64_t i = 8 * n8 + first; i < n; i += stride) {
+        f32x2 v[1];
+        values(i, v);
+        dst[i] = lo_of(v[0]);
     }
 }
 
-__global__ void fill_i8_kernel(int8_t *dst, uint64_t n, uint64_t seed)
+__global__ void __launch_bounds__(kFillThreads) fill_i8_kernel(int8_t *dst, uint64_t n16, uint64_t n, uint64_t mixed_seed)
 {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        dst[i] = (int8_t)clpk_uniform_i4(seed, i);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint64_t g = first; g < n16; g += stride) {
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            w[j] = 0;
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                w[j] |= ((uint32_t)((int)(rand64_at(mixed_seed, 16 * g + 4 * j + t) >> 60) - 8) & 0xFFu) << (8 * t);
+        }
+        *reinterpret_cast<uint4 *>(dst + 16 * g) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    for (uint64_t i = 16 * n16 + first; i < n; i += stride)
+        dst[i] = (int8_t)((int)(rand64_at(mixed_seed, i) >> 60) - 8);
 }
 
-__global__ void convert_kernel(void *dst, const float *src, uint64_t n, int dtype)
+// One element in its narrow format, as bits.
+template <int DT>
+__device__ __forceinline__ uint64_t narrow(float x)
 {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const float x = src[i];
-        switch (dtype) {
-        case CLPK_DT_F16:
-            reinterpret_cast<__half *>(dst)[i] = __float2half_rn(x);
-            break;
-        case CLPK_DT_BF16:
-            reinterpret_cast<__nv_bfloat16 *>(dst)[i] = __float2bfloat16_rn(x);
-            break;
-        case CLPK_DT_E4M3:
-            reinterpret_cast<uint8_t *>(dst)[i] = __nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3);
-            break;
-        case CLPK_DT_E5M2:
-            reinterpret_cast<uint8_t *>(dst)[i] = __nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E5M2);
-            break;
-        case CLPK_DT_TF32: {
-            // nearest even at bit 13 in integer arithmetic (infinities and NaNs keep their class)
-            uint32_t b = __float_as_uint(x);
-            if ((b & 0x7F800000u) != 0x7F800000u)
-                b += 0xFFFu + ((b >> 13) & 1u);
-            reinterpret_cast<uint32_t *>(dst)[i] = b & 0xFFFFE000u;
-            break;
+    if constexpr (DT == CLPK_DT_F16) {
+        return __half_as_ushort(__float2half_rn(x));
+    } else if constexpr (DT == CLPK_DT_BF16) {
+        return __bfloat16_as_ushort(__float2bfloat16_rn(x));
+    } else if constexpr (DT == CLPK_DT_E4M3) {
+        return __nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3);
+    } else if constexpr (DT == CLPK_DT_E5M2) {
+        return __nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E5M2);
+    } else if constexpr (DT == CLPK_DT_TF32) {
+        // nearest even at bit 13 in integer arithmetic (infinities and NaNs keep their class)
+        uint32_t b = __float_as_uint(x);
+        if ((b & 0x7F800000u) != 0x7F800000u)
+            b += 0xFFFu + ((b >> 13) & 1u);
+        return b & 0xFFFFE000u;
+    } else if constexpr (DT == CLPK_DT_F64) {
+        return (uint64_t)__double_as_longlong((double)x);
+    } else if constexpr (DT == CLPK_DT_I8) {
+        const int v = __float2int_rn(x);
+        return (uint8_t)(int8_t)(v < -128 ? -128 : (v > 127 ? 127 : v));
+    } else {
+        return clpk_e2m1_encode(x);
+    }
+}
+
+// two neighbours; the 8-bit floats have an instruction for that
+template <int DT>
+__device__ __forceinline__ uint64_t narrow2(float x0, float x1)
+{
+    if constexpr (DT == CLPK_DT_E4M3 || DT == CLPK_DT_E5M2)
+        return __nv_cvt_float2_to_fp8x2(make_float2(x0, x1), __NV_SATFINITE, DT == CLPK_DT_E4M3 ? __NV_E4M3 : __NV_E5M2);
+    else
+        return 0;
+}
+
+template <int DT> struct Narrow {
+    static constexpr int bits = DT == CLPK_DT_F64 ? 64 : DT == CLPK_DT_TF32 ? 32 : DT == CLPK_DT_F16 || DT == CLPK_DT_BF16 ? 16 : DT == CLPK_DT_E2M1 ? 4 : 8;
+    static constexpr int bytes8 = bits;                        // bytes of eight elements
+};
+
+// Bound by memory: 4 bytes in and bits / 8 out per element.  8192 x 8192: to fp8 122 -> 50 us (6.7 TB/s), 16 bits
+// 129 -> 60, tf32 147 -> 82.
+template <int DT>
+__global__ void __launch_bounds__(kFillThreads) convert_kernel(void *dst, const float *src, uint64_t n8, uint64_t n)
+{
+    constexpr int bits = Narrow<DT>::bits;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint64_t g = first; g < n8; g += stride) {
+        const Float8 x = ld_float8(src + 8 * g);
+        constexpr int kWords = (8 * bits + 63) / 64;
+        uint64_t w[kWords];
+#pragma unroll
+        for (int j = 0; j < kWords; j++)
+            w[j] = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            if constexpr (DT == CLPK_DT_E4M3 || DT == CLPK_DT_E5M2) {
+                if ((i & 1) == 0)
+                    w[0] |= narrow2<DT>(x.v[i], x.v[i + 1]) << (8 * i);
+            } else {
+                w[i * bits / 64] |= narrow<DT>(x.v[i]) << (i * bits % 64);
+            }
         }
-        case CLPK_DT_F64:
-            reinterpret_cast<double *>(dst)[i] = (double)x;
-            break;
-        case CLPK_DT_I8: {
-            int v = __float2int_rn(x);
-            v = v < -128 ? -128 : (v > 127 ? 127 : v);
-            reinterpret_cast<int8_t *>(dst)[i] = (int8_t)v;
-            break;
+        uint8_t *p = static_cast<uint8_t *>(dst) + g * Narrow<DT>::bytes8;
+        if constexpr (bits == 4) {
+            *reinterpret_cast<uint32_t *>(p) = (uint32_t)w[0];
+        } else if constexpr (bits == 8) {
+            *reinterpret_cast<uint64_t *>(p) = w[0];
+        } else if constexpr (bits == 16) {
+            *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(w[0], w[1]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < kWords; j += 4)
+                st_float8(reinterpret_cast<float *>(p + 8 * j), w[j], w[j + 1], w[j + 2], w[j + 3]);
         }
-        default:
-            break;
+    }
+    if constexpr (bits == 4) {
+        for (uint64_t i = 4 * n8 + first; i < n / 2; i += stride)
+            static_cast<uint8_t *>(dst)[i] = (uint8_t)(narrow<DT>(src[2 * i]) | (narrow<DT>(src[2 * i + 1]) << 4));
+    } else {
+        for (uint64_t i = 8 * n8 + first; i < n; i += stride) {
+            const uint64_t v = narrow<DT>(src[i]);
+            if constexpr (bits == 8)
+                static_cast<uint8_t *>(dst)[i] = (uint8_t)v;
+            else if constexpr (bits == 16)
+                static_cast<uint16_t *>(dst)[i] = (uint16_t)v;
+            else if constexpr (bits == 32)
+                static_cast<uint32_t *>(dst)[i] = (uint32_t)v;
+            else
+                static_cast<uint64_t *>(dst)[i] = v;
         }
     }
 }
 
-__global__ void convert_e2m1_kernel(uint8_t *dst, const float *src, uint64_t n_pairs)
-{
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_pairs; i += stride)
-        dst[i] = (uint8_t)(clpk_e2m1_encode(src[2 * i]) | (clpk_e2m1_encode(src[2 * i + 1]) << 4));
-}
+// Bound by memory (8192 x 8192: 111 -> 42 us, 6.4 TB/s); a CTA takes four accesses per thread of one contiguous range (8 Ki floats), so that the chip walks
+// the array in address order.  SINGLE: one CTA reads everything and writes the result itself; otherwise the CTAs meet
+// in an atomicMax on a word that has been cleared.
+constexpr int kAbsmaxLoads = 4;
 
-__global__ void absmax_kernel(float *out, const float *src, uint64_t n)
+template <bool SINGLE>
+__global__ void __launch_bounds__(kFillThreads) absmax_kernel(float *out, const float *src, uint64_t n8, uint64_t n)
 {
     float m = 0.0f;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+    const uint64_t step = (uint64_t)gridDim.x * kFillThreads * kAbsmaxLoads;
+    for (uint64_t g = (uint64_t)blockIdx.x * kFillThreads * kAbsmaxLoads + threadIdx.x; g < n8; g += step) {
+        Float8 x[kAbsmaxLoads];
+#pragma unroll
+        for (int u = 0; u < kAbsmaxLoads; u++)
+            x[u] = g + u * kFillThreads < n8 ? ld_float8(src + 8 * (g + u * kFillThreads)) : Float8{};
+#pragma unroll
+        for (int u = 0; u < kAbsmaxLoads; u++)
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                m = fmaxf(m, fabsf(x[u].v[i]));
+    }
+    for (uint64_t i = 8 * n8 + (uint64_t)blockIdx.x * kFillThreads + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kFillThreads)
         m = fmaxf(m, fabsf(src[i]));
-    for (int o = 16; o > 0; o >>= 1)
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     // |x| >= 0, so the float ordering equals the ordering of the bit patterns.
+    uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    __shared__ uint32_t warp_top[kFillThreads / 32];
     if ((threadIdx.x & 31) == 0)
-        atomicMax(reinterpret_cast<unsigned int *>(out), __float_as_uint(m));
+        warp_top[threadIdx.x >> 5] = top;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < kFillThreads / 32; w++)
+            top = max(top, warp_top[w]);
+        if (SINGLE)
+            *reinterpret_cast<uint32_t *>(out) = top;
+        else
+            atomicMax(reinterpret_cast<uint32_t *>(out), top);
+    }
 }
 
-// One thread per scale block of BLOCK elements; UE8M0 selects the scale format
-// (power-of-two MX scale) against ue4m3 (NVFP4 scale, after the tensor scale).
+// ---- block-scaled FP4 -------------------------------------------------------------------------------------------------
+//
+// BLOCK elements share a scale; UE8M0 selects the scale format (power-of-two MX scale) against ue4m3 (NVFP4 scale,
+// after the tensor scale).  A lane takes 16 neighbouring elements -- an NVFP4 block -- and BLOCK / 16 lanes share a
+// scale.  Bound by memory (4.6 bytes an element) once the two quotients of an element, x / tensor scale and that /
+// block scale, are no IEEE division each: both divisors are shared, so each is a multiplication by the divisor's
+// reciprocal with the residual correction of clpk_rng_fast.cuh -- done twice for the first, whose exact rounding
+// decides ties later; the block scale has four significand bits, so one correction leaves nothing to a tie.  That
+// holds while nothing under- or overflows: magnitudes and tensor scales within 2^+-60.  A warp that meets any other
+// block (zeros, NaN, infinities) takes the divisions.  8192 x 8192: NVFP4 171 -> 50 us, MXFP4 270 -> 46 (6.3 and 6.6 TB/s).
+
+// divisor and reciprocal for the whole tensor; plain: outside the range above
+struct TensorScale {
+    float scale, inv;
+    bool plain;
+};
+
+__device__ __forceinline__ uint32_t e2m1x2(float x0, float x1)
+{
+    uint32_t r;
+    asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+        "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+        : "=r"(r)
+        : "f"(x0), "f"(x1));
+    return r & 0xFFu;
+}
+
+// x / b from inv = RN(1 / b), correctly rounded (see above)
+__device__ __forceinline__ float shared_quotient(float x, float b, float inv)
+{
+    float q = __fmul_rn(x, inv);
+    q = __fmaf_rn(__fmaf_rn(-b, q, x), inv, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, x), inv, q);
+}
+
+template <bool UE8M0>
+__device__ __forceinline__ uint8_t fp4_block_scale(float amax, float *decoded)
+{
+    uint8_t s;
+    if (UE8M0) {
+        s = clpk_ue8m0_for_absmax(amax);
+        *decoded = clpk_ue8m0_decode(s);
+    } else {
+        s = __nv_cvt_float_to_fp8(__fdiv_rn(amax, 6.0f), __NV_SATFINITE, __NV_E4M3);
+        *decoded = clpk_e4m3_decode(s);
+    }
+    return s;
+}
+
+constexpr int kQuantPerLane = 16;
+
 template <int BLOCK, bool UE8M0>
-__global__ void quantize_fp4_kernel(uint8_t *packed, uint8_t *scales, const float *src,
-                                    uint64_t n_blocks, float tensor_scale)
+__global__ void __launch_bounds__(kFillThreads) quantize_fp4_kernel(uint8_t *packed, uint8_t *scales, const float *src, uint64_t n16, TensorScale ts)
+{
+    constexpr int kLanes = BLOCK / kQuantPerLane;              // lanes of one block
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31;
+    // whole warps step together: n16 is a multiple of 4, so a block's lanes are inside or outside as one
+    for (uint64_t g0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); g0 < n16; g0 += stride) {
+        const uint64_t g = g0 + lane;
+        const bool inside = g < n16;
+        float x[kQuantPerLane] = {};
+        if (inside) {
+            const Float8 a = ld_float8(src + 16 * g), b = ld_float8(src + 16 * g + 8);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                x[i] = a.v[i];
+                x[8 + i] = b.v[i];
+            }
+        }
+        uint32_t top = 0;                                      // largest magnitude's bits; NaNs come out largest
+#pragma unroll
+        for (int i = 0; i < kQuantPerLane; i++)
+            top = max(top, __float_as_uint(x[i]) & 0x7FFFFFFFu);
+#pragma unroll
+        for (int o = 1; o < kLanes; o *= 2)
+            top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+        const bool tame = top - 0x21800000u <= 0x5D800000u - 0x21800000u;      // 2^-60 ... 2^60
+        uint64_t codes = 0;
+        uint8_t sbyte;
+        float sdec;
+        if (!ts.plain && __all_sync(0xffffffffu, tame || !inside)) {
+            float sinv, amax = __uint_as_float(top);
+            if (UE8M0) {
+                sbyte = clpk_ue8m0_for_absmax(amax);
+                sdec = 1.0f;
+                sinv = __uint_as_float((254u - sbyte) << 23);  // a power of two's reciprocal is exact (2^-58 ... 2^62)
+            } else {
+                // rounding is monotone: the quotient of the largest is the largest quotient
+                amax = shared_quotient(amax, ts.scale, ts.inv);
+                sbyte = __nv_cvt_float_to_fp8(shared_quotient(amax, 6.0f, 0x1.555556p-3f), __NV_SATFINITE, __NV_E4M3);
+                sdec = __half2float(__half(__nv_cvt_fp8_to_halfraw(sbyte, __NV_E4M3)));
+                sinv = rcp_approx(sdec);
+                sinv = __fmaf_rn(__fmaf_rn(-sdec, sinv, 1.0f), sinv, sinv);
+            }
+#pragma unroll
+            for (int i = 0; i < kQuantPerLane; i += 2) {
+                const f32x2 xx = pk(x[i], x[i + 1]);
+                f32x2 q;
+                if (!UE8M0) {
+                    q = mul2(xx, pk(ts.inv));
+                    q = fma2(fma2(pk(-ts.scale), q, xx), pk(ts.inv), q);
+                    const f32x2 v = fma2(fma2(pk(-ts.scale), q, xx), pk(ts.inv), q);
+                    q = mul2(v, pk(sinv));
+                    q = fma2(fma2(pk(-sdec), q, v), pk(sinv), q);
+                } else {
+                    q = mul2(xx, pk(sinv));
+                }
+                // the sign is x's, also where a residual lost that of a zero
+                const float q0 = __uint_as_float(((uint32_t)q & 0x7FFFFFFFu) | (__float_as_uint(x[i]) & 0x80000000u));
+                const float q1 = __uint_as_float(((uint32_t)(q >> 32) & 0x7FFFFFFFu) | (__float_as_uint(x[i + 1]) & 0x80000000u));
+                codes |= (uint64_t)e2m1x2(q0, q1) << (4 * i);
+            }
+            if (!UE8M0 && sdec == 0.0f)
+                codes = 0;
+        } else {
+            float amax = 0.0f;
+#pragma unroll
+            for (int i = 0; i < kQuantPerLane; i++) {
+                if (!UE8M0)
+                    x[i] = __fdiv_rn(x[i], ts.scale);
+                amax = fmaxf(amax, fabsf(x[i]));
+            }
+#pragma unroll
+            for (int o = 1; o < kLanes; o *= 2)
+                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            sbyte = fp4_block_scale<UE8M0>(amax, &sdec);
+            if (sdec > 0.0f)
+#pragma unroll
+                for (int i = 0; i < kQuantPerLane; i++)
+                    codes |= (uint64_t)clpk_e2m1_encode(__fdiv_rn(x[i], sdec)) << (4 * i);
+        }
+        if (inside) {
+            reinterpret_cast<uint64_t *>(packed)[g] = codes;
+            if (lane % kLanes == 0)
+                scales[g / kLanes] = sbyte;
+        }
+    }
+}
+
+// The same for pointers that are not aligned for it: one thread per scale block.
+template <int BLOCK, bool UE8M0>
+__global__ void quantize_fp4_unaligned_kernel(uint8_t *packed, uint8_t *scales, const float *src, uint64_t n_blocks, float tensor_scale)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < n_blocks; b += stride) {
         const float *x = src + b * BLOCK;
-        float v[BLOCK];
         float amax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < BLOCK; i++) {
-            v[i] = UE8M0 ? x[i] : __fdiv_rn(x[i], tensor_scale);
-            amax = fmaxf(amax, fabsf(v[i]));
-        }
-        uint8_t sbyte;
+        for (int i = 0; i < BLOCK; i++)
+            amax = fmaxf(amax, fabsf(UE8M0 ? x[i] : __fdiv_rn(x[i], tensor_scale)));
         float sdec;
-        if (UE8M0) {
-            sbyte = clpk_ue8m0_for_absmax(amax);
-            sdec = clpk_ue8m0_decode(sbyte);
-        } else {
-            sbyte = __nv_cvt_float_to_fp8(__fdiv_rn(amax, 6.0f), __NV_SATFINITE, __NV_E4M3);
-            sdec = clpk_e4m3_decode(sbyte);
-        }
-        scales[b] = sbyte;
-        uint8_t *p = packed + b * (BLOCK / 2);
-#pragma unroll
-        for (int i = 0; i < BLOCK; i += 2) {
-            uint8_t lo = 0, hi = 0;
-            if (sdec > 0.0f) {
-                lo = clpk_e2m1_encode(__fdiv_rn(v[i], sdec));
-                hi = clpk_e2m1_encode(__fdiv_rn(v[i + 1], sdec));
-            }
-            p[i / 2] = (uint8_t)(lo | (hi << 4));
-        }
+        scales[b] = fp4_block_scale<UE8M0>(amax, &sdec);
+        auto code = [&](float v) -> uint8_t {
+            return sdec > 0.0f ? clpk_e2m1_encode(__fdiv_rn(UE8M0 ? v : __fdiv_rn(v, tensor_scale), sdec)) : 0;
+        };
+        for (int i = 0; i < BLOCK; i += 2)
+            packed[b * (BLOCK / 2) + i / 2] = (uint8_t)(code(x[i]) | (code(x[i + 1]) << 4));
     }
 }
 
@@ -141,10 +401,34 @@ __global__ void flush_kernel(uint4 *p, uint64_t n16, uint32_t tag)
         p[i] = make_uint4(tag, tag, tag, tag);
 }
 
-static int fill_grid()
+// One step of one thread per item: CTAs start in address order as others end, which keeps the chip inside a few MiB of
+// memory and has no last round of a few CTAs (a grid of 8 CTAs per SM, of which 6 are resident, ran the normal
+// deviates at 57 % of the warps).
+static unsigned fill_grid(uint64_t items)
 {
-    int sms = num_sms();
-    return sms > 0 ? sms * 8 : 1024;
+    const uint64_t want = (items + kFillThreads - 1) / kFillThreads;
+    return (unsigned)(want == 0 ? 1 : want < 0x7FFFFFFFull ? want : 0x7FFFFFFFull);
+}
+
+static bool aligned(const void *p, size_t bytes) { return ((uintptr_t)p % bytes) == 0; }
+
+template <int DT>
+static void launch_convert(void *d_dst, const float *d_src, uint64_t n, cudaStream_t s)
+{
+    constexpr size_t dst_align = Narrow<DT>::bytes8 < 32 ? Narrow<DT>::bytes8 : 32;
+    const uint64_t n8 = aligned(d_src, 32) && aligned(d_dst, dst_align) ? n / 8 : 0;
+    convert_kernel<DT><<<fill_grid(n8 ? n8 : n), kFillThreads, 0, s>>>(d_dst, d_src, n8, n);
+}
+
+template <int BLOCK, bool UE8M0>
+static void launch_quantize(uint8_t *d_packed, uint8_t *d_scales, const float *d_src, uint64_t n, float tensor_scale, cudaStream_t s)
+{
+    if (!aligned(d_src, 32) || !aligned(d_packed, 8)) {
+        quantize_fp4_unaligned_kernel<BLOCK, UE8M0><<<fill_grid(n / BLOCK), kFillThreads, 0, s>>>(d_packed, d_scales, d_src, n / BLOCK, tensor_scale);
+        return;
+    }
+    TensorScale ts = {tensor_scale, 1.0f / tensor_scale, !UE8M0 && !(tensor_scale >= 0x1p-60f && tensor_scale <= 0x1p60f)};
+    quantize_fp4_kernel<BLOCK, UE8M0><<<fill_grid(n / kQuantPerLane), kFillThreads, 0, s>>>(d_packed, d_scales, d_src, n / kQuantPerLane, ts);
 }
 
 } // namespace clpk
@@ -160,7 +444,15 @@ int clpk_fill_f32(float *d_dst, uint64_t n, uint64_t seed, int dist, float mean,
     CLPK_REQUIRE(dist >= 0 && dist <= 2, "unknown distribution %d", dist);
     if (n == 0)
         return CLPK_OK;
-    fill_f32_kernel<<<fill_grid(), 256, 0, as_stream(stream)>>>(d_dst, n, seed, dist, mean, std);
+    const uint64_t n8 = aligned(d_dst, 32) ? n / 8 : 0, mixed = clpk_mix64(seed);
+    const unsigned grid = fill_grid(n8 ? n8 : n);
+    cudaStream_t s = as_stream(stream);
+    if (dist == CLPK_DIST_UNIFORM01)
+        fill_f32_kernel<CLPK_DIST_UNIFORM01><<<grid, kFillThreads, 0, s>>>(d_dst, n8, n, mixed, mean, std);
+    else if (dist == CLPK_DIST_UNIFORM_PM1)
+        fill_f32_kernel<CLPK_DIST_UNIFORM_PM1><<<grid, kFillThreads, 0, s>>>(d_dst, n8, n, mixed, mean, std);
+    else
+        fill_f32_kernel<CLPK_DIST_NORMAL><<<grid, kFillThreads, 0, s>>>(d_dst, n8, n, mixed, mean, std);
     CLPK_LAUNCH_CHECK("fill_f32");
     return CLPK_OK;
 }
@@ -170,7 +462,8 @@ int clpk_fill_i8(int8_t *d_dst, uint64_t n, uint64_t seed, void *stream)
     CLPK_REQUIRE(d_dst || n == 0, "d_dst is NULL");
     if (n == 0)
         return CLPK_OK;
-    fill_i8_kernel<<<fill_grid(), 256, 0, as_stream(stream)>>>(d_dst, n, seed);
+    const uint64_t n16 = aligned(d_dst, 16) ? n / 16 : 0;
+    fill_i8_kernel<<<fill_grid(n16 ? n16 : n), kFillThreads, 0, as_stream(stream)>>>(d_dst, n16, n, clpk_mix64(seed));
     CLPK_LAUNCH_CHECK("fill_i8");
     return CLPK_OK;
 }
@@ -184,13 +477,18 @@ int clpk_convert_f32(void *d_dst, const float *d_src, uint64_t n, int dtype, voi
                  "clpk_convert_f32: dtype %d has no plain conversion", dtype);
     if (n == 0)
         return CLPK_OK;
-    if (dtype == CLPK_DT_E2M1) {
-        CLPK_REQUIRE(n % 2 == 0, "E2M1 packs two elements per byte: n (%llu) must be even", (unsigned long long)n);
-        convert_e2m1_kernel<<<fill_grid(), 256, 0, as_stream(stream)>>>(static_cast<uint8_t *>(d_dst), d_src, n / 2);
-        CLPK_LAUNCH_CHECK("convert_e2m1");
-        return CLPK_OK;
+    CLPK_REQUIRE(dtype != CLPK_DT_E2M1 || n % 2 == 0, "E2M1 packs two elements per byte: n (%llu) must be even", (unsigned long long)n);
+    cudaStream_t s = as_stream(stream);
+    switch (dtype) {
+    case CLPK_DT_F16:  launch_convert<CLPK_DT_F16>(d_dst, d_src, n, s); break;
+    case CLPK_DT_BF16: launch_convert<CLPK_DT_BF16>(d_dst, d_src, n, s); break;
+    case CLPK_DT_E4M3: launch_convert<CLPK_DT_E4M3>(d_dst, d_src, n, s); break;
+    case CLPK_DT_E5M2: launch_convert<CLPK_DT_E5M2>(d_dst, d_src, n, s); break;
+    case CLPK_DT_I8:   launch_convert<CLPK_DT_I8>(d_dst, d_src, n, s); break;
+    case CLPK_DT_TF32: launch_convert<CLPK_DT_TF32>(d_dst, d_src, n, s); break;
+    case CLPK_DT_F64:  launch_convert<CLPK_DT_F64>(d_dst, d_src, n, s); break;
+    default:           launch_convert<CLPK_DT_E2M1>(d_dst, d_src, n, s); break;
     }
-    convert_kernel<<<fill_grid(), 256, 0, as_stream(stream)>>>(d_dst, d_src, n, dtype);
     CLPK_LAUNCH_CHECK("convert");
     return CLPK_OK;
 }
@@ -198,11 +496,19 @@ int clpk_convert_f32(void *d_dst, const float *d_src, uint64_t n, int dtype, voi
 int clpk_absmax_f32(float *d_absmax, const float *d_src, uint64_t n, void *stream)
 {
     CLPK_REQUIRE(d_absmax, "d_absmax is NULL");
-    CLPK_CUDA(cudaMemsetAsync(d_absmax, 0, sizeof(float), as_stream(stream)));
+    cudaStream_t s = as_stream(stream);
+    const uint64_t n8 = aligned(d_src, 32) ? n / 8 : 0;
+    // up to 32 Ki floats one CTA reads in the time that clearing the word would take
+    if (n > 0 && n <= 32768 && d_src) {
+        absmax_kernel<true><<<1, kFillThreads, 0, s>>>(d_absmax, d_src, n8, n);
+        CLPK_LAUNCH_CHECK("absmax");
+        return CLPK_OK;
+    }
+    CLPK_CUDA(cudaMemsetAsync(d_absmax, 0, sizeof(float), s));
     if (n == 0)
         return CLPK_OK;
     CLPK_REQUIRE(d_src, "d_src is NULL");
-    absmax_kernel<<<fill_grid(), 256, 0, as_stream(stream)>>>(d_absmax, d_src, n);
+    absmax_kernel<false><<<fill_grid((n8 ? n8 : n) / kAbsmaxLoads + 1), kFillThreads, 0, s>>>(d_absmax, d_src, n8, n);
     CLPK_LAUNCH_CHECK("absmax");
     return CLPK_OK;
 }
@@ -218,13 +524,12 @@ int clpk_quantize_fp4(uint8_t *d_packed, uint8_t *d_scales, const float *d_src, 
     const uint64_t n = rows * cols;
     if (n == 0)
         return CLPK_OK;
-    const int g = fill_grid();
     cudaStream_t s = as_stream(stream);
     switch (dtype) {
-    case CLPK_DT_MXF4:     quantize_fp4_kernel<32, true><<<g, 128, 0, s>>>(d_packed, d_scales, d_src, n / 32, 1.0f); break;
-    case CLPK_DT_MXF4_B64: quantize_fp4_kernel<64, true><<<g, 128, 0, s>>>(d_packed, d_scales, d_src, n / 64, 1.0f); break;
-    case CLPK_DT_NVF4:     quantize_fp4_kernel<16, false><<<g, 128, 0, s>>>(d_packed, d_scales, d_src, n / 16, tensor_scale); break;
-    default:               quantize_fp4_kernel<32, false><<<g, 128, 0, s>>>(d_packed, d_scales, d_src, n / 32, tensor_scale); break;
+    case CLPK_DT_MXF4:     launch_quantize<32, true>(d_packed, d_scales, d_src, n, 1.0f, s); break;
+    case CLPK_DT_MXF4_B64: launch_quantize<64, true>(d_packed, d_scales, d_src, n, 1.0f, s); break;
+    case CLPK_DT_NVF4:     launch_quantize<16, false>(d_packed, d_scales, d_src, n, tensor_scale, s); break;
+    default:               launch_quantize<32, false>(d_packed, d_scales, d_src, n, tensor_scale, s); break;
     }
     CLPK_LAUNCH_CHECK("quantize_fp4");
     return CLPK_OK;
@@ -234,7 +539,7 @@ int clpk_flush_l2(void *d_scratch, size_t bytes, void *stream)
 {
     CLPK_REQUIRE(d_scratch, "d_scratch is NULL");
     static unsigned tag = 0;
-    flush_kernel<<<fill_grid(), 256, 0, as_stream(stream)>>>(reinterpret_cast<uint4 *>(d_scratch),
+    flush_kernel<<<num_sms() > 0 ? num_sms() * 8 : 1024, kFillThreads, 0, as_stream(stream)>>>(reinterpret_cast<uint4 *>(d_scratch),
                                                             bytes / 16, ++tag);
     CLPK_LAUNCH_CHECK("flush_l2");
     return CLPK_OK;
