@@ -682,38 +682,67 @@ struct NvGemmSmem {
 };
 static_assert(sizeof(NvGemmSmem) <= 512, "NvGemmSmem");
 
-// Row-major scale bytes [rows][k / block] -> 512-byte blocks in tensor-memory order, one
-// 32-bit word (four factors) per row per block.  NVFP4: 16 factors per row per stage =
-// 4 words; MXFP4: 8 factors = 2 words.  words = words per row per stage.
-// is_b = 0: blocks ordered [rows/128][k/256][words];  is_b = 1: [rows/256][k/256][words][2].
-// One CTA moves 128 rows x 32 words through shared memory: coalesced 128-byte reads along a
-// row, coalesced 512-byte writes of whole blocks (a byte-per-thread scatter took 64 us per
-// 16 MiB operand, 7 % of a 16384^3 NVFP4 GEMM; this takes a tenth of that).
-// Rows at and beyond `rows` (the operand padded up to whole tiles) get zero factors: their elements arrive
-// as zeros from the operand's tensor map, and zero times any finite factor is zero.
-__global__ void __launch_bounds__(256) pack_scales_kernel(uint32_t *__restrict__ out, const uint32_t *__restrict__ in, uint32_t rows,
-                                                          uint32_t words_per_row, uint32_t kblocks, int is_b, uint32_t words)
+// Row-major scale bytes [rows][k / block] of both operands -> 512-byte blocks in tensor-memory order, one 32-bit word
+// (four factors) per row per block.  NVFP4: 16 factors per row per stage = 4 words; MXFP4: 8 factors = 2 words.
+// A's blocks are ordered [rows/128][k/256][words]; B's [rows/256][k/256][words][2] for the 256-wide tile (b_pairs),
+// like A's for the 128-wide one.  Rows at and beyond an operand's `rows` (it is padded up to whole tiles) get zero
+// factors: their elements arrive as zeros from the operand's tensor map, and zero times any finite factor is zero.
+//
+// One warp takes 128 rows x one stage: a lane loads the stage's words of rows r, r + 32, r + 64, r + 96 and holds
+// their transpose, one 16-byte piece of every block.  Eight neighbouring stages are one CTA, so that a row's 128-byte
+// line is read once.  The kernel is latency: launched with the programmatic attribute like the GEMM behind it, so that
+// both set up under the tail of what precedes.  NVFP4 one-call GEMM, device time at 2048^3 / 4096^3: 20.4 / 55.3 us with
+// one launch per operand through shared memory, 10.9 / 37.5 now, 8.1 / 31.2 with the scales already packed.
+struct PackOperand {
+    const uint32_t *in;
+    uint32_t *out;
+    uint32_t rows, row_groups;          // row groups of 128 after padding
+    uint32_t vector;                    // 1: `in` is aligned to a stage's words
+};
+
+template <int WORDS>
+__global__ void __launch_bounds__(256) pack_scales_kernel(PackOperand oa, PackOperand ob, uint32_t kblocks, uint32_t b_pairs)
 {
-    __shared__ uint32_t tile[128][33];
-    const uint32_t row0 = blockIdx.y * 128, w0 = blockIdx.x * 32;
-    for (uint32_t i = threadIdx.x; i < 128 * 32; i += 256) {
-        const uint32_t r = i >> 5, c = i & 31;
-        tile[r][c] = (w0 + c < words_per_row && row0 + r < rows) ? in[(uint64_t)(row0 + r) * words_per_row + w0 + c] : 0u;
+    griddep_wait();
+    griddep_launch_dependents();
+    const uint32_t lane = threadIdx.x & 31, kgroups = (kblocks + 7) / 8;
+    const uint32_t kb = blockIdx.x % kgroups * 8 + (threadIdx.x >> 5);
+    uint32_t group = blockIdx.x / kgroups;
+    const bool is_b = group >= oa.row_groups;
+    const PackOperand &op = is_b ? ob : oa;
+    group -= is_b ? oa.row_groups : 0;
+    if (kb >= kblocks)
+        return;
+    uint32_t w[4][WORDS];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t row = group * 128 + i * 32 + lane;
+        const uint32_t *src = op.in + ((uint64_t)row * kblocks + kb) * WORDS;
+#pragma unroll
+        for (int j = 0; j < WORDS; j++)
+            w[i][j] = 0;
+        if (row < op.rows) {
+            if (op.vector) {
+                if constexpr (WORDS == 4) {
+                    const uint4 v = *reinterpret_cast<const uint4 *>(src);
+                    w[i][0] = v.x; w[i][1] = v.y; w[i][2] = v.z; w[i][3] = v.w;
+                } else {
+                    const uint2 v = *reinterpret_cast<const uint2 *>(src);
+                    w[i][0] = v.x; w[i][1] = v.y;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < WORDS; j++)
+                    w[i][j] = src[j];
+            }
+        }
     }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < 32 * 128; i += 256) {
-        const uint32_t c = i >> 7, o = i & 127;            // word column of the tile, word of the 512-byte block
-        const uint32_t wd = w0 + c;
-        if (wd >= words_per_row)
-            continue;
-        const uint32_t kb = wd / words, kk = wd % words;
-        const uint32_t r = (o & 3) * 32 + (o >> 2);         // block byte (r%32)*16 + (r/32)*4 <-> word (r%32)*4 + r/32
-        uint64_t block;
-        if (!is_b)
-            block = ((uint64_t)blockIdx.y * kblocks + kb) * words + kk;
-        else
-            block = (((uint64_t)(blockIdx.y >> 1) * kblocks + kb) * words + kk) * 2 + (blockIdx.y & 1);
-        out[block * 128 + o] = tile[r][c];
+#pragma unroll
+    for (int j = 0; j < WORDS; j++) {
+        const uint64_t block = is_b && b_pairs ? (((uint64_t)(group >> 1) * kblocks + kb) * WORDS + j) * 2 + (group & 1)
+                                               : ((uint64_t)group * kblocks + kb) * WORDS + j;
+        // block byte (r % 32) * 16 + (r / 32) * 4 of row r
+        reinterpret_cast<uint4 *>(op.out)[block * 32 + lane] = make_uint4(w[0][j], w[1][j], w[2][j], w[3][j]);
     }
 }
 
@@ -1271,15 +1300,26 @@ static int pack_scales(const clpk_gemm_args_t *a, cudaStream_t s)
                  "block-scaled FP4 needs a 16-byte aligned workspace of clpk_gemm_workspace_bytes() bytes");
     CLPK_REQUIRE(((uintptr_t)a->d_sfa % 4) == 0 && ((uintptr_t)a->d_sfb % 4) == 0, "scale arrays must be 4-byte aligned");
     uint8_t *wsa = static_cast<uint8_t *>(a->d_workspace), *wsb = wsa + sfa_bytes;
-    const uint32_t words_per_row = a->k / 256 * words, kblocks = a->k / 256;
-    const dim3 ga((words_per_row + 31) / 32, padded_rows(a->m) / 128), gb((words_per_row + 31) / 32, padded_rows(a->n) / 128);
-    pack_scales_kernel<<<ga, 256, 0, s>>>(reinterpret_cast<uint32_t *>(wsa), static_cast<const uint32_t *>(a->d_sfa), a->m,
-                                          words_per_row, kblocks, 0, words);
-    // B's blocks: per 256 columns [k block][instruction][column half] for the 256-wide tile, per 128 columns
-    // [k block][instruction] (A's order) for the 128-wide one
-    pack_scales_kernel<<<gb, 256, 0, s>>>(reinterpret_cast<uint32_t *>(wsb), static_cast<const uint32_t *>(a->d_sfb), a->n,
-                                          words_per_row, kblocks, fp4_tile_n(a->m, a->n, a->k) == 256 ? 1 : 0, words);
-    CLPK_LAUNCH_CHECK("pack_scales");
+    const uint32_t kblocks = a->k / 256;
+    auto operand = [&](const void *in, uint8_t *out, uint32_t rows) {
+        return PackOperand{static_cast<const uint32_t *>(in), reinterpret_cast<uint32_t *>(out), rows, padded_rows(rows) / 128,
+                           (uintptr_t)in % (words * 4) == 0 ? 1u : 0u};
+    };
+    const PackOperand oa = operand(a->d_sfa, wsa, a->m), ob = operand(a->d_sfb, wsb, a->n);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((oa.row_groups + ob.row_groups) * ((kblocks + 7) / 8));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute pdl[1];
+    pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl[0].val.programmaticStreamSerializationAllowed = tuning(CLPK_TUNE_GEMM_NO_PDL) == 1 ? 0 : 1;
+    cfg.attrs = pdl;
+    cfg.numAttrs = 1;
+    const uint32_t b_pairs = fp4_tile_n(a->m, a->n, a->k) == 256 ? 1 : 0;
+    const cudaError_t e = words == 4 ? cudaLaunchKernelEx(&cfg, pack_scales_kernel<4>, oa, ob, kblocks, b_pairs)
+                                     : cudaLaunchKernelEx(&cfg, pack_scales_kernel<2>, oa, ob, kblocks, b_pairs);
+    if (e != cudaSuccess)
+        return cuda_fail(e, "launch pack_scales");
     return CLPK_OK;
 }
 
