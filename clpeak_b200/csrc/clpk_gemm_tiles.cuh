@@ -1,4 +1,4 @@
-// The dense GEMM for shapes that do not fill the chip with 512 x 256 tiles (included by gemm.cu).
+// The GEMM for shapes that do not fill the chip with the large kernels' tiles (included by gemm.cu).
 //
 // Same pieces as gemm_kernel -- CTA pairs, TMA ring, elected-lane issue, bounded waits -- with the split of the work
 // left to the launch:
@@ -17,6 +17,10 @@
 // 128 x 8192 x 8192 42.4 -> 18.6, bf16 64 x 64 x 16384 147 -> 13.3.  Tried: four K blocks per stage (slower from
 // TN = 64 on), asking the next stage's barrier ahead of the instructions (no effect), clusters of 16 for eight splits
 // (10 % for single tiles of K > 8000, slower elsewhere).
+//
+// Block-scaled kinds: TN = 64, 128 or 256 (split), one K block and its scale factors per stage; a block is 13 (NVFP4,
+// TN = 128) issued instructions and costs 0.25 us, so that splitting K pays early: NVFP4 95 x 352 x 8960 14.7 -> 8.0 us,
+// MXFP4 2654 x 120 x 16384 22.4 -> 11.8, NVFP4 458 x 1176 x 6400 12.4 -> 10.2.
 #pragma once
 
 constexpr int kTilesMaxStages = 16;
@@ -31,6 +35,24 @@ struct TilesSmem {
     uint64_t tmem_empty[2];
     uint32_t tmem_base;
 };
+
+// The block-scaled kinds carry 2 KiB of A's factors and 2 KiB per 128 columns of B's with every K block (MXFP4 fills
+// half of that), in the blocks that pack_scales_kernel makes; they go to tensor memory in front of the K block's
+// instructions as in gemm_block_scaled_kernel, in columns of their own per stage behind 256 accumulator columns.
+template <int DT> struct TilesKind {
+    static constexpr bool fp4 = DT == CLPK_DT_NVF4 || DT == CLPK_DT_MXF4;
+    static constexpr uint32_t words = DT == CLPK_DT_MXF4 ? 2 : 4;          // 512-byte blocks per 128 rows and K block
+};
+__host__ __device__ constexpr uint32_t tiles_sf_bytes(uint32_t tn) { return 2048 + (tn + 127) / 128 * 2048; }
+__host__ __device__ constexpr uint32_t tiles_sf_cols(uint32_t tn) { return 16 + (tn + 127) / 128 * 16; }
+
+struct TilesMaps {
+    CUtensorMap a, b, c;
+};
+struct TilesScaleMaps {
+    CUtensorMap a, b, c, sfa, sfb;
+};
+template <int DT> using TilesMapsOf = std::conditional_t<TilesKind<DT>::fp4, TilesScaleMaps, TilesMaps>;
 
 struct TilesParams {
     uint32_t tiles_m, tiles_n, group;
@@ -102,14 +124,24 @@ __device__ __forceinline__ uint32_t cluster_addr(const void *p, uint32_t cta)
     return a;
 }
 
-template <int DT>
-__global__ void __launch_bounds__(kGemmThreads)
-    gemm_tiles_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                      const __grid_constant__ CUtensorMap tmap_c, TilesParams p)
+// 3-D tile load whose completion bytes go to the leader's barrier
+__device__ __forceinline__ void tma_load_pair_3d_at(void *smem_dst, const CUtensorMap *tmap, int32_t x, int32_t y, int32_t z, uint32_t leader_bar)
 {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
+        "l"(tmap), "r"(leader_bar), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+
+template <int DT>
+__global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_constant__ TilesMapsOf<DT> maps, TilesParams p)
+{
+    constexpr bool kFp4 = TilesKind<DT>::fp4;
+    constexpr uint32_t kWords = TilesKind<DT>::words;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const uint32_t block_bytes = tiles_block_bytes(p.tn), stage_bytes = p.kps * block_bytes;
+    const uint32_t block_bytes = tiles_block_bytes(p.tn), stage_bytes = p.kps * block_bytes + (kFp4 ? tiles_sf_bytes(p.tn) : 0);
     uint8_t *staging = smem + (size_t)p.stages * stage_bytes;
     TilesSmem *sh = reinterpret_cast<TilesSmem *>(staging + kEpilogueWarps * kStagingBytes);
 
@@ -129,9 +161,13 @@ __global__ void __launch_bounds__(kGemmThreads)
             mbar_init(&sh->tmem_empty[acc], 2 * kEpilogueWarps);
         }
         mbar_fence_init();
-        tma_prefetch_desc(&tmap_a);
-        tma_prefetch_desc(&tmap_b);
-        tma_prefetch_desc(&tmap_c);
+        tma_prefetch_desc(&maps.a);
+        tma_prefetch_desc(&maps.b);
+        tma_prefetch_desc(&maps.c);
+        if constexpr (kFp4) {
+            tma_prefetch_desc(&maps.sfa);
+            tma_prefetch_desc(&maps.sfb);
+        }
     }
     if (warp == 1)
         tmem_alloc<2>(&sh->tmem_base, p.tmem_cols);
@@ -153,8 +189,8 @@ __global__ void __launch_bounds__(kGemmThreads)
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        uint32_t full0;
-        full0 = cluster_addr(&sh->full[0], leader);
+        const uint32_t full0 = cluster_addr(&sh->full[0], leader);
+        const uint32_t b_blocks = (p.tn + 127) / 128 * kWords;       // scale blocks of B per K block
         uint32_t s = 0, parity = 1;                            // parity of the empty barrier's previous phase
         bool ok = true;
         for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters) {
@@ -173,14 +209,22 @@ __global__ void __launch_bounds__(kGemmThreads)
                 const uint32_t nk = kb1 - kb < p.kps ? kb1 - kb : p.kps;
                 if (elect_one()) {
                     if (r == 0)
-                        mbar_expect_tx(&sh->full[s], nk * 2 * block_bytes);
+                        mbar_expect_tx(&sh->full[s], nk * 2 * block_bytes + (kFp4 ? 2 * (kWords * 512 + b_blocks * 512) : 0));
 #pragma unroll
                     for (uint32_t h = 0; h < 2; h++)
                         if (h < nk) {
                             uint8_t *blk = st + h * block_bytes;
-                            tma_load_pair_at(blk, &tmap_a, x + h * kRowBytesK, row_a, full0 + 8 * s);
-                            tma_load_pair_at(blk + kHalfTileBytes, &tmap_b, x + h * kRowBytesK, row_b, full0 + 8 * s);
+                            tma_load_pair_at(blk, &maps.a, x + h * kRowBytesK, row_a, full0 + 8 * s);
+                            tma_load_pair_at(blk + kHalfTileBytes, &maps.b, x + h * kRowBytesK, row_b, full0 + 8 * s);
                         }
+                    if constexpr (kFp4) {
+                        // A's blocks lie [rows / 128][K block][word], B's [rows / 256][K block][word][half of the 256]
+                        uint8_t *sf = st + block_bytes;
+                        tma_load_pair_at(sf, &maps.sfa, 0, (int32_t)(((mb * 2 + r) * p.k_blocks + kb) * kWords), full0 + 8 * s);
+                        const uint32_t col = nb * p.tn;
+                        tma_load_pair_3d_at(sf + 2048, &maps.sfb, 0, (int32_t)(col / 128 & 1), (int32_t)((col / 256 * p.k_blocks + kb) * kWords),
+                                            full0 + 8 * s);
+                    }
                 }
                 __syncwarp();
                 if (++s == p.stages) {
@@ -195,7 +239,12 @@ __global__ void __launch_bounds__(kGemmThreads)
             constexpr uint32_t kAFmt = DT == CLPK_DT_BF16 ? kFmtBF16 : DT == CLPK_DT_F16 ? kFmtF16 : DT == CLPK_DT_TF32 ? kFmtTF32
                                      : DT == CLPK_DT_I8 ? kFmtS8 : DT == CLPK_DT_E5M2 ? kFmtE5M2 : kFmtE4M3;
             constexpr uint32_t kBFmt = DT == CLPK_DT_E5M2 ? kFmtE4M3 : kAFmt;
-            const uint32_t idesc = make_idesc(256, p.tn, kAFmt, kBFmt, DT == CLPK_DT_I8 ? kAccS32 : kAccF32);
+            constexpr bool kMx = DT == CLPK_DT_MXF4;
+            // MXFP4: instruction kk reads bytes 0-1 (id 0) or 2-3 (id 2) of word kk / 2
+            const uint32_t idesc = kFp4 ? make_idesc_block_scaled(256, p.tn, kFmtE2M1, kFmtE2M1, kMx ? 1u : 0u, 0, 0)
+                                        : make_idesc(256, p.tn, kAFmt, kBFmt, DT == CLPK_DT_I8 ? kAccS32 : kAccF32);
+            const uint32_t idesc_hi = make_idesc_block_scaled(256, p.tn, kFmtE2M1, kFmtE2M1, 1u, 2, 2);
+            const uint32_t b_halves = (p.tn + 127) / 128;
             const uint16_t pair_mask = (uint16_t)(3u << leader);
             uint32_t s = 0, parity = 0, tcount = 0;
             bool ok = true;
@@ -208,6 +257,9 @@ __global__ void __launch_bounds__(kGemmThreads)
                 }
                 tc_fence_after_sync();
                 const uint32_t d = tmem + acc * p.tn;
+                [[maybe_unused]] uint32_t mb, nb = 0;
+                if constexpr (kFp4)
+                    dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
                 for (uint32_t kb = kb0; kb < kb1; kb += p.kps) {
                     if (!warp_wait(&sh->full[s], parity)) {
                         if (lane == 0)
@@ -224,9 +276,30 @@ __global__ void __launch_bounds__(kGemmThreads)
                         parity ^= 1;
                     }
                     if (elect_one()) {
+                        if constexpr (kFp4) {
+                            const uint32_t sf_s = base + block_bytes, sfa_t = tmem + 256 + s_now * tiles_sf_cols(p.tn);
+                            const uint64_t ad = make_smem_desc(base, 16, 1024, kSwizzle128B);
+                            const uint64_t bd = make_smem_desc(base + kHalfTileBytes, 16, 1024, kSwizzle128B);
+#pragma unroll
+                            for (uint32_t w = 0; w < kWords; w++)
+                                tmem_cp_32x128b_warpx4<2>(sfa_t + 4 * w, make_smem_desc(sf_s + w * 512, 16, 128, kSwizzleNone));
+                            for (uint32_t w = 0; w < kWords * b_halves; w++)
+                                tmem_cp_32x128b_warpx4<2>(sfa_t + 16 + 4 * w, make_smem_desc(sf_s + 2048 + w * 512, 16, 128, kSwizzleNone));
+                            // a 64-column tile in the upper half of its 128 reads the upper two of a word's four columns
+                            const uint32_t sfb_t = sfa_t + 16 + (nb * p.tn % 128) / 32;
+#pragma unroll
+                            for (uint32_t kk = 0; kk < 4; kk++) {
+                                const uint32_t accumulate = (kb != kb0 || kk != 0) ? 1u : 0u;
+                                if constexpr (kMx)
+                                    mma2_mxf4_bs(d, ad + 2 * kk, bd + 2 * kk, (kk & 1) ? idesc_hi : idesc, sfa_t + 4 * (kk / 2),
+                                                 sfb_t + 4 * b_halves * (kk / 2), accumulate);
+                                else
+                                    mma2_nvf4_bs(d, ad + 2 * kk, bd + 2 * kk, idesc, sfa_t + 4 * kk, sfb_t + 4 * b_halves * kk, accumulate);
+                            }
+                        }
 #pragma unroll
                         for (uint32_t h = 0; h < 2; h++) {
-                            if (h >= nk)
+                            if (kFp4 || h >= nk)
                                 break;
                             const uint32_t blk = base + h * block_bytes;
                             const uint64_t ad = make_smem_desc(blk, 16, 1024, kSwizzle128B);
@@ -240,7 +313,7 @@ __global__ void __launch_bounds__(kGemmThreads)
                                     mma2_tf32_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
                                 else if constexpr (DT == CLPK_DT_I8)
                                     mma2_i8_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-                                else
+                                else if constexpr (!kFp4)
                                     mma2_f16_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
                             }
                         }
@@ -286,9 +359,9 @@ __global__ void __launch_bounds__(kGemmThreads)
                 tmem_ld_wait();
                 if (c + 4 >= n_chunks)
                     release();
-                tiles_store_chunk<DT>(v0, p.alpha, boxes, n_stored, &tmap_c, nb * p.tn + c * kTilesChunk, row, lane);
+                tiles_store_chunk<DT>(v0, p.alpha, boxes, n_stored, &maps.c, nb * p.tn + c * kTilesChunk, row, lane);
                 if (two)
-                    tiles_store_chunk<DT>(v1, p.alpha, boxes, n_stored, &tmap_c, nb * p.tn + (c + 2) * kTilesChunk, row, lane);
+                    tiles_store_chunk<DT>(v1, p.alpha, boxes, n_stored, &maps.c, nb * p.tn + (c + 2) * kTilesChunk, row, lane);
             }
         }
     } else if (!warp_wait(&sh->tmem_full[0], 0)) {
@@ -351,7 +424,7 @@ __global__ void __launch_bounds__(kGemmThreads)
                         }
                     }
                 }
-                tiles_store_chunk<DT>(sum, p.alpha, boxes, n_stored, &tmap_c, nb * p.tn + c * kTilesChunk, row, lane);
+                tiles_store_chunk<DT>(sum, p.alpha, boxes, n_stored, &maps.c, nb * p.tn + c * kTilesChunk, row, lane);
             }
         }
     }

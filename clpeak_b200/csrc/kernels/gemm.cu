@@ -28,6 +28,7 @@
 
 #include <atomic>
 #include <cstdlib>
+#include <type_traits>
 
 #include "../clpk_internal.h"
 #include "../clpk_ptx.cuh"
@@ -642,6 +643,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads)
 //    mbarrier waits, one polling lane per epilogue warp, raster group widths from 4 to 32, four stages instead of
 //    five (3 %), C stored with the L2 evict-first policy.
 
+// rows of a block-scaled operand rounded up to whole 256-row tiles
+static inline uint32_t padded_rows(uint32_t rows) { return (rows + 255u) / 256u * 256u; }
+
 constexpr int kNvMaxStages = 6;
 constexpr int kNvGemmThreads = 32 * (3 + kEpilogueWarps);                   // operand producer, MMA, 8 epilogue warps, scale producer
 constexpr uint32_t kNvSfCol = 256;                             // first scale column: after the accumulator(s)
@@ -1057,6 +1061,28 @@ static int make_scale_map(CUtensorMap *map, const void *base, uint64_t n_rows, u
 }
 
 
+// B's packed scale factors for gemm_tiles_kernel: [rows / 256 * K blocks * words][half of the 256 rows][512 bytes]; a box
+// is one K block's words of one half, or of both.
+static int make_scale_map_b(CUtensorMap *map, const void *base, uint64_t n_rows, uint32_t words, uint32_t halves)
+{
+    EncodeTiledFn enc;
+    int rc = get_encode_fn(&enc);
+    if (rc != CLPK_OK)
+        return rc;
+    const cuuint64_t dims[3] = {128, 2, n_rows / 2};
+    const cuuint64_t strides[2] = {512, 1024};
+    const cuuint32_t box[3] = {128, halves, words};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void *>(base), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled (scales) failed with CUresult %d", (int)r);
+        return CLPK_ERR_CUDA;
+    }
+    return CLPK_OK;
+}
+
 constexpr size_t kGemmSmemBytes = (size_t)kDenseStages * kDenseStageBytes + kEpilogueWarps * kStagingBytes + sizeof(DenseSmem) + 1024;
 
 // One wave counter per launch, from a ring of 32 per device so that launches on different streams
@@ -1134,39 +1160,52 @@ static int launch_persistent(Kernel kernel, const char *what, int threads, size_
     return CLPK_OK;
 }
 
-// How gemm_tiles_kernel splits a problem; tn = 0: leave it to gemm_kernel.
+// How gemm_tiles_kernel splits a problem; tn = 0: leave it to gemm_kernel or gemm_block_scaled_kernel.
 struct TilesPlan {
     uint32_t tn, splits;
 };
 
-// The plan is the cheapest by a cost estimate in microseconds, fitted to 2500 timed launches of both kernels: 120
-// shapes with M and N from 64 to 14000, K from 256 to 16000 in all six dense types, every tile width and split
-// (residual 13 %; the chosen plan is 1 % slower than the fastest one in the geometric mean, 19 % at worst).
-//   gemm_kernel        3.6 + waves * (0.57 per 128-byte K block of a 512 x 256 tile + 2.9), and 9.3 for the cooperative
-//                      launch and its memsets when there are more than two waves
-//   gemm_tiles_kernel  3.9 + waves * (K blocks * (0.118 to issue a block + 0.175 TN / 256 for its instructions + the bytes
-//                      all SMs fetch for it at 54 TB/s) + 1.1 TN / 256 of epilogue) and, split, 1 + the exchange
+// The plan is the cheapest by a cost estimate in microseconds, fitted to timed launches of both kernels: 2500 for 120
+// shapes with M and N from 64 to 14000, K from 256 to 16000 in the six dense types, 300 for 90 block-scaled ones, every
+// tile width and split of each (residuals 13 and 6 %; the chosen plans are 1 % slower than the fastest in the geometric
+// mean, 19 % at worst).  With W = TN / 256 and T the time to fetch what all SMs load for one K block of 128 bytes:
+//   gemm_kernel               3.6 + waves * (0.57 per K block of a 512 x 256 tile + 2.9), and 9.3 for the cooperative
+//                             launch and its memsets when there are more than two waves
+//   gemm_tiles_kernel, dense  3.9 + waves * (K blocks * (0.118 to issue a block + 0.175 W for its instructions + T at
+//                             54 TB/s) + 1.1 W of epilogue) and, split, 1 + 4.3 W per exchanged share of the tile
+//   gemm_block_scaled_kernel  4.0 + waves * (K blocks * (0.275 + T at 43 TB/s) + 0.7)
+//   gemm_tiles_kernel, FP4    3.3 + waves * (K blocks * (0.25 + 0.06 W + T at 62 TB/s) + 1.4 W) and the same exchange
 // Splits of 2 and 4 are clusters of 4 and 8 CTAs, of which the chip holds 33 and 15 at a time.  From the fifth wave of
-// 512 x 256 tiles on that kernel's smaller operand traffic wins at every K (16384 x 16384 x 256: 140 against 142 us).
-static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks)
+// 512 x 256 tiles on (16384 x 16384 x 256: 140 against 142 us) and the third of block-scaled ones the large tiles'
+// smaller operand traffic wins at every K; an FP4 tile 256 wide that is not split is the large kernel's own.
+static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4)
 {
     const uint32_t pairs = (uint32_t)num_sms() / 2;
     auto ceil_div = [](uint32_t a, uint32_t b) { return (a - 1) / b + 1; };
-    const uint64_t big_tiles = (uint64_t)ceil_div(m, kDenseTileM) * ceil_div(n, kTileMN);
+    // bytes that `clusters` clusters of `splits` pairs load for one K block of a 256 x tn tile each
+    auto fetched = [&](uint64_t clusters, uint32_t splits, uint32_t tn) {
+        return (float)clusters * splits * ((m < 256 ? m : 256) + (n < tn ? n : tn)) * kRowBytesK;
+    };
+    const uint64_t big_tiles = (uint64_t)ceil_div(m, fp4 ? kTileMN : kDenseTileM) * ceil_div(n, kTileMN);
     TilesPlan plan = {0, 1};
-    if (pairs == 0 || big_tiles > 4ull * pairs)
+    if (pairs == 0 || big_tiles > (fp4 ? 2ull : 4ull) * pairs)
         return plan;
-    const uint32_t big_waves = ceil_div((uint32_t)big_tiles, pairs);
-    float best = 0.97f * (3.6f + (big_waves > 2 ? 9.3f : 0.0f) + big_waves * (k_blocks * 0.57f + 2.9f));
+    const float big_waves = (float)((big_tiles - 1) / pairs + 1);
+    const float big = fp4 ? 4.0f + big_waves * (k_blocks * (0.275f + fetched(big_tiles < pairs ? big_tiles : pairs, 1, 256) / 43.2e6f) + 0.7f)
+                          : 3.6f + (big_waves > 2 ? 9.3f : 0.0f) + big_waves * (k_blocks * 0.57f + 2.9f);
+    float best = 0.97f * big;
+    const float launch = fp4 ? 3.3f : 3.9f, issue = fp4 ? 0.25f : 0.118f, wide_issue = fp4 ? 0.06f : 0.175f;
+    const float rate = fp4 ? 62.4e6f : 53.8e6f, drain = fp4 ? 1.36f : 1.14f;
     for (uint32_t splits = 1; splits <= 4; splits *= 2) {
         const uint32_t resident = splits == 1 ? pairs : splits == 2 ? pairs * 33 / 74 : pairs * 15 / 74;
         if (resident == 0 || k_blocks < splits)
             break;
-        for (uint32_t tn = 32; tn <= kTileMN; tn += 32) {
+        // scale factors come in blocks of 128 columns, of which a 64-wide tile uses half
+        for (uint32_t tn = fp4 ? 64 : 32; tn <= (fp4 && splits == 1 ? 128u : 256u); tn = fp4 ? 2 * tn : tn + 32) {
             const uint64_t tiles = (uint64_t)ceil_div(m, kTilesM) * ceil_div(n, tn);
             const float waves = (float)((tiles - 1) / resident + 1), wide = (float)tn / 256.0f;
-            const float fetched = (float)(tiles < resident ? tiles : resident) * splits * ((m < kTilesM ? m : kTilesM) + (n < tn ? n : tn)) * kRowBytesK;
-            float t = 3.9f + waves * (ceil_div(k_blocks, splits) * (0.118f + 0.175f * wide + fetched / 53.8e6f) + 1.14f * wide);
+            const float block = issue + wide_issue * wide + fetched(tiles < resident ? tiles : resident, splits, tn) / rate;
+            float t = launch + waves * (ceil_div(k_blocks, splits) * block + drain * wide);
             if (splits > 1)
                 t += waves * (1.0f + 4.3f * wide * (splits - 1) / splits);
             if (t < best) {
@@ -1178,16 +1217,28 @@ static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks)
     return plan;
 }
 
+// wsa, wsb: the packed scale factors (block-scaled kinds)
 template <int DT>
-static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64_t row_bytes, uint32_t k_blocks, TilesPlan plan, cudaStream_t s)
+static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64_t row_bytes, uint32_t k_blocks, TilesPlan plan, cudaStream_t s,
+                        const uint8_t *wsa = nullptr, const uint8_t *wsb = nullptr)
 {
-    CUtensorMap tb, tc;
-    int rc = make_operand_map(&tb, a->d_b, a->n, row_bytes, plan.tn / 2);
+    TilesMapsOf<DT> maps;
+    maps.a = ta;
+    int rc = make_operand_map(&maps.b, a->d_b, a->n, row_bytes, plan.tn / 2);
     if (rc != CLPK_OK)
         return rc;
-    rc = make_output_map(&tc, a->d_c, a->m, a->n, DT, true);
+    rc = make_output_map(&maps.c, a->d_c, a->m, a->n, DT, true);
     if (rc != CLPK_OK)
         return rc;
+    if constexpr (TilesKind<DT>::fp4) {
+        constexpr uint32_t words = TilesKind<DT>::words;
+        rc = make_scale_map(&maps.sfa, wsa, (uint64_t)padded_rows(a->m) / 128 * k_blocks * words, words);
+        if (rc != CLPK_OK)
+            return rc;
+        rc = make_scale_map_b(&maps.sfb, wsb, (uint64_t)padded_rows(a->n) / 128 * k_blocks * words, words, (plan.tn + 127) / 128);
+        if (rc != CLPK_OK)
+            return rc;
+    }
     TilesParams p;
     p.tiles_m = (a->m + kTilesM - 1) / kTilesM;
     p.tiles_n = (a->n + plan.tn - 1) / plan.tn;
@@ -1202,15 +1253,18 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
     const size_t fixed = kEpilogueWarps * kStagingBytes + sizeof(TilesSmem) + 1024;
     // two K blocks per stage halve the hand-overs (0.195 -> 0.137 us per block at TN = 32), but from TN = 160 on leave
     // too few stages (2048^3 bf16 at TN = 192: 19.3 -> 20.7 us)
-    p.kps = plan.tn <= 128 ? 2 : 1;
-    p.stages = (uint32_t)((kTilesSmemMax - fixed) / (p.kps * tiles_block_bytes(plan.tn)));
-    if (p.stages > kTilesMaxStages)
-        p.stages = kTilesMaxStages;
-    p.tmem_cols = 32;
+    constexpr bool fp4 = TilesKind<DT>::fp4;
+    p.kps = plan.tn <= 128 && !fp4 ? 2 : 1;
+    const uint32_t stage_bytes = p.kps * tiles_block_bytes(plan.tn) + (fp4 ? tiles_sf_bytes(plan.tn) : 0);
+    p.stages = (uint32_t)((kTilesSmemMax - fixed) / stage_bytes);
+    const uint32_t most = fp4 ? 256 / tiles_sf_cols(plan.tn) : kTilesMaxStages;      // scale factors: 256 tensor-memory columns
+    if (p.stages > most)
+        p.stages = most;
+    p.tmem_cols = fp4 ? 512 : 32;
     while (p.tmem_cols < (n_tiles > clusters ? 2 : 1) * plan.tn)
         p.tmem_cols *= 2;
     CLPK_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&p.clock), g_gemm_clock));
-    const size_t smem = p.stages * p.kps * tiles_block_bytes(plan.tn) + fixed;
+    const size_t smem = p.stages * stage_bytes + fixed;
     CLPK_CUDA(cudaFuncSetAttribute(gemm_tiles_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTilesSmemMax));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(clusters * 2 * plan.splits);
@@ -1226,7 +1280,7 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
     cfg.attrs = attr;
     cfg.numAttrs = 2;
     g_last_aligned = 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tiles_kernel<DT>, ta, tb, tc, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tiles_kernel<DT>, maps, p);
     if (e != cudaSuccess)
         return cuda_fail(e, "gemm_tiles");
     return CLPK_OK;
@@ -1259,9 +1313,6 @@ int clpk_gemm_last_clock(unsigned long long *h_cycles, unsigned long long *h_ns,
     *h_ns = v[1];
     return CLPK_OK;
 }
-
-// rows of a block-scaled operand rounded up to whole 256-row tiles
-static inline uint32_t padded_rows(uint32_t rows) { return (rows + 255u) / 256u * 256u; }
 
 int clpk_gemm_workspace_bytes(int dtype, uint32_t m, uint32_t n, uint32_t k, size_t *bytes)
 {
@@ -1421,6 +1472,10 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
                 return rc;
         }
         const uint32_t tn = fp4_tile_n(a->m, a->n, a->k);
+        if (tuning(CLPK_TUNE_GEMM_FP4_TILE) <= 0)                // the knob's forced tiles are the large kernel's
+            if (const TilesPlan plan = plan_tiles(a->m, a->n, p.k_blocks, true); plan.tn)
+                return mx ? launch_tiles<CLPK_DT_MXF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb)
+                          : launch_tiles<CLPK_DT_NVF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb);
         CUtensorMap tsa, tsb;
         rc = make_scale_map(&tsa, wsa, sfa_bytes / 512, words);
         if (rc != CLPK_OK)
@@ -1450,7 +1505,7 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
                   : launch_persistent(gemm_block_scaled_kernel<false, 256>, "gemm_nvf4", kNvGemmThreads,
                                       BlockScaled<false, 256>::smem_bytes, s, p, n_tiles, ta, tb, tsa, tsb, tc);
     }
-    if (const TilesPlan plan = plan_tiles(a->m, a->n, p.k_blocks); plan.tn) {
+    if (const TilesPlan plan = plan_tiles(a->m, a->n, p.k_blocks, false); plan.tn) {
         switch (a->dtype) {
         case CLPK_DT_BF16: return launch_tiles<CLPK_DT_BF16>(a, ta, row_bytes, p.k_blocks, plan, s);
         case CLPK_DT_F16:  return launch_tiles<CLPK_DT_F16>(a, ta, row_bytes, p.k_blocks, plan, s);

@@ -47,3 +47,34 @@ def test_scales_at_any_word_alignment(K, cuda, dtype, m, n, k):
         results.append((ws, c))
     for ws, c in results[1:]:
         assert bool((ws == results[0][0]).all()) and bool((c == results[0][1]).all())
+
+
+def decoded(cuda, dtype, q, sf, rows, k):
+    """The operand's values in fp64."""
+    codes = cuda.stack((q & 15, q >> 4), dim=-1).view(rows, k).long()
+    mags = cuda.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0], dtype=cuda.float64, device="cuda")
+    values = mags[codes & 7] * cuda.where(codes >= 8, -1.0, 1.0)
+    block = 16 if dtype == N.DT_NVF4 else 32
+    scale = sf.view(cuda.float8_e4m3fn).double() if dtype == N.DT_NVF4 else cuda.exp2(sf.double() - 127)
+    return values * scale.view(rows, k // block).repeat_interleave(block, dim=1)
+
+
+# one stage; 64-wide tiles in both halves of a scale block, with ragged last tiles; K split in two and four with ranges
+# of unequal length; several tiles per CTA pair; the 256-wide split tile; the large kernel's whole tiles
+@pytest.mark.parametrize("m,n,k", [(1, 8, 256), (64, 64, 256), (200, 200, 512), (384, 480, 256), (95, 352, 8960), (300, 136, 11008),
+                                   (350, 416, 3328), (458, 1176, 6400), (2656, 120, 16384), (72, 1136, 13568), (8404, 216, 1024),
+                                   (6976, 544, 5376), (512, 512, 2048)])
+@pytest.mark.parametrize("dtype", [N.DT_NVF4, N.DT_MXF4])
+def test_every_element(K, cuda, dtype, m, n, k):
+    a, sfa, ta, _ = make_nvfp4_operand(K, cuda, m, k, 40, dtype)
+    b, sfb, tb, _ = make_nvfp4_operand(K, cuda, n, k, 41, dtype)
+    alpha, ws = ta * tb, workspace(K, cuda, dtype, m, n, k)
+    c = run(K, cuda, dtype, m, n, k, a, sfa.data_ptr(), b, sfb.data_ptr(), alpha, ws)
+    fa, fb = decoded(cuda, dtype, a, sfa, m, k), decoded(cuda, dtype, b, sfb, n, k)
+    want = alpha * (fa @ fb.T)
+    # K roundings of the accumulator (truncating adder: one ulp each), one of alpha, one of the bf16 result
+    tol = (k + 1) * 2.0 ** -23 * alpha * (fa.abs() @ fb.abs().T) + 2.0 ** -8 * want.abs() + 1e-30
+    worst = float(((c.view(cuda.bfloat16).double().view(m, n) - want).abs() / tol).max())
+    assert worst <= 1.0, f"worst error over all of C is {worst:.3g}x the stated tolerance"
+    again = run(K, cuda, dtype, m, n, k, a, None, b, None, alpha, ws)       # scales already arranged
+    assert bool((again == c).all()), "partial sums are added in a fixed order: the same bits every time"
