@@ -26,9 +26,9 @@ int smem_optin_bytes(); // of the current device
 // clpk_set_tuning has set it.
 int tuning(int knob);
 
-// fp32 (CUDA cores) and fp64 (DMMA) GEMMs, simt_gemm.cu; dtype is CLPK_DT_F32 or CLPK_DT_F64.
+// fp32 (CUDA cores) and fp64 (DMMA) GEMMs, simt_gemm.cu; dtype is CLPK_DT_F32 or CLPK_DT_F64; *status is cleared.
 int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t m, uint32_t n, uint32_t k, float alpha,
-                     cudaStream_t s);
+                     uint32_t *status, cudaStream_t s);
 
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 

@@ -1395,9 +1395,8 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
     CLPK_REQUIRE(a->d_a && a->d_b && a->d_c && a->d_status, "NULL buffer");
     if (a->dtype == CLPK_DT_F32 || a->dtype == CLPK_DT_F64) {
         // no tcgen05 kind for these: the CUDA-core fp32 and DMMA fp64 kernels of simt_gemm.cu
-        CLPK_CUDA(cudaMemsetAsync(a->d_status, 0, sizeof(uint32_t), as_stream(stream)));
         g_last_aligned = 0;
-        return launch_simt_gemm(a->dtype, a->d_a, a->d_b, a->d_c, a->m, a->n, a->k, a->alpha, as_stream(stream));
+        return launch_simt_gemm(a->dtype, a->d_a, a->d_b, a->d_c, a->m, a->n, a->k, a->alpha, a->d_status, as_stream(stream));
     }
     CLPK_REQUIRE(a->m > 0 && a->n > 0 && a->k > 0, "M, N and K must be positive");
     const bool block_scaled = a->dtype == CLPK_DT_NVF4 || a->dtype == CLPK_DT_MXF4;

@@ -34,14 +34,20 @@
 // k lane%4) fall in 16 distinct 8-byte banks per half warp.  Bound: the DMMA pipe, 64
 // fp64 FMA / clock / SM, the same rate as the scalar DFMA pipe (37.2 TFLOPS at 1.965 GHz).
 //
-// Both take any M, N > 0 and any K that keeps operand rows 16-byte aligned (a multiple of 4
-// floats, 2 doubles): a second instantiation of each kernel zero-fills the chunks a tile
-// reaches beyond A or B (cp.async with a source size of 0) and skips the stores beyond C;
+// Shapes of which those tiles make too few CTAs take 64 x 64 (fp32, fp64) or 32 x 32 (fp64) tiles with K split over the
+// CTAs of a cluster and over groups of warps inside a CTA (sgemm64_kernel, dgemm_split_kernel; plan_simt has the rule).
+// Device time before -> after: fp32 64 x 64 x 16384 1545 -> 69 us, 459 x 349 x 4636 474 -> 52, 2048^3 342 -> 323; fp64
+// 64 x 64 x 16384 1388 -> 33, 863 x 251 x 2456 228 -> 51, 2048 x 2048 x 512 151 -> 143.
+//
+// All take any M, N > 0 and any K that keeps operand rows 16-byte aligned (a multiple of 4
+// floats, 2 doubles): a second instantiation of the large kernels, and the others always, zero-fill the chunks a tile
+// reaches beyond A or B (cp.async with a source size of 0) and skip the stores beyond C;
 // whole tiles and k blocks take the instantiation without the checks.
 //
 // CTAs walk C in groups of 16 tile rows so that the operand panels a wave of CTAs needs
 // stay in L2.  Work 2*M*N*K flop; minimum HBM bytes (M*K + N*K + M*N) * element.
 #include "../clpk_internal.h"
+#include "../clpk_ptx.cuh"
 
 namespace clpk {
 
@@ -49,14 +55,84 @@ constexpr int kSimtTile = 128;
 constexpr int kSimtBK = 16;
 constexpr int kRasterGroup = 16;
 
-// blockIdx.x -> (tile row, tile column), column-major inside groups of kRasterGroup tile rows
-__device__ __forceinline__ void raster(uint32_t tiles_m, uint32_t tiles_n, uint32_t *tm, uint32_t *tn)
+// tile -> (tile row, tile column), column-major inside groups of kRasterGroup tile rows
+__device__ __forceinline__ void raster(uint32_t tile, uint32_t tiles_m, uint32_t tiles_n, uint32_t *tm, uint32_t *tn)
 {
     const uint32_t per_group = kRasterGroup * tiles_n;
-    const uint32_t g = blockIdx.x / per_group, r = blockIdx.x % per_group;
+    const uint32_t g = tile / per_group, r = tile % per_group;
     const uint32_t rows = min((uint32_t)kRasterGroup, tiles_m - g * kRasterGroup);
     *tm = g * kRasterGroup + r % rows;
     *tn = r / rows;
+}
+
+// The launches carry the programmatic-serialisation attribute: a CTA may start under the tail of the kernel before it
+// in the stream and waits here until that has completed.  The status word is cleared by the kernel, so that nothing
+// sits between two launches.
+__device__ __forceinline__ void join_stream(uint32_t *status)
+{
+    griddep_wait();
+    griddep_launch_dependents();
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *status = 0u;
+}
+
+// ---- K split over the CTAs of a cluster -----------------------------------------------------------------------------
+//
+// Each of the S CTAs leaves its partial tiles in its own shared memory ([parts][rows][cols], parts = K groups inside the
+// CTA) and sums a share of the rows over all of them, in rank order: the same bits whatever the timing.
+
+template <typename T> struct Vec16;
+template <> struct Vec16<float> { using type = float4; };
+template <> struct Vec16<double> { using type = double2; };
+__device__ __forceinline__ void add_to(float4 &a, const float4 &b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+__device__ __forceinline__ void add_to(double2 &a, const double2 &b) { a.x += b.x; a.y += b.y; }
+__device__ __forceinline__ float4 ld_cluster(uint32_t addr, float4)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ double2 ld_cluster(uint32_t addr, double2)
+{
+    double2 v;
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+
+// `part`: this CTA's partial tiles, just written; called by all threads.
+template <typename T, int ROWS, int COLS, int PARTS, int THREADS>
+__device__ __forceinline__ void sum_partial_tiles(const T *part, uint32_t S, uint32_t rank, T *C, uint32_t row0, uint32_t col0, uint32_t M,
+                                                  uint32_t N, T alpha)
+{
+    using V = typename Vec16<T>::type;
+    constexpr uint32_t per = 16 / sizeof(T), row_vecs = COLS / per, vecs = ROWS * row_vecs;
+    cluster_sync();
+    const uint32_t local = smem_u32(part);
+    for (uint32_t i = rank * vecs / S + threadIdx.x; i < (rank + 1) * vecs / S; i += THREADS) {
+        V sum;
+        for (uint32_t src = 0; src < S; src++) {
+            uint32_t addr;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local + i * 16), "r"(src));
+#pragma unroll
+            for (int q = 0; q < PARTS; q++) {
+                const V v = ld_cluster(addr + q * (ROWS * COLS * (uint32_t)sizeof(T)), V{});
+                if (src == 0 && q == 0)
+                    sum = v;
+                else
+                    add_to(sum, v);
+            }
+        }
+        const uint32_t row = row0 + i / row_vecs, col = col0 + i % row_vecs * per;
+        if (row < M) {
+            const T *e = reinterpret_cast<const T *>(&sum);
+            T *dst = C + (size_t)row * N + col;
+#pragma unroll
+            for (uint32_t t = 0; t < per; t++)
+                if (col + t < N)
+                    dst[t] = alpha * e[t];
+        }
+    }
+    cluster_sync();                     // nobody leaves while its shared memory is being read
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -108,13 +184,14 @@ __device__ __forceinline__ void cp_async_16_or_zeros(void *dst_shared, const voi
 template <bool RAGGED>
 __global__ void __launch_bounds__(kSgemmThreads, 2)
 sgemm_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ C, uint32_t M, uint32_t N,
-             uint32_t K, float alpha)
+             uint32_t K, float alpha, uint32_t *status)
 {
     extern __shared__ __align__(16) float ssm[];
     float *const tiles = ssm;                                   // [buffer][A, B][k][kSgemmLd]
     float *const staging = ssm + 4 * kSgemmTileFloats;          // [buffer][chunk][thread] of float4
     uint32_t tm, tn;
-    raster((M + kSimtTile - 1) / kSimtTile, (N + kSimtTile - 1) / kSimtTile, &tm, &tn);
+    raster(blockIdx.x, (M + kSimtTile - 1) / kSimtTile, (N + kSimtTile - 1) / kSimtTile, &tm, &tn);
+    join_stream(status);
     // Four warps in a 2 x 2 grid, 64 x 64 outputs per warp, a warp 8 (rows) x 4 (columns) threads, 8 rows x 16
     // columns per thread as 4 x 4 blocks.  A 128-bit shared-memory load takes two passes of the data pipe per warp
     // when every group of four consecutive lanes asks for at most two different 16-byte words, and four passes
@@ -245,6 +322,129 @@ sgemm_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__
     }
 }
 
+// The same product in 64 x 64 tiles for shapes of which 128 x 128 tiles make too few, K split over the CTAs of a cluster
+// and over two groups of two warps inside a CTA.  A group takes every other k block of its CTA's range through staging
+// and tile buffers of its own and meets only its own 64 threads.  64 x 32 outputs per warp, 8 x 8 per thread: four
+// 128-bit fragment loads per 32 packed FMAs.
+constexpr int kSgemm64 = 64;
+constexpr int kSgemm64Ld = kSgemm64 + 4;
+constexpr int kSgemm64Groups = 2, kSgemm64GroupThreads = kSgemmThreads / kSgemm64Groups;
+constexpr size_t kSgemm64TileFloats = (size_t)kSimtBK * kSgemm64Ld;
+constexpr size_t kSgemm64StagingFloats = 8 * 4 * (size_t)kSgemm64GroupThreads; // eight chunks per thread
+constexpr size_t kSgemm64GroupFloats = 4 * kSgemm64TileFloats + 2 * kSgemm64StagingFloats;
+constexpr size_t kSgemm64SmemBytes = kSgemm64Groups * kSgemm64GroupFloats * sizeof(float);
+static_assert(kSgemm64 * kSgemm64 <= kSgemm64GroupFloats, "the partial tiles take the buffers' place");
+
+__global__ void __launch_bounds__(kSgemmThreads, 3)
+sgemm64_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ C, uint32_t M, uint32_t N,
+               uint32_t K, float alpha, uint32_t S, uint32_t *status)
+{
+    extern __shared__ __align__(16) float ssm[];
+    const int group = threadIdx.x / kSgemm64GroupThreads, tid = threadIdx.x % kSgemm64GroupThreads;
+    float *const tiles = ssm + group * kSgemm64GroupFloats;     // [buffer][A, B][k][kSgemm64Ld]
+    float *const staging = tiles + 4 * kSgemm64TileFloats;      // [buffer][chunk][thread] of float4
+    uint32_t tm, tn;
+    const uint32_t rank = blockIdx.x % S;
+    raster(blockIdx.x / S, (M + kSgemm64 - 1) / kSgemm64, (N + kSgemm64 - 1) / kSgemm64, &tm, &tn);
+    join_stream(status);
+    const uint32_t nk_all = (K + kSimtBK - 1) / kSimtBK, kb0 = rank * nk_all / S, kb1 = (rank + 1) * nk_all / S;
+    const uint32_t nk = kb1 - kb0 > (uint32_t)group ? (kb1 - kb0 - group - 1) / kSgemm64Groups + 1 : 0;   // this group's k blocks
+    auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kSgemm64GroupThreads) : "memory"); };
+
+    // the lane map of sgemm_kernel: 8 (rows) x 4 (columns) threads per warp
+    const int lane = tid & 31, lx = (lane & 1) | ((lane >> 1) & 2), ly = ((lane >> 1) & 1) | ((lane >> 2) & 6);
+    const int fa = ly * 4, fb = (tid >> 5) * 32 + lx * 4;
+    const int lrow = tid >> 2, lk = (tid & 3) * 4;
+    const uint32_t row_a = tm * kSgemm64 + lrow, row_b = tn * kSgemm64 + lrow;
+    const float *srcA = A + (size_t)row_a * K + lk, *srcB = B + (size_t)row_b * K + lk;
+    auto fetch = [&](uint32_t i) {                              // the group's i-th k block into staging buffer i % 2
+        float *st = staging + (i & 1) * kSgemm64StagingFloats + tid * 4;
+        const uint32_t k0 = (kb0 + i * kSgemm64Groups + group) * kSimtBK;
+        const bool in_k = k0 + lk < K;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const bool in_a = in_k && row_a + 16 * c < M, in_b = in_k && row_b + 16 * c < N;
+            cp_async_16_or_zeros(st + c * 4 * kSgemm64GroupThreads, in_a ? srcA + (size_t)c * 16 * K + k0 : A, in_a);
+            cp_async_16_or_zeros(st + (4 + c) * 4 * kSgemm64GroupThreads, in_b ? srcB + (size_t)c * 16 * K + k0 : B, in_b);
+        }
+    };
+    auto transpose = [&](uint32_t i) {
+        const float *st = staging + (i & 1) * kSgemm64StagingFloats + tid * 4;
+        float *sA = tiles + (i & 1) * 2 * kSgemm64TileFloats, *sB = sA + kSgemm64TileFloats;
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const float4 v = *reinterpret_cast<const float4 *>(st + c * 4 * kSgemm64GroupThreads);
+            float *dst = (c < 4 ? sA : sB) + lk * kSgemm64Ld + ((lrow + 16 * (c & 3)) ^ (lk & 8));     // see sgemm_kernel
+            dst[0] = v.x; dst[kSgemm64Ld] = v.y; dst[2 * kSgemm64Ld] = v.z; dst[3 * kSgemm64Ld] = v.w;
+        }
+    };
+    unsigned long long acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            acc[i][j] = 0ull;
+
+#pragma unroll
+    for (uint32_t i = 0; i < 2; i++) {
+        if (i < nk)
+            fetch(i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (nk > 0)
+        transpose(0);
+    group_sync();
+    for (uint32_t kb = 0; kb < nk; kb++) {
+        // this thread emptied its part of staging buffer kb % 2 into the tile
+        if (kb + 2 < nk)
+            fetch(kb + 2);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float *sA = tiles + (kb & 1) * 2 * kSgemm64TileFloats, *sB = sA + kSgemm64TileFloats;
+#pragma unroll
+        for (int k = 0; k < kSimtBK; k++) {
+            const int ca = fa ^ (k & 8), cb = fb ^ (k & 8);
+            float a[8];
+            unsigned long long b[4];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const float4 v = *reinterpret_cast<const float4 *>(sA + k * kSgemm64Ld + ca + 32 * q);
+                a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float4 v = *reinterpret_cast<const float4 *>(sB + k * kSgemm64Ld + cb + 16 * h);
+                b[2 * h] = pack2(v.x, v.y);
+                b[2 * h + 1] = pack2(v.z, v.w);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const unsigned long long aa = pack2(a[i], a[i]);
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    ffma2(acc[i][j], aa, b[j]);
+            }
+        }
+        if (kb + 1 < nk) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            transpose(kb + 1);
+            group_sync();
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+    __syncthreads();
+    float *part = ssm + group * (kSgemm64 * kSgemm64);          // [group][64][64]
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const float2 lo = unpack2(acc[i][2 * h]), hi = unpack2(acc[i][2 * h + 1]);
+            *reinterpret_cast<float4 *>(part + (fa + 32 * (i >> 2) + (i & 3)) * kSgemm64 + fb + 16 * h) = make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+    sum_partial_tiles<float, kSgemm64, kSgemm64, kSgemm64Groups, kSgemmThreads>(ssm, S, rank, C, tm * kSgemm64, tn * kSgemm64, M, N, alpha);
+}
+
 // ---------------------------------------------------------------------------------------------
 // fp64
 // ---------------------------------------------------------------------------------------------
@@ -269,13 +469,14 @@ __device__ __forceinline__ void dmma_m8n8k4(double &d0, double &d1, double a, do
 template <int CN, bool RAGGED>
 __global__ void __launch_bounds__(Dgemm<CN>::threads, 128 / CN)
 dgemm_kernel(const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C, uint32_t M, uint32_t N,
-             uint32_t K, double alpha)
+             uint32_t K, double alpha, uint32_t *status)
 {
     extern __shared__ __align__(16) double dsm[];
     constexpr int kThreads = Dgemm<CN>::threads;
     constexpr size_t kDgemmStageDoubles = Dgemm<CN>::stage_doubles;
     uint32_t tm, tn;
-    raster((M + kSimtTile - 1) / kSimtTile, (N + CN - 1) / CN, &tm, &tn);
+    raster(blockIdx.x, (M + kSimtTile - 1) / kSimtTile, (N + CN - 1) / CN, &tm, &tn);
+    join_stream(status);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int kWarpsN = CN / 32;
     const int wm = (warp / kWarpsN) * 64, wn = (warp % kWarpsN) * 32;   // this warp's 64 x 32 corner inside the tile
@@ -371,8 +572,179 @@ dgemm_kernel(const double *__restrict__ A, const double *__restrict__ B, double 
         }
 }
 
+// Smaller tiles, K split over the CTAs of a cluster and over WK groups of WM x WN warps inside a CTA; 32 x 32 outputs
+// per warp (4 x 4 accumulator tiles, eight fragment loads per 16 DMMAs of 16 cycles each).  A group takes every WK-th
+// block of eight k of its CTA's range through a ring of its own, four stages deep; a group of one warp meets nobody.
+// Rows of 12 doubles put the fragment reads of a half warp into 16 different 8-byte banks.
+constexpr int kDsplitBK = 8, kDsplitLd = kDsplitBK + 4, kDsplitStages = 4;
+template <int WM, int WN, int WK> struct DgemmSplit {
+    static constexpr int rows = 32 * WM, cols = 32 * WN, group_threads = 32 * WM * WN, threads = group_threads * WK;
+    static constexpr size_t stage_doubles = (size_t)(rows + cols) * kDsplitLd, group_doubles = kDsplitStages * stage_doubles;
+    static constexpr size_t smem_bytes = WK * group_doubles * sizeof(double);
+    static constexpr int ctas_per_sm = (int)(220 * 1024 / smem_bytes);
+    static_assert((size_t)rows * cols <= group_doubles, "the partial tiles take the rings' place");
+    static_assert(WK == 1 || WM * WN == 1, "groups of several warps would need named barriers");
+};
+
+template <int WM, int WN, int WK>
+__global__ void __launch_bounds__(DgemmSplit<WM, WN, WK>::threads, DgemmSplit<WM, WN, WK>::ctas_per_sm)
+dgemm_split_kernel(const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C, uint32_t M, uint32_t N,
+                   uint32_t K, double alpha, uint32_t S, uint32_t *status)
+{
+    extern __shared__ __align__(16) double dsm[];
+    using D = DgemmSplit<WM, WN, WK>;
+    uint32_t tm, tn;
+    const uint32_t rank = blockIdx.x % S;
+    raster(blockIdx.x / S, (M + D::rows - 1) / D::rows, (N + D::cols - 1) / D::cols, &tm, &tn);
+    join_stream(status);
+    const int group = threadIdx.x / D::group_threads, tid = threadIdx.x % D::group_threads, lane = tid & 31, warp = tid >> 5;
+    const uint32_t nk_all = (K + kDsplitBK - 1) / kDsplitBK, kb0 = rank * nk_all / S, kb1 = (rank + 1) * nk_all / S;
+    const uint32_t nk = kb1 - kb0 > (uint32_t)group ? (kb1 - kb0 - group - 1) / WK + 1 : 0;       // this group's blocks
+    const int wm = warp / WN * 32, wn = warp % WN * 32;
+    double *ring = dsm + group * D::group_doubles;
+    auto group_sync = [&]() {
+        if constexpr (D::group_threads == 32)
+            __syncwarp();
+        else
+            __syncthreads();
+    };
+
+    auto load_stage = [&](uint32_t i) {                          // the group's i-th block
+        double *st = ring + (size_t)(i % kDsplitStages) * D::stage_doubles;
+        const uint32_t k0 = (kb0 + i * WK + group) * kDsplitBK;
+#pragma unroll
+        for (int u = 0; u < (D::rows + D::cols) * 4 / D::group_threads; u++) {
+            const int c = tid + D::group_threads * u, r = c >> 2, kc = (c & 3) * 2;
+            const bool is_a = r < D::rows;
+            const uint32_t row = is_a ? tm * D::rows + r : tn * D::cols + (r - D::rows);
+            const bool inside = row < (is_a ? M : N) && k0 + kc < K;
+            const double *base = is_a ? A : B;
+            cp_async_16_or_zeros(st + r * kDsplitLd + kc, inside ? base + (size_t)row * K + k0 + kc : base, inside);
+        }
+    };
+    double acc[4][4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            acc[i][j][0] = acc[i][j][1] = 0.0;
+#pragma unroll
+    for (int d = 0; d < kDsplitStages - 1; d++) {
+        if ((uint32_t)d < nk)
+            load_stage(d);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const int fr = lane >> 2, fk = lane & 3;
+    for (uint32_t kb = 0; kb < nk; kb++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kDsplitStages - 2) : "memory");
+        group_sync();                                            // block kb has landed; the stage of kb - 1 is free
+        if (kb + kDsplitStages - 1 < nk)
+            load_stage(kb + kDsplitStages - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const double *sa = ring + (size_t)(kb % kDsplitStages) * D::stage_doubles, *sb = sa + D::rows * kDsplitLd;
+#pragma unroll
+        for (int k4 = 0; k4 < kDsplitBK; k4 += 4) {
+            double a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                a[i] = sa[(wm + 8 * i + fr) * kDsplitLd + k4 + fk];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                b[j] = sb[(wn + 8 * j + fr) * kDsplitLd + k4 + fk];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    dmma_m8n8k4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    double *part = dsm + (size_t)group * D::rows * D::cols;      // [group][rows][cols]
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            *reinterpret_cast<double2 *>(part + (wm + 8 * i + fr) * D::cols + wn + 8 * j + 2 * fk) = make_double2(acc[i][j][0], acc[i][j][1]);
+    sum_partial_tiles<double, D::rows, D::cols, WK, D::threads>(dsm, S, rank, C, tm * D::rows, tn * D::cols, M, N, alpha);
+}
+
+// CTAs that clusters of this size can have running at one per SM: GPCs of 16 to 20 SMs leave some over
+static uint64_t simt_capacity(uint32_t cluster)
+{
+    const uint64_t sms = num_sms() > 0 ? (uint64_t)num_sms() : 148;
+    return cluster <= 2 ? sms : cluster == 4 ? sms * 132 / 148 : sms * 120 / 148;
+}
+
+template <typename... Params, typename... Args>
+static int launch_simt(void (*kernel)(Params...), const char *what, uint64_t ctas, int threads, size_t smem, uint32_t cluster, bool even_share,
+                       cudaStream_t s, Args... args)
+{
+    // An even share per SM: a CTA that may start under the tail of the previous kernel goes where that has ended, and
+    // some SMs would take three while others get none.  No more CTAs fit an SM than its share when they ask for enough
+    // shared memory (fp32 4195 x 225 x 1980, 264 CTAs of 64 x 64: 151 -> 113 us, fp64 902 x 868 x 2356 182 -> 146).
+    if (even_share) {
+        const uint64_t share = (ctas - 1) / simt_capacity(cluster) + 1;
+        const size_t fill = 227 * 1024 / (share + 1) + 1024;
+        if (share < 8 && fill > smem)
+            smem = fill;
+    }
+    CLPK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = tuning(CLPK_TUNE_GEMM_NO_PDL) == 1 ? 0 : 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    if (e != cudaSuccess)
+        return cuda_fail(e, what);
+    return CLPK_OK;
+}
+
+// Tile edge (128: the large kernels) and K ranges for a problem: the cheapest by an estimate in microseconds, fitted to
+// 400 timed launches of all kernels on 90 shapes (M and N from 64 to 15000, K to 16000; residuals 5 to 9 %, 17 % for the
+// 32-wide fp64 tile; the chosen plans are 3 to 4 % slower than the fastest in the geometric mean).  With L CTAs on the
+// busiest SM, a block of 16 k costs its CTA  max(alone, L * shared):
+//   fp32  128 x 128  max(1.62, 1.43 L)    64 x 64  max(0.51, 0.40 L)    (the pipe's own time: 1.07 and 0.27 L)
+//   fp64  128 x 64   max(1.48, 1.24 L)    64 x 64  max(0.91, 0.62 L)    32 x 32  max(0.22, 0.20 L)    (1.08, 0.54, 0.13 L)
+// The large tiles are kept unless the estimate is 8 % better; a K range has at least four blocks.
+struct SimtPlan {
+    uint32_t tile, splits;
+};
+
+static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
+{
+    const uint32_t blocks = (k - 1) / kSimtBK + 1;
+    auto estimate = [&](uint32_t rows, uint32_t cols, uint32_t splits, float alone, float shared) {
+        const uint64_t ctas = (uint64_t)((m - 1) / rows + 1) * ((n - 1) / cols + 1) * splits;
+        const float busiest = shared * (float)((ctas - 1) / simt_capacity(splits) + 1);
+        return (float)((blocks - 1) / splits + 1) * (alone > busiest ? alone : busiest);
+    };
+    float best = f64 ? 0.92f * (3.8f + estimate(128, 64, 1, 1.48f, 1.24f)) : 0.92f * (2.0f + estimate(128, 128, 1, 1.62f, 1.43f));
+    SimtPlan plan = {128, 1};
+    for (uint32_t splits = 1; splits <= 8 && (splits == 1 || blocks >= 4 * splits); splits *= 2)
+        for (uint32_t tile = f64 ? 32 : 64; tile <= 64; tile *= 2) {
+            float t = !f64 ? 4.1f + estimate(64, 64, splits, 0.507f, 0.404f) + (splits > 1 ? 1.1f + 0.08f * splits : 0.0f)
+                    : tile == 64 ? 4.56f + estimate(64, 64, splits, 0.907f, 0.616f)
+                                 : 4.25f + estimate(32, 32, splits, 0.217f, 0.196f) + (splits > 1 ? 0.23f + 0.35f * splits : 0.0f);
+            if (t < best) {
+                best = t;
+                plan = {tile, splits};
+            }
+        }
+    return plan;
+}
+
 int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t m, uint32_t n, uint32_t k, float alpha,
-                     cudaStream_t s)
+                     uint32_t *status, cudaStream_t s)
 {
     CLPK_REQUIRE(m > 0 && n > 0 && k > 0, "M, N and K must be positive");
     const uint32_t k_unit = dtype == CLPK_DT_F32 ? 4 : 2;            // elements per 16 bytes: operand rows stay aligned
@@ -383,21 +755,28 @@ int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t 
     CLPK_REQUIRE(tiles <= 0x3FFFFFFFull, "too many tiles");
     // whole tiles and whole k blocks take the kernel without the bounds checks
     const bool ragged = m % kSimtTile != 0 || n % tile_n != 0 || k % kSimtBK != 0;
+    const SimtPlan plan = plan_simt(dtype == CLPK_DT_F64, m, n, k);
+    const uint64_t ctas = (uint64_t)((m - 1) / plan.tile + 1) * ((n - 1) / plan.tile + 1) * plan.splits;
     if (dtype == CLPK_DT_F32) {
-        auto kernel = ragged ? sgemm_kernel<true> : sgemm_kernel<false>;
-        CLPK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSgemmSmemBytes));
-        kernel<<<(unsigned)tiles, kSgemmThreads, kSgemmSmemBytes, s>>>(static_cast<const float *>(a), static_cast<const float *>(b),
-                                                                      static_cast<float *>(c), m, n, k, alpha);
-        CLPK_LAUNCH_CHECK("sgemm");
-    } else {
-        // 128 x 64 CTA tiles: 34.2-34.5 TFLOPS at 4096^3 / 8192^3 against 31.9-32.1 with 128 x 128 tiles of 8 warps
-        auto kernel = ragged ? dgemm_kernel<64, true> : dgemm_kernel<64, false>;
-        CLPK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Dgemm<64>::smem_bytes));
-        kernel<<<(unsigned)tiles, Dgemm<64>::threads, Dgemm<64>::smem_bytes, s>>>(
-            static_cast<const double *>(a), static_cast<const double *>(b), static_cast<double *>(c), m, n, k, (double)alpha);
-        CLPK_LAUNCH_CHECK("dgemm");
+        const float *fa = static_cast<const float *>(a), *fb = static_cast<const float *>(b);
+        float *fc = static_cast<float *>(c);
+        if (plan.tile == 64)
+            return launch_simt(sgemm64_kernel, "launch sgemm64", ctas, kSgemmThreads, kSgemm64SmemBytes, plan.splits, true, s, fa, fb, fc, m, n, k, alpha,
+                               plan.splits, status);
+        return launch_simt(ragged ? sgemm_kernel<true> : sgemm_kernel<false>, "launch sgemm", tiles, kSgemmThreads, kSgemmSmemBytes, 1, false, s, fa, fb,
+                           fc, m, n, k, alpha, status);
     }
-    return CLPK_OK;
+    const double *da = static_cast<const double *>(a), *db = static_cast<const double *>(b);
+    double *dc = static_cast<double *>(c);
+    if (plan.tile == 64)
+        return launch_simt(dgemm_split_kernel<2, 2, 1>, "launch dgemm 64", ctas, DgemmSplit<2, 2, 1>::threads, DgemmSplit<2, 2, 1>::smem_bytes, plan.splits,
+                           true, s, da, db, dc, m, n, k, alpha, plan.splits, status);
+    if (plan.tile == 32)
+        return launch_simt(dgemm_split_kernel<1, 1, 4>, "launch dgemm 32", ctas, DgemmSplit<1, 1, 4>::threads, DgemmSplit<1, 1, 4>::smem_bytes, plan.splits,
+                           true, s, da, db, dc, m, n, k, alpha, plan.splits, status);
+    // 128 x 64 CTA tiles: 34.2-34.5 TFLOPS at 4096^3 / 8192^3 against 31.9-32.1 with 128 x 128 tiles of 8 warps
+    return launch_simt(ragged ? dgemm_kernel<64, true> : dgemm_kernel<64, false>, "launch dgemm", tiles, Dgemm<64>::threads, Dgemm<64>::smem_bytes, 1, false,
+                       s, da, db, dc, m, n, k, alpha, status);
 }
 
 } // namespace clpk

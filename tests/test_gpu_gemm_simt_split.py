@@ -1,0 +1,61 @@
+"""fp32 / fp64 GEMM shapes that take the small tiles and the split of K: every element of C against the fp64 product."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from clpeak_b200 import native as N
+from tests.gpu_util import dev_empty, stream_ptr, sync
+
+pytestmark = pytest.mark.gpu
+
+
+def operand(K, cuda, dtype, rows, k, seed):
+    f = dev_empty(rows * k, cuda.float32)
+    K.clpk_fill_f32(f.data_ptr(), rows * k, seed, N.DIST_NORMAL, 0.0, 0.02, stream_ptr())
+    if dtype == N.DT_F32:
+        return f
+    d = dev_empty(rows * k, cuda.float64)
+    K.clpk_convert_f32(d.data_ptr(), f.data_ptr(), rows * k, N.DT_F64, stream_ptr())
+    return d
+
+
+# fewer k blocks than groups and ranks could take; ranges and groups of unequal length; ragged tiles in both directions;
+# N odd (no vector store); one and several CTAs per SM; the large tiles' side of the rule
+@pytest.mark.parametrize("m,n,k", [(1, 1, 4), (33, 65, 20), (64, 64, 16384), (129, 131, 36), (131, 102, 7688), (201, 73, 2828), (863, 251, 2456),
+                                   (1315, 363, 956), (440, 434, 520), (64, 868, 1036), (719, 366, 688), (459, 349, 4636), (3720, 110, 596),
+                                   (2254, 496, 464), (1024, 1024, 512)])
+@pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F64])
+def test_every_element(K, cuda, dtype, m, n, k):
+    a, b = operand(K, cuda, dtype, m, k, 40), operand(K, cuda, dtype, n, k, 41)
+    alpha, results = 0.75, []
+    for _ in range(2):
+        c = cuda.full((m * n + 1024,), float("nan"), dtype=a.dtype, device="cuda")
+        status = cuda.full((1,), 7, dtype=cuda.int32, device="cuda")
+        args = N.GemmArgs(dtype=dtype, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=alpha,
+                          d_status=status.data_ptr())
+        K.clpk_gemm(C.byref(args), stream_ptr())
+        sync()
+        assert int(status.item()) == 0
+        assert bool(cuda.isnan(c[m * n:]).all()), "the kernel wrote beyond C"
+        results.append(c[:m * n])
+    assert bool((results[0] == results[1]).all()), "partial sums are added in a fixed order: the same bits every time"
+    fa, fb = a.double().view(m, k), b.double().view(n, k)
+    want, s_abs = alpha * (fa @ fb.T), alpha * (fa.abs() @ fb.abs().T)
+    # K roundings of the accumulator and one of alpha; fp64: the reference sum rounds as often
+    u = 2.0 ** -24 if dtype == N.DT_F32 else 2.0 ** -52
+    worst = float(((results[0].double().view(m, n) - want).abs() / ((k + 2) * u * s_abs + 1e-300)).max())
+    assert worst <= 1.0, f"worst error over all of C is {worst:.3g}x the stated tolerance"
+
+
+def test_nan_and_infinity_stay_in_their_rows_and_columns(K, cuda):
+    """Zero fill beyond K and beyond the operands must not meet them: 0 * inf would spread."""
+    m, n, k = 70, 66, 1028
+    a, b = operand(K, cuda, N.DT_F32, m, k, 1), operand(K, cuda, N.DT_F32, n, k, 2)
+    a[3 * k + 5], b[7 * k + k - 1] = float("inf"), float("nan")
+    c, status = dev_empty(m * n, cuda.float32), dev_empty(1, cuda.int32)
+    args = N.GemmArgs(dtype=N.DT_F32, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=1.0, d_status=status.data_ptr())
+    K.clpk_gemm(C.byref(args), stream_ptr())
+    sync()
+    bad = ~np.isfinite(c.view(m, n).cpu().numpy())
+    assert bad[3].all() and bad[:, 7].all() and bad.sum() == m + n - 1
