@@ -59,6 +59,14 @@ __global__ void __launch_bounds__(256) global_bandwidth_kernel(const V *__restri
     out[gid] = lane_sum(sum);
 }
 
+// Every stream kernel is launched with the programmatic-serialisation attribute: its first CTAs take their places under
+// the tail of the kernel before it in the stream and wait here until that has completed.
+__device__ __forceinline__ void join_stream()
+{
+    griddep_wait();
+    griddep_launch_dependents();
+}
+
 // ---- LDG flavour ---------------------------------------------------------------------
 
 constexpr int kLdgThreads = 512;
@@ -88,6 +96,7 @@ __global__ void __launch_bounds__(kLdgThreads) stream_read_ldg(const uint4 *__re
                                                                uint64_t n16,
                                                                uint32_t *__restrict__ partials)
 {
+    join_stream();
     constexpr uint64_t kTile = (uint64_t)kLdgThreads * kLdgUnroll;
     uint32_t acc = 0;
     const uint64_t n_full = n16 / kTile;
@@ -112,6 +121,7 @@ __global__ void __launch_bounds__(kLdgThreads) stream_copy_ldg(uint4 *__restrict
                                                                const uint4 *__restrict__ src,
                                                                uint64_t n16)
 {
+    join_stream();
     constexpr uint64_t kTile = (uint64_t)kLdgThreads * kLdgUnroll;
     const uint64_t n_full = n16 / kTile;
     for (uint64_t t = blockIdx.x; t < n_full; t += gridDim.x) {
@@ -144,6 +154,7 @@ __global__ void __launch_bounds__(kLdgThreads) stream_triad_ldg(float4 *__restri
                                                                 float s, uint64_t n4,
                                                                 uint64_t n_tail_floats)
 {
+    join_stream();
     constexpr int kU = 2;   // two b + two c loads in flight per thread
     constexpr uint64_t kTile = (uint64_t)kLdgThreads * kU;
     const uint64_t n_full = n4 / kTile;
@@ -210,14 +221,31 @@ __device__ __forceinline__ void st_stream32(Vec32 *p, const Vec32 &v)
                  : "memory");
 }
 
-// n_tiles full tiles, one per CTA; CTA 0 also takes the tail of n_tail16 16-byte pieces.
+// n_tiles full tiles; CTA 0 also takes the tail of n_tail16 16-byte pieces.  ATOMIC: one tile per CTA, the CTAs of a
+// slot meet in an atomicXor on slots that have been cleared.  Otherwise (up to kWideRounds tiles per slot) CTA b owns
+// slot b and takes tiles b, b + grid, ..., and stores what it found; slots without a CTA are cleared by the others.
+// Clearing first is an operation of its own in the stream: 45 against 36 us for a read, copy and triad pass over 1 MiB
+// arrays with the checksum read back, 156 against 148 over 128 MiB.  Beyond that many rounds the CTAs drift apart and the open memory pages with them.
+constexpr uint64_t kWideRounds = 8;
+
+template <bool ATOMIC>
 __global__ void __launch_bounds__(kWideThreads) stream_read_wide(const Vec32 *__restrict__ src, uint64_t n_tiles,
                                                                  uint64_t n_tail16, uint32_t *__restrict__ slots)
 {
+    join_stream();
     unsigned long long x = 0;
-    if (blockIdx.x < n_tiles) {
-        const Vec32 v = ld_stream32(src + (uint64_t)blockIdx.x * kWideThreads + threadIdx.x);
-        x = v.a ^ v.b ^ v.c ^ v.d;
+    if (ATOMIC) {
+        if (blockIdx.x < n_tiles) {
+            const Vec32 v = ld_stream32(src + (uint64_t)blockIdx.x * kWideThreads + threadIdx.x);
+            x = v.a ^ v.b ^ v.c ^ v.d;
+        }
+    } else {
+        for (uint64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+            const Vec32 v = ld_stream32(src + t * kWideThreads + threadIdx.x);
+            x ^= v.a ^ v.b ^ v.c ^ v.d;
+        }
+        for (uint32_t i = blockIdx.x + gridDim.x * (threadIdx.x + 1); i < kWideSlots; i += gridDim.x * kWideThreads)
+            slots[i] = 0u;
     }
     uint32_t y = (uint32_t)x ^ (uint32_t)(x >> 32);
     if (blockIdx.x == 0) {
@@ -236,13 +264,17 @@ __global__ void __launch_bounds__(kWideThreads) stream_read_wide(const Vec32 *__
 #pragma unroll
         for (int i = 0; i < kWideThreads / 32; i++)
             z ^= warp_x[i];
-        atomicXor(slots + (blockIdx.x & (kWideSlots - 1)), z);       // XOR: the order does not matter
+        if (ATOMIC)
+            atomicXor(slots + (blockIdx.x & (kWideSlots - 1)), z);   // XOR: the order does not matter
+        else
+            slots[blockIdx.x] = z;
     }
 }
 
 __global__ void __launch_bounds__(kWideThreads) stream_copy_wide(Vec32 *__restrict__ dst, const Vec32 *__restrict__ src,
                                                                  uint64_t n_tiles, uint64_t n_tail16)
 {
+    join_stream();
     if (blockIdx.x < n_tiles) {
         const uint64_t i = (uint64_t)blockIdx.x * kWideThreads + threadIdx.x;
         st_stream32(dst + i, ld_stream32(src + i));
@@ -277,13 +309,23 @@ __device__ __forceinline__ void report_timeout(uint32_t *status, uint32_t where)
 // as a whole walks the array in address order whatever the relative speed of the SMs (a
 // fixed tile-to-CTA map lets the CTAs drift apart and costs about 10 % of the bandwidth).
 // The producer leaves each stage's byte count in shared memory; a count of zero ends the
-// consumers' loop.
+// consumers' loop.  Arrays of a few tiles per CTA are dealt out after all (next_tile NULL): nothing drifts that far
+// in kTmaDealtRounds tiles, and clearing the counter is an operation of its own in the stream (the pass over 8 MiB
+// arrays: 47 -> 34 us).
+constexpr uint64_t kTmaDealtRounds = 4;
+
+__device__ __forceinline__ uint64_t claim_tile(unsigned long long *next_tile, uint64_t round)
+{
+    return next_tile ? atomicAdd(next_tile, 1ull) : blockIdx.x + round * gridDim.x;
+}
+
 __global__ void __launch_bounds__(160) stream_read_tma(const uint8_t *__restrict__ src,
                                                        uint64_t n_bytes,
                                                        uint32_t *__restrict__ partials,
                                                        uint32_t *__restrict__ status,
                                                        unsigned long long *__restrict__ next_tile)
 {
+    join_stream();
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)kTmaStages * kTmaTile);
     uint64_t *empty = full + kTmaStages;
@@ -310,7 +352,7 @@ __global__ void __launch_bounds__(160) stream_read_tma(const uint8_t *__restrict
                     report_timeout(status, 0);
                     break;
                 }
-                const uint64_t t = atomicAdd(next_tile, 1ull);
+                const uint64_t t = claim_tile(next_tile, j);
                 if (t >= n_tiles) {
                     stage_bytes[s] = 0;
                     mbar_arrive(&full[s]);
@@ -351,6 +393,7 @@ __global__ void __launch_bounds__(32) stream_copy_tma(uint8_t *__restrict__ dst,
                                                       uint32_t *__restrict__ status,
                                                       unsigned long long *__restrict__ next_tile)
 {
+    join_stream();
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)kTmaStages * kTmaTile);
     const uint64_t n_tiles = (n_bytes + kTmaTile - 1) / kTmaTile;
@@ -365,7 +408,7 @@ __global__ void __launch_bounds__(32) stream_copy_tma(uint8_t *__restrict__ dst,
     uint64_t issued = 0;
     bool more = true;
     auto issue_load = [&]() {
-        const uint64_t t = atomicAdd(next_tile, 1ull);
+        const uint64_t t = claim_tile(next_tile, issued);
         if (t >= n_tiles) {
             more = false;
             return;
@@ -401,6 +444,7 @@ __global__ void __launch_bounds__(kWideThreads) stream_triad_wide(Vec32 *__restr
                                                                   const Vec32 *__restrict__ c, float s,
                                                                   uint64_t n_tiles, uint64_t n_tail_floats)
 {
+    join_stream();
     if (blockIdx.x < n_tiles) {
         const uint64_t i = (uint64_t)blockIdx.x * kWideThreads + threadIdx.x;
         Vec32 vb = ld_stream32(b + i);
@@ -427,6 +471,7 @@ __global__ void __launch_bounds__(192) stream_triad_tma(float *__restrict__ a,
                                                         uint32_t *__restrict__ status,
                                                         unsigned long long *__restrict__ next_tile)
 {
+    join_stream();
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr uint32_t kStage = 2 * kTmaTriadTile;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)kTmaTriadStages * kStage);
@@ -461,7 +506,7 @@ __global__ void __launch_bounds__(192) stream_triad_tma(float *__restrict__ a,
                     report_timeout(status, 3);
                     break;
                 }
-                const uint64_t t = atomicAdd(next_tile, 1ull);
+                const uint64_t t = claim_tile(next_tile, j);
                 if (t >= n_tiles) {
                     stage_bytes[st] = 0;
                     mbar_arrive(&full[st]);
@@ -565,8 +610,11 @@ constexpr int kCounterRing = 32;
 static unsigned long long *g_counters[64] = {nullptr};
 static std::atomic<unsigned> g_next_counter{0};
 
-static int tile_counter(cudaStream_t s, unsigned long long **out)
+static int tile_counter(cudaStream_t s, uint64_t n_bytes, uint32_t tile, unsigned long long **out)
 {
+    *out = nullptr;
+    if (n_bytes <= kTmaDealtRounds * num_sms() * tile)
+        return CLPK_OK;
     int dev = 0;
     CLPK_CUDA(cudaGetDevice(&dev));
     CLPK_REQUIRE(dev >= 0 && dev < 64, "device ordinal %d out of range", dev);
@@ -577,6 +625,25 @@ static int tile_counter(cudaStream_t s, unsigned long long **out)
     }
     *out = g_counters[dev] + g_next_counter.fetch_add(1) % kCounterRing;
     CLPK_CUDA(cudaMemsetAsync(*out, 0, sizeof(unsigned long long), s));
+    return CLPK_OK;
+}
+
+template <typename... Params, typename... Args>
+static int launch_stream(void (*kernel)(Params...), const char *what, unsigned grid, int threads, size_t smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    if (e != cudaSuccess)
+        return cuda_fail(e, what);
     return CLPK_OK;
 }
 
@@ -637,27 +704,28 @@ int clpk_stream_read(int variant, const void *d_src, uint64_t n_bytes, uint32_t 
         CLPK_REQUIRE(((uintptr_t)d_src % 32) == 0, "the 256-bit variant needs a 32-byte aligned pointer");
         const uint64_t n_tiles = n_bytes / kWideTileBytes;
         CLPK_REQUIRE(n_tiles < 0x7FFFFFFFull, "n_bytes too large for one CTA per 8 KiB tile");
+        const Vec32 *src = reinterpret_cast<const Vec32 *>(d_src);
+        const uint64_t tail = (n_bytes % kWideTileBytes) / 16;
+        if (n_tiles <= kWideRounds * kWideSlots)
+            return launch_stream(stream_read_wide<false>, "launch stream_read", wide_grid(n_tiles < kWideSlots ? n_tiles : kWideSlots), kWideThreads, 0, s,
+                                 src, n_tiles, tail, d_partials);
         CLPK_CUDA(cudaMemsetAsync(d_partials, 0, kWideSlots * sizeof(uint32_t), s));
-        stream_read_wide<<<wide_grid(n_tiles), kWideThreads, 0, s>>>(reinterpret_cast<const Vec32 *>(d_src), n_tiles,
-                                                                     (n_bytes % kWideTileBytes) / 16, d_partials);
-    } else if (variant == CLPK_STREAM_LDG) {
-        stream_read_ldg<<<grid, kLdgThreads, 0, s>>>(reinterpret_cast<const uint4 *>(d_src), n_bytes / 16,
-                                                     d_partials);
-    } else {
-        uint32_t *st;
-        rc = status_word(&st);
-        if (rc != CLPK_OK)
-            return rc;
-        CLPK_CUDA(cudaFuncSetAttribute(stream_read_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaSmem));
-        unsigned long long *ctr;
-        rc = tile_counter(s, &ctr);
-        if (rc != CLPK_OK)
-            return rc;
-        stream_read_tma<<<grid, 160, kTmaSmem, s>>>(reinterpret_cast<const uint8_t *>(d_src), n_bytes,
-                                                    d_partials, st, ctr);
+        return launch_stream(stream_read_wide<true>, "launch stream_read", wide_grid(n_tiles), kWideThreads, 0, s, src, n_tiles, tail, d_partials);
     }
-    CLPK_LAUNCH_CHECK("stream_read");
-    return CLPK_OK;
+    if (variant == CLPK_STREAM_LDG)
+        return launch_stream(stream_read_ldg, "launch stream_read", grid, kLdgThreads, 0, s, reinterpret_cast<const uint4 *>(d_src), n_bytes / 16,
+                             d_partials);
+    uint32_t *st;
+    rc = status_word(&st);
+    if (rc != CLPK_OK)
+        return rc;
+    CLPK_CUDA(cudaFuncSetAttribute(stream_read_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaSmem));
+    unsigned long long *ctr;
+    rc = tile_counter(s, n_bytes, kTmaTile, &ctr);
+    if (rc != CLPK_OK)
+        return rc;
+    return launch_stream(stream_read_tma, "launch stream_read", grid, 160, kTmaSmem, s, reinterpret_cast<const uint8_t *>(d_src), n_bytes, d_partials,
+                         st, ctr);
 }
 
 int clpk_stream_copy(int variant, void *d_dst, const void *d_src, uint64_t n_bytes, void *stream)
@@ -675,27 +743,23 @@ int clpk_stream_copy(int variant, void *d_dst, const void *d_src, uint64_t n_byt
                      "the 256-bit variant needs 32-byte aligned pointers");
         const uint64_t n_tiles = n_bytes / kWideTileBytes;
         CLPK_REQUIRE(n_tiles < 0x7FFFFFFFull, "n_bytes too large for one CTA per 8 KiB tile");
-        stream_copy_wide<<<wide_grid(n_tiles), kWideThreads, 0, s>>>(reinterpret_cast<Vec32 *>(d_dst),
-                                                                     reinterpret_cast<const Vec32 *>(d_src), n_tiles,
-                                                                     (n_bytes % kWideTileBytes) / 16);
-    } else if (variant == CLPK_STREAM_LDG) {
-        stream_copy_ldg<<<num_sms() * kLdgCtasPerSm, kLdgThreads, 0, s>>>(
-            reinterpret_cast<uint4 *>(d_dst), reinterpret_cast<const uint4 *>(d_src), n_bytes / 16);
-    } else {
-        uint32_t *st;
-        rc = status_word(&st);
-        if (rc != CLPK_OK)
-            return rc;
-        CLPK_CUDA(cudaFuncSetAttribute(stream_copy_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaSmem));
-        unsigned long long *ctr;
-        rc = tile_counter(s, &ctr);
-        if (rc != CLPK_OK)
-            return rc;
-        stream_copy_tma<<<num_sms(), 32, kTmaSmem, s>>>(reinterpret_cast<uint8_t *>(d_dst),
-                                                        reinterpret_cast<const uint8_t *>(d_src), n_bytes, st, ctr);
+        return launch_stream(stream_copy_wide, "launch stream_copy", wide_grid(n_tiles), kWideThreads, 0, s, reinterpret_cast<Vec32 *>(d_dst),
+                             reinterpret_cast<const Vec32 *>(d_src), n_tiles, (n_bytes % kWideTileBytes) / 16);
     }
-    CLPK_LAUNCH_CHECK("stream_copy");
-    return CLPK_OK;
+    if (variant == CLPK_STREAM_LDG)
+        return launch_stream(stream_copy_ldg, "launch stream_copy", num_sms() * kLdgCtasPerSm, kLdgThreads, 0, s, reinterpret_cast<uint4 *>(d_dst),
+                             reinterpret_cast<const uint4 *>(d_src), n_bytes / 16);
+    uint32_t *st;
+    rc = status_word(&st);
+    if (rc != CLPK_OK)
+        return rc;
+    CLPK_CUDA(cudaFuncSetAttribute(stream_copy_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaSmem));
+    unsigned long long *ctr;
+    rc = tile_counter(s, n_bytes, kTmaTile, &ctr);
+    if (rc != CLPK_OK)
+        return rc;
+    return launch_stream(stream_copy_tma, "launch stream_copy", num_sms(), 32, kTmaSmem, s, reinterpret_cast<uint8_t *>(d_dst),
+                         reinterpret_cast<const uint8_t *>(d_src), n_bytes, st, ctr);
 }
 
 int clpk_stream_triad(int variant, float *d_a, const float *d_b, const float *d_c, float sc,
@@ -714,28 +778,24 @@ int clpk_stream_triad(int variant, float *d_a, const float *d_b, const float *d_
                      "the 256-bit variant needs 32-byte aligned pointers");
         const uint64_t n_tiles = n_floats * 4 / kWideTileBytes;
         CLPK_REQUIRE(n_tiles < 0x7FFFFFFFull, "n_floats too large for one CTA per 8 KiB tile");
-        stream_triad_wide<<<wide_grid(n_tiles), kWideThreads, 0, s>>>(
-            reinterpret_cast<Vec32 *>(d_a), reinterpret_cast<const Vec32 *>(d_b), reinterpret_cast<const Vec32 *>(d_c), sc,
-            n_tiles, n_floats - n_tiles * (kWideTileBytes / 4));
-    } else if (variant == CLPK_STREAM_LDG) {
-        stream_triad_ldg<<<num_sms() * kLdgCtasPerSm, kLdgThreads, 0, s>>>(
-            reinterpret_cast<float4 *>(d_a), reinterpret_cast<const float4 *>(d_b),
-            reinterpret_cast<const float4 *>(d_c), sc, n_floats / 4, n_floats % 4);
-    } else {
-        CLPK_REQUIRE(n_floats % 4 == 0, "the TMA variant needs n_floats to be a multiple of 4");
-        uint32_t *st;
-        rc = status_word(&st);
-        if (rc != CLPK_OK)
-            return rc;
-        CLPK_CUDA(cudaFuncSetAttribute(stream_triad_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaTriadSmem));
-        unsigned long long *ctr;
-        rc = tile_counter(s, &ctr);
-        if (rc != CLPK_OK)
-            return rc;
-        stream_triad_tma<<<num_sms(), 192, kTmaTriadSmem, s>>>(d_a, d_b, d_c, sc, n_floats * 4, st, ctr);
+        return launch_stream(stream_triad_wide, "launch stream_triad", wide_grid(n_tiles), kWideThreads, 0, s, reinterpret_cast<Vec32 *>(d_a),
+                             reinterpret_cast<const Vec32 *>(d_b), reinterpret_cast<const Vec32 *>(d_c), sc, n_tiles,
+                             n_floats - n_tiles * (kWideTileBytes / 4));
     }
-    CLPK_LAUNCH_CHECK("stream_triad");
-    return CLPK_OK;
+    if (variant == CLPK_STREAM_LDG)
+        return launch_stream(stream_triad_ldg, "launch stream_triad", num_sms() * kLdgCtasPerSm, kLdgThreads, 0, s, reinterpret_cast<float4 *>(d_a),
+                             reinterpret_cast<const float4 *>(d_b), reinterpret_cast<const float4 *>(d_c), sc, n_floats / 4, n_floats % 4);
+    CLPK_REQUIRE(n_floats % 4 == 0, "the TMA variant needs n_floats to be a multiple of 4");
+    uint32_t *st;
+    rc = status_word(&st);
+    if (rc != CLPK_OK)
+        return rc;
+    CLPK_CUDA(cudaFuncSetAttribute(stream_triad_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTmaTriadSmem));
+    unsigned long long *ctr;
+    rc = tile_counter(s, n_floats * 4, kTmaTriadTile, &ctr);
+    if (rc != CLPK_OK)
+        return rc;
+    return launch_stream(stream_triad_tma, "launch stream_triad", num_sms(), 192, kTmaTriadSmem, s, d_a, d_b, d_c, sc, n_floats * 4, st, ctr);
 }
 
 /* Reads and clears the device-side status word of the TMA streaming kernels
