@@ -37,7 +37,7 @@
 // Shapes of which those tiles make too few CTAs take 64 x 64 (fp32, fp64) or 32 x 32 (fp64) tiles with K split over the
 // CTAs of a cluster and over groups of warps inside a CTA (sgemm64_kernel, dgemm_split_kernel; plan_simt has the rule).
 // Device time before -> after: fp32 64 x 64 x 16384 1545 -> 69 us, 459 x 349 x 4636 474 -> 52, 2048^3 342 -> 323; fp64
-// 64 x 64 x 16384 1388 -> 33, 863 x 251 x 2456 228 -> 51, 2048 x 2048 x 512 151 -> 143.
+// 64 x 64 x 16384 1388 -> 33, 863 x 251 x 2456 228 -> 42, 2048 x 2048 x 512 151 -> 143.
 //
 // All take any M, N > 0 and any K that keeps operand rows 16-byte aligned (a multiple of 4
 // floats, 2 doubles): a second instantiation of the large kernels, and the others always, zero-fill the chunks a tile
@@ -574,14 +574,16 @@ dgemm_kernel(const double *__restrict__ A, const double *__restrict__ B, double 
 
 // Smaller tiles, K split over the CTAs of a cluster and over WK groups of WM x WN warps inside a CTA; 32 x 32 outputs
 // per warp (4 x 4 accumulator tiles, eight fragment loads per 16 DMMAs of 16 cycles each).  A group takes every WK-th
-// block of eight k of its CTA's range through a ring of its own, four stages deep; a group of one warp meets nobody.
+// block of eight k of its CTA's range through a ring of its own; a group of one warp meets nobody.  Three stages, so that
+// three CTAs of four one-warp groups fit an SM: with four stages and two CTAs 10215 x 138 x 872 took 122 us against 103,
+// 863 x 251 x 2456 50 against 42.
 // Rows of 12 doubles put the fragment reads of a half warp into 16 different 8-byte banks.
-constexpr int kDsplitBK = 8, kDsplitLd = kDsplitBK + 4, kDsplitStages = 4;
+constexpr int kDsplitBK = 8, kDsplitLd = kDsplitBK + 4, kDsplitStages = 3;
 template <int WM, int WN, int WK> struct DgemmSplit {
     static constexpr int rows = 32 * WM, cols = 32 * WN, group_threads = 32 * WM * WN, threads = group_threads * WK;
     static constexpr size_t stage_doubles = (size_t)(rows + cols) * kDsplitLd, group_doubles = kDsplitStages * stage_doubles;
     static constexpr size_t smem_bytes = WK * group_doubles * sizeof(double);
-    static constexpr int ctas_per_sm = (int)(220 * 1024 / smem_bytes);
+    static constexpr int ctas_per_sm = 220 * 1024 / smem_bytes < 4 ? (int)(220 * 1024 / smem_bytes) : 4;
     static_assert((size_t)rows * cols <= group_doubles, "the partial tiles take the rings' place");
     static_assert(WK == 1 || WM * WN == 1, "groups of several warps would need named barriers");
 };
@@ -710,11 +712,11 @@ static int launch_simt(void (*kernel)(Params...), const char *what, uint64_t cta
 }
 
 // Tile edge (128: the large kernels) and K ranges for a problem: the cheapest by an estimate in microseconds, fitted to
-// 400 timed launches of all kernels on 90 shapes (M and N from 64 to 15000, K to 16000; residuals 5 to 9 %, 17 % for the
-// 32-wide fp64 tile; the chosen plans are 3 to 4 % slower than the fastest in the geometric mean).  With L CTAs on the
+// 400 timed launches of all kernels on 90 shapes (M and N from 64 to 15000, K to 16000; residuals 5 to 9 %, 13 % for the
+// 32-wide fp64 tile; the chosen plans are 2 to 3 % slower than the fastest in the geometric mean).  With L CTAs on the
 // busiest SM, a block of 16 k costs its CTA  max(alone, L * shared):
 //   fp32  128 x 128  max(1.62, 1.43 L)    64 x 64  max(0.51, 0.40 L)    (the pipe's own time: 1.07 and 0.27 L)
-//   fp64  128 x 64   max(1.48, 1.24 L)    64 x 64  max(0.91, 0.62 L)    32 x 32  max(0.22, 0.20 L)    (1.08, 0.54, 0.13 L)
+//   fp64  128 x 64   max(1.48, 1.24 L)    64 x 64  max(0.91, 0.62 L)    32 x 32  max(0.22, 0.17 L)    (1.08, 0.54, 0.13 L)
 // The large tiles are kept unless the estimate is 8 % better; a K range has at least four blocks.
 struct SimtPlan {
     uint32_t tile, splits;
@@ -734,7 +736,7 @@ static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
         for (uint32_t tile = f64 ? 32 : 64; tile <= 64; tile *= 2) {
             float t = !f64 ? 4.1f + estimate(64, 64, splits, 0.507f, 0.404f) + (splits > 1 ? 1.1f + 0.08f * splits : 0.0f)
                     : tile == 64 ? 4.56f + estimate(64, 64, splits, 0.907f, 0.616f)
-                                 : 4.25f + estimate(32, 32, splits, 0.217f, 0.196f) + (splits > 1 ? 0.23f + 0.35f * splits : 0.0f);
+                                 : 3.9f + estimate(32, 32, splits, 0.223f, 0.174f) + (splits > 1 ? 0.5f * splits : 0.0f);
             if (t < best) {
                 best = t;
                 plan = {tile, splits};
