@@ -34,6 +34,29 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 
 } // namespace clpk
 
+namespace clpk {
+
+// Launches a kernel with the programmatic-serialisation attribute: its first CTAs take their places under the tail of
+// the kernel before it in the stream.  The kernel must therefore wait (griddep_wait) before it touches memory.
+template <typename... Params, typename... Args>
+int launch_behind(void (*kernel)(Params...), const char *what, unsigned grid, int threads, size_t smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    return e == cudaSuccess ? CLPK_OK : cuda_fail(e, what);
+}
+
+} // namespace clpk
+
 #define CLPK_CUDA(call)                                          \
     do {                                                         \
         cudaError_t e__ = (call);                                \

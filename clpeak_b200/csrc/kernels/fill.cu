@@ -9,12 +9,20 @@
 #include <math.h>
 
 #include "../clpk_internal.h"
+#include "../clpk_ptx.cuh"
 #include "../clpk_rng_fast.cuh"
 #include "../clpk_formats.h"
 
 namespace clpk {
 
 constexpr int kFillThreads = 256;
+
+// every kernel here is launched behind the one before it in the stream (launch_behind)
+__device__ __forceinline__ void join_stream()
+{
+    griddep_wait();
+    griddep_launch_dependents();
+}
 
 struct __align__(32) Float8 {
     float v[8];
@@ -45,6 +53,7 @@ __device__ __forceinline__ void st_float8(float *p, f32x2 a, f32x2 b, f32x2 c, f
 template <int DIST>
 __global__ void __launch_bounds__(kFillThreads) fill_f32_kernel(float *dst, uint64_t n8, uint64_t n, uint64_t mixed_seed, float mean, float stdv)
 {
+    griddep_launch_dependents();                               // the stores wait, the values need no memory
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     // the 2 P values from element i on
     auto values = [&](uint64_t i, auto &out) {
@@ -69,17 +78,20 @@ __global__ void __launch_bounds__(kFillThreads) fill_f32_kernel(float *dst, uint
     for (uint64_t g = first; g < n8; g += stride) {
         f32x2 v[4];
         values(8 * g, v);
+        griddep_wait();
         st_float8(dst + 8 * g, v[0], v[1], v[2], v[3]);
     }
     for (uint64_t i = 8 * n8 + first; i < n; i += stride) {
         f32x2 v[1];
         values(i, v);
+        griddep_wait();
         dst[i] = lo_of(v[0]);
     }
 }
 
 __global__ void __launch_bounds__(kFillThreads) fill_i8_kernel(int8_t *dst, uint64_t n16, uint64_t n, uint64_t mixed_seed)
 {
+    griddep_launch_dependents();                               // the stores wait, the values need no memory
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (uint64_t g = first; g < n16; g += stride) {
         uint32_t w[4];
@@ -90,10 +102,13 @@ __global__ void __launch_bounds__(kFillThreads) fill_i8_kernel(int8_t *dst, uint
             for (int t = 0; t < 4; t++)
                 w[j] |= ((uint32_t)((int)(rand64_at(mixed_seed, 16 * g + 4 * j + t) >> 60) - 8) & 0xFFu) << (8 * t);
         }
+        griddep_wait();
         *reinterpret_cast<uint4 *>(dst + 16 * g) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    for (uint64_t i = 16 * n16 + first; i < n; i += stride)
+    for (uint64_t i = 16 * n16 + first; i < n; i += stride) {
+        griddep_wait();
         dst[i] = (int8_t)((int)(rand64_at(mixed_seed, i) >> 60) - 8);
+    }
 }
 
 // One element in its narrow format, as bits.
@@ -144,6 +159,7 @@ template <int DT> struct Narrow {
 template <int DT>
 __global__ void __launch_bounds__(kFillThreads) convert_kernel(void *dst, const float *src, uint64_t n8, uint64_t n)
 {
+    join_stream();
     constexpr int bits = Narrow<DT>::bits;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (uint64_t g = first; g < n8; g += stride) {
@@ -201,6 +217,7 @@ constexpr int kAbsmaxLoads = 4;
 template <bool SINGLE>
 __global__ void __launch_bounds__(kFillThreads) absmax_kernel(float *out, const float *src, uint64_t n8, uint64_t n)
 {
+    join_stream();
     float m = 0.0f;
     const uint64_t step = (uint64_t)gridDim.x * kFillThreads * kAbsmaxLoads;
     for (uint64_t g = (uint64_t)blockIdx.x * kFillThreads * kAbsmaxLoads + threadIdx.x; g < n8; g += step) {
@@ -288,6 +305,7 @@ constexpr int kQuantPerLane = 16;
 template <int BLOCK, bool UE8M0>
 __global__ void __launch_bounds__(kFillThreads) quantize_fp4_kernel(uint8_t *packed, uint8_t *scales, const float *src, uint64_t n16, TensorScale ts)
 {
+    join_stream();
     constexpr int kLanes = BLOCK / kQuantPerLane;              // lanes of one block
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
@@ -378,6 +396,7 @@ __global__ void __launch_bounds__(kFillThreads) quantize_fp4_kernel(uint8_t *pac
 template <int BLOCK, bool UE8M0>
 __global__ void quantize_fp4_unaligned_kernel(uint8_t *packed, uint8_t *scales, const float *src, uint64_t n_blocks, float tensor_scale)
 {
+    join_stream();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < n_blocks; b += stride) {
         const float *x = src + b * BLOCK;
@@ -413,22 +432,22 @@ static unsigned fill_grid(uint64_t items)
 static bool aligned(const void *p, size_t bytes) { return ((uintptr_t)p % bytes) == 0; }
 
 template <int DT>
-static void launch_convert(void *d_dst, const float *d_src, uint64_t n, cudaStream_t s)
+static int launch_convert(void *d_dst, const float *d_src, uint64_t n, cudaStream_t s)
 {
     constexpr size_t dst_align = Narrow<DT>::bytes8 < 32 ? Narrow<DT>::bytes8 : 32;
     const uint64_t n8 = aligned(d_src, 32) && aligned(d_dst, dst_align) ? n / 8 : 0;
-    convert_kernel<DT><<<fill_grid(n8 ? n8 : n), kFillThreads, 0, s>>>(d_dst, d_src, n8, n);
+    return launch_behind(convert_kernel<DT>, "launch convert", fill_grid(n8 ? n8 : n), kFillThreads, 0, s, d_dst, d_src, n8, n);
 }
 
 template <int BLOCK, bool UE8M0>
-static void launch_quantize(uint8_t *d_packed, uint8_t *d_scales, const float *d_src, uint64_t n, float tensor_scale, cudaStream_t s)
+static int launch_quantize(uint8_t *d_packed, uint8_t *d_scales, const float *d_src, uint64_t n, float tensor_scale, cudaStream_t s)
 {
-    if (!aligned(d_src, 32) || !aligned(d_packed, 8)) {
-        quantize_fp4_unaligned_kernel<BLOCK, UE8M0><<<fill_grid(n / BLOCK), kFillThreads, 0, s>>>(d_packed, d_scales, d_src, n / BLOCK, tensor_scale);
-        return;
-    }
+    if (!aligned(d_src, 32) || !aligned(d_packed, 8))
+        return launch_behind(quantize_fp4_unaligned_kernel<BLOCK, UE8M0>, "launch quantize_fp4", fill_grid(n / BLOCK), kFillThreads, 0, s, d_packed, d_scales,
+                             d_src, n / BLOCK, tensor_scale);
     TensorScale ts = {tensor_scale, 1.0f / tensor_scale, !UE8M0 && !(tensor_scale >= 0x1p-60f && tensor_scale <= 0x1p60f)};
-    quantize_fp4_kernel<BLOCK, UE8M0><<<fill_grid(n / kQuantPerLane), kFillThreads, 0, s>>>(d_packed, d_scales, d_src, n / kQuantPerLane, ts);
+    return launch_behind(quantize_fp4_kernel<BLOCK, UE8M0>, "launch quantize_fp4", fill_grid(n / kQuantPerLane), kFillThreads, 0, s, d_packed, d_scales, d_src,
+                         n / kQuantPerLane, ts);
 }
 
 } // namespace clpk
@@ -448,13 +467,10 @@ int clpk_fill_f32(float *d_dst, uint64_t n, uint64_t seed, int dist, float mean,
     const unsigned grid = fill_grid(n8 ? n8 : n);
     cudaStream_t s = as_stream(stream);
     if (dist == CLPK_DIST_UNIFORM01)
-        fill_f32_kernel<CLPK_DIST_UNIFORM01><<<grid, kFillThreads, 0, s>>>(d_dst, n8, n, mixed, mean, std);
-    else if (dist == CLPK_DIST_UNIFORM_PM1)
-        fill_f32_kernel<CLPK_DIST_UNIFORM_PM1><<<grid, kFillThreads, 0, s>>>(d_dst, n8, n, mixed, mean, std);
-    else
-        fill_f32_kernel<CLPK_DIST_NORMAL><<<grid, kFillThreads, 0, s>>>(d_dst, n8, n, mixed, mean, std);
-    CLPK_LAUNCH_CHECK("fill_f32");
-    return CLPK_OK;
+        return launch_behind(fill_f32_kernel<CLPK_DIST_UNIFORM01>, "launch fill_f32", grid, kFillThreads, 0, s, d_dst, n8, n, mixed, mean, std);
+    if (dist == CLPK_DIST_UNIFORM_PM1)
+        return launch_behind(fill_f32_kernel<CLPK_DIST_UNIFORM_PM1>, "launch fill_f32", grid, kFillThreads, 0, s, d_dst, n8, n, mixed, mean, std);
+    return launch_behind(fill_f32_kernel<CLPK_DIST_NORMAL>, "launch fill_f32", grid, kFillThreads, 0, s, d_dst, n8, n, mixed, mean, std);
 }
 
 int clpk_fill_i8(int8_t *d_dst, uint64_t n, uint64_t seed, void *stream)
@@ -463,9 +479,7 @@ int clpk_fill_i8(int8_t *d_dst, uint64_t n, uint64_t seed, void *stream)
     if (n == 0)
         return CLPK_OK;
     const uint64_t n16 = aligned(d_dst, 16) ? n / 16 : 0;
-    fill_i8_kernel<<<fill_grid(n16 ? n16 : n), kFillThreads, 0, as_stream(stream)>>>(d_dst, n16, n, clpk_mix64(seed));
-    CLPK_LAUNCH_CHECK("fill_i8");
-    return CLPK_OK;
+    return launch_behind(fill_i8_kernel, "launch fill_i8", fill_grid(n16 ? n16 : n), kFillThreads, 0, as_stream(stream), d_dst, n16, n, clpk_mix64(seed));
 }
 
 int clpk_convert_f32(void *d_dst, const float *d_src, uint64_t n, int dtype, void *stream)
@@ -480,17 +494,15 @@ int clpk_convert_f32(void *d_dst, const float *d_src, uint64_t n, int dtype, voi
     CLPK_REQUIRE(dtype != CLPK_DT_E2M1 || n % 2 == 0, "E2M1 packs two elements per byte: n (%llu) must be even", (unsigned long long)n);
     cudaStream_t s = as_stream(stream);
     switch (dtype) {
-    case CLPK_DT_F16:  launch_convert<CLPK_DT_F16>(d_dst, d_src, n, s); break;
-    case CLPK_DT_BF16: launch_convert<CLPK_DT_BF16>(d_dst, d_src, n, s); break;
-    case CLPK_DT_E4M3: launch_convert<CLPK_DT_E4M3>(d_dst, d_src, n, s); break;
-    case CLPK_DT_E5M2: launch_convert<CLPK_DT_E5M2>(d_dst, d_src, n, s); break;
-    case CLPK_DT_I8:   launch_convert<CLPK_DT_I8>(d_dst, d_src, n, s); break;
-    case CLPK_DT_TF32: launch_convert<CLPK_DT_TF32>(d_dst, d_src, n, s); break;
-    case CLPK_DT_F64:  launch_convert<CLPK_DT_F64>(d_dst, d_src, n, s); break;
-    default:           launch_convert<CLPK_DT_E2M1>(d_dst, d_src, n, s); break;
+    case CLPK_DT_F16:  return launch_convert<CLPK_DT_F16>(d_dst, d_src, n, s);
+    case CLPK_DT_BF16: return launch_convert<CLPK_DT_BF16>(d_dst, d_src, n, s);
+    case CLPK_DT_E4M3: return launch_convert<CLPK_DT_E4M3>(d_dst, d_src, n, s);
+    case CLPK_DT_E5M2: return launch_convert<CLPK_DT_E5M2>(d_dst, d_src, n, s);
+    case CLPK_DT_I8:   return launch_convert<CLPK_DT_I8>(d_dst, d_src, n, s);
+    case CLPK_DT_TF32: return launch_convert<CLPK_DT_TF32>(d_dst, d_src, n, s);
+    case CLPK_DT_F64:  return launch_convert<CLPK_DT_F64>(d_dst, d_src, n, s);
+    default:           return launch_convert<CLPK_DT_E2M1>(d_dst, d_src, n, s);
     }
-    CLPK_LAUNCH_CHECK("convert");
-    return CLPK_OK;
 }
 
 int clpk_absmax_f32(float *d_absmax, const float *d_src, uint64_t n, void *stream)
@@ -499,18 +511,13 @@ int clpk_absmax_f32(float *d_absmax, const float *d_src, uint64_t n, void *strea
     cudaStream_t s = as_stream(stream);
     const uint64_t n8 = aligned(d_src, 32) ? n / 8 : 0;
     // up to 32 Ki floats one CTA reads in the time that clearing the word would take
-    if (n > 0 && n <= 32768 && d_src) {
-        absmax_kernel<true><<<1, kFillThreads, 0, s>>>(d_absmax, d_src, n8, n);
-        CLPK_LAUNCH_CHECK("absmax");
-        return CLPK_OK;
-    }
+    if (n > 0 && n <= 32768 && d_src)
+        return launch_behind(absmax_kernel<true>, "launch absmax", 1, kFillThreads, 0, s, d_absmax, d_src, n8, n);
     CLPK_CUDA(cudaMemsetAsync(d_absmax, 0, sizeof(float), s));
     if (n == 0)
         return CLPK_OK;
     CLPK_REQUIRE(d_src, "d_src is NULL");
-    absmax_kernel<false><<<fill_grid((n8 ? n8 : n) / kAbsmaxLoads + 1), kFillThreads, 0, s>>>(d_absmax, d_src, n8, n);
-    CLPK_LAUNCH_CHECK("absmax");
-    return CLPK_OK;
+    return launch_behind(absmax_kernel<false>, "launch absmax", fill_grid((n8 ? n8 : n) / kAbsmaxLoads + 1), kFillThreads, 0, s, d_absmax, d_src, n8, n);
 }
 
 int clpk_quantize_fp4(uint8_t *d_packed, uint8_t *d_scales, const float *d_src, uint64_t rows,
@@ -526,13 +533,11 @@ int clpk_quantize_fp4(uint8_t *d_packed, uint8_t *d_scales, const float *d_src, 
         return CLPK_OK;
     cudaStream_t s = as_stream(stream);
     switch (dtype) {
-    case CLPK_DT_MXF4:     launch_quantize<32, true>(d_packed, d_scales, d_src, n, 1.0f, s); break;
-    case CLPK_DT_MXF4_B64: launch_quantize<64, true>(d_packed, d_scales, d_src, n, 1.0f, s); break;
-    case CLPK_DT_NVF4:     launch_quantize<16, false>(d_packed, d_scales, d_src, n, tensor_scale, s); break;
-    default:               launch_quantize<32, false>(d_packed, d_scales, d_src, n, tensor_scale, s); break;
+    case CLPK_DT_MXF4:     return launch_quantize<32, true>(d_packed, d_scales, d_src, n, 1.0f, s);
+    case CLPK_DT_MXF4_B64: return launch_quantize<64, true>(d_packed, d_scales, d_src, n, 1.0f, s);
+    case CLPK_DT_NVF4:     return launch_quantize<16, false>(d_packed, d_scales, d_src, n, tensor_scale, s);
+    default:               return launch_quantize<32, false>(d_packed, d_scales, d_src, n, tensor_scale, s);
     }
-    CLPK_LAUNCH_CHECK("quantize_fp4");
-    return CLPK_OK;
 }
 
 int clpk_flush_l2(void *d_scratch, size_t bytes, void *stream)

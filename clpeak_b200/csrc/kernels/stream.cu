@@ -628,25 +628,6 @@ static int tile_counter(cudaStream_t s, uint64_t n_bytes, uint32_t tile, unsigne
     return CLPK_OK;
 }
 
-template <typename... Params, typename... Args>
-static int launch_stream(void (*kernel)(Params...), const char *what, unsigned grid, int threads, size_t smem, cudaStream_t s, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-    if (e != cudaSuccess)
-        return cuda_fail(e, what);
-    return CLPK_OK;
-}
-
 } // namespace clpk
 
 using namespace clpk;
@@ -707,13 +688,13 @@ int clpk_stream_read(int variant, const void *d_src, uint64_t n_bytes, uint32_t 
         const Vec32 *src = reinterpret_cast<const Vec32 *>(d_src);
         const uint64_t tail = (n_bytes % kWideTileBytes) / 16;
         if (n_tiles <= kWideRounds * kWideSlots)
-            return launch_stream(stream_read_wide<false>, "launch stream_read", wide_grid(n_tiles < kWideSlots ? n_tiles : kWideSlots), kWideThreads, 0, s,
+            return launch_behind(stream_read_wide<false>, "launch stream_read", wide_grid(n_tiles < kWideSlots ? n_tiles : kWideSlots), kWideThreads, 0, s,
                                  src, n_tiles, tail, d_partials);
         CLPK_CUDA(cudaMemsetAsync(d_partials, 0, kWideSlots * sizeof(uint32_t), s));
-        return launch_stream(stream_read_wide<true>, "launch stream_read", wide_grid(n_tiles), kWideThreads, 0, s, src, n_tiles, tail, d_partials);
+        return launch_behind(stream_read_wide<true>, "launch stream_read", wide_grid(n_tiles), kWideThreads, 0, s, src, n_tiles, tail, d_partials);
     }
     if (variant == CLPK_STREAM_LDG)
-        return launch_stream(stream_read_ldg, "launch stream_read", grid, kLdgThreads, 0, s, reinterpret_cast<const uint4 *>(d_src), n_bytes / 16,
+        return launch_behind(stream_read_ldg, "launch stream_read", grid, kLdgThreads, 0, s, reinterpret_cast<const uint4 *>(d_src), n_bytes / 16,
                              d_partials);
     uint32_t *st;
     rc = status_word(&st);
@@ -724,7 +705,7 @@ int clpk_stream_read(int variant, const void *d_src, uint64_t n_bytes, uint32_t 
     rc = tile_counter(s, n_bytes, kTmaTile, &ctr);
     if (rc != CLPK_OK)
         return rc;
-    return launch_stream(stream_read_tma, "launch stream_read", grid, 160, kTmaSmem, s, reinterpret_cast<const uint8_t *>(d_src), n_bytes, d_partials,
+    return launch_behind(stream_read_tma, "launch stream_read", grid, 160, kTmaSmem, s, reinterpret_cast<const uint8_t *>(d_src), n_bytes, d_partials,
                          st, ctr);
 }
 
@@ -743,11 +724,11 @@ int clpk_stream_copy(int variant, void *d_dst, const void *d_src, uint64_t n_byt
                      "the 256-bit variant needs 32-byte aligned pointers");
         const uint64_t n_tiles = n_bytes / kWideTileBytes;
         CLPK_REQUIRE(n_tiles < 0x7FFFFFFFull, "n_bytes too large for one CTA per 8 KiB tile");
-        return launch_stream(stream_copy_wide, "launch stream_copy", wide_grid(n_tiles), kWideThreads, 0, s, reinterpret_cast<Vec32 *>(d_dst),
+        return launch_behind(stream_copy_wide, "launch stream_copy", wide_grid(n_tiles), kWideThreads, 0, s, reinterpret_cast<Vec32 *>(d_dst),
                              reinterpret_cast<const Vec32 *>(d_src), n_tiles, (n_bytes % kWideTileBytes) / 16);
     }
     if (variant == CLPK_STREAM_LDG)
-        return launch_stream(stream_copy_ldg, "launch stream_copy", num_sms() * kLdgCtasPerSm, kLdgThreads, 0, s, reinterpret_cast<uint4 *>(d_dst),
+        return launch_behind(stream_copy_ldg, "launch stream_copy", num_sms() * kLdgCtasPerSm, kLdgThreads, 0, s, reinterpret_cast<uint4 *>(d_dst),
                              reinterpret_cast<const uint4 *>(d_src), n_bytes / 16);
     uint32_t *st;
     rc = status_word(&st);
@@ -758,7 +739,7 @@ int clpk_stream_copy(int variant, void *d_dst, const void *d_src, uint64_t n_byt
     rc = tile_counter(s, n_bytes, kTmaTile, &ctr);
     if (rc != CLPK_OK)
         return rc;
-    return launch_stream(stream_copy_tma, "launch stream_copy", num_sms(), 32, kTmaSmem, s, reinterpret_cast<uint8_t *>(d_dst),
+    return launch_behind(stream_copy_tma, "launch stream_copy", num_sms(), 32, kTmaSmem, s, reinterpret_cast<uint8_t *>(d_dst),
                          reinterpret_cast<const uint8_t *>(d_src), n_bytes, st, ctr);
 }
 
@@ -778,12 +759,12 @@ int clpk_stream_triad(int variant, float *d_a, const float *d_b, const float *d_
                      "the 256-bit variant needs 32-byte aligned pointers");
         const uint64_t n_tiles = n_floats * 4 / kWideTileBytes;
         CLPK_REQUIRE(n_tiles < 0x7FFFFFFFull, "n_floats too large for one CTA per 8 KiB tile");
-        return launch_stream(stream_triad_wide, "launch stream_triad", wide_grid(n_tiles), kWideThreads, 0, s, reinterpret_cast<Vec32 *>(d_a),
+        return launch_behind(stream_triad_wide, "launch stream_triad", wide_grid(n_tiles), kWideThreads, 0, s, reinterpret_cast<Vec32 *>(d_a),
                              reinterpret_cast<const Vec32 *>(d_b), reinterpret_cast<const Vec32 *>(d_c), sc, n_tiles,
                              n_floats - n_tiles * (kWideTileBytes / 4));
     }
     if (variant == CLPK_STREAM_LDG)
-        return launch_stream(stream_triad_ldg, "launch stream_triad", num_sms() * kLdgCtasPerSm, kLdgThreads, 0, s, reinterpret_cast<float4 *>(d_a),
+        return launch_behind(stream_triad_ldg, "launch stream_triad", num_sms() * kLdgCtasPerSm, kLdgThreads, 0, s, reinterpret_cast<float4 *>(d_a),
                              reinterpret_cast<const float4 *>(d_b), reinterpret_cast<const float4 *>(d_c), sc, n_floats / 4, n_floats % 4);
     CLPK_REQUIRE(n_floats % 4 == 0, "the TMA variant needs n_floats to be a multiple of 4");
     uint32_t *st;
@@ -795,7 +776,7 @@ int clpk_stream_triad(int variant, float *d_a, const float *d_b, const float *d_
     rc = tile_counter(s, n_floats * 4, kTmaTriadTile, &ctr);
     if (rc != CLPK_OK)
         return rc;
-    return launch_stream(stream_triad_tma, "launch stream_triad", num_sms(), 192, kTmaTriadSmem, s, d_a, d_b, d_c, sc, n_floats * 4, st, ctr);
+    return launch_behind(stream_triad_tma, "launch stream_triad", num_sms(), 192, kTmaTriadSmem, s, d_a, d_b, d_c, sc, n_floats * 4, st, ctr);
 }
 
 /* Reads and clears the device-side status word of the TMA streaming kernels

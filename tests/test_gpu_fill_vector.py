@@ -152,3 +152,27 @@ def test_quantize_generated_operands(K, orc, cuda, dtype):
     sync()
     assert_bits_equal(to_np(scales), want_scales.ravel(), "fp4 scales")
     assert_bits_equal(to_np(packed), want_packed.ravel(), "fp4 codes")
+
+
+def test_operand_kernels_under_each_others_tails(K, orc, cuda):
+    """fill -> absmax -> quantise -> fill again into the same buffer, back to back: each kernel may start before the one in
+    front of it has ended, and has to wait for it before it reads or overwrites its data."""
+    rows, cols = 512, 2048
+    n = rows * cols
+    f, top = dev_empty(n, cuda.float32), dev_empty(16, cuda.float32)
+    packed = [dev_empty(n // 2, cuda.uint8) for _ in range(8)]
+    scales = [dev_empty(n // 16, cuda.uint8) for _ in range(8)]
+    halves = [dev_empty(n, cuda.bfloat16) for _ in range(8)]
+    for i in range(8):
+        K.clpk_fill_f32(f.data_ptr(), n, 60 + i, N.DIST_NORMAL, 0.0, 0.02, stream_ptr())
+        K.clpk_absmax_f32(top.data_ptr() + 4 * i, f.data_ptr(), n, stream_ptr())
+        K.clpk_quantize_fp4(packed[i].data_ptr(), scales[i].data_ptr(), f.data_ptr(), rows, cols, N.DT_NVF4, 4e-5, stream_ptr())
+        K.clpk_convert_f32(halves[i].data_ptr(), f.data_ptr(), n, N.DT_BF16, stream_ptr())
+    sync()
+    for i in range(8):
+        want = orc.fill_f32(n, 60 + i, N.DIST_NORMAL, 0.0, 0.02)
+        assert float(top[i].item()) == float(np.abs(want).max())
+        want_packed, want_scales = orc.quantize_fp4(want.reshape(rows, cols), N.DT_NVF4, float(np.float32(4e-5)))
+        assert_bits_equal(to_np(packed[i]), want_packed.ravel(), "fp4 codes")
+        assert_bits_equal(to_np(scales[i]), want_scales.ravel(), "fp4 scales")
+        assert_bits_equal(to_np(halves[i].view(cuda.int16)), orc.convert_f32(want, N.DT_BF16), "bf16")
