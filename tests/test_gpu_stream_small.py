@@ -52,3 +52,38 @@ def test_dependent_kernels_back_to_back(K, cuda, variant, n):
         want_b = want_b + one * 1.5
         assert checksum(p) == int(np.bitwise_xor.reduce(want_b.cpu().numpy().view(np.uint32)))
     assert bool((b == want_b).all())
+
+
+def test_the_launches_can_be_captured(K, cuda):
+    """Operands, a small GEMM with scales to arrange and a stream pass as one graph, replayed on new contents."""
+    rows = cols = 256
+    n = rows * cols
+    f, top = dev_empty(n, cuda.float32), dev_empty(1, cuda.float32)
+    q, sf, c = dev_empty(n // 2, cuda.uint8), dev_empty(n // 16, cuda.uint8), dev_empty(n, cuda.bfloat16)
+    ws, st, out = dev_empty(2 * n // 16, cuda.uint8), dev_empty(1, cuda.int32), dev_empty(n, cuda.float32)
+    parts = dev_empty(SLOTS, cuda.int32)
+    single = N.GemmArgs(dtype=N.DT_F32, m=rows, n=rows, k=cols, d_a=f.data_ptr(), d_b=f.data_ptr(), d_c=out.data_ptr(), alpha=1.0, d_status=st.data_ptr())
+    scaled = N.GemmArgs(dtype=N.DT_NVF4, m=rows, n=rows, k=cols, d_a=q.data_ptr(), d_b=q.data_ptr(), d_c=c.data_ptr(), d_sfa=sf.data_ptr(),
+                        d_sfb=sf.data_ptr(), alpha=1.0, d_workspace=ws.data_ptr(), workspace_bytes=ws.numel(), d_status=st.data_ptr())
+
+    def run(s):
+        K.clpk_fill_f32(f.data_ptr(), n, 17, N.DIST_NORMAL, 0.0, 0.02, s)
+        K.clpk_absmax_f32(top.data_ptr(), f.data_ptr(), n, s)
+        K.clpk_quantize_fp4(q.data_ptr(), sf.data_ptr(), f.data_ptr(), rows, cols, N.DT_NVF4, 3e-5, s)
+        K.clpk_gemm(C.byref(scaled), s)
+        K.clpk_gemm(C.byref(single), s)
+        K.clpk_stream_read(N.STREAM_WIDE, out.data_ptr(), 4 * n, parts.data_ptr(), s)
+
+    run(stream_ptr())
+    sync()
+    want = [t.clone() for t in (f, top, q, sf, c, out, parts)]
+    stream = cuda.cuda.Stream()
+    graph = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(graph, stream=stream):
+        run(stream.cuda_stream)
+    for _ in range(3):
+        for t in (f, top, q, sf, c, out, parts):
+            t.zero_()
+        graph.replay()
+        sync()
+        assert all(bool((t == w).all()) for t, w in zip((f, top, q, sf, c, out, parts), want))
