@@ -49,23 +49,22 @@ struct GemmParams {
     float alpha;
     uint32_t *status;
     uint32_t group;             // tile columns per raster group (both kernels)
-    unsigned int *wave_sync;    // one counter for this launch, or NULL: see wave_align()
+    unsigned int *wave_sync;    // {arrivals, CTAs that are done} of this launch, or NULL: see wave_align()
     uint32_t align_at;          // K block of a tile before which the producers meet
     uint32_t align_period;      // ... in every align_period-th wave
     unsigned long long *clock;  // two words: CTA 0 stores the SM cycles and nanoseconds it ran for (clpk_gemm_last_clock)
-    uint32_t zero_status;       // 1: the kernel clears *status itself (launches that may overlap the previous kernel's tail)
 };
 
 // Launches of a small GEMM repeat every 40-100 us, and 6-7 us of each are the CTA's set-up (barriers, tensor
-// memory, descriptor prefetch) and the launch gap.  The plain (non-cooperative) launches therefore carry the
+// memory, descriptor prefetch) and the launch gap.  The launches therefore carry the
 // programmatic-serialisation attribute: a CTA of launch i + 1 takes an SM as soon as launch i's CTA there has
 // exited, does its set-up, and then waits here until launch i has completed as a whole and its writes are visible.
 // Nothing of global memory is read or written before that point.
 __device__ __forceinline__ void join_previous_launch(const GemmParams &p)
 {
     griddep_wait();
-    if (p.zero_status && blockIdx.x == 0 && threadIdx.x == 0)
-        *p.status = 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *p.status = 0u;             // by the kernel: no stream operation sits between two launches
     griddep_launch_dependents();
 }
 
@@ -387,10 +386,12 @@ __device__ __forceinline__ void drain_warp_tile_early(uint32_t taddr0, uint32_t 
 // that share an operand panel then ask for it that far apart, the L2 has long replaced
 // it, and every panel is fetched from DRAM several times per wave.  So the producers
 // meet before each wave: every CTA adds one to a counter and waits until the counter
-// shows that all CTAs of the wave have arrived.  The kernel is launched cooperatively
-// (all CTAs resident), and the wait is bounded all the same: a CTA that has waited
-// 40 us stops taking part, after which the others time out once each and the kernel
-// finishes unaligned.
+// shows that all CTAs of the wave have arrived.  There is one CTA per SM, so they are normally all resident; the wait
+// is bounded all the same: a CTA that has waited 40 us (another stream's kernel holds an SM) stops taking part, after
+// which the others time out once each and the kernel finishes unaligned.  The last CTA to leave clears the counter for
+// the launch that gets it next (leave_wave_sync).  A cooperative launch behind two clearing operations, the first form
+// of this, cost about 5 us a GEMM: e4m3 8192 x 8192 x 512 40.3 -> 35.8 us, x 1024 67 -> 62, bf16 x 1024 113 -> 105, NVFP4
+// 16384 x 16384 x 1024 196 -> 170, back to back.
 __device__ __forceinline__ void wave_align(const GemmParams &p, uint32_t wave, uint32_t n_tiles, uint32_t n_clusters,
                                            bool &enabled)
 {
@@ -416,6 +417,16 @@ __device__ __forceinline__ void wave_align(const GemmParams &p, uint32_t wave, u
         }
         __nanosleep(64);
     }
+}
+
+// By the thread that arrived for its CTA's producer, at the end of the kernel.
+__device__ __forceinline__ void leave_wave_sync(const GemmParams &p)
+{
+    if (!p.wave_sync)
+        return;
+    __threadfence();                                        // this CTA's arrivals come before its leaving
+    if (atomicInc(p.wave_sync + 1, gridDim.x - 1) == gridDim.x - 1)
+        atomicExch(p.wave_sync, 0u);
 }
 
 template <int DT>
@@ -585,6 +596,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads)
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync();
+    if (threadIdx.x == 0)
+        leave_wave_sync(p);
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.clock) {
         p.clock[0] = clock64() - clk0;
         p.clock[1] = globaltimer_ns() - ns0;
@@ -960,6 +973,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNvGemmThreads)
     tc_fence_before_sync();
     __syncthreads();
     cluster_sync();
+    if (threadIdx.x == 0)
+        leave_wave_sync(p);
     if (blockIdx.x == 0 && threadIdx.x == 0 && p.clock) {
         p.clock[0] = clock64() - clk0;
         p.clock[1] = globaltimer_ns() - ns0;
@@ -1085,21 +1100,20 @@ static int make_scale_map_b(CUtensorMap *map, const void *base, uint64_t n_rows,
 
 constexpr size_t kGemmSmemBytes = (size_t)kDenseStages * kDenseStageBytes + kEpilogueWarps * kStagingBytes + sizeof(DenseSmem) + 1024;
 
-// One wave counter per launch, from a ring of 32 per device so that launches on different streams
-// do not share one; zeroed in stream order before the kernel.  The slot index comes from one
-// process-wide counter, so a slot is handed out again 32 launches later: with more than 32 aligned
-// GEMMs in flight at once on one device (across streams) two running kernels would share a counter.
-// That costs alignment, not correctness -- a producer that does not see its wave complete within
-// 40 us stops taking part -- but callers that want the alignment keep at most 32 in flight.
+// One pair of wave counters per launch, from a ring of 32 per device so that launches on different streams do not share
+// one; zero between launches.  The slot index comes from one process-wide counter, so a slot is handed out again 32
+// launches later: with more than 32 aligned GEMMs in flight at once on one device (across streams) two running kernels
+// would share a slot.  That costs alignment, not correctness -- a producer that does not see its wave complete within
+// 40 us stops taking part, and the slot is zero again when both have ended -- but callers that want the alignment keep
+// at most 32 in flight.
 constexpr int kSyncSlots = 32;
-__device__ unsigned int g_wave_sync[kSyncSlots];
+__device__ unsigned int g_wave_sync[kSyncSlots][2];
 static std::atomic<unsigned> g_next_sync_slot{0};
 static thread_local int g_last_aligned = -1;
 // {SM cycles, nanoseconds} CTA 0 of the last GEMM launch on this device ran for (both tensor kernels write it).
 __device__ unsigned long long g_gemm_clock[2];
 
-// Launches a persistent cluster kernel whose last parameter is GemmParams: cooperatively with a
-// fresh wave counter when the alignment is on, plainly (and unaligned) otherwise.
+// Launches a persistent cluster kernel whose last parameter is GemmParams, with a wave counter when the alignment is on.
 template <typename Kernel, typename... Maps>
 static int launch_persistent(Kernel kernel, const char *what, int threads, size_t smem, cudaStream_t s, GemmParams p,
                              uint32_t n_tiles, const Maps &...maps)
@@ -1107,43 +1121,15 @@ static int launch_persistent(Kernel kernel, const char *what, int threads, size_
     CLPK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int grid = (num_sms() / 2) * 2;
     p.wave_sync = nullptr;
-    p.zero_status = 0;
-    g_last_aligned = 0;
     CLPK_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&p.clock), g_gemm_clock));
-    // nothing to keep in step in the first two waves: small problems skip the counter and its memset
+    // nothing to keep in step in the first two waves: small problems skip the counter
     const bool worth_aligning = n_tiles > 2u * (uint32_t)(grid / 2) * p.align_period;
     if (worth_aligning && tuning(CLPK_TUNE_GEMM_NO_ALIGN) != 1) {
         unsigned int *base = nullptr;
         CLPK_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&base), g_wave_sync));
-        p.wave_sync = base + g_next_sync_slot.fetch_add(1) % kSyncSlots;
-        CLPK_CUDA(cudaMemsetAsync(p.wave_sync, 0, sizeof(unsigned int), s));
-        CLPK_CUDA(cudaMemsetAsync(p.status, 0, sizeof(uint32_t), s));
-        // cooperative: every CTA is resident before any runs, so the wave counter can fill up
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)grid);
-        cfg.blockDim = dim3((unsigned)threads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        const cudaError_t ce = cudaLaunchKernelEx(&cfg, kernel, maps..., p);
-        if (ce == cudaSuccess) {
-            g_last_aligned = 1;
-            return CLPK_OK;
-        }
-        // Only "the grid cannot be co-resident here" (another context holds SMs, MPS limits) is a
-        // reason to run without the alignment; anything else is a real error and is reported as one.
-        if (ce != cudaErrorCooperativeLaunchTooLarge && ce != cudaErrorLaunchOutOfResources)
-            return cuda_fail(ce, what);
-        (void)cudaGetLastError();
-        p.wave_sync = nullptr;
+        p.wave_sync = base + 2 * (g_next_sync_slot.fetch_add(1) % kSyncSlots);
     }
-    // No stream operation between two such launches (the kernel clears the status word itself), so that the
-    // programmatic serialisation can overlap this launch's set-up with the tail of the one before.
-    p.zero_status = 1;
+    g_last_aligned = p.wave_sync ? 1 : 0;
     cudaLaunchConfig_t plain = {};
     plain.gridDim = dim3((unsigned)grid);
     plain.blockDim = dim3((unsigned)threads);
@@ -1169,8 +1155,8 @@ struct TilesPlan {
 // shapes with M and N from 64 to 14000, K from 256 to 16000 in the six dense types, 300 for 90 block-scaled ones, every
 // tile width and split of each (residuals 13 and 6 %; the chosen plans are 1 % slower than the fastest in the geometric
 // mean, 19 % at worst).  With W = TN / 256 and T the time to fetch what all SMs load for one K block of 128 bytes:
-//   gemm_kernel               3.6 + waves * (0.57 per K block of a 512 x 256 tile + 2.9), and 9.3 for the cooperative
-//                             launch and its memsets when there are more than two waves
+//   gemm_kernel               3.6 + waves * (0.57 per K block of a 512 x 256 tile + 2.9), and 4 for the producers'
+//                             meetings when there are more than two waves
 //   gemm_tiles_kernel, dense  3.9 + waves * (K blocks * (0.118 to issue a block + 0.175 W for its instructions + T at
 //                             54 TB/s) + 1.1 W of epilogue) and, split, 1 + 4.3 W per exchanged share of the tile
 //   gemm_block_scaled_kernel  4.0 + waves * (K blocks * (0.275 + T at 43 TB/s) + 0.7)
@@ -1192,7 +1178,7 @@ static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4)
         return plan;
     const float big_waves = (float)((big_tiles - 1) / pairs + 1);
     const float big = fp4 ? 4.0f + big_waves * (k_blocks * (0.275f + fetched(big_tiles < pairs ? big_tiles : pairs, 1, 256) / 43.2e6f) + 0.7f)
-                          : 3.6f + (big_waves > 2 ? 9.3f : 0.0f) + big_waves * (k_blocks * 0.57f + 2.9f);
+                          : 3.6f + (big_waves > 2 ? 4.0f : 0.0f) + big_waves * (k_blocks * 0.57f + 2.9f);
     float best = 0.97f * big;
     const float launch = fp4 ? 3.3f : 3.9f, issue = fp4 ? 0.25f : 0.118f, wide_issue = fp4 ? 0.06f : 0.175f;
     const float rate = fp4 ? 62.4e6f : 53.8e6f, drain = fp4 ? 1.36f : 1.14f;

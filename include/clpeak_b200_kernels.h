@@ -106,7 +106,7 @@ CLPK_API int clpk_flush_l2(void *d_scratch, size_t bytes, void *stream);
  *   GEMM_FP4_TILE  block-scaled GEMM tile: 0 = by size, 1 = 256x256 one accumulator,
  *                  2 = 256x128 two accumulators (the epilogue overlaps the next tile)
  *   MMA_LONE_LANE  1 = the peak probes issue from one thread instead of an elected lane of a whole warp
- *   GEMM_NO_PDL    1 = GEMMs too small for the per-wave alignment are launched plainly; by default they carry
+ *   GEMM_NO_PDL    1 = GEMMs are launched plainly; by default they carry
  *                  the programmatic-serialisation attribute, so that a launch's set-up overlaps the tail of
  *                  the kernel before it in the stream (it waits for that kernel before touching memory) */
 #define CLPK_TUNE_GEMM_NO_ALIGN 0
@@ -115,7 +115,7 @@ CLPK_API int clpk_flush_l2(void *d_scratch, size_t bytes, void *stream);
 #define CLPK_TUNE_MMA_PAIR      3
 #define CLPK_TUNE_GEMM_FP4_TILE 4
 #define CLPK_TUNE_MMA_LONE_LANE 5   /* 1 = the peak probes issue from one thread instead of an elected lane of a whole warp */
-#define CLPK_TUNE_GEMM_NO_PDL   6   /* 1 = small GEMMs are launched without programmatic stream serialisation */
+#define CLPK_TUNE_GEMM_NO_PDL   6   /* 1 = GEMMs are launched without programmatic stream serialisation */
 #define CLPK_TUNE_COUNT         7
 CLPK_API int clpk_set_tuning(int knob, int value);
 CLPK_API int clpk_get_tuning(int knob, int *value);
@@ -446,9 +446,8 @@ typedef struct clpk_gemm_args {
 CLPK_API int clpk_gemm_workspace_bytes(int dtype, uint32_t m, uint32_t n, uint32_t k, size_t *bytes);
 CLPK_API int clpk_gemm_pack_scales(const clpk_gemm_args_t *args, void *stream);
 CLPK_API int clpk_gemm(const clpk_gemm_args_t *args, void *stream);
-/* 1 if the calling thread's last clpk_gemm launch ran with the per-wave producer meeting (a
- * cooperative launch), 0 if it ran without (small problem, knob, or the cooperative launch did
- * not fit), -1 before any launch.  Lets a benchmark record which schedule it timed. */
+/* 1 if the calling thread's last clpk_gemm launch ran with the per-wave producer meeting, 0 if
+ * it ran without (small problem, knob), -1 before any launch.  Lets a benchmark record which schedule it timed. */
 CLPK_API int clpk_gemm_last_launch_aligned(void);
 /* SM cycles (clock64) and nanoseconds (%globaltimer) that CTA 0 of the last tensor-core GEMM
  * launched on the current device ran for; cycles / ns is the SM clock the kernel really had, which
