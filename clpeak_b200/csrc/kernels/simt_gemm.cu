@@ -36,8 +36,8 @@
 //
 // Shapes of which those tiles make too few CTAs take 64 x 64 (fp32, fp64) or 32 x 32 (fp64) tiles with K split over the
 // CTAs of a cluster and over groups of warps inside a CTA (sgemm64_kernel, dgemm_split_kernel; plan_simt has the rule).
-// Device time before -> after: fp32 64 x 64 x 16384 1545 -> 69 us, 459 x 349 x 4636 474 -> 52, 2048^3 342 -> 323; fp64
-// 64 x 64 x 16384 1388 -> 33, 863 x 251 x 2456 228 -> 42, 2048 x 2048 x 512 151 -> 143.
+// Device time before -> after: fp32 64 x 64 x 16384 1545 -> 57 us, 459 x 349 x 4636 474 -> 68; fp64
+// 64 x 64 x 16384 1388 -> 26, 863 x 251 x 2456 228 -> 42, 2048 x 2048 x 512 151 -> 143.
 //
 // All take any M, N > 0 and any K that keeps operand rows 16-byte aligned (a multiple of 4
 // floats, 2 doubles): a second instantiation of the large kernels, and the others always, zero-fill the chunks a tile
@@ -323,19 +323,22 @@ sgemm_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__
 }
 
 // The same product in 64 x 64 tiles for shapes of which 128 x 128 tiles make too few, K split over the CTAs of a cluster
-// and over two groups of two warps inside a CTA.  A group takes every other k block of its CTA's range through staging
+// and over G groups of two warps inside a CTA.  A group takes every G-th k block of its CTA's range through staging
 // and tile buffers of its own and meets only its own 64 threads.  64 x 32 outputs per warp, 8 x 8 per thread: four
-// 128-bit fragment loads per 32 packed FMAs.
+// 128-bit fragment loads per 32 packed FMAs.  Two groups and three CTAs per SM, or four groups for a CTA that has its
+// SM to itself and a long range: with one warp per scheduler the FMA pipe waits on every load (64 x 64 x 16384 in eight
+// ranges 68 -> 56 us, 719 x 368 x 6380 116 -> 87).
 constexpr int kSgemm64 = 64;
 constexpr int kSgemm64Ld = kSgemm64 + 4;
-constexpr int kSgemm64Groups = 2, kSgemm64GroupThreads = kSgemmThreads / kSgemm64Groups;
+constexpr int kSgemm64GroupThreads = 64;
 constexpr size_t kSgemm64TileFloats = (size_t)kSimtBK * kSgemm64Ld;
 constexpr size_t kSgemm64StagingFloats = 8 * 4 * (size_t)kSgemm64GroupThreads; // eight chunks per thread
 constexpr size_t kSgemm64GroupFloats = 4 * kSgemm64TileFloats + 2 * kSgemm64StagingFloats;
-constexpr size_t kSgemm64SmemBytes = kSgemm64Groups * kSgemm64GroupFloats * sizeof(float);
+template <int G> constexpr size_t kSgemm64SmemBytes = G * kSgemm64GroupFloats * sizeof(float);
 static_assert(kSgemm64 * kSgemm64 <= kSgemm64GroupFloats, "the partial tiles take the buffers' place");
 
-__global__ void __launch_bounds__(kSgemmThreads, 3)
+template <int G>
+__global__ void __launch_bounds__(G *kSgemm64GroupThreads, G == 2 ? 3 : 1)
 sgemm64_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ C, uint32_t M, uint32_t N,
                uint32_t K, float alpha, uint32_t S, uint32_t *status)
 {
@@ -348,7 +351,7 @@ sgemm64_kernel(const float *__restrict__ A, const float *__restrict__ B, float *
     raster(blockIdx.x / S, (M + kSgemm64 - 1) / kSgemm64, (N + kSgemm64 - 1) / kSgemm64, &tm, &tn);
     join_stream(status);
     const uint32_t nk_all = (K + kSimtBK - 1) / kSimtBK, kb0 = rank * nk_all / S, kb1 = (rank + 1) * nk_all / S;
-    const uint32_t nk = kb1 - kb0 > (uint32_t)group ? (kb1 - kb0 - group - 1) / kSgemm64Groups + 1 : 0;   // this group's k blocks
+    const uint32_t nk = kb1 - kb0 > (uint32_t)group ? (kb1 - kb0 - group - 1) / G + 1 : 0;   // this group's k blocks
     auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kSgemm64GroupThreads) : "memory"); };
 
     // the lane map of sgemm_kernel: 8 (rows) x 4 (columns) threads per warp
@@ -359,7 +362,7 @@ sgemm64_kernel(const float *__restrict__ A, const float *__restrict__ B, float *
     const float *srcA = A + (size_t)row_a * K + lk, *srcB = B + (size_t)row_b * K + lk;
     auto fetch = [&](uint32_t i) {                              // the group's i-th k block into staging buffer i % 2
         float *st = staging + (i & 1) * kSgemm64StagingFloats + tid * 4;
-        const uint32_t k0 = (kb0 + i * kSgemm64Groups + group) * kSimtBK;
+        const uint32_t k0 = (kb0 + i * G + group) * kSimtBK;
         const bool in_k = k0 + lk < K;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
@@ -442,7 +445,7 @@ sgemm64_kernel(const float *__restrict__ A, const float *__restrict__ B, float *
             const float2 lo = unpack2(acc[i][2 * h]), hi = unpack2(acc[i][2 * h + 1]);
             *reinterpret_cast<float4 *>(part + (fa + 32 * (i >> 2) + (i & 3)) * kSgemm64 + fb + 16 * h) = make_float4(lo.x, lo.y, hi.x, hi.y);
         }
-    sum_partial_tiles<float, kSgemm64, kSgemm64, kSgemm64Groups, kSgemmThreads>(ssm, S, rank, C, tm * kSgemm64, tn * kSgemm64, M, N, alpha);
+    sum_partial_tiles<float, kSgemm64, kSgemm64, G, G * kSgemm64GroupThreads>(ssm, S, rank, C, tm * kSgemm64, tn * kSgemm64, M, N, alpha);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -717,29 +720,39 @@ static int launch_simt(void (*kernel)(Params...), const char *what, uint64_t cta
 // busiest SM, a block of 16 k costs its CTA  max(alone, L * shared):
 //   fp32  128 x 128  max(1.62, 1.43 L)    64 x 64  max(0.51, 0.40 L)    (the pipe's own time: 1.07 and 0.27 L)
 //   fp64  128 x 64   max(1.48, 1.24 L)    64 x 64  max(0.91, 0.62 L)    32 x 32  max(0.22, 0.17 L)    (1.08, 0.54, 0.13 L)
+// A CTA alone on its SM with a range of 32 blocks (fp32) or 24 (fp64) takes twice the K groups: 0.41 and 0.18 a block,
+// and 1.5 and 0.6 us more for the longer sum at the end (shorter ranges lose up to 20 % by it, long ones gain up to 33 %).
 // The large tiles are kept unless the estimate is 8 % better; a K range has at least four blocks.
 struct SimtPlan {
     uint32_t tile, splits;
+    bool wide;                  // twice the K groups
 };
 
 static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
 {
     const uint32_t blocks = (k - 1) / kSimtBK + 1;
+    auto ctas = [&](uint32_t rows, uint32_t cols, uint32_t splits) { return (uint64_t)((m - 1) / rows + 1) * ((n - 1) / cols + 1) * splits; };
     auto estimate = [&](uint32_t rows, uint32_t cols, uint32_t splits, float alone, float shared) {
-        const uint64_t ctas = (uint64_t)((m - 1) / rows + 1) * ((n - 1) / cols + 1) * splits;
-        const float busiest = shared * (float)((ctas - 1) / simt_capacity(splits) + 1);
+        const float busiest = shared * (float)((ctas(rows, cols, splits) - 1) / simt_capacity(splits) + 1);
         return (float)((blocks - 1) / splits + 1) * (alone > busiest ? alone : busiest);
     };
     float best = f64 ? 0.92f * (3.8f + estimate(128, 64, 1, 1.48f, 1.24f)) : 0.92f * (2.0f + estimate(128, 128, 1, 1.62f, 1.43f));
-    SimtPlan plan = {128, 1};
+    SimtPlan plan = {128, 1, false};
     for (uint32_t splits = 1; splits <= 8 && (splits == 1 || blocks >= 4 * splits); splits *= 2)
         for (uint32_t tile = f64 ? 32 : 64; tile <= 64; tile *= 2) {
-            float t = !f64 ? 4.1f + estimate(64, 64, splits, 0.507f, 0.404f) + (splits > 1 ? 1.1f + 0.08f * splits : 0.0f)
-                    : tile == 64 ? 4.56f + estimate(64, 64, splits, 0.907f, 0.616f)
-                                 : 3.9f + estimate(32, 32, splits, 0.223f, 0.174f) + (splits > 1 ? 0.5f * splits : 0.0f);
+            const bool wide = !(f64 && tile == 64) && ctas(tile, tile, splits) <= simt_capacity(splits) && blocks >= (f64 ? 24 : 32) * splits;
+            float t;
+            if (!f64)
+                t = (wide ? 5.6f + estimate(64, 64, splits, 0.405f, 0.0f) : 4.1f + estimate(64, 64, splits, 0.507f, 0.404f)) +
+                    (splits > 1 ? 1.1f + 0.08f * splits : 0.0f);
+            else if (tile == 64)
+                t = 4.56f + estimate(64, 64, splits, 0.907f, 0.616f);
+            else
+                t = (wide ? 4.5f + estimate(32, 32, splits, 0.178f, 0.0f) : 3.9f + estimate(32, 32, splits, 0.223f, 0.174f)) +
+                    (splits > 1 ? 0.5f * splits : 0.0f);
             if (t < best) {
                 best = t;
-                plan = {tile, splits};
+                plan = {tile, splits, wide};
             }
         }
     return plan;
@@ -763,8 +776,10 @@ int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t 
         const float *fa = static_cast<const float *>(a), *fb = static_cast<const float *>(b);
         float *fc = static_cast<float *>(c);
         if (plan.tile == 64)
-            return launch_simt(sgemm64_kernel, "launch sgemm64", ctas, kSgemmThreads, kSgemm64SmemBytes, plan.splits, true, s, fa, fb, fc, m, n, k, alpha,
-                               plan.splits, status);
+            return plan.wide ? launch_simt(sgemm64_kernel<4>, "launch sgemm64", ctas, 4 * kSgemm64GroupThreads, kSgemm64SmemBytes<4>, plan.splits, false, s, fa, fb,
+                                       fc, m, n, k, alpha, plan.splits, status)
+                         : launch_simt(sgemm64_kernel<2>, "launch sgemm64", ctas, 2 * kSgemm64GroupThreads, kSgemm64SmemBytes<2>, plan.splits, true, s, fa, fb,
+                                       fc, m, n, k, alpha, plan.splits, status);
         return launch_simt(ragged ? sgemm_kernel<true> : sgemm_kernel<false>, "launch sgemm", tiles, kSgemmThreads, kSgemmSmemBytes, 1, false, s, fa, fb,
                            fc, m, n, k, alpha, status);
     }
@@ -773,6 +788,9 @@ int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t 
     if (plan.tile == 64)
         return launch_simt(dgemm_split_kernel<2, 2, 1>, "launch dgemm 64", ctas, DgemmSplit<2, 2, 1>::threads, DgemmSplit<2, 2, 1>::smem_bytes, plan.splits,
                            true, s, da, db, dc, m, n, k, alpha, plan.splits, status);
+    if (plan.tile == 32 && plan.wide)
+        return launch_simt(dgemm_split_kernel<1, 1, 8>, "launch dgemm 32", ctas, DgemmSplit<1, 1, 8>::threads, DgemmSplit<1, 1, 8>::smem_bytes, plan.splits,
+                           false, s, da, db, dc, m, n, k, alpha, plan.splits, status);
     if (plan.tile == 32)
         return launch_simt(dgemm_split_kernel<1, 1, 4>, "launch dgemm 32", ctas, DgemmSplit<1, 1, 4>::threads, DgemmSplit<1, 1, 4>::smem_bytes, plan.splits,
                            true, s, da, db, dc, m, n, k, alpha, plan.splits, status);

@@ -24,7 +24,7 @@ def operand(K, cuda, dtype, rows, k, seed):
 # N odd (no vector store); one and several CTAs per SM; the large tiles' side of the rule
 @pytest.mark.parametrize("m,n,k", [(1, 1, 4), (33, 65, 20), (64, 64, 16384), (129, 131, 36), (131, 102, 7688), (201, 73, 2828), (863, 251, 2456),
                                    (1315, 363, 956), (440, 434, 520), (64, 868, 1036), (719, 366, 688), (459, 349, 4636), (3720, 110, 596),
-                                   (2254, 496, 464), (1024, 1024, 512)])
+                                   (2254, 496, 464), (1024, 1024, 512), (97, 106, 5732), (719, 368, 6380), (64, 64, 4100)])
 @pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F64])
 def test_every_element(K, cuda, dtype, m, n, k):
     a, b = operand(K, cuda, dtype, m, k, 40), operand(K, cuda, dtype, n, k, 41)
