@@ -56,3 +56,35 @@ def test_every_element(K, cuda, dtype, m, n, k_bytes):
         assert worst <= 1.0, f"worst error over all of C is {worst:.3g}x the stated tolerance"
     again = run_into(K, cuda, dtype, m, n, k, d_a, d_b, alpha)
     assert bool((again == c).all()), "partial sums are added in a fixed order: the same bits every time"
+
+
+def test_aligned_launches_on_two_streams(K, cuda):
+    """GEMMs whose producers meet once per wave, back to back on two streams and over more launches than there are wave
+    counters: whoever holds the SMs, the bits are those of a launch by itself, and the counters serve the next launch."""
+    m, n, k = 8192, 8192, 256
+    d_a, d_b = make_gemm_operands(K, cuda, N.DT_BF16, m, n, k)
+    want = run_into(K, cuda, N.DT_BF16, m, n, k, d_a, d_b, 1.0).clone()
+    assert K.raw("clpk_gemm_last_launch_aligned")() == 1
+    streams = [cuda.cuda.Stream() for _ in range(2)]
+    out = [dev_empty(m * n, cuda.int16) for _ in streams]
+    status = [dev_empty(1, cuda.int32) for _ in streams]
+    sync()
+    for _ in range(20):
+        for s, c, st in zip(streams, out, status):
+            args = N.GemmArgs(dtype=N.DT_BF16, m=m, n=n, k=k, d_a=d_a.data_ptr(), d_b=d_b.data_ptr(), d_c=c.data_ptr(), alpha=1.0,
+                              d_status=st.data_ptr())
+            K.clpk_gemm(C.byref(args), s.cuda_stream)
+    sync()
+    for c, st in zip(out, status):
+        assert int(st.item()) == 0 and bool((c == want).all())
+    # a counter that had not come back to zero would let the producers pass unmet or make them wait 40 us a wave
+    e0, e1 = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
+    times = []
+    for _ in range(40):
+        e0.record()
+        K.clpk_gemm(C.byref(args), stream_ptr())
+        e1.record()
+        sync()
+        times.append(e0.elapsed_time(e1))
+    assert sorted(times)[20] < 4 * sorted(times)[0], times
+    assert bool((out[1] == want).all())
