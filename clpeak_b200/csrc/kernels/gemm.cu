@@ -37,7 +37,6 @@ namespace clpk {
 
 constexpr uint32_t kRowBytesK = 128;                        // K bytes per row per stage
 constexpr uint32_t kHalfTileBytes = 128 * kRowBytesK;       // 16 KiB: 128 rows x 128 B
-constexpr uint32_t kStageBytes = 2 * kHalfTileBytes;        // A half + B half (block-scaled kernel)
 constexpr uint32_t kTileMN = 256;
 constexpr int kGemmThreads = 320;                          // dense kernel: producer, MMA, 8 epilogue warps
 
@@ -71,50 +70,7 @@ __device__ __forceinline__ void join_previous_launch(const GemmParams &p)
 // Output element of a GEMM dtype: fp32 for TF32, int32 for I8, bf16 for everything else.
 template <int DT> struct OutBytes { static constexpr uint32_t value = (DT == CLPK_DT_TF32 || DT == CLPK_DT_I8) ? 4u : 2u; };
 
-// Thread-local epilogue step: 32 consecutive accumulator columns of one row -> global memory.
-template <int DT>
-__device__ __forceinline__ void store_columns(uint8_t *dst_bytes, const uint32_t (&r)[32], float alpha)
-{
-    if constexpr (DT == CLPK_DT_I8) {
-        uint4 *dst = reinterpret_cast<uint4 *>(dst_bytes);
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-            dst[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
-    } else if constexpr (DT == CLPK_DT_TF32) {
-        uint4 *dst = reinterpret_cast<uint4 *>(dst_bytes);
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-            dst[i] = make_uint4(__float_as_uint(__uint_as_float(r[4 * i]) * alpha), __float_as_uint(__uint_as_float(r[4 * i + 1]) * alpha),
-                                __float_as_uint(__uint_as_float(r[4 * i + 2]) * alpha), __float_as_uint(__uint_as_float(r[4 * i + 3]) * alpha));
-    } else {
-        uint32_t w[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
-            w[i] = *reinterpret_cast<uint32_t *>(&v);
-        }
-        uint4 *dst = reinterpret_cast<uint4 *>(dst_bytes);
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-            dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-    }
-}
-
-// 2-D tile load whose completion bytes go to the barrier at the same offset in
-// the pair's leader CTA (cluster rank 0).
-__device__ __forceinline__ void tma_load_pair(void *smem_dst, const CUtensorMap *tmap, int32_t x,
-                                              int32_t y, uint64_t *bar)
-{
-    uint32_t leader_bar;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(leader_bar) : "r"(smem_u32(bar)));
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(smem_dst)),
-        "l"(tmap), "r"(leader_bar), "r"(x), "r"(y)
-        : "memory");
-}
-
-// The same with the leader's barrier address already mapped (mapa hoisted out of the loop).
+// 2-D tile load whose completion bytes go to the pair's leader CTA: leader_bar is its barrier's address (leader_addr).
 __device__ __forceinline__ void tma_load_pair_at(void *smem_dst, const CUtensorMap *tmap, int32_t x, int32_t y,
                                                  uint32_t leader_bar)
 {
