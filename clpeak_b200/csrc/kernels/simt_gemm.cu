@@ -54,6 +54,7 @@ namespace clpk {
 constexpr int kSimtTile = 128;
 constexpr int kSimtBK = 16;
 constexpr int kRasterGroup = 16;
+constexpr int kSimtSmemMax = 227 * 1024;                // the most dynamic shared memory that a CTA may ask for
 
 // tile -> (tile row, tile column), column-major inside groups of kRasterGroup tile rows
 __device__ __forceinline__ void raster(uint32_t tile, uint32_t tiles_m, uint32_t tiles_n, uint32_t *tm, uint32_t *tn)
@@ -690,11 +691,13 @@ static int launch_simt(void (*kernel)(Params...), const char *what, uint64_t cta
     // shared memory (fp32 4195 x 225 x 1980, 264 CTAs of 64 x 64: 151 -> 113 us, fp64 902 x 868 x 2356 182 -> 146).
     if (even_share) {
         const uint64_t share = (ctas - 1) / simt_capacity(cluster) + 1;
-        const size_t fill = 227 * 1024 / (share + 1) + 1024;
+        const size_t fill = kSimtSmemMax / (share + 1) + 1024;
         if (share < 8 && fill > smem)
             smem = fill;
     }
-    CLPK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // The attribute is the kernel's, not the call's: a limit of this call's size would refuse the larger request of
+    // another host thread between its own setting and its launch.
+    CLPK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSimtSmemMax));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3((unsigned)threads);
