@@ -32,7 +32,7 @@ struct __align__(32) Float8 {
 __device__ __forceinline__ Float8 ld_float8(const float *p)
 {
     unsigned long long w[4];
-    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]) : "l"(p));
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]) : "l"(p) : "memory");
     Float8 r;
 #pragma unroll
     for (int i = 0; i < 4; i++) {

@@ -68,7 +68,8 @@ __device__ __forceinline__ void raster(uint32_t tile, uint32_t tiles_m, uint32_t
 
 // The launches carry the programmatic-serialisation attribute: a CTA may start under the tail of the kernel before it
 // in the stream and waits here until that has completed.  The status word is cleared by the kernel, so that nothing
-// sits between two launches.
+// sits between two launches.  No operand is `const __restrict__`: the kernel before may still be writing it when this
+// one starts, and the read-only path that the qualifier allows wants data that does not change while the kernel runs.
 __device__ __forceinline__ void join_stream(uint32_t *status)
 {
     griddep_wait();
@@ -184,7 +185,7 @@ __device__ __forceinline__ void cp_async_16_or_zeros(void *dst_shared, const voi
 // aligned): chunks outside the operands arrive as zeros, stores outside C are skipped.
 template <bool RAGGED>
 __global__ void __launch_bounds__(kSgemmThreads, 2)
-sgemm_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ C, uint32_t M, uint32_t N,
+sgemm_kernel(const float *A, const float *B, float *C, uint32_t M, uint32_t N,
              uint32_t K, float alpha, uint32_t *status)
 {
     extern __shared__ __align__(16) float ssm[];
@@ -340,7 +341,7 @@ static_assert(kSgemm64 * kSgemm64 <= kSgemm64GroupFloats, "the partial tiles tak
 
 template <int G>
 __global__ void __launch_bounds__(G *kSgemm64GroupThreads, G == 2 ? 3 : 1)
-sgemm64_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ C, uint32_t M, uint32_t N,
+sgemm64_kernel(const float *A, const float *B, float *C, uint32_t M, uint32_t N,
                uint32_t K, float alpha, uint32_t S, uint32_t *status)
 {
     extern __shared__ __align__(16) float ssm[];
@@ -472,7 +473,7 @@ __device__ __forceinline__ void dmma_m8n8k4(double &d0, double &d1, double a, do
 
 template <int CN, bool RAGGED>
 __global__ void __launch_bounds__(Dgemm<CN>::threads, 128 / CN)
-dgemm_kernel(const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C, uint32_t M, uint32_t N,
+dgemm_kernel(const double *A, const double *B, double *C, uint32_t M, uint32_t N,
              uint32_t K, double alpha, uint32_t *status)
 {
     extern __shared__ __align__(16) double dsm[];
@@ -594,7 +595,7 @@ template <int WM, int WN, int WK> struct DgemmSplit {
 
 template <int WM, int WN, int WK>
 __global__ void __launch_bounds__(DgemmSplit<WM, WN, WK>::threads, DgemmSplit<WM, WN, WK>::ctas_per_sm)
-dgemm_split_kernel(const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C, uint32_t M, uint32_t N,
+dgemm_split_kernel(const double *A, const double *B, double *C, uint32_t M, uint32_t N,
                    uint32_t K, double alpha, uint32_t S, uint32_t *status)
 {
     extern __shared__ __align__(16) double dsm[];

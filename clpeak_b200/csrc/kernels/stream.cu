@@ -67,6 +67,23 @@ __device__ __forceinline__ void join_stream()
     griddep_launch_dependents();
 }
 
+// 16 bytes that are read once.  The kernel before may be writing them while this one starts, so no parameter here is
+// `const __restrict__` (its data may go through the read-only path, whose condition is that it does not change while
+// the kernel runs), and the load is volatile, which keeps it behind join_stream().
+__device__ __forceinline__ uint4 ld_once(const uint4 *p)
+{
+    uint4 v;
+    asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ float4 ld_once(const float4 *p)
+{
+    float4 v;
+    asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 // ---- LDG flavour ---------------------------------------------------------------------
 
 constexpr int kLdgThreads = 512;
@@ -92,9 +109,9 @@ __device__ __forceinline__ void cta_xor_store(uint32_t x, uint32_t *slot)
     }
 }
 
-__global__ void __launch_bounds__(kLdgThreads) stream_read_ldg(const uint4 *__restrict__ src,
+__global__ void __launch_bounds__(kLdgThreads) stream_read_ldg(const uint4 *src,
                                                                uint64_t n16,
-                                                               uint32_t *__restrict__ partials)
+                                                               uint32_t *partials)
 {
     join_stream();
     constexpr uint64_t kTile = (uint64_t)kLdgThreads * kLdgUnroll;
@@ -105,20 +122,20 @@ __global__ void __launch_bounds__(kLdgThreads) stream_read_ldg(const uint4 *__re
         uint4 v[kLdgUnroll];
 #pragma unroll
         for (int u = 0; u < kLdgUnroll; u++)
-            v[u] = __ldcs(p + u * kLdgThreads);
+            v[u] = ld_once(p + u * kLdgThreads);
 #pragma unroll
         for (int u = 0; u < kLdgUnroll; u++)
             acc ^= xor4(v[u]);
     }
     if (blockIdx.x == 0) {
         for (uint64_t i = n_full * kTile + threadIdx.x; i < n16; i += kLdgThreads)
-            acc ^= xor4(__ldcs(src + i));
+            acc ^= xor4(ld_once(src + i));
     }
     cta_xor_store(acc, partials + blockIdx.x);
 }
 
-__global__ void __launch_bounds__(kLdgThreads) stream_copy_ldg(uint4 *__restrict__ dst,
-                                                               const uint4 *__restrict__ src,
+__global__ void __launch_bounds__(kLdgThreads) stream_copy_ldg(uint4 *dst,
+                                                               const uint4 *src,
                                                                uint64_t n16)
 {
     join_stream();
@@ -129,14 +146,14 @@ __global__ void __launch_bounds__(kLdgThreads) stream_copy_ldg(uint4 *__restrict
         uint4 v[kLdgUnroll];
 #pragma unroll
         for (int u = 0; u < kLdgUnroll; u++)
-            v[u] = __ldcs(src + base + u * kLdgThreads);
+            v[u] = ld_once(src + base + u * kLdgThreads);
 #pragma unroll
         for (int u = 0; u < kLdgUnroll; u++)
             __stcs(dst + base + u * kLdgThreads, v[u]);
     }
     if (blockIdx.x == 0) {
         for (uint64_t i = n_full * kTile + threadIdx.x; i < n16; i += kLdgThreads)
-            __stcs(dst + i, __ldcs(src + i));
+            __stcs(dst + i, ld_once(src + i));
     }
 }
 
@@ -148,9 +165,9 @@ __device__ __forceinline__ float4 triad4(const float4 &b, const float4 &c, float
                        __fadd_rn(b.z, __fmul_rn(s, c.z)), __fadd_rn(b.w, __fmul_rn(s, c.w)));
 }
 
-__global__ void __launch_bounds__(kLdgThreads) stream_triad_ldg(float4 *__restrict__ a,
-                                                                const float4 *__restrict__ b,
-                                                                const float4 *__restrict__ c,
+__global__ void __launch_bounds__(kLdgThreads) stream_triad_ldg(float4 *a,
+                                                                const float4 *b,
+                                                                const float4 *c,
                                                                 float s, uint64_t n4,
                                                                 uint64_t n_tail_floats)
 {
@@ -163,8 +180,8 @@ __global__ void __launch_bounds__(kLdgThreads) stream_triad_ldg(float4 *__restri
         float4 vb[kU], vc[kU];
 #pragma unroll
         for (int u = 0; u < kU; u++) {
-            vb[u] = __ldcs(b + base + u * kLdgThreads);
-            vc[u] = __ldcs(c + base + u * kLdgThreads);
+            vb[u] = ld_once(b + base + u * kLdgThreads);
+            vc[u] = ld_once(c + base + u * kLdgThreads);
         }
 #pragma unroll
         for (int u = 0; u < kU; u++)
@@ -172,7 +189,7 @@ __global__ void __launch_bounds__(kLdgThreads) stream_triad_ldg(float4 *__restri
     }
     if (blockIdx.x == 0) {
         for (uint64_t i = n_full * kTile + threadIdx.x; i < n4; i += kLdgThreads)
-            __stcs(a + i, triad4(__ldcs(b + i), __ldcs(c + i), s));
+            __stcs(a + i, triad4(ld_once(b + i), ld_once(c + i), s));
         // floats beyond the last whole float4
         const float *bf = reinterpret_cast<const float *>(b) + n4 * 4;
         const float *cf = reinterpret_cast<const float *>(c) + n4 * 4;
@@ -210,7 +227,8 @@ __device__ __forceinline__ Vec32 ld_stream32(const Vec32 *p)
     Vec32 v;
     asm volatile("ld.global.L1::no_allocate.L2::evict_first.v4.b64 {%0, %1, %2, %3}, [%4];"
                  : "=l"(v.a), "=l"(v.b), "=l"(v.c), "=l"(v.d)
-                 : "l"(p));
+                 : "l"(p)
+                 : "memory");
     return v;
 }
 
@@ -229,8 +247,8 @@ __device__ __forceinline__ void st_stream32(Vec32 *p, const Vec32 &v)
 constexpr uint64_t kWideRounds = 8;
 
 template <bool ATOMIC>
-__global__ void __launch_bounds__(kWideThreads) stream_read_wide(const Vec32 *__restrict__ src, uint64_t n_tiles,
-                                                                 uint64_t n_tail16, uint32_t *__restrict__ slots)
+__global__ void __launch_bounds__(kWideThreads) stream_read_wide(const Vec32 *src, uint64_t n_tiles,
+                                                                 uint64_t n_tail16, uint32_t *slots)
 {
     join_stream();
     unsigned long long x = 0;
@@ -251,7 +269,7 @@ __global__ void __launch_bounds__(kWideThreads) stream_read_wide(const Vec32 *__
     if (blockIdx.x == 0) {
         const uint4 *tail = reinterpret_cast<const uint4 *>(src + n_tiles * kWideThreads);
         for (uint64_t i = threadIdx.x; i < n_tail16; i += kWideThreads)
-            y ^= xor4(__ldcs(tail + i));
+            y ^= xor4(ld_once(tail + i));
     }
     for (int o = 16; o > 0; o >>= 1)
         y ^= __shfl_xor_sync(0xffffffffu, y, o);
@@ -271,7 +289,7 @@ __global__ void __launch_bounds__(kWideThreads) stream_read_wide(const Vec32 *__
     }
 }
 
-__global__ void __launch_bounds__(kWideThreads) stream_copy_wide(Vec32 *__restrict__ dst, const Vec32 *__restrict__ src,
+__global__ void __launch_bounds__(kWideThreads) stream_copy_wide(Vec32 *dst, const Vec32 *src,
                                                                  uint64_t n_tiles, uint64_t n_tail16)
 {
     join_stream();
@@ -283,7 +301,7 @@ __global__ void __launch_bounds__(kWideThreads) stream_copy_wide(Vec32 *__restri
         const uint4 *ts = reinterpret_cast<const uint4 *>(src + n_tiles * kWideThreads);
         uint4 *td = reinterpret_cast<uint4 *>(dst + n_tiles * kWideThreads);
         for (uint64_t i = threadIdx.x; i < n_tail16; i += kWideThreads)
-            __stcs(td + i, __ldcs(ts + i));
+            __stcs(td + i, ld_once(ts + i));
     }
 }
 
@@ -319,11 +337,11 @@ __device__ __forceinline__ uint64_t claim_tile(unsigned long long *next_tile, ui
     return next_tile ? atomicAdd(next_tile, 1ull) : blockIdx.x + round * gridDim.x;
 }
 
-__global__ void __launch_bounds__(160) stream_read_tma(const uint8_t *__restrict__ src,
+__global__ void __launch_bounds__(160) stream_read_tma(const uint8_t *src,
                                                        uint64_t n_bytes,
-                                                       uint32_t *__restrict__ partials,
-                                                       uint32_t *__restrict__ status,
-                                                       unsigned long long *__restrict__ next_tile)
+                                                       uint32_t *partials,
+                                                       uint32_t *status,
+                                                       unsigned long long *next_tile)
 {
     join_stream();
     extern __shared__ __align__(128) uint8_t smem[];
@@ -387,11 +405,11 @@ __global__ void __launch_bounds__(160) stream_read_tma(const uint8_t *__restrict
     cta_xor_store(acc, partials + blockIdx.x);
 }
 
-__global__ void __launch_bounds__(32) stream_copy_tma(uint8_t *__restrict__ dst,
-                                                      const uint8_t *__restrict__ src,
+__global__ void __launch_bounds__(32) stream_copy_tma(uint8_t *dst,
+                                                      const uint8_t *src,
                                                       uint64_t n_bytes,
-                                                      uint32_t *__restrict__ status,
-                                                      unsigned long long *__restrict__ next_tile)
+                                                      uint32_t *status,
+                                                      unsigned long long *next_tile)
 {
     join_stream();
     extern __shared__ __align__(128) uint8_t smem[];
@@ -440,8 +458,8 @@ __global__ void __launch_bounds__(32) stream_copy_tma(uint8_t *__restrict__ dst,
     bulk_wait<0>();
 }
 
-__global__ void __launch_bounds__(kWideThreads) stream_triad_wide(Vec32 *__restrict__ a, const Vec32 *__restrict__ b,
-                                                                  const Vec32 *__restrict__ c, float s,
+__global__ void __launch_bounds__(kWideThreads) stream_triad_wide(Vec32 *a, const Vec32 *b,
+                                                                  const Vec32 *c, float s,
                                                                   uint64_t n_tiles, uint64_t n_tail_floats)
 {
     join_stream();
@@ -464,12 +482,12 @@ __global__ void __launch_bounds__(kWideThreads) stream_triad_wide(Vec32 *__restr
     }
 }
 
-__global__ void __launch_bounds__(192) stream_triad_tma(float *__restrict__ a,
-                                                        const float *__restrict__ b,
-                                                        const float *__restrict__ c, float s,
+__global__ void __launch_bounds__(192) stream_triad_tma(float *a,
+                                                        const float *b,
+                                                        const float *c, float s,
                                                         uint64_t n_bytes,
-                                                        uint32_t *__restrict__ status,
-                                                        unsigned long long *__restrict__ next_tile)
+                                                        uint32_t *status,
+                                                        unsigned long long *next_tile)
 {
     join_stream();
     extern __shared__ __align__(128) uint8_t smem[];
