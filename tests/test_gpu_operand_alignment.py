@@ -1,0 +1,72 @@
+"""Operand kernels on pointers that are not aligned for their wide accesses: the same elements, and about the same time."""
+import numpy as np
+import pytest
+
+from clpeak_b200 import native as N
+from tests.gpu_util import assert_bits_equal, dev_empty, stream_ptr, sync, to_np
+
+pytestmark = pytest.mark.gpu
+
+
+def best_us(cuda, fn, rounds=25, calls=4):
+    for _ in range(3):
+        fn()
+    sync()
+    times = []
+    for _ in range(rounds):
+        e0, e1 = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
+        e0.record()
+        for _ in range(calls):
+            fn()
+        e1.record()
+        sync()
+        times.append(e0.elapsed_time(e1) * 1e3 / calls)
+    return min(times)
+
+
+def assert_about_as_fast(cuda, at_offset, offsets, factor):
+    """Best of many bursts on both sides: what else the machine does only adds time, and rarely to all of them."""
+    base = best_us(cuda, lambda: at_offset(0))
+    for off in offsets:
+        t = best_us(cuda, lambda: at_offset(off))
+        assert t < factor * base, f"{t:.1f} us at an offset of {off} elements, {base:.1f} at none"
+
+
+N_TIMED = 8192 * 4096              # two to three times the L2 in floats
+
+
+@pytest.mark.parametrize("dist", [0, 1, 2])
+@pytest.mark.parametrize("n", [3, 8, 13, 4100])
+def test_fill_at_every_offset(K, orc, cuda, dist, n):
+    want = orc.fill_f32(n, 31, dist, 0.5, 3.0)
+    for offset in range(9):
+        buf = cuda.full((n + offset + 8,), 77.0, dtype=cuda.float32, device="cuda")
+        K.clpk_fill_f32(buf.data_ptr() + 4 * offset, n, 31, dist, 0.5, 3.0, stream_ptr())
+        sync()
+        got = to_np(buf)
+        assert_bits_equal(got[offset:offset + n], want, "fill")
+        assert np.all(got[:offset] == 77.0) and np.all(got[offset + n:] == 77.0), "the fill wrote outside its range"
+
+
+@pytest.mark.parametrize("n", [5, 16, 29, 5000])
+def test_fill_i8_at_every_offset(K, orc, cuda, n):
+    want = orc.fill_i8(n, 9)
+    for offset in range(17):
+        buf = cuda.full((n + offset + 8,), 77, dtype=cuda.int8, device="cuda")
+        K.clpk_fill_i8(buf.data_ptr() + offset, n, 9, stream_ptr())
+        sync()
+        got = to_np(buf)
+        assert_bits_equal(got[offset:offset + n], want, "fill_i8")
+        assert np.all(got[:offset] == 77) and np.all(got[offset + n:] == 77)
+
+
+# cut at the first aligned address it is the same work; one element at a time took 1.8 to 4 times as long
+@pytest.mark.parametrize("dist", [0, 1, 2])
+def test_fill_is_as_fast_from_any_offset(K, cuda, dist):
+    d = dev_empty(N_TIMED + 8, cuda.float32)
+    assert_about_as_fast(cuda, lambda off: K.clpk_fill_f32(d.data_ptr() + 4 * off, N_TIMED, 3, dist, 0.0, 1.0, stream_ptr()), (1, 4), 1.3)
+
+
+def test_fill_i8_is_as_fast_from_any_offset(K, cuda):
+    d = dev_empty(N_TIMED + 16, cuda.int8)
+    assert_about_as_fast(cuda, lambda off: K.clpk_fill_i8(d.data_ptr() + off, N_TIMED, 3, stream_ptr()), (1, 8), 1.3)
