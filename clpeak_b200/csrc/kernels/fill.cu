@@ -228,30 +228,30 @@ __global__ void __launch_bounds__(kFillThreads) convert_kernel(void *dst, const 
     }
 }
 
-// Bound by memory (8192 x 8192: 111 -> 42 us, 6.4 TB/s); a CTA takes four accesses per thread of one contiguous range (8 Ki floats), so that the chip walks
-// the array in address order.  SINGLE: one CTA reads everything and writes the result itself; otherwise the CTAs meet
-// in an atomicMax on a word that has been cleared.
+// Bound by memory (8192 x 8192: 111 -> 42 us, 6.4 TB/s, from any address); a CTA takes four accesses per thread of one
+// contiguous range (8 Ki floats), so that the chip walks the array in address order.  SINGLE: one CTA reads everything and
+// writes the result itself; otherwise the CTAs meet in an atomicMax on a word that has been cleared.
 constexpr int kAbsmaxLoads = 4;
 
 template <bool SINGLE>
-__global__ void __launch_bounds__(kFillThreads) absmax_kernel(float *out, const float *src, uint64_t n8, uint64_t n)
+__global__ void __launch_bounds__(kFillThreads) absmax_kernel(float *out, const float *src, Split part)
 {
     join_stream();
     float m = 0.0f;
     const uint64_t step = (uint64_t)gridDim.x * kFillThreads * kAbsmaxLoads;
-    for (uint64_t g = (uint64_t)blockIdx.x * kFillThreads * kAbsmaxLoads + threadIdx.x; g < n8; g += step) {
+    for (uint64_t g = (uint64_t)blockIdx.x * kFillThreads * kAbsmaxLoads + threadIdx.x; g < part.whole; g += step) {
         Float8 x[kAbsmaxLoads];
 #pragma unroll
         for (int u = 0; u < kAbsmaxLoads; u++)
-            x[u] = g + u * kFillThreads < n8 ? ld_float8(src + 8 * (g + u * kFillThreads)) : Float8{};
+            x[u] = g + u * kFillThreads < part.whole ? ld_float8(src + 8 * (g + u * kFillThreads)) : Float8{};
 #pragma unroll
         for (int u = 0; u < kAbsmaxLoads; u++)
 #pragma unroll
             for (int i = 0; i < 8; i++)
                 m = fmaxf(m, fabsf(x[u].v[i]));
     }
-    for (uint64_t i = 8 * n8 + (uint64_t)blockIdx.x * kFillThreads + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kFillThreads)
-        m = fmaxf(m, fabsf(src[i]));
+    if (part.has_single())
+        m = fmaxf(m, fabsf(src[part.single(8)]));
     // |x| >= 0, so the float ordering equals the ordering of the bit patterns.
     uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
     __shared__ uint32_t warp_top[kFillThreads / 32];
@@ -451,7 +451,7 @@ static unsigned fill_grid(uint64_t items)
 static bool aligned(const void *p, size_t bytes) { return ((uintptr_t)p % bytes) == 0; }
 
 // One element at a time is bound by how fast CTAs start, whatever the type: 8192 x 8192 from an address 4 bytes off,
-// uniform 270 us, normal 292, int8 269; cut at the boundary 64, 161 and 56, as from an aligned one.
+// uniform 270 us, normal 292, int8 269, absmax 129; cut at the boundary 64, 161, 56 and 42, as from an aligned one.
 static Split split_at(const void *p, uint32_t align, uint32_t element, uint32_t per, uint64_t n)
 {
     const uint32_t head = (align - (uint32_t)((uintptr_t)p % align)) % align / element;
@@ -542,15 +542,17 @@ int clpk_absmax_f32(float *d_absmax, const float *d_src, uint64_t n, void *strea
 {
     CLPK_REQUIRE(d_absmax, "d_absmax is NULL");
     cudaStream_t s = as_stream(stream);
-    const uint64_t n8 = aligned(d_src, 32) ? n / 8 : 0;
+    const Split part = split_at(d_src, 32, sizeof(float), 8, n);
     // up to 32 Ki floats one CTA reads in the time that clearing the word would take
     if (n > 0 && n <= 32768 && d_src)
-        return launch_behind(absmax_kernel<true>, "launch absmax", 1, kFillThreads, 0, s, d_absmax, d_src, n8, n);
+        return launch_behind(absmax_kernel<true>, "launch absmax", 1, kFillThreads, 0, s, d_absmax, d_src + part.head,
+                             part);
     CLPK_CUDA(cudaMemsetAsync(d_absmax, 0, sizeof(float), s));
     if (n == 0)
         return CLPK_OK;
     CLPK_REQUIRE(d_src, "d_src is NULL");
-    return launch_behind(absmax_kernel<false>, "launch absmax", fill_grid((n8 ? n8 : n) / kAbsmaxLoads + 1), kFillThreads, 0, s, d_absmax, d_src, n8, n);
+    return launch_behind(absmax_kernel<false>, "launch absmax", fill_grid(part.whole / kAbsmaxLoads + 1), kFillThreads, 0, s, d_absmax,
+                         d_src + part.head, part);
 }
 
 int clpk_quantize_fp4(uint8_t *d_packed, uint8_t *d_scales, const float *d_src, uint64_t rows,

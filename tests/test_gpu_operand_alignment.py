@@ -60,6 +60,23 @@ def test_fill_i8_at_every_offset(K, orc, cuda, n):
         assert np.all(got[:offset] == 77) and np.all(got[offset + n:] == 77)
 
 
+@pytest.mark.parametrize("n", [1, 6, 8, 15, 40, 32768, 32769, 70001])
+def test_absmax_at_every_offset(K, orc, cuda, n):
+    """The largest in the head, in the steps and at the very end, from every offset."""
+    src = orc.fill_f32(n, 8, N.DIST_UNIFORM_PM1)
+    buf = cuda.full((n + 32,), 50.0, dtype=cuda.float32, device="cuda")        # larger than all of the operand's own
+    out = dev_empty(1, cuda.float32)
+    for offset in range(9):
+        for at in {0, min(5, n - 1), n // 2, n - 1}:
+            x = src.copy()
+            x[at] = -9.5
+            buf.fill_(50.0)
+            buf[offset:offset + n] = cuda.from_numpy(x).cuda()
+            K.clpk_absmax_f32(out.data_ptr(), buf.data_ptr() + 4 * offset, n, stream_ptr())
+            sync()
+            assert float(out.item()) == 9.5, (offset, at)
+
+
 # cut at the first aligned address it is the same work; one element at a time took 1.8 to 4 times as long
 @pytest.mark.parametrize("dist", [0, 1, 2])
 def test_fill_is_as_fast_from_any_offset(K, cuda, dist):
@@ -70,3 +87,11 @@ def test_fill_is_as_fast_from_any_offset(K, cuda, dist):
 def test_fill_i8_is_as_fast_from_any_offset(K, cuda):
     d = dev_empty(N_TIMED + 16, cuda.int8)
     assert_about_as_fast(cuda, lambda off: K.clpk_fill_i8(d.data_ptr() + off, N_TIMED, 3, stream_ptr()), (1, 8), 1.3)
+
+
+# a small array is one CTA's, which took twice the time over one element per thread and step; a large one 1.2 to 3 times
+@pytest.mark.parametrize("n", [32768, N_TIMED])
+def test_absmax_is_as_fast_from_any_offset(K, cuda, n):
+    src, out = dev_empty(n + 8, cuda.float32), dev_empty(1, cuda.float32)
+    src.zero_()
+    assert_about_as_fast(cuda, lambda off: K.clpk_absmax_f32(out.data_ptr(), src.data_ptr() + 4 * off, n, stream_ptr()), (1, 4), 1.3)
