@@ -1,7 +1,7 @@
 // Seeded operand generation, format conversion and block-scaled FP4 quantisation.
 //
-// Eight consecutive elements per thread and step, moved with the widest access their type and alignment allow.  The fills
-// take the elements in front of the first aligned address, and those left over at the end, one at a time.
+// Eight consecutive elements per thread and step, moved with the widest access their type and alignment allow.  The
+// elements in front of the first aligned address, and those left over at the end, go one at a time.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -57,6 +57,27 @@ __device__ __forceinline__ Float8 ld_float8(const float *p)
         r.v[2 * i + 1] = hi_of(w[i]);
     }
     return r;
+}
+
+// eight floats from an address that is a multiple of ALIGN bytes
+template <int ALIGN>
+__device__ __forceinline__ Float8 ld_float8(const float *p)
+{
+    if constexpr (ALIGN == 32) {
+        return ld_float8(p);
+    } else {
+        Float8 r;
+        if constexpr (ALIGN == 16) {
+            const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
+            r.v[0] = a.x; r.v[1] = a.y; r.v[2] = a.z; r.v[3] = a.w;
+            r.v[4] = b.x; r.v[5] = b.y; r.v[6] = b.z; r.v[7] = b.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                r.v[i] = p[i];
+        }
+        return r;
+    }
 }
 
 __device__ __forceinline__ void st_float8(float *p, f32x2 a, f32x2 b, f32x2 c, f32x2 d)
@@ -175,14 +196,14 @@ template <int DT> struct Narrow {
 
 // Bound by memory: 4 bytes in and bits / 8 out per element.  8192 x 8192: to fp8 122 -> 50 us (6.7 TB/s), 16 bits
 // 129 -> 60, tf32 147 -> 82.
-template <int DT>
-__global__ void __launch_bounds__(kFillThreads) convert_kernel(void *dst, const float *src, uint64_t n8, uint64_t n)
+template <int DT, int SRC_ALIGN>
+__global__ void __launch_bounds__(kFillThreads) convert_kernel(void *dst, const float *src, Split part)
 {
     join_stream();
     constexpr int bits = Narrow<DT>::bits;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (uint64_t g = first; g < n8; g += stride) {
-        const Float8 x = ld_float8(src + 8 * g);
+    for (uint64_t g = first; g < part.whole; g += stride) {
+        const Float8 x = ld_float8<SRC_ALIGN>(src + 8 * g);
         constexpr int kWords = (8 * bits + 63) / 64;
         uint64_t w[kWords];
 #pragma unroll
@@ -211,20 +232,22 @@ __global__ void __launch_bounds__(kFillThreads) convert_kernel(void *dst, const 
         }
     }
     if constexpr (bits == 4) {
-        for (uint64_t i = 4 * n8 + first; i < n / 2; i += stride)
-            static_cast<uint8_t *>(dst)[i] = (uint8_t)(narrow<DT>(src[2 * i]) | (narrow<DT>(src[2 * i + 1]) << 4));
-    } else {
-        for (uint64_t i = 8 * n8 + first; i < n; i += stride) {
-            const uint64_t v = narrow<DT>(src[i]);
-            if constexpr (bits == 8)
-                static_cast<uint8_t *>(dst)[i] = (uint8_t)v;
-            else if constexpr (bits == 16)
-                static_cast<uint16_t *>(dst)[i] = (uint16_t)v;
-            else if constexpr (bits == 32)
-                static_cast<uint32_t *>(dst)[i] = (uint32_t)v;
-            else
-                static_cast<uint64_t *>(dst)[i] = v;
+        // two elements a byte: an even number of them, on both sides
+        if (part.has_single() && threadIdx.x % 2 == 0) {
+            const int64_t i = part.single(8);
+            static_cast<uint8_t *>(dst)[i / 2] = (uint8_t)(narrow<DT>(src[i]) | (narrow<DT>(src[i + 1]) << 4));
         }
+    } else if (part.has_single()) {
+        const int64_t i = part.single(8);
+        const uint64_t v = narrow<DT>(src[i]);
+        if constexpr (bits == 8)
+            static_cast<uint8_t *>(dst)[i] = (uint8_t)v;
+        else if constexpr (bits == 16)
+            static_cast<uint16_t *>(dst)[i] = (uint16_t)v;
+        else if constexpr (bits == 32)
+            static_cast<uint32_t *>(dst)[i] = (uint32_t)v;
+        else
+            static_cast<uint64_t *>(dst)[i] = v;
     }
 }
 
@@ -452,21 +475,29 @@ static bool aligned(const void *p, size_t bytes) { return ((uintptr_t)p % bytes)
 
 // One element at a time is bound by how fast CTAs start, whatever the type: 8192 x 8192 from an address 4 bytes off,
 // uniform 270 us, normal 292, int8 269, absmax 129; cut at the boundary 64, 161, 56 and 42, as from an aligned one.
-static Split split_at(const void *p, uint32_t align, uint32_t element, uint32_t per, uint64_t n)
+static Split split_at(const void *p, uint32_t align, uint32_t element_bits, uint32_t per, uint64_t n)
 {
-    const uint32_t head = (align - (uint32_t)((uintptr_t)p % align)) % align / element;
+    const uint32_t head = (align - (uint32_t)((uintptr_t)p % align)) % align * 8 / element_bits;
     if (head >= n)
         return {0, (uint32_t)n, (uint32_t)n};
     const uint64_t whole = (n - head) / per;
     return {whole, head, (uint32_t)(n - per * whole)};
 }
 
+// Cut where the destination is aligned; the source's alignment there picks the loads.  A warp's narrow loads find the rest
+// of their lines in L1, its narrow stores would be partial writes.  8192 x 8192 from a source 16 bytes off: to bf16
+// 58 us, fp8 49, as from an aligned one; 4 bytes off 72 and 67 (one element at a time, bound by the start of CTAs, 272).
 template <int DT>
 static int launch_convert(void *d_dst, const float *d_src, uint64_t n, cudaStream_t s)
 {
-    constexpr size_t dst_align = Narrow<DT>::bytes8 < 32 ? Narrow<DT>::bytes8 : 32;
-    const uint64_t n8 = aligned(d_src, 32) && aligned(d_dst, dst_align) ? n / 8 : 0;
-    return launch_behind(convert_kernel<DT>, "launch convert", fill_grid(n8 ? n8 : n), kFillThreads, 0, s, d_dst, d_src, n8, n);
+    constexpr uint32_t dst_align = Narrow<DT>::bytes8 < 32 ? Narrow<DT>::bytes8 : 32;
+    const Split part = split_at(d_dst, dst_align, Narrow<DT>::bits, 8, n);
+    void *dst = static_cast<uint8_t *>(d_dst) + (uint64_t)part.head * Narrow<DT>::bits / 8;
+    const float *src = d_src + part.head;
+    auto launch = [&](auto kernel) {
+        return launch_behind(kernel, "launch convert", fill_grid(part.whole), kFillThreads, 0, s, dst, src, part);
+    };
+    return aligned(src, 32) ? launch(convert_kernel<DT, 32>) : aligned(src, 16) ? launch(convert_kernel<DT, 16>) : launch(convert_kernel<DT, 4>);
 }
 
 template <int BLOCK, bool UE8M0>
@@ -493,7 +524,7 @@ int clpk_fill_f32(float *d_dst, uint64_t n, uint64_t seed, int dist, float mean,
     CLPK_REQUIRE(dist >= 0 && dist <= 2, "unknown distribution %d", dist);
     if (n == 0)
         return CLPK_OK;
-    const Split part = split_at(d_dst, 32, sizeof(float), 8, n);
+    const Split part = split_at(d_dst, 32, 32, 8, n);
     const uint64_t mixed = clpk_mix64(seed) + part.head;       // the generator's index is added to it
     d_dst += part.head;
     const unsigned grid = fill_grid(part.whole);
@@ -510,7 +541,7 @@ int clpk_fill_i8(int8_t *d_dst, uint64_t n, uint64_t seed, void *stream)
     CLPK_REQUIRE(d_dst || n == 0, "d_dst is NULL");
     if (n == 0)
         return CLPK_OK;
-    const Split part = split_at(d_dst, 16, 1, 16, n);
+    const Split part = split_at(d_dst, 16, 8, 16, n);
     return launch_behind(fill_i8_kernel, "launch fill_i8", fill_grid(part.whole), kFillThreads, 0, as_stream(stream), d_dst + part.head,
                          part, clpk_mix64(seed) + part.head);
 }
@@ -542,7 +573,7 @@ int clpk_absmax_f32(float *d_absmax, const float *d_src, uint64_t n, void *strea
 {
     CLPK_REQUIRE(d_absmax, "d_absmax is NULL");
     cudaStream_t s = as_stream(stream);
-    const Split part = split_at(d_src, 32, sizeof(float), 8, n);
+    const Split part = split_at(d_src, 32, 32, 8, n);
     // up to 32 Ki floats one CTA reads in the time that clearing the word would take
     if (n > 0 && n <= 32768 && d_src)
         return launch_behind(absmax_kernel<true>, "launch absmax", 1, kFillThreads, 0, s, d_absmax, d_src + part.head,

@@ -77,6 +77,29 @@ def test_absmax_at_every_offset(K, orc, cuda, n):
             assert float(out.item()) == 9.5, (offset, at)
 
 
+# bits of an element; the source's offset decides the loads (32, 16 or 4 bytes), the destination's where the array is cut
+@pytest.mark.parametrize("dtype,bits", [(N.DT_F16, 16), (N.DT_BF16, 16), (N.DT_E4M3, 8), (N.DT_E5M2, 8), (N.DT_I8, 8), (N.DT_TF32, 32),
+                                        (N.DT_F64, 64), (N.DT_E2M1, 4)])
+@pytest.mark.parametrize("n", [2, 8, 22, 2062])
+def test_convert_at_every_pair_of_offsets(K, orc, cuda, dtype, bits, n):
+    x = orc.fill_f32(n, 6, N.DIST_NORMAL, 0.0, 2.0)
+    want = x.astype(np.float64) if dtype == N.DT_F64 else orc.convert_f32(x, dtype)
+    want = np.ascontiguousarray(want).view(np.uint8).ravel()
+    unit, size = max(bits // 8, 1), n * bits // 8
+    src = cuda.empty(n + 16, dtype=cuda.float32, device="cuda")
+    for src_offset in range(9):
+        src.fill_(1e6)
+        src[src_offset:src_offset + n] = cuda.from_numpy(x).cuda()
+        for dst_offset in range(0, 32 // unit + 1):
+            first = unit * dst_offset
+            buf = cuda.full((first + size + 64,), 0x5A, dtype=cuda.uint8, device="cuda")
+            K.clpk_convert_f32(buf.data_ptr() + first, src.data_ptr() + 4 * src_offset, n, dtype, stream_ptr())
+            sync()
+            got = to_np(buf)
+            assert np.array_equal(got[first:first + size], want), (src_offset, dst_offset)
+            assert np.all(got[:first] == 0x5A) and np.all(got[first + size:] == 0x5A), "the conversion wrote outside its range"
+
+
 # cut at the first aligned address it is the same work; one element at a time took 1.8 to 4 times as long
 @pytest.mark.parametrize("dist", [0, 1, 2])
 def test_fill_is_as_fast_from_any_offset(K, cuda, dist):
@@ -95,3 +118,17 @@ def test_absmax_is_as_fast_from_any_offset(K, cuda, n):
     src, out = dev_empty(n + 8, cuda.float32), dev_empty(1, cuda.float32)
     src.zero_()
     assert_about_as_fast(cuda, lambda off: K.clpk_absmax_f32(out.data_ptr(), src.data_ptr() + 4 * off, n, stream_ptr()), (1, 4), 1.3)
+
+
+# the loads are narrower where source and destination are not aligned at once; one element at a time took 3 to 5 times as long
+@pytest.mark.parametrize("dtype,bits", [(N.DT_BF16, 16), (N.DT_E4M3, 8), (N.DT_TF32, 32), (N.DT_F64, 64), (N.DT_E2M1, 4)])
+def test_convert_is_nearly_as_fast_from_any_offset(K, cuda, dtype, bits):
+    src, dst = dev_empty(N_TIMED + 16, cuda.float32), dev_empty(N_TIMED * bits // 8 + 64, cuda.uint8)
+    src.zero_()
+    unit = max(bits // 8, 1)
+
+    def convert(offsets):
+        src_offset, dst_offset = offsets or (0, 0)
+        K.clpk_convert_f32(dst.data_ptr() + unit * dst_offset, src.data_ptr() + 4 * src_offset, N_TIMED, dtype, stream_ptr())
+
+    assert_about_as_fast(cuda, convert, ((1, 0), (4, 0), (0, 1), (3, 1)), 1.6)
