@@ -494,10 +494,12 @@ static int launch_convert(void *d_dst, const float *d_src, uint64_t n, cudaStrea
     const Split part = split_at(d_dst, dst_align, Narrow<DT>::bits, 8, n);
     void *dst = static_cast<uint8_t *>(d_dst) + (uint64_t)part.head * Narrow<DT>::bits / 8;
     const float *src = d_src + part.head;
-    auto launch = [&](auto kernel) {
-        return launch_behind(kernel, "launch convert", fill_grid(part.whole), kFillThreads, 0, s, dst, src, part);
-    };
-    return aligned(src, 32) ? launch(convert_kernel<DT, 32>) : aligned(src, 16) ? launch(convert_kernel<DT, 16>) : launch(convert_kernel<DT, 4>);
+    const unsigned grid = fill_grid(part.whole);
+    if (aligned(src, 32))
+        return launch_behind(convert_kernel<DT, 32>, "launch convert", grid, kFillThreads, 0, s, dst, src, part);
+    if (aligned(src, 16))
+        return launch_behind(convert_kernel<DT, 16>, "launch convert", grid, kFillThreads, 0, s, dst, src, part);
+    return launch_behind(convert_kernel<DT, 4>, "launch convert", grid, kFillThreads, 0, s, dst, src, part);
 }
 
 template <int BLOCK, bool UE8M0>
