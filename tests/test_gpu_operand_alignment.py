@@ -100,6 +100,30 @@ def test_convert_at_every_pair_of_offsets(K, orc, cuda, dtype, bits, n):
             assert np.all(got[:first] == 0x5A) and np.all(got[first + size:] == 0x5A), "the conversion wrote outside its range"
 
 
+BLOCK = {N.DT_MXF4: 32, N.DT_MXF4_B64: 64, N.DT_NVF4: 16, N.DT_NVF4_B32: 32}
+
+
+@pytest.mark.parametrize("dtype", list(BLOCK))
+@pytest.mark.parametrize("rows,cols", [(1, 64), (7, 192), (33, 320)])
+def test_quantize_at_every_pair_of_offsets(K, orc, cuda, dtype, rows, cols):
+    n, ts = rows * cols, 1.0 if dtype in (N.DT_MXF4, N.DT_MXF4_B64) else float(np.float32(2.5e-4))
+    x = orc.fill_f32(n, 6, N.DIST_NORMAL).reshape(rows, cols)
+    x[0, :64] = 0.0                                                 # a warp that takes the divisions
+    want_packed, want_scales = orc.quantize_fp4(x, dtype, ts)
+    src, scales = cuda.empty(n + 16, dtype=cuda.float32, device="cuda"), dev_empty(n // BLOCK[dtype], cuda.uint8)
+    for src_offset in range(9):
+        src.fill_(1e6)
+        src[src_offset:src_offset + n] = cuda.from_numpy(x.ravel()).cuda()
+        for first in range(9):
+            packed = cuda.full((first + n // 2 + 16,), 0x5A, dtype=cuda.uint8, device="cuda")
+            K.clpk_quantize_fp4(packed.data_ptr() + first, scales.data_ptr(), src.data_ptr() + 4 * src_offset, rows, cols, dtype, ts, stream_ptr())
+            sync()
+            got = to_np(packed)
+            assert_bits_equal(got[first:first + n // 2], want_packed.ravel(), "fp4 codes")
+            assert_bits_equal(to_np(scales), want_scales.ravel(), "fp4 scales")
+            assert np.all(got[:first] == 0x5A) and np.all(got[first + n // 2:] == 0x5A)
+
+
 # cut at the first aligned address it is the same work; one element at a time took 1.8 to 4 times as long
 @pytest.mark.parametrize("dist", [0, 1, 2])
 def test_fill_is_as_fast_from_any_offset(K, cuda, dist):
@@ -132,3 +156,17 @@ def test_convert_is_nearly_as_fast_from_any_offset(K, cuda, dtype, bits):
         K.clpk_convert_f32(dst.data_ptr() + unit * dst_offset, src.data_ptr() + 4 * src_offset, N_TIMED, dtype, stream_ptr())
 
     assert_about_as_fast(cuda, convert, ((1, 0), (4, 0), (0, 1), (3, 1)), 1.6)
+
+
+# narrower loads and stores (2.5 times at most); one thread per scale block, every quotient computed twice, took 5 to 12 times as long
+@pytest.mark.parametrize("dtype", list(BLOCK))
+def test_quantize_is_nearly_as_fast_from_any_offset(K, cuda, dtype):
+    src, packed, scales = dev_empty(N_TIMED + 16, cuda.float32), dev_empty(N_TIMED // 2 + 16, cuda.uint8), dev_empty(N_TIMED // 16, cuda.uint8)
+    K.clpk_fill_f32(src.data_ptr(), N_TIMED + 16, 3, N.DIST_NORMAL, 0.0, 0.02, stream_ptr())
+
+    def quantize(offsets):
+        src_offset, dst_offset = offsets or (0, 0)
+        K.clpk_quantize_fp4(packed.data_ptr() + dst_offset, scales.data_ptr(), src.data_ptr() + 4 * src_offset, 4096, N_TIMED // 4096, dtype, 2e-5,
+                            stream_ptr())
+
+    assert_about_as_fast(cuda, quantize, ((1, 0), (4, 0), (0, 4), (0, 1), (3, 1)), 3.5)
