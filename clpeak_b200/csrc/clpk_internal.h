@@ -30,6 +30,9 @@ int tuning(int knob);
 int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t m, uint32_t n, uint32_t k, float alpha,
                      uint32_t *status, cudaStream_t s);
 
+// clpk_gemm_plan of those two types
+void simt_gemm_plan(bool f64, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile_n, uint32_t *splits, uint32_t *wide);
+
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 } // namespace clpk

@@ -1159,6 +1159,33 @@ static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4)
     return plan;
 }
 
+// bits of an element of the tcgen05 kinds, 0 for anything else
+static uint32_t tensor_elem_bits(int dtype)
+{
+    switch (dtype) {
+    case CLPK_DT_BF16:
+    case CLPK_DT_F16:  return 16;
+    case CLPK_DT_TF32: return 32;
+    case CLPK_DT_E4M3:
+    case CLPK_DT_E5M2:
+    case CLPK_DT_I8:   return 8;
+    case CLPK_DT_MXF4:
+    case CLPK_DT_NVF4: return 4;
+    default:           return 0;
+    }
+}
+
+static uint32_t k_blocks_of(uint32_t k, uint32_t elem_bits) { return (uint32_t)(((uint64_t)k * elem_bits / 8 + kRowBytesK - 1) / kRowBytesK); }
+
+// What clpk_gemm does with a problem of a tcgen05 kind; the GEMM_FP4_TILE knob's forced tiles are the large kernel's.
+static TilesPlan gemm_plan(uint32_t m, uint32_t n, uint32_t k, uint32_t elem_bits)
+{
+    const bool fp4 = elem_bits == 4;
+    if (fp4 && tuning(CLPK_TUNE_GEMM_FP4_TILE) > 0)
+        return {0, 1};
+    return plan_tiles(m, n, k_blocks_of(k, elem_bits), fp4);
+}
+
 // wsa, wsb: the packed scale factors (block-scaled kinds)
 template <int DT>
 static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64_t row_bytes, uint32_t k_blocks, TilesPlan plan, cudaStream_t s,
@@ -1240,6 +1267,28 @@ static int launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, const CUten
 using namespace clpk;
 
 extern "C" {
+
+int clpk_gemm_plan(int dtype, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile_n, uint32_t *splits, uint32_t *wide)
+{
+    int rc = require_sm100();
+    if (rc != CLPK_OK)
+        return rc;
+    CLPK_REQUIRE(tile_n && splits, "NULL output");
+    CLPK_REQUIRE(m > 0 && n > 0 && k > 0, "M, N and K must be positive");
+    uint32_t no_wide = 0;
+    if (dtype == CLPK_DT_F32 || dtype == CLPK_DT_F64) {
+        simt_gemm_plan(dtype == CLPK_DT_F64, m, n, k, tile_n, splits, wide ? wide : &no_wide);
+        return CLPK_OK;
+    }
+    const uint32_t elem_bits = tensor_elem_bits(dtype);
+    CLPK_REQUIRE(elem_bits > 0, "clpk_gemm_plan: dtype %d has no GEMM", dtype);
+    const TilesPlan plan = gemm_plan(m, n, k, elem_bits);
+    *tile_n = plan.tn;
+    *splits = plan.splits;
+    if (wide)
+        *wide = 0;
+    return CLPK_OK;
+}
 
 int clpk_gemm_last_launch_aligned(void) { return g_last_aligned; }
 
@@ -1349,17 +1398,8 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
     CLPK_REQUIRE(!block_scaled || a->k % 256 == 0, "block-scaled FP4 needs K to be a multiple of 256 (got %u)", a->k);
     CLPK_REQUIRE(((uintptr_t)a->d_a % 16) == 0 && ((uintptr_t)a->d_b % 16) == 0 && ((uintptr_t)a->d_c % 16) == 0,
                  "operands must be 16-byte aligned");
-    uint32_t elem_bits;
-    switch (a->dtype) {
-    case CLPK_DT_BF16:
-    case CLPK_DT_F16:  elem_bits = 16; break;
-    case CLPK_DT_TF32: elem_bits = 32; break;
-    case CLPK_DT_E4M3:
-    case CLPK_DT_E5M2:
-    case CLPK_DT_I8:   elem_bits = 8; break;
-    case CLPK_DT_MXF4:
-    case CLPK_DT_NVF4: elem_bits = 4; break;
-    default:
+    const uint32_t elem_bits = tensor_elem_bits(a->dtype);
+    if (elem_bits == 0) {
         set_error("clpk_gemm: dtype %d is not available in this build", a->dtype);
         return CLPK_ERR_UNSUPPORTED;
     }
@@ -1383,7 +1423,7 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
     p.n = a->n;
     p.k = a->k;
     p.k_block_elems = kRowBytesK;          // x coordinate is in bytes: the maps are typed UINT8
-    p.k_blocks = (uint32_t)((row_bytes + kRowBytesK - 1) / kRowBytesK);
+    p.k_blocks = k_blocks_of(a->k, elem_bits);
     p.c = a->d_c;
     p.alpha = a->alpha;
     p.status = a->d_status;
@@ -1413,10 +1453,9 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
                 return rc;
         }
         const uint32_t tn = fp4_tile_n(a->m, a->n, a->k);
-        if (tuning(CLPK_TUNE_GEMM_FP4_TILE) <= 0)                // the knob's forced tiles are the large kernel's
-            if (const TilesPlan plan = plan_tiles(a->m, a->n, p.k_blocks, true); plan.tn)
-                return mx ? launch_tiles<CLPK_DT_MXF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb)
-                          : launch_tiles<CLPK_DT_NVF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb);
+        if (const TilesPlan plan = gemm_plan(a->m, a->n, a->k, elem_bits); plan.tn)
+            return mx ? launch_tiles<CLPK_DT_MXF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb)
+                      : launch_tiles<CLPK_DT_NVF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb);
         CUtensorMap tsa, tsb;
         rc = make_scale_map(&tsa, wsa, sfa_bytes / 512, words);
         if (rc != CLPK_OK)
@@ -1446,7 +1485,7 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
                   : launch_persistent(gemm_block_scaled_kernel<false, 256>, "gemm_nvf4", kNvGemmThreads,
                                       BlockScaled<false, 256>::smem_bytes, s, p, n_tiles, ta, tb, tsa, tsb, tc);
     }
-    if (const TilesPlan plan = plan_tiles(a->m, a->n, p.k_blocks, false); plan.tn) {
+    if (const TilesPlan plan = gemm_plan(a->m, a->n, a->k, elem_bits); plan.tn) {
         switch (a->dtype) {
         case CLPK_DT_BF16: return launch_tiles<CLPK_DT_BF16>(a, ta, row_bytes, p.k_blocks, plan, s);
         case CLPK_DT_F16:  return launch_tiles<CLPK_DT_F16>(a, ta, row_bytes, p.k_blocks, plan, s);

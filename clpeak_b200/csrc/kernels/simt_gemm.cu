@@ -762,6 +762,14 @@ static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
     return plan;
 }
 
+void simt_gemm_plan(bool f64, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile_n, uint32_t *splits, uint32_t *wide)
+{
+    const SimtPlan plan = plan_simt(f64, m, n, k);
+    *tile_n = plan.tile == 128 ? 0 : plan.tile;
+    *splits = plan.splits;
+    *wide = plan.wide ? 1 : 0;
+}
+
 int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t m, uint32_t n, uint32_t k, float alpha,
                      uint32_t *status, cudaStream_t s)
 {

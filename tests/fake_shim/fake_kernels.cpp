@@ -511,6 +511,14 @@ int clpk_dmma_peak(const double *a, const double *b, uint32_t n_mma, uint32_t gr
     return CLPK_OK;
 }
 
+int clpk_gemm_plan(int, uint32_t, uint32_t, uint32_t, uint32_t *tile_n, uint32_t *splits, uint32_t *wide)
+{
+    *tile_n = 0;
+    *splits = 1;
+    if (wide)
+        *wide = 0;
+    return CLPK_OK;
+}
 int clpk_gemm_last_launch_aligned(void) { return -1; }
 int clpk_gemm_last_clock(unsigned long long *c, unsigned long long *n, void *) { *c = 0; *n = 0; return CLPK_OK; }
 int clpk_set_tuning(int, int) { return CLPK_OK; }

@@ -50,3 +50,10 @@ def assert_floats_equal_nan_aware(got: np.ndarray, want: np.ndarray, what: str):
     if not same.all():
         bad = np.flatnonzero(~same)
         raise AssertionError(f"{what}: {bad.size} differing values, first at {bad[0]}: {g[bad[0]]!r} vs {w[bad[0]]!r}")
+
+
+def gemm_plan(K, dtype, m, n, k):
+    """(tile width or 0 for the large kernel, K ranges, twice the K groups) that clpk_gemm takes."""
+    out = [C.c_uint32(99) for _ in range(3)]
+    K.clpk_gemm_plan(dtype, m, n, k, *(C.byref(v) for v in out))
+    return tuple(v.value for v in out)

@@ -4,7 +4,7 @@ import ctypes as C
 import pytest
 
 from clpeak_b200 import native as N
-from tests.gpu_util import dev_empty, stream_ptr, sync
+from tests.gpu_util import dev_empty, gemm_plan, stream_ptr, sync
 from tests.test_gpu_gemm import make_nvfp4_operand
 
 pytestmark = pytest.mark.gpu
@@ -59,13 +59,36 @@ def decoded(cuda, dtype, q, sf, rows, k):
     return values * scale.view(rows, k // block).repeat_interleave(block, dim=1)
 
 
-# one stage; 64-wide tiles in both halves of a scale block, with ragged last tiles; K split in two and four with ranges
-# of unequal length; several tiles per CTA pair; the 256-wide split tile; the large kernel's whole tiles
+# one stage; 64-wide tiles in both halves of a scale block, with ragged last tiles; K split in four with ranges of unequal
+# length; several tiles per CTA pair; whole tiles (PLANS below names the tiles)
 @pytest.mark.parametrize("m,n,k", [(1, 8, 256), (64, 64, 256), (200, 200, 512), (384, 480, 256), (95, 352, 8960), (300, 136, 11008),
                                    (350, 416, 3328), (458, 1176, 6400), (2656, 120, 16384), (72, 1136, 13568), (8404, 216, 1024),
                                    (6976, 544, 5376), (512, 512, 2048)])
 @pytest.mark.parametrize("dtype", [N.DT_NVF4, N.DT_MXF4])
 def test_every_element(K, cuda, dtype, m, n, k):
+    check_every_element(K, cuda, dtype, m, n, k)
+
+
+# every tile with K whole, in two and in four: a 64-wide tile uses half of a block of B's scale factors, a 256-wide one
+# two blocks in one box, 48 tensor-memory columns and five stages; and several tiles per CTA pair
+PLANS = [(64, 1, 1, (33, 144, 256)), (128, 1, 1, (33, 5456, 768)), (64, 1, 2, (795, 2344, 256)), (128, 1, 2, (883, 4648, 256)),
+         (64, 2, 1, (33, 1072, 3072)), (128, 2, 1, (34, 2128, 5376)), (256, 2, 1, (34, 4808, 8448)), (256, 2, 1, (512, 2304, 8192)),
+         (64, 4, 1, (33, 128, 2816)), (128, 4, 1, (35, 1016, 5888)), (256, 4, 1, (33, 2136, 12288)), (256, 4, 1, (512, 1024, 16384)),
+         (0, 1, 1, (2048, 5000, 1024))]
+
+
+@pytest.mark.parametrize("tile_n,splits,tiles_per_pair,shape", PLANS)
+@pytest.mark.parametrize("dtype", [N.DT_NVF4, N.DT_MXF4])
+def test_every_plan(K, cuda, dtype, tile_n, splits, tiles_per_pair, shape):
+    m, n, k = shape
+    assert gemm_plan(K, dtype, m, n, k) == (tile_n, splits, 0)
+    if tile_n:
+        pairs = cuda.cuda.get_device_properties(0).multi_processor_count // 2
+        assert (splits == 1 and -(-m // 256) * -(-n // tile_n) > pairs) == (tiles_per_pair > 1)
+    check_every_element(K, cuda, dtype, m, n, k)
+
+
+def check_every_element(K, cuda, dtype, m, n, k):
     a, sfa, ta, _ = make_nvfp4_operand(K, cuda, m, k, 40, dtype)
     b, sfb, tb, _ = make_nvfp4_operand(K, cuda, n, k, 41, dtype)
     alpha, ws = ta * tb, workspace(K, cuda, dtype, m, n, k)
