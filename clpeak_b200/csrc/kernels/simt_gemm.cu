@@ -726,15 +726,51 @@ static int launch_simt(void (*kernel)(Params...), const char *what, uint64_t cta
 //   fp64  128 x 64   max(1.48, 1.24 L)    64 x 64  max(0.91, 0.62 L)    32 x 32  max(0.22, 0.17 L)    (1.08, 0.54, 0.13 L)
 // A CTA alone on its SM with a range of 32 blocks (fp32) or 24 (fp64) takes twice the K groups: 0.41 and 0.18 a block,
 // and 1.5 and 0.6 us more for the longer sum at the end (shorter ranges lose up to 20 % by it, long ones gain up to 33 %).
-// The large tiles are kept unless the estimate is 8 % better; a K range has at least four blocks.
+// The large tiles are kept unless the estimate is 8 % better; a K range has at least four blocks.  Short fp64 sums have an
+// estimate of their own (plan_short_f64).
 struct SimtPlan {
     uint32_t tile, splits;
     bool wide;                  // twice the K groups
 };
 
+// fp64 with fewer than 24 blocks: what a CTA costs besides them -- start, pipeline fill, sum, stores -- is then a good part
+// of its time.  Small tiles pay it once per round of the CTAs that an SM holds (4 of 64 x 64, 3 of 32 x 32), the large
+// kernel, whose odd rows of C are stored in 8-byte pieces, with every CTA.  Fitted to 490 shapes with K from 2 to 368
+// (residuals 10, 6 and 7 %; the chosen plans are 1 % slower than the fastest in the geometric mean, where the estimate
+// above was 10 % slower and 2.7 times at worst: 4153 x 558 x 6 took 23.5 us in 32 x 32 tiles against 9.3 in the large
+// ones, 12879 x 166 x 12 23.9 against 9.9, 963 x 955 x 248 35.9 against 24.3 in 64 x 64 ones).
+static SimtPlan plan_short_f64(uint32_t m, uint32_t n, uint32_t blocks)
+{
+    auto per_sm = [&](uint32_t rows, uint32_t cols, uint32_t splits) {
+        return (uint32_t)(((uint64_t)((m - 1) / rows + 1) * ((n - 1) / cols + 1) * splits - 1) / simt_capacity(splits) + 1);
+    };
+    // `held` CTAs at a time, `alone` us for one by itself and `shared` for each of several
+    auto rounds = [](uint32_t ctas, uint32_t held, float alone, float shared) {
+        auto round = [&](uint32_t c) { return c == 0 ? 0.0f : alone > c * shared ? alone : c * shared; };
+        return (float)(ctas / held) * round(held) + round(ctas % held);
+    };
+    SimtPlan plan = {128, 1, false};
+    const uint32_t large = per_sm(128, 64, 1);
+    float best = (large > 1 ? 0.90f : 0.95f) * (1.2f + (float)large * (1.45f * (float)blocks + 1.57f + (n % 2 ? 1.32f : 0.0f)));
+    for (uint32_t splits = 1; splits <= 4 && (splits == 1 || blocks >= 4 * splits); splits *= 2)
+        for (uint32_t tile = 32; tile <= 64; tile *= 2) {
+            const uint32_t ctas = per_sm(tile, tile, splits);
+            const float range = (float)((blocks - 1) / splits + 1);
+            const float t = tile == 64 ? 3.4f + rounds(ctas, 4, 0.92f * range + 1.54f, 0.60f * range + 1.05f)
+                                       : 2.0f + rounds(ctas, 3, 0.254f * range + 1.67f, 0.18f * range + 1.12f) + (splits > 1 ? 0.29f * splits : 0.0f);
+            if (t < best) {
+                best = t;
+                plan = {tile, splits, false};
+            }
+        }
+    return plan;
+}
+
 static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
 {
     const uint32_t blocks = (k - 1) / kSimtBK + 1;
+    if (f64 && blocks < 24)
+        return plan_short_f64(m, n, blocks);
     auto ctas = [&](uint32_t rows, uint32_t cols, uint32_t splits) { return (uint64_t)((m - 1) / rows + 1) * ((n - 1) / cols + 1) * splits; };
     auto estimate = [&](uint32_t rows, uint32_t cols, uint32_t splits, float alone, float shared) {
         const float busiest = shared * (float)((ctas(rows, cols, splits) - 1) / simt_capacity(splits) + 1);

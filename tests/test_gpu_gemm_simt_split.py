@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from clpeak_b200 import native as N
-from tests.gpu_util import dev_empty, stream_ptr, sync
+from tests.gpu_util import dev_empty, gemm_plan, stream_ptr, sync
 
 pytestmark = pytest.mark.gpu
 
@@ -21,12 +21,39 @@ def operand(K, cuda, dtype, rows, k, seed):
 
 
 # fewer k blocks than groups and ranks could take; ranges and groups of unequal length; ragged tiles in both directions;
-# N odd (no vector store); one and several CTAs per SM; the large tiles' side of the rule
+# N odd (no vector store); one and several CTAs per SM
 @pytest.mark.parametrize("m,n,k", [(1, 1, 4), (33, 65, 20), (64, 64, 16384), (129, 131, 36), (131, 102, 7688), (201, 73, 2828), (863, 251, 2456),
                                    (1315, 363, 956), (440, 434, 520), (64, 868, 1036), (719, 366, 688), (459, 349, 4636), (3720, 110, 596),
                                    (2254, 496, 464), (1024, 1024, 512), (97, 106, 5732), (719, 368, 6380), (64, 64, 4100)])
 @pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F64])
 def test_every_element(K, cuda, dtype, m, n, k):
+    check_every_element(K, cuda, dtype, m, n, k)
+
+
+# (tile, K ranges, twice the K groups) and a shape that takes them
+PLANS = [(N.DT_F32, (0, 1, 0), (1135, 1699, 36)), (N.DT_F32, (64, 1, 0), (52, 36, 64)), (N.DT_F32, (64, 2, 0), (42, 58, 128)),
+         (N.DT_F32, (64, 4, 0), (127, 33, 256)), (N.DT_F32, (64, 8, 0), (94, 36, 512)), (N.DT_F32, (64, 8, 1), (64, 64, 16384)),
+         (N.DT_F64, (32, 1, 0), (47, 70, 64)), (N.DT_F64, (32, 1, 1), (2287, 33, 512)), (N.DT_F64, (32, 4, 0), (68, 61, 512)),
+         (N.DT_F64, (32, 8, 1), (64, 64, 16384)), (N.DT_F64, (64, 8, 0), (130, 197, 512))]
+
+
+@pytest.mark.parametrize("dtype,plan,shape", PLANS)
+def test_every_plan(K, cuda, dtype, plan, shape):
+    assert gemm_plan(K, dtype, *shape) == plan
+    check_every_element(K, cuda, dtype, *shape)
+
+
+# short fp64 sums: shapes that 32-wide tiles made 1.1 to 2.5 times slower than the large ones take those or 64-wide ones,
+# an odd N also in more CTAs than run at once, and shapes that small tiles serve best keep them
+@pytest.mark.parametrize("tile,shape", [(0, (4153, 558, 6)), (0, (2888, 782, 2)), (0, (12879, 166, 12)), (0, (11657, 120, 14)), (64, (394, 15109, 38)),
+                                        (64, (963, 955, 248)), (0, (12127, 1916, 10)), (64, (1674, 807, 4)), (32, (863, 251, 248)), (32, (64, 64, 128)),
+                                        (64, (661, 6775, 24)), (32, (1481, 215, 40))])
+def test_short_fp64_sums(K, cuda, tile, shape):
+    assert gemm_plan(K, N.DT_F64, *shape)[0] == tile
+    check_every_element(K, cuda, N.DT_F64, *shape)
+
+
+def check_every_element(K, cuda, dtype, m, n, k):
     a, b = operand(K, cuda, dtype, m, k, 40), operand(K, cuda, dtype, n, k, 41)
     alpha, results = 0.75, []
     for _ in range(2):
