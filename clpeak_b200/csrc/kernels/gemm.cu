@@ -1119,7 +1119,10 @@ struct TilesPlan {
 //   gemm_tiles_kernel, FP4    3.3 + waves * (K blocks * (0.25 + 0.06 W + T at 62 TB/s) + 1.4 W) and the same exchange
 // Splits of 2 and 4 are clusters of 4 and 8 CTAs, of which the chip holds 33 and 15 at a time.  From the fifth wave of
 // 512 x 256 tiles on (16384 x 16384 x 256: 140 against 142 us) and the third of block-scaled ones the large tiles'
-// smaller operand traffic wins at every K; an FP4 tile 256 wide that is not split is the large kernel's own.
+// smaller operand traffic wins at every K; an FP4 tile 256 wide that is not split is the large kernel's own.  An FP4 A of a few
+// rows, whose lines more than half the pairs ask for at once, costs them 0.04 a block more, up to eight rows 0.15 (mxf4
+// 9 x 9336 x 14592: 32 us in 128-wide tiles, 26 in large ones; of 1400 shapes with few rows 87 were more than 3 % slower
+// than in large tiles, at worst 1.31 times, and with the term 14, at worst 1.09).
 static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4)
 {
     const uint32_t pairs = (uint32_t)num_sms() / 2;
@@ -1146,7 +1149,9 @@ static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4)
         for (uint32_t tn = fp4 ? 64 : 32; tn <= (fp4 && splits == 1 ? 128u : 256u); tn = fp4 ? 2 * tn : tn + 32) {
             const uint64_t tiles = (uint64_t)ceil_div(m, kTilesM) * ceil_div(n, tn);
             const float waves = (float)((tiles - 1) / resident + 1), wide = (float)tn / 256.0f;
-            const float block = issue + wide_issue * wide + fetched(tiles < resident ? tiles : resident, splits, tn) / rate;
+            float block = issue + wide_issue * wide + fetched(tiles < resident ? tiles : resident, splits, tn) / rate;
+            if (fp4 && splits == 1 && m <= 48 && tiles > pairs / 2)
+                block += m <= 8 ? 0.15f : 0.04f;
             float t = launch + waves * (ceil_div(k_blocks, splits) * block + drain * wide);
             if (splits > 1)
                 t += waves * (1.0f + 4.3f * wide * (splits - 1) / splits);

@@ -88,6 +88,15 @@ def test_every_plan(K, cuda, dtype, tile_n, splits, tiles_per_pair, shape):
     check_every_element(K, cuda, dtype, m, n, k)
 
 
+# an A of a few rows and tiles for most of the chip: many pairs asking for the same lines made small tiles up to 1.3 times
+# slower than the large kernel's; half the pairs, or more rows, and they are faster
+@pytest.mark.parametrize("tile_n,shape", [(0, (9, 9336, 14592)), (0, (1, 9128, 12032)), (0, (28, 6680, 4352)), (128, (2, 4456, 3328)),
+                                          (128, (64, 6680, 4352)), (64, (9, 1024, 1536))])
+def test_operands_of_a_few_rows(K, cuda, tile_n, shape):
+    assert gemm_plan(K, N.DT_NVF4, *shape)[0] == tile_n
+    check_every_element(K, cuda, N.DT_NVF4, *shape)
+
+
 def check_every_element(K, cuda, dtype, m, n, k):
     a, sfa, ta, _ = make_nvfp4_operand(K, cuda, m, k, 40, dtype)
     b, sfb, tb, _ = make_nvfp4_operand(K, cuda, n, k, 41, dtype)
