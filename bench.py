@@ -7,8 +7,12 @@ algorithmic HBM traffic per step.  `value` is whole-job GB/s with the buffers
 resident in HBM; `e2e` is the same three kernels driven through the C ABI from
 pinned HOST buffers (H2D of b and c and a D2H of the read checksum inside the
 timed region).  The tensor-core and GEMM rows of the same backend are measured
-after the timed region and reported under "rows" (they explain the headline
+after the timed region and reported as "rows" of the details (they explain the headline
 metric's "TFLOPS/TOPS per dtype" part; each carries its own roofline fraction).
+
+Standard output is one short JSON line with the headline numbers; the rows, the plugin call and the baselines' own
+rows are one JSON line on standard error (and in a file, with --details): all in one line they were 25 KB, of which
+whoever keeps the end of an output has no headline.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
@@ -372,6 +376,21 @@ def reference_arm(args):
 # our arm
 # ---------------------------------------------------------------------------------
 
+DETAIL_KEYS = ("rows", "e2e_plugin", "spec_peaks_per_gpu")
+DETAIL_BASELINE_KEYS = ("rows", "other_reference_cpu_rows", "reference_cuda_kernels_on_this_gpu")
+
+
+def split_line(line):
+    """(the headline's line, everything that explains it)"""
+    headline = {k: v for k, v in line.items() if k not in DETAIL_KEYS}
+    details = {k: line[k] for k in DETAIL_KEYS if k in line}
+    if headline.get("cpu_baseline"):
+        base = headline["cpu_baseline"]
+        headline["cpu_baseline"] = {k: v for k, v in base.items() if k not in DETAIL_BASELINE_KEYS}
+        details["cpu_baseline"] = {k: base[k] for k in DETAIL_BASELINE_KEYS if k in base}
+    return headline, details
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -381,6 +400,7 @@ def main():
     ap.add_argument("--size-gib", type=float, default=8.0, help="bytes per array (default: the 8 GiB of the config)")
     ap.add_argument("--no-rows", action="store_true", help="skip the tensor-core / GEMM rows")
     ap.add_argument("--no-e2e", action="store_true")
+    ap.add_argument("--details", metavar="FILE", help="also write the details to this file")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3) if args.impl == "ours" else args.warmup
     if args.impl == "reference":
@@ -634,7 +654,11 @@ def main():
         "e2e": e2e, "e2e_plugin": plugin, "gpu_launches": 3 * args.steps, "clocks": clocks, "read_checksum": read_xor, "verified_at_full_size": checks,
         "rows": rows, "spec_peaks_per_gpu": SPEC,
     }
-    print(json.dumps(line), flush=True)
+    headline, details = split_line(line)
+    print(json.dumps({"details": details}), file=sys.stderr, flush=True)
+    if args.details:
+        Path(args.details).write_text(json.dumps(details))
+    print(json.dumps(headline), flush=True)
     reps.close()
     return 0
 
