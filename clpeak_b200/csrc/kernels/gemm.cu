@@ -348,6 +348,8 @@ __device__ __forceinline__ void drain_warp_tile_early(uint32_t taddr0, uint32_t 
 // the launch that gets it next (leave_wave_sync).  A cooperative launch behind two clearing operations, the first form
 // of this, cost about 5 us a GEMM: e4m3 8192 x 8192 x 512 40.3 -> 35.8 us, x 1024 67 -> 62, bf16 x 1024 113 -> 105, NVFP4
 // 16384 x 16384 x 1024 196 -> 170, back to back.
+__device__ unsigned int g_wave_dropouts;       // producers that have stopped taking part since the library was loaded
+
 __device__ __forceinline__ void wave_align(const GemmParams &p, uint32_t wave, uint32_t n_tiles, uint32_t n_clusters,
                                            bool &enabled)
 {
@@ -369,6 +371,7 @@ __device__ __forceinline__ void wave_align(const GemmParams &p, uint32_t wave, u
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
         if (t1 - t0 > 40000ull) {
             enabled = false;
+            atomicAdd(&g_wave_dropouts, 1u);
             return;
         }
         __nanosleep(64);
@@ -1057,11 +1060,12 @@ static int make_scale_map_b(CUtensorMap *map, const void *base, uint64_t n_rows,
 constexpr size_t kGemmSmemBytes = (size_t)kDenseStages * kDenseStageBytes + kEpilogueWarps * kStagingBytes + sizeof(DenseSmem) + 1024;
 
 // One pair of wave counters per launch, from a ring of 32 per device so that launches on different streams do not share
-// one; zero between launches.  The slot index comes from one process-wide counter, so a slot is handed out again 32
-// launches later: with more than 32 aligned GEMMs in flight at once on one device (across streams) two running kernels
-// would share a slot.  That costs alignment, not correctness -- a producer that does not see its wave complete within
-// 40 us stops taking part, and the slot is zero again when both have ended -- but callers that want the alignment keep
-// at most 32 in flight.
+// one; zero between launches.  The slot is chosen by the host, from one process-wide index: 32 launches later, on whatever
+// device, it is handed out again, and a launch captured in a graph keeps its slot for every replay.  So two running
+// kernels can share a slot -- eager launches only with more than 32 of them in flight, a replay with any other launch.
+// That costs alignment, not correctness: whoever does not see its wave complete within 40 us stops taking part, a wave
+// that is counted too soon runs unaligned, and the slot is zero again when all its kernels have ended (every CTA arrives
+// before it leaves, and the grids of a device are all the same size, so the last CTA of all clears it).
 constexpr int kSyncSlots = 32;
 __device__ unsigned int g_wave_sync[kSyncSlots][2];
 static std::atomic<unsigned> g_next_sync_slot{0};
@@ -1296,6 +1300,23 @@ int clpk_gemm_plan(int dtype, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile
 }
 
 int clpk_gemm_last_launch_aligned(void) { return g_last_aligned; }
+
+int clpk_gemm_wave_state(uint32_t *h_counters_set, uint32_t *h_dropouts, void *stream)
+{
+    CLPK_REQUIRE(h_counters_set && h_dropouts, "NULL output");
+    unsigned int counters[kSyncSlots][2], dropouts = 0;
+    void *sym = nullptr;
+    CLPK_CUDA(cudaGetSymbolAddress(&sym, g_wave_sync));
+    CLPK_CUDA(cudaMemcpyAsync(counters, sym, sizeof counters, cudaMemcpyDeviceToHost, as_stream(stream)));
+    CLPK_CUDA(cudaGetSymbolAddress(&sym, g_wave_dropouts));
+    CLPK_CUDA(cudaMemcpyAsync(&dropouts, sym, sizeof dropouts, cudaMemcpyDeviceToHost, as_stream(stream)));
+    CLPK_CUDA(cudaStreamSynchronize(as_stream(stream)));
+    *h_counters_set = 0;
+    for (const auto &slot : counters)
+        *h_counters_set += (slot[0] != 0) + (slot[1] != 0);
+    *h_dropouts = dropouts;
+    return CLPK_OK;
+}
 
 int clpk_gemm_last_clock(unsigned long long *h_cycles, unsigned long long *h_ns, void *stream)
 {

@@ -141,6 +141,7 @@ KERNEL_API = {
     "clpk_gemm_pack_scales": [C.POINTER(GemmArgs), _vp],
     "clpk_gemm_plan": [_i, _u32, _u32, _u32, C.POINTER(_u32), C.POINTER(_u32), C.POINTER(_u32)],
     "clpk_gemm_last_launch_aligned": [],
+    "clpk_gemm_wave_state": [C.POINTER(_u32), C.POINTER(_u32), _vp],
     "clpk_gemm_last_clock": [C.POINTER(C.c_ulonglong), C.POINTER(C.c_ulonglong), _vp],
     "clpk_set_tuning": [_i, _i],
     "clpk_get_tuning": [_i, C.POINTER(_i)],

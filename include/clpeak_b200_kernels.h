@@ -454,6 +454,10 @@ CLPK_API int clpk_gemm_plan(int dtype, uint32_t m, uint32_t n, uint32_t k, uint3
 /* 1 if the calling thread's last clpk_gemm launch ran with the per-wave producer meeting, 0 if
  * it ran without (small problem, knob), -1 before any launch.  Lets a benchmark record which schedule it timed. */
 CLPK_API int clpk_gemm_last_launch_aligned(void);
+/* The state of those meetings on the current device: how many of the counters are not zero (none, while no GEMM runs)
+ * and how many producers have given up waiting for the others since the library was loaded (none, while every GEMM has
+ * the chip to itself).  Waits for `stream`. */
+CLPK_API int clpk_gemm_wave_state(uint32_t *h_counters_set, uint32_t *h_dropouts, void *stream);
 /* SM cycles (clock64) and nanoseconds (%globaltimer) that CTA 0 of the last tensor-core GEMM
  * launched on the current device ran for; cycles / ns is the SM clock the kernel really had, which
  * under the power cap is well below the nominal one.  Waits for `stream`.  The fp32 / fp64 kernels

@@ -520,6 +520,7 @@ int clpk_gemm_plan(int, uint32_t, uint32_t, uint32_t, uint32_t *tile_n, uint32_t
     return CLPK_OK;
 }
 int clpk_gemm_last_launch_aligned(void) { return -1; }
+int clpk_gemm_wave_state(uint32_t *set, uint32_t *dropouts, void *) { *set = 0; *dropouts = 0; return CLPK_OK; }
 int clpk_gemm_last_clock(unsigned long long *c, unsigned long long *n, void *) { *c = 0; *n = 0; return CLPK_OK; }
 int clpk_set_tuning(int, int) { return CLPK_OK; }
 int clpk_get_tuning(int, int *value) { if (value) *value = -1; return CLPK_OK; }

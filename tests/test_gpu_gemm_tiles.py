@@ -99,7 +99,7 @@ def test_plans_that_no_kernel_takes_are_refused(K):
 
 def test_aligned_launches_on_two_streams(K, cuda):
     """GEMMs whose producers meet once per wave, back to back on two streams and over more launches than there are wave
-    counters: whoever holds the SMs, the bits are those of a launch by itself, and the counters serve the next launch."""
+    counters: whoever holds the SMs, the bits are those of a launch by itself, and the counters are zero again."""
     m, n, k = 8192, 8192, 256
     d_a, d_b = make_gemm_operands(K, cuda, N.DT_BF16, m, n, k)
     want = run_into(K, cuda, N.DT_BF16, m, n, k, d_a, d_b, 1.0).clone()
@@ -116,14 +116,28 @@ def test_aligned_launches_on_two_streams(K, cuda):
     sync()
     for c, st in zip(out, status):
         assert int(st.item()) == 0 and bool((c == want).all())
-    # a counter that had not come back to zero would let the producers pass unmet or make them wait 40 us a wave
-    e0, e1 = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
-    times = []
+    assert wave_state(K)[0] == 0, "a counter did not come back to zero"
+
+
+def wave_state(K):
+    counters_set, dropouts = C.c_uint32(99), C.c_uint32(99)
+    K.clpk_gemm_wave_state(C.byref(counters_set), C.byref(dropouts), stream_ptr())
+    return counters_set.value, dropouts.value
+
+
+def test_producers_meet_and_leave_the_counters_at_zero(K, cuda):
+    """More launches than there are counters, each with the chip to itself: no producer gives up waiting for the others, and
+    after each launch every counter is zero again -- one left above zero would let the producers of the launch that gets
+    it next pass unmet, which no result shows."""
+    m, n, k = 8192, 8192, 256
+    d_a, d_b = make_gemm_operands(K, cuda, N.DT_BF16, m, n, k)
+    c, status = dev_empty(m * n, cuda.int16), dev_empty(1, cuda.int32)
+    args = N.GemmArgs(dtype=N.DT_BF16, m=m, n=n, k=k, d_a=d_a.data_ptr(), d_b=d_b.data_ptr(), d_c=c.data_ptr(), alpha=1.0,
+                      d_status=status.data_ptr())
+    sync()
+    before = wave_state(K)
+    assert before[0] == 0
     for _ in range(40):
-        e0.record()
         K.clpk_gemm(C.byref(args), stream_ptr())
-        e1.record()
-        sync()
-        times.append(e0.elapsed_time(e1))
-    assert sorted(times)[20] < 4 * sorted(times)[0], times
-    assert bool((out[1] == want).all())
+        assert K.raw("clpk_gemm_last_launch_aligned")() == 1
+        assert wave_state(K) == before
