@@ -1126,8 +1126,10 @@ struct TilesPlan {
 // smaller operand traffic wins at every K; an FP4 tile 256 wide that is not split is the large kernel's own.  An FP4 A of a few
 // rows, whose lines more than half the pairs ask for at once, costs them 0.04 a block more, up to eight rows 0.15 (mxf4
 // 9 x 9336 x 14592: 32 us in 128-wide tiles, 26 in large ones; of 1400 shapes with few rows 87 were more than 3 % slower
-// than in large tiles, at worst 1.31 times, and with the term 14, at worst 1.09).
-static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4)
+// than in large tiles, at worst 1.31 times, and with the term 17, at worst 1.10).  Behind the launch that arranges the
+// scales it does not show (nvf4 5 x 5632 x 3840: 11.1 us in 128-wide tiles, 14.0 in large ones), so `arranged`: FP4 whose
+// scales lie in the workspace already.
+static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4, bool arranged)
 {
     const uint32_t pairs = (uint32_t)num_sms() / 2;
     auto ceil_div = [](uint32_t a, uint32_t b) { return (a - 1) / b + 1; };
@@ -1154,7 +1156,7 @@ static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4)
             const uint64_t tiles = (uint64_t)ceil_div(m, kTilesM) * ceil_div(n, tn);
             const float waves = (float)((tiles - 1) / resident + 1), wide = (float)tn / 256.0f;
             float block = issue + wide_issue * wide + fetched(tiles < resident ? tiles : resident, splits, tn) / rate;
-            if (fp4 && splits == 1 && m <= 48 && tiles > pairs / 2)
+            if (arranged && splits == 1 && m <= 48 && tiles > pairs * 40 / 74)
                 block += m <= 8 ? 0.15f : 0.04f;
             float t = launch + waves * (ceil_div(k_blocks, splits) * block + drain * wide);
             if (splits > 1)
@@ -1187,12 +1189,12 @@ static uint32_t tensor_elem_bits(int dtype)
 static uint32_t k_blocks_of(uint32_t k, uint32_t elem_bits) { return (uint32_t)(((uint64_t)k * elem_bits / 8 + kRowBytesK - 1) / kRowBytesK); }
 
 // What clpk_gemm does with a problem of a tcgen05 kind; the GEMM_FP4_TILE knob's forced tiles are the large kernel's.
-static TilesPlan gemm_plan(uint32_t m, uint32_t n, uint32_t k, uint32_t elem_bits)
+static TilesPlan gemm_plan(uint32_t m, uint32_t n, uint32_t k, uint32_t elem_bits, bool arranged)
 {
     const bool fp4 = elem_bits == 4;
     if (fp4 && tuning(CLPK_TUNE_GEMM_FP4_TILE) > 0)
         return {0, 1};
-    return plan_tiles(m, n, k_blocks_of(k, elem_bits), fp4);
+    return plan_tiles(m, n, k_blocks_of(k, elem_bits), fp4, arranged);
 }
 
 // wsa, wsb: the packed scale factors (block-scaled kinds)
@@ -1291,7 +1293,7 @@ int clpk_gemm_plan(int dtype, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile
     }
     const uint32_t elem_bits = tensor_elem_bits(dtype);
     CLPK_REQUIRE(elem_bits > 0, "clpk_gemm_plan: dtype %d has no GEMM", dtype);
-    const TilesPlan plan = gemm_plan(m, n, k, elem_bits);
+    const TilesPlan plan = gemm_plan(m, n, k, elem_bits, elem_bits == 4);
     *tile_n = plan.tn;
     *splits = plan.splits;
     if (wide)
@@ -1479,7 +1481,7 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
                 return rc;
         }
         const uint32_t tn = fp4_tile_n(a->m, a->n, a->k);
-        if (const TilesPlan plan = gemm_plan(a->m, a->n, a->k, elem_bits); plan.tn)
+        if (const TilesPlan plan = gemm_plan(a->m, a->n, a->k, elem_bits, a->d_sfa == nullptr); plan.tn)
             return mx ? launch_tiles<CLPK_DT_MXF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb)
                       : launch_tiles<CLPK_DT_NVF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb);
         CUtensorMap tsa, tsb;
@@ -1511,7 +1513,7 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
                   : launch_persistent(gemm_block_scaled_kernel<false, 256>, "gemm_nvf4", kNvGemmThreads,
                                       BlockScaled<false, 256>::smem_bytes, s, p, n_tiles, ta, tb, tsa, tsb, tc);
     }
-    if (const TilesPlan plan = gemm_plan(a->m, a->n, a->k, elem_bits); plan.tn) {
+    if (const TilesPlan plan = gemm_plan(a->m, a->n, a->k, elem_bits, false); plan.tn) {
         switch (a->dtype) {
         case CLPK_DT_BF16: return launch_tiles<CLPK_DT_BF16>(a, ta, row_bytes, p.k_blocks, plan, s);
         case CLPK_DT_F16:  return launch_tiles<CLPK_DT_F16>(a, ta, row_bytes, p.k_blocks, plan, s);
