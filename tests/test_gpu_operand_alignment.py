@@ -8,28 +8,24 @@ from tests.gpu_util import assert_bits_equal, dev_empty, stream_ptr, sync, to_np
 pytestmark = pytest.mark.gpu
 
 
-def best_us(cuda, fn, rounds=25, calls=4):
-    for _ in range(3):
-        fn()
-    sync()
-    times = []
+def assert_about_as_fast(cuda, at_offset, offsets, factor, rounds=25, calls=4):
+    """Best of many bursts on both sides, taken in turn: what else the machine does only adds time, and rarely to all of
+    one side's."""
+    best = {}
+    for off in (0, *offsets):
+        for _ in range(3):
+            at_offset(off)
     for _ in range(rounds):
-        e0, e1 = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
-        e0.record()
-        for _ in range(calls):
-            fn()
-        e1.record()
-        sync()
-        times.append(e0.elapsed_time(e1) * 1e3 / calls)
-    return min(times)
-
-
-def assert_about_as_fast(cuda, at_offset, offsets, factor):
-    """Best of many bursts on both sides: what else the machine does only adds time, and rarely to all of them."""
-    base = best_us(cuda, lambda: at_offset(0))
-    for off in offsets:
-        t = best_us(cuda, lambda: at_offset(off))
-        assert t < factor * base, f"{t:.1f} us at an offset of {off} elements, {base:.1f} at none"
+        for off in (0, *offsets):
+            e0, e1 = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(calls):
+                at_offset(off)
+            e1.record()
+            sync()
+            best[off] = min(best.get(off, 1e9), e0.elapsed_time(e1) * 1e3 / calls)
+    slow = {off: us for off, us in best.items() if us >= factor * best[0]}
+    assert not slow, f"us at these offsets: {slow}; {best[0]:.1f} at none"
 
 
 N_TIMED = 8192 * 4096              # two to three times the L2 in floats
@@ -136,12 +132,14 @@ def test_fill_i8_is_as_fast_from_any_offset(K, cuda):
     assert_about_as_fast(cuda, lambda off: K.clpk_fill_i8(d.data_ptr() + off, N_TIMED, 3, stream_ptr()), (1, 8), 1.3)
 
 
-# a small array is one CTA's, which took twice the time over one element per thread and step; a large one 1.2 to 3 times
-@pytest.mark.parametrize("n", [32768, N_TIMED])
-def test_absmax_is_as_fast_from_any_offset(K, cuda, n):
+# a small array is one CTA's, which took five times the time (a burst of launches as fast as the host issues them, so with
+# more room than the others); a large one took three times
+@pytest.mark.parametrize("n,factor", [(32768, 2.5), (N_TIMED, 1.3)])
+def test_absmax_is_as_fast_from_any_offset(K, cuda, n, factor):
     src, out = dev_empty(n + 8, cuda.float32), dev_empty(1, cuda.float32)
     src.zero_()
-    assert_about_as_fast(cuda, lambda off: K.clpk_absmax_f32(out.data_ptr(), src.data_ptr() + 4 * off, n, stream_ptr()), (1, 4), 1.3)
+    assert_about_as_fast(cuda, lambda off: K.clpk_absmax_f32(out.data_ptr(), src.data_ptr() + 4 * off, n, stream_ptr()), (1, 4), factor,
+                         calls=40 if n < N_TIMED else 4)
 
 
 # the loads are narrower where source and destination are not aligned at once; one element at a time took 3 to 5 times as long
