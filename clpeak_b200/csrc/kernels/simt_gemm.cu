@@ -36,7 +36,7 @@
 //
 // Shapes of which those tiles make too few CTAs take 64 x 64 (fp32, fp64) or 32 x 32 (fp64) tiles with K split over the
 // CTAs of a cluster and over groups of warps inside a CTA (sgemm64_kernel, dgemm_split_kernel; plan_simt has the rule).
-// Device time before -> after: fp32 64 x 64 x 16384 1545 -> 57 us, 459 x 349 x 4636 474 -> 68; fp64
+// Device time before -> after: fp32 64 x 64 x 16384 1545 -> 57 us, 459 x 349 x 4636 474 -> 69; fp64
 // 64 x 64 x 16384 1388 -> 26, 863 x 251 x 2456 228 -> 42, 2048 x 2048 x 512 151 -> 143.
 //
 // All take any M, N > 0 and any K that keeps operand rows 16-byte aligned (a multiple of 4
