@@ -886,7 +886,8 @@ def measure_rows(K, N, torch, stream, time_once, world=1, clocked=None, all_rank
                                 "rate_at_max_clock_T(FL)OPS": (per_ms / sms_ms * 1965.0 / true_mhz) if true_mhz else None}
         rows[f"mma_{name}"] = row
 
-    # the reference's fp32 and fp64 GEMM rows (CUDA cores / DMMA), 8192^3, with the library beside them
+    # the reference's fp32 and fp64 GEMM rows (bf16 pieces on the tensor cores, against the CUDA cores' rate / DMMA), 8192^3, with
+    # the library beside them
     for dt, tdt, name, spec_tf in ((N.DT_F32, torch.float32, "fp32", 75.0), (N.DT_F64, torch.float64, "fp64", 37.0)):
         try:
             m = 8192

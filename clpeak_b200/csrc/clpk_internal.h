@@ -30,6 +30,12 @@ int tuning(int knob);
 int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t m, uint32_t n, uint32_t k, float alpha,
                      uint32_t *status, cudaStream_t s);
 
+// what those two types ask of their operands
+int check_simt_gemm(int dtype, const void *a, const void *b, const void *c, uint32_t m, uint32_t n, uint32_t k);
+
+// microseconds that its plan for an fp32 product is estimated at
+float simt_f32_estimate(uint32_t m, uint32_t n, uint32_t k);
+
 // clpk_gemm_plan of those two types
 void simt_gemm_plan(bool f64, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile_n, uint32_t *splits, uint32_t *wide);
 

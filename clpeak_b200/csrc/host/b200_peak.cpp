@@ -725,7 +725,9 @@ struct B200Harness {
         int rc = operand(A, sfa, 40, false);
         rc |= operand(B, sfb, 41, true);
         clpk_gemm_args_t g{};
-        g.dtype = dt; g.m = g.n = g.k = d;
+        // this row measures the CUDA cores, as the reference's does; CLPK_DT_F32 would take the tensor cores
+        g.dtype = dt == CLPK_DT_F32 ? CLPK_DT_F32_FFMA : dt;
+        g.m = g.n = g.k = d;
         g.d_a = A.p; g.d_b = B.p; g.d_c = C.p; g.d_status = st.as<uint32_t>();
         g.alpha = nv ? tensorScale * tensorScale : 1.0f;
         g.d_sfa = sfa.p; g.d_sfb = sfb.p; g.d_workspace = ws.p; g.workspace_bytes = wsBytes;

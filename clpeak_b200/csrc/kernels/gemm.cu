@@ -32,6 +32,7 @@
 
 #include "../clpk_internal.h"
 #include "../clpk_ptx.cuh"
+#include "../clpk_rng_fast.cuh"
 
 namespace clpk {
 
@@ -566,6 +567,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads)
 }
 
 #include "../clpk_gemm_tiles.cuh"
+#include "../clpk_gemm_f32.cuh"
 
 
 // ---------------------------------------------------------------------------------
@@ -1197,6 +1199,30 @@ static TilesPlan gemm_plan(uint32_t m, uint32_t n, uint32_t k, uint32_t elem_bit
     return plan_tiles(m, n, k_blocks_of(k, elem_bits), fp4, arranged);
 }
 
+// CTAs in clusters of `cluster`, behind the kernel before them
+template <typename Maps, typename Params>
+static int launch_clusters(void (*kernel)(Maps, Params), const char *what, uint32_t ctas, int threads, size_t smem, uint32_t cluster, cudaStream_t s,
+                           const Maps &maps, const Params &p)
+{
+    CLPK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTilesSmemMax));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = tuning(CLPK_TUNE_GEMM_NO_PDL) == 1 ? 0 : 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    g_last_aligned = 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, maps, p);
+    return e == cudaSuccess ? CLPK_OK : cuda_fail(e, what);
+}
+
 // wsa, wsb: the packed scale factors (block-scaled kinds)
 template <int DT>
 static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64_t row_bytes, uint32_t k_blocks, TilesPlan plan, cudaStream_t s,
@@ -1245,25 +1271,7 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
         p.tmem_cols *= 2;
     CLPK_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&p.clock), g_gemm_clock));
     const size_t smem = p.stages * stage_bytes + fixed;
-    CLPK_CUDA(cudaFuncSetAttribute(gemm_tiles_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTilesSmemMax));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(clusters * 2 * plan.splits);
-    cfg.blockDim = dim3(kGemmThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2 * plan.splits;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = tuning(CLPK_TUNE_GEMM_NO_PDL) == 1 ? 0 : 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    g_last_aligned = 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tiles_kernel<DT>, maps, p);
-    if (e != cudaSuccess)
-        return cuda_fail(e, "gemm_tiles");
-    return CLPK_OK;
+    return launch_clusters(gemm_tiles_kernel<DT>, "gemm_tiles", clusters * 2 * plan.splits, kGemmThreads, smem, 2 * plan.splits, s, maps, p);
 }
 
 template <int DT>
@@ -1271,6 +1279,78 @@ static int launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, const CUten
 {
     const uint32_t n_tiles = ((p.m + kDenseTileM - 1) / kDenseTileM) * ((p.n + kTileMN - 1) / kTileMN);
     return launch_persistent(gemm_kernel<DT>, "gemm", kGemmThreads, kGemmSmemBytes, s, p, n_tiles, ta, tb, tc);
+}
+
+// TN and K ranges of gemm_f32_kernel; tn = 0: leave it to the kernels of simt_gemm.cu.  Like plan_tiles the cheapest by an
+// estimate in microseconds, from timed launches of every width and split: with W = TN / 256
+//   5.0 + waves * (chunks of 32 per range * max(0.44, 0.22 + 0.92 W) + 5 W of epilogue) and, split, 1 + 7 W per exchange.
+// A chunk is what the converters and the turns of the accumulators take; its instructions alone would be 0.22 to 0.46.  The
+// CUDA-core kernels keep what they are estimated to do as fast, sums of few chunks and products of a few tiles, whose
+// launch is shorter (688 x 140 x 268: 7.4 us against 9.0; 64 x 64 x 16384 57 against 62).  Beyond 2^28 elements of K, or
+// 2^31 rows, coordinates would not fit a tensor map's 32 bits.
+static TilesPlan plan_f32(uint32_t m, uint32_t n, uint32_t k)
+{
+    const uint32_t pairs = (uint32_t)num_sms() / 2, chunks = (k - 1) / kF32Chunk + 1;
+    TilesPlan plan = {0, 1};
+    if (pairs == 0 || k < 2 * kF32Chunk || k >= 1u << 28 || m >= 1u << 31 || n >= 1u << 31)
+        return plan;
+    float best = 0.95f * simt_f32_estimate(m, n, k);
+    for (uint32_t splits = 1; splits <= 4 && chunks >= 2 * splits; splits *= 2) {
+        const uint32_t resident = splits == 1 ? pairs : splits == 2 ? pairs * 33 / 74 : pairs * 15 / 74;
+        if (resident == 0)
+            break;
+        for (uint32_t tn = 32; tn <= 128; tn += 32) {
+            const uint64_t tiles = (uint64_t)((m - 1) / kF32M + 1) * ((n - 1) / tn + 1);
+            const float waves = (float)((tiles - 1) / resident + 1), wide = (float)tn / 256.0f;
+            const float chunk = 0.22f + 0.92f * wide > 0.44f ? 0.22f + 0.92f * wide : 0.44f;
+            const float t = 5.0f + waves * ((float)((chunks - 1) / splits + 1) * chunk + 5.0f * wide + (splits > 1 ? 1.0f + 7.0f * wide : 0.0f));
+            if (t < best) {
+                best = t;
+                plan = {tn, splits};
+            }
+        }
+    }
+    return plan;
+}
+
+template <uint32_t TN>
+static int launch_f32(const clpk_gemm_args_t *a, uint32_t splits, cudaStream_t s)
+{
+    using T = F32Tile<TN>;
+    F32Maps maps;
+    int rc = make_operand_map(&maps.a, a->d_a, a->m, (uint64_t)a->k * 4);
+    if (rc != CLPK_OK)
+        return rc;
+    rc = make_operand_map(&maps.b, a->d_b, a->n, (uint64_t)a->k * 4, TN / 2);
+    if (rc != CLPK_OK)
+        return rc;
+    F32Params p;
+    p.m = a->m;
+    p.n = a->n;
+    p.k = a->k;
+    p.tiles_m = (a->m + kF32M - 1) / kF32M;
+    p.tiles_n = (a->n + TN - 1) / TN;
+    p.group = tuning(CLPK_TUNE_GEMM_GROUP) > 0 ? (uint32_t)tuning(CLPK_TUNE_GEMM_GROUP) : 8;
+    p.chunks = (a->k + kF32Chunk - 1) / kF32Chunk;
+    p.splits = splits;
+    p.a = static_cast<const float *>(a->d_a);
+    p.b = static_cast<const float *>(a->d_b);
+    p.c = static_cast<float *>(a->d_c);
+    p.alpha = a->alpha;
+    p.status = a->d_status;
+    const uint32_t n_tiles = p.tiles_m * p.tiles_n, pairs = (uint32_t)num_sms() / 2;
+    const uint32_t clusters = splits > 1 ? n_tiles : (n_tiles < pairs ? n_tiles : pairs);
+    return launch_clusters(gemm_f32_kernel<TN>, "gemm_f32", clusters * 2 * splits, kF32Threads, T::smem_bytes, 2 * splits, s, maps, p);
+}
+
+static int launch_f32_tiles(const clpk_gemm_args_t *a, TilesPlan plan, cudaStream_t s)
+{
+    switch (plan.tn) {
+    case 32:  return launch_f32<32>(a, plan.splits, s);
+    case 64:  return launch_f32<64>(a, plan.splits, s);
+    case 96:  return launch_f32<96>(a, plan.splits, s);
+    default:  return launch_f32<128>(a, plan.splits, s);
+    }
 }
 
 } // namespace clpk
@@ -1287,7 +1367,16 @@ int clpk_gemm_plan(int dtype, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile
     CLPK_REQUIRE(tile_n && splits, "NULL output");
     CLPK_REQUIRE(m > 0 && n > 0 && k > 0, "M, N and K must be positive");
     uint32_t no_wide = 0;
-    if (dtype == CLPK_DT_F32 || dtype == CLPK_DT_F64) {
+    if (dtype == CLPK_DT_F32) {
+        if (const TilesPlan plan = plan_f32(m, n, k); plan.tn) {
+            *tile_n = plan.tn;
+            *splits = plan.splits;
+            if (wide)
+                *wide = 2;
+            return CLPK_OK;
+        }
+    }
+    if (dtype == CLPK_DT_F32 || dtype == CLPK_DT_F32_FFMA || dtype == CLPK_DT_F64) {
         simt_gemm_plan(dtype == CLPK_DT_F64, m, n, k, tile_n, splits, wide ? wide : &no_wide);
         return CLPK_OK;
     }
@@ -1412,10 +1501,17 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
         return rc;
     CLPK_REQUIRE(a, "args is NULL");
     CLPK_REQUIRE(a->d_a && a->d_b && a->d_c && a->d_status, "NULL buffer");
-    if (a->dtype == CLPK_DT_F32 || a->dtype == CLPK_DT_F64) {
-        // no tcgen05 kind for these: the CUDA-core fp32 and DMMA fp64 kernels of simt_gemm.cu
+    if (a->dtype == CLPK_DT_F32 || a->dtype == CLPK_DT_F32_FFMA || a->dtype == CLPK_DT_F64) {
+        const int type = a->dtype == CLPK_DT_F64 ? CLPK_DT_F64 : CLPK_DT_F32;
+        rc = check_simt_gemm(type, a->d_a, a->d_b, a->d_c, a->m, a->n, a->k);
+        if (rc != CLPK_OK)
+            return rc;
+        if (a->dtype == CLPK_DT_F32)
+            if (const TilesPlan plan = plan_f32(a->m, a->n, a->k); plan.tn)
+                return launch_f32_tiles(a, plan, as_stream(stream));
+        // the CUDA-core fp32 and DMMA fp64 kernels of simt_gemm.cu
         g_last_aligned = 0;
-        return launch_simt_gemm(a->dtype, a->d_a, a->d_b, a->d_c, a->m, a->n, a->k, a->alpha, a->d_status, as_stream(stream));
+        return launch_simt_gemm(type, a->d_a, a->d_b, a->d_c, a->m, a->n, a->k, a->alpha, a->d_status, as_stream(stream));
     }
     CLPK_REQUIRE(a->m > 0 && a->n > 0 && a->k > 0, "M, N and K must be positive");
     const bool block_scaled = a->dtype == CLPK_DT_NVF4 || a->dtype == CLPK_DT_MXF4;

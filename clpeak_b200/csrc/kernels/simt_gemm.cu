@@ -1,5 +1,5 @@
-// The two GEMM rows that have no tcgen05 kind: fp32 on the CUDA cores and fp64 on the
-// warp-level DMMA path.  They take the place of the reference's cuBLASLt "fp32" and
+// The two GEMM rows that have no tcgen05 kind: fp32 on the CUDA cores (small products and sums of less than 64 numbers;
+// the others are gemm_f32_kernel's) and fp64 on the warp-level DMMA path.  They take the place of the reference's cuBLASLt "fp32" and
 // "fp64" rows (src/cuda/cuda_blas.cpp:567-581) behind the same clpk_gemm entry point:
 // C[M][N] = alpha * A[M][K] * B[N][K]^T, both operands K-contiguous, C row-major in the
 // operand type.
@@ -731,6 +731,7 @@ static int launch_simt(void (*kernel)(Params...), const char *what, uint64_t cta
 struct SimtPlan {
     uint32_t tile, splits;
     bool wide;                  // twice the K groups
+    float us = 0.0f;            // the estimate it was chosen by (fp32 and long fp64 sums)
 };
 
 // fp64 with fewer than 24 blocks: what a CTA costs besides them -- start, pipeline fill, sum, stores -- is then a good part
@@ -776,8 +777,9 @@ static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
         const float busiest = shared * (float)((ctas(rows, cols, splits) - 1) / simt_capacity(splits) + 1);
         return (float)((blocks - 1) / splits + 1) * (alone > busiest ? alone : busiest);
     };
-    float best = f64 ? 0.92f * (3.8f + estimate(128, 64, 1, 1.48f, 1.24f)) : 0.92f * (2.0f + estimate(128, 128, 1, 1.62f, 1.43f));
-    SimtPlan plan = {128, 1, false};
+    const float large = f64 ? 3.8f + estimate(128, 64, 1, 1.48f, 1.24f) : 2.0f + estimate(128, 128, 1, 1.62f, 1.43f);
+    float best = 0.92f * large;
+    SimtPlan plan = {128, 1, false, large};
     for (uint32_t splits = 1; splits <= 8 && (splits == 1 || blocks >= 4 * splits); splits *= 2)
         for (uint32_t tile = f64 ? 32 : 64; tile <= 64; tile *= 2) {
             const bool wide = !(f64 && tile == 64) && ctas(tile, tile, splits) <= simt_capacity(splits) && blocks >= (f64 ? 24 : 32) * splits;
@@ -792,11 +794,13 @@ static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
                     (splits > 1 ? 0.5f * splits : 0.0f);
             if (t < best) {
                 best = t;
-                plan = {tile, splits, wide};
+                plan = {tile, splits, wide, t};
             }
         }
     return plan;
 }
+
+float simt_f32_estimate(uint32_t m, uint32_t n, uint32_t k) { return plan_simt(false, m, n, k).us; }
 
 void simt_gemm_plan(bool f64, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile_n, uint32_t *splits, uint32_t *wide)
 {
@@ -806,16 +810,27 @@ void simt_gemm_plan(bool f64, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile
     *wide = plan.wide ? 1 : 0;
 }
 
-int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t m, uint32_t n, uint32_t k, float alpha,
-                     uint32_t *status, cudaStream_t s)
+static uint64_t large_tiles(int dtype, uint32_t m, uint32_t n)
+{
+    const uint32_t tile_n = dtype == CLPK_DT_F32 ? kSimtTile : 64;
+    return (uint64_t)((m + kSimtTile - 1) / kSimtTile) * ((n + tile_n - 1) / tile_n);
+}
+
+int check_simt_gemm(int dtype, const void *a, const void *b, const void *c, uint32_t m, uint32_t n, uint32_t k)
 {
     CLPK_REQUIRE(m > 0 && n > 0 && k > 0, "M, N and K must be positive");
     const uint32_t k_unit = dtype == CLPK_DT_F32 ? 4 : 2;            // elements per 16 bytes: operand rows stay aligned
     CLPK_REQUIRE(k % k_unit == 0, "K = %u: a row of A and B must be a multiple of 16 bytes", k);
     CLPK_REQUIRE(((uintptr_t)a % 16) == 0 && ((uintptr_t)b % 16) == 0 && ((uintptr_t)c % 16) == 0, "operands must be 16-byte aligned");
+    CLPK_REQUIRE(large_tiles(dtype, m, n) <= 0x3FFFFFFFull, "too many tiles");
+    return CLPK_OK;
+}
+
+int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t m, uint32_t n, uint32_t k, float alpha,
+                     uint32_t *status, cudaStream_t s)
+{
     const uint32_t tile_n = dtype == CLPK_DT_F32 ? kSimtTile : 64;
-    const uint64_t tiles = (uint64_t)((m + kSimtTile - 1) / kSimtTile) * ((n + tile_n - 1) / tile_n);
-    CLPK_REQUIRE(tiles <= 0x3FFFFFFFull, "too many tiles");
+    const uint64_t tiles = large_tiles(dtype, m, n);
     // whole tiles and whole k blocks take the kernel without the bounds checks
     const bool ragged = m % kSimtTile != 0 || n % tile_n != 0 || k % kSimtBK != 0;
     const SimtPlan plan = plan_simt(dtype == CLPK_DT_F64, m, n, k);

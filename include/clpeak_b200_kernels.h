@@ -146,6 +146,7 @@ CLPK_API int clpk_fill_i8(int8_t *d_dst, uint64_t n, uint64_t seed, void *stream
 #define CLPK_DT_TF32  10  /* fp32 word rounded (nearest even) to 10 mantissa bits, low 13 bits clear       */
 #define CLPK_DT_E2M1  11  /* plain e2m1, two per byte (element 2i in the low nibble), saturating at +-6   */
 #define CLPK_DT_F64   12  /* double; clpk_convert_f32 widens exactly                                      */
+#define CLPK_DT_F32_FFMA 13  /* clpk_gemm: fp32 on the CUDA cores at every size, for a row that measures them */
 
 /* Round-to-nearest-even conversion of n floats to a plain (unscaled) format:
  * F16, BF16, E4M3 / E5M2 (saturating to the largest finite value), I8
@@ -404,7 +405,8 @@ CLPK_API int clpk_dmma_peak(const double *d_a, const double *d_b, uint32_t n_mma
  * (src/cuda/cuda_blas.cpp:275-287).  Accumulation in tensor memory, no epilogue
  * beyond the multiplication by `alpha` (the product of the NVF4 tensor scales).
  *   dtype            A / B elements                  accumulate   C element
- *   CLPK_DT_F32      fp32, CUDA cores (FFMA)         fp32         fp32   the reference's "fp32" row
+ *   CLPK_DT_F32      fp32: tensor cores, or FFMA     fp32         fp32
+ *   CLPK_DT_F32_FFMA fp32, CUDA cores (FFMA)         fp32         fp32   the reference's "fp32" row
  *   CLPK_DT_F64      fp64, mma.sync.m8n8k4 (DMMA)    fp64         fp64   the reference's "fp64" row
  *                    (src/cuda/cuda_blas.cpp:567-581); any M, N > 0, K a multiple of 4 (fp32) or 2 (fp64)
  *   CLPK_DT_BF16     bf16                            fp32         bf16
@@ -416,6 +418,9 @@ CLPK_API int clpk_dmma_peak(const double *d_a, const double *d_b, uint32_t n_mma
  *   CLPK_DT_I8       int8                            int32        int32 (alpha ignored)
  *   CLPK_DT_MXF4     e2m1 + ue8m0 per 32             fp32         bf16
  *   CLPK_DT_NVF4     e2m1 + ue4m3 per 16             fp32         bf16
+ * CLPK_DT_F32: small products and short sums run on the CUDA cores (FFMA); the others multiply three bf16 pieces of each
+ * element on the tensor cores and add fp32 sums of 32 products with fp32 rounding, which leaves a smaller error than K
+ * fused multiply-adds.  Infinities, NaNs, overflows and magnitudes below 2^-100 are multiplied by FFMA in either case.
  * tcgen05 kinds: any M, N, K > 0 such that a row of A / B and a row of C are multiples of 16
  * bytes (partial tiles are computed whole and clipped; whole 512 x 256 tiles and K a multiple
  * of 128 bytes waste nothing).  FP4 kinds: K a multiple of 256; the workspace holds scale
@@ -448,7 +453,8 @@ CLPK_API int clpk_gemm_pack_scales(const clpk_gemm_args_t *args, void *stream);
 CLPK_API int clpk_gemm(const clpk_gemm_args_t *args, void *stream);
 /* How clpk_gemm splits a problem of these sizes on the current device: the tile's width in columns and the number of
  * K ranges.  A width of 0 is the kernel for large shapes, whose tiles are its own.  For CLPK_DT_F32 and CLPK_DT_F64
- * tiles are square; *wide (may be NULL) is 1 where a CTA takes twice the K groups.  For the FP4 kinds: of a call without
+ * tiles are square; *wide (may be NULL) is 1 where a CTA takes twice the K groups, and 2 where an fp32 product runs on the
+ * tensor cores, in tiles of 256 rows.  For the FP4 kinds: of a call without
  * scale pointers.  Lets a benchmark or a test record which kernel it ran; needs no GPU work. */
 CLPK_API int clpk_gemm_plan(int dtype, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile_n, uint32_t *splits, uint32_t *wide);
 /* 1 if the calling thread's last clpk_gemm launch ran with the per-wave producer meeting, 0 if

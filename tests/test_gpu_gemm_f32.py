@@ -1,0 +1,116 @@
+"""The fp32 GEMM on the tensor cores: every tile width and K split, edges of tiles and of chunks, and the numbers that three
+bf16 pieces cannot hold."""
+import ctypes as C
+
+import pytest
+
+from clpeak_b200 import native as N
+from tests.gpu_util import dev_empty, gemm_plan, stream_ptr, sync
+
+pytestmark = pytest.mark.gpu
+
+
+def operands(K, cuda, m, n, k):
+    out = []
+    for rows, seed in ((m, 50), (n, 51)):
+        f = dev_empty(rows * k, cuda.float32)
+        K.clpk_fill_f32(f.data_ptr(), rows * k, seed, N.DIST_NORMAL, 0.0, 0.02, stream_ptr())
+        out.append(f.view(rows, k))
+    return out
+
+
+def multiply(K, cuda, a, b, alpha=1.0):
+    (m, k), n = a.shape, b.shape[0]
+    c = cuda.full((m * n + 1024,), 7.0, dtype=cuda.float32, device="cuda")
+    status = cuda.full((1,), 7, dtype=cuda.int32, device="cuda")
+    args = N.GemmArgs(dtype=N.DT_F32, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=alpha, d_status=status.data_ptr())
+    K.clpk_gemm(C.byref(args), stream_ptr())
+    sync()
+    assert int(status.item()) == 0
+    assert bool((c[m * n:] == 7.0).all()), "the kernel wrote beyond C"
+    return c[:m * n].view(m, n)
+
+
+def worst(c, a, b, alpha=1.0):
+    """Largest error in units of 2^-24 sum |a b|."""
+    want, s_abs = alpha * (a.double() @ b.double().T), abs(alpha) * (a.double().abs() @ b.double().abs().T)
+    return float(((c.double() - want).abs() / (2.0 ** -24 * s_abs + 1e-300)).max())
+
+
+def bound(k):
+    """One rounding per chunk of 32, one of alpha, and at most eight units for what an instruction cuts when it aligns its
+    products (two per chunk cut a sum of full size, in a chunk that is a part of the sum)."""
+    return -(-k // 32) + 9
+
+
+# (tile width, K ranges) and a shape that takes them: ragged rows, columns and chunks, odd N, several tiles per pair
+PLANS = [((32, 1), (2618, 67, 188)), ((32, 2), (2644, 65, 324)), ((32, 4), (1067, 65, 396)), ((64, 1), (67, 2381, 228)), ((64, 1), (2577, 829, 164)),
+         ((64, 2), (2819, 73, 488)), ((64, 4), (1655, 67, 580)), ((96, 1), (273, 2387, 180)), ((96, 1), (1090, 1867, 164)), ((96, 2), (66, 2435, 816)),
+         ((96, 4), (2914, 65, 604)), ((128, 1), (529, 2327, 172)), ((128, 1), (1544, 2051, 176)), ((128, 2), (264, 1629, 1848)), ((128, 4), (65, 1447, 1732))]
+
+
+@pytest.mark.parametrize("plan,shape", PLANS)
+def test_every_plan(K, cuda, plan, shape):
+    assert gemm_plan(K, N.DT_F32, *shape) == (*plan, 2)
+    a, b = operands(K, cuda, *shape)
+    c = multiply(K, cuda, a, b, 0.75)
+    assert worst(c, a, b, 0.75) <= bound(shape[2])
+    assert bool((c == multiply(K, cuda, a, b, 0.75)).all()), "partial sums are added in a fixed order: the same bits every time"
+
+
+@pytest.mark.parametrize("m,n,k", [(256, 128, 256), (257, 129, 260), (255, 127, 252), (128, 1000, 288), (1000, 131, 1028), (300, 202, 2044), (2000, 2001, 512)])
+def test_edges(K, cuda, m, n, k):
+    a, b = operands(K, cuda, m, n, k)
+    assert worst(multiply(K, cuda, a, b), a, b) <= bound(k)
+
+
+@pytest.mark.parametrize("shape", [(300, 200, 1024), (2000, 1500, 260)])
+def test_infinities_nans_and_overflow(K, cuda, shape):
+    """They reach what a product in 64 bits says they reach, and nothing else."""
+    a, b = operands(K, cuda, *shape)
+    a[3, 5], a[130, 0], a[131, 7], b[7, shape[2] - 1] = float("inf"), float("nan"), 3.4e38, float("-inf")
+    a[200] = 1e30
+    b[9] = 1e30                           # 1e60 overflows, 1e30 * 0.02 does not
+    c = multiply(K, cuda, a, b)
+    want = (a.double() @ b.double().T).float()
+    finite = cuda.isfinite(want)
+    assert bool((cuda.isfinite(c) == finite).all())
+    assert bool((cuda.isnan(c) == cuda.isnan(want)).all()) and bool((c[~finite & ~cuda.isnan(want)] == want[~finite & ~cuda.isnan(want)]).all())
+    s_abs = a.double().abs() @ b.double().abs().T
+    assert bool(((c.double() - want.double()).abs()[finite] <= (shape[2] + 2) * 2.0 ** -24 * s_abs[finite]).all())
+
+
+@pytest.mark.parametrize("shape", [(300, 200, 1024), (2000, 1500, 260)])
+@pytest.mark.parametrize("small,large", [(2.0 ** -96, 2.0 ** 90), (2.0 ** -110, 2.0 ** 100), (2.0 ** -140, 2.0 ** 120)])
+def test_small_magnitudes_keep_their_bits(K, cuda, shape, small, large):
+    """Where the third bf16 piece of an element would leave bf16's range the tile is multiplied as it is; zeros stay zeros."""
+    a, b = operands(K, cuda, *shape)
+    a[5:9] *= small
+    a[100] = 0.0
+    b *= large
+    b[11] = 0.0
+    c = multiply(K, cuda, a, b)
+    assert worst(c, a, b) <= shape[2] + 2
+    assert bool((c[100] == 0.0).all()) and bool((c[:, 11] == 0.0).all())
+
+
+def test_wide_range_of_magnitudes(K, cuda):
+    """Every element of its own binade between 2^-40 and 2^40: the error stays relative to the products."""
+    m, n, k = 513, 260, 1000
+    a, b = operands(K, cuda, m, n, k)
+    for t, seed in ((a, 3), (b, 4)):
+        g = cuda.Generator(device="cuda").manual_seed(seed)
+        t *= 2.0 ** cuda.randint(-40, 41, t.shape, generator=g, device="cuda").float()
+    assert worst(multiply(K, cuda, a, b), a, b) <= bound(k)
+
+
+def test_the_cuda_cores_on_request(K, cuda):
+    """DT_F32_FFMA: no tile of the tensor cores at any size, the same product within fp32 rounding."""
+    m, n, k = 300, 202, 2044
+    assert gemm_plan(K, N.DT_F32, m, n, k)[2] == 2 and gemm_plan(K, N.DT_F32_FFMA, m, n, k)[2] != 2
+    a, b = operands(K, cuda, m, n, k)
+    c, status = dev_empty(m * n, cuda.float32), dev_empty(1, cuda.int32)
+    args = N.GemmArgs(dtype=N.DT_F32_FFMA, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=1.0, d_status=status.data_ptr())
+    K.clpk_gemm(C.byref(args), stream_ptr())
+    sync()
+    assert worst(c.view(m, n), a, b) <= k + 2
