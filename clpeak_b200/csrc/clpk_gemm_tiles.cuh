@@ -3,6 +3,11 @@
 // Same pieces as gemm_kernel -- CTA pairs, TMA ring, elected-lane issue, bounded waits -- with the split of the work
 // left to the launch:
 //  * Tile 256 x TN per CTA pair, TN = 32 ... 256 in steps of 32, one M = 256 row block (CTA r holds its 128 rows).
+//  * Dense kinds, K not split: also 512 x TN, a second row block that shares the tile's B.  The 512 x 256 tiles of gemm_kernel
+//    leave the chip idle where they are few or their last wave is nearly empty, and where N is just above a multiple of
+//    256; narrower ones of the same height read as little of A.  Up to TN = 128 there are two accumulators, beyond one,
+//    whose reading the next tile waits for.  bf16 10149 x 456 x 2176 28.6 -> 19.6 us, e4m3 2882 x 1544 x 4864 29.6 -> 21.3, i8
+//    9909 x 488 x 2304 19.6 -> 16.0, tf32 8248 x 1576 x 640 36.8 -> 31.0.
 //  * K over 1, 2 or 4 pairs of one cluster.  Every pair accumulates its own K range in tensor memory; then the pairs
 //    exchange partial sums through distributed shared memory (each owns every splits-th 32-column chunk of the tile),
 //    add them in pair order -- the same order whoever owns the chunk -- and store what they own.  Nothing goes through
@@ -58,6 +63,8 @@ struct TilesParams {
     uint32_t tiles_m, tiles_n, group;
     uint32_t k_blocks;                  // of 128 bytes
     uint32_t tn, splits, stages;
+    uint32_t row_blocks;                // of 256 rows that share a tile's B: 1, or 2 where K is not split (dense kinds)
+    uint32_t accs;                      // accumulators: 2, or 1 where two would not fit
     uint32_t kps;                       // K blocks per stage: 1 or 2
     uint32_t tmem_cols;                 // power of two: one accumulator, or two when a cluster has several tiles
     float alpha;
@@ -65,8 +72,8 @@ struct TilesParams {
     unsigned long long *clock;
 };
 
-// bytes of one K block in a CTA: its 128 rows of A and its half of the tile's rows of B
-__host__ __device__ constexpr uint32_t tiles_block_bytes(uint32_t tn) { return kHalfTileBytes + tn / 2 * kRowBytesK; }
+// bytes of one K block in a CTA: its 128 rows of each row block of A and its half of the tile's rows of B
+__host__ __device__ constexpr uint32_t tiles_block_bytes(uint32_t tn, uint32_t row_blocks = 1) { return row_blocks * kHalfTileBytes + tn / 2 * kRowBytesK; }
 
 // 32 columns of one row per lane -> the warp's staging box (32 rows x 64 bytes of bf16 in the 64-byte swizzle, or
 // x 128 bytes of fp32 / int32 in the 128-byte swizzle) -> one TMA store that clips what lies beyond C.
@@ -141,14 +148,15 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
     constexpr uint32_t kWords = TilesKind<DT>::words;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const uint32_t block_bytes = tiles_block_bytes(p.tn), stage_bytes = p.kps * block_bytes + (kFp4 ? tiles_sf_bytes(p.tn) : 0);
+    const uint32_t row_blocks = kFp4 ? 1 : p.row_blocks, b_at = row_blocks * kHalfTileBytes;
+    const uint32_t block_bytes = tiles_block_bytes(p.tn, row_blocks), stage_bytes = p.kps * block_bytes + (kFp4 ? tiles_sf_bytes(p.tn) : 0);
     uint8_t *staging = smem + (size_t)p.stages * stage_bytes;
     TilesSmem *sh = reinterpret_cast<TilesSmem *>(staging + kEpilogueWarps * kStagingBytes);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank(), r = rank & 1, leader = rank & ~1u, split = rank >> 1;
     const uint32_t cluster_id = blockIdx.x / (2 * p.splits), n_clusters = gridDim.x / (2 * p.splits);
-    const uint32_t n_tiles = p.tiles_m * p.tiles_n;
+    const uint32_t n_tiles = p.tiles_m * p.tiles_n, accs = kFp4 ? 2 : p.accs;
     const uint32_t kb0 = split * p.k_blocks / p.splits, kb1 = (split + 1) * p.k_blocks / p.splits;
 
     if (threadIdx.x == 0) {
@@ -196,7 +204,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
         for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters) {
             uint32_t mb, nb;
             dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
-            const int32_t row_a = (int32_t)(mb * kTilesM + r * 128), row_b = (int32_t)(nb * p.tn + r * (p.tn / 2));
+            const int32_t row_a = (int32_t)(mb * row_blocks * kTilesM + r * 128), row_b = (int32_t)(nb * p.tn + r * (p.tn / 2));
             for (uint32_t kb = kb0; kb < kb1; kb += p.kps) {
                 if (!warp_wait(&sh->empty[s], parity)) {       // a fresh barrier's preceding phase counts as complete
                     if (lane == 0)
@@ -215,7 +223,9 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
                         if (h < nk) {
                             uint8_t *blk = st + h * block_bytes;
                             tma_load_pair_at(blk, &maps.a, x + h * kRowBytesK, row_a, full0 + 8 * s);
-                            tma_load_pair_at(blk + kHalfTileBytes, &maps.b, x + h * kRowBytesK, row_b, full0 + 8 * s);
+                            if (row_blocks == 2)
+                                tma_load_pair_at(blk + kHalfTileBytes, &maps.a, x + h * kRowBytesK, row_a + (int32_t)kTilesM, full0 + 8 * s);
+                            tma_load_pair_at(blk + b_at, &maps.b, x + h * kRowBytesK, row_b, full0 + 8 * s);
                         }
                     if constexpr (kFp4) {
                         // A's blocks lie [rows / 128][K block][word], B's [rows / 256][K block][word][half of the 256]
@@ -249,14 +259,14 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
             uint32_t s = 0, parity = 0, tcount = 0;
             bool ok = true;
             for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters, tcount++) {
-                const uint32_t acc = tcount & 1, use = tcount >> 1;
+                const uint32_t acc = tcount % accs, use = tcount / accs;
                 if (use > 0 && !warp_wait(&sh->tmem_empty[acc], (use - 1) & 1)) {
                     if (lane == 0)
                         atomicCAS(p.status, 0u, 0x222u);
                     break;
                 }
                 tc_fence_after_sync();
-                const uint32_t d = tmem + acc * p.tn;
+                const uint32_t d = tmem + acc * row_blocks * p.tn;
                 [[maybe_unused]] uint32_t mb, nb = 0;
                 if constexpr (kFp4)
                     dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
@@ -302,20 +312,24 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
                             if (kFp4 || h >= nk)
                                 break;
                             const uint32_t blk = base + h * block_bytes;
-                            const uint64_t ad = make_smem_desc(blk, 16, 1024, kSwizzle128B);
-                            const uint64_t bd = make_smem_desc(blk + kHalfTileBytes, 16, 1024, kSwizzle128B);
+                            const uint64_t bd = make_smem_desc(blk + b_at, 16, 1024, kSwizzle128B);
+                            auto multiply = [&](uint32_t dd, uint64_t ad) {
 #pragma unroll
-                            for (uint32_t kk = 0; kk < 4; kk++) {
-                                const uint32_t accumulate = (kb != kb0 || h != 0 || kk != 0) ? 1u : 0u;
-                                if constexpr (DT == CLPK_DT_E4M3 || DT == CLPK_DT_E5M2)
-                                    mma2_f8f6f4_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-                                else if constexpr (DT == CLPK_DT_TF32)
-                                    mma2_tf32_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-                                else if constexpr (DT == CLPK_DT_I8)
-                                    mma2_i8_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-                                else if constexpr (!kFp4)
-                                    mma2_f16_ss(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-                            }
+                                for (uint32_t kk = 0; kk < 4; kk++) {
+                                    const uint32_t accumulate = (kb != kb0 || h != 0 || kk != 0) ? 1u : 0u;
+                                    if constexpr (DT == CLPK_DT_E4M3 || DT == CLPK_DT_E5M2)
+                                        mma2_f8f6f4_ss(dd, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                                    else if constexpr (DT == CLPK_DT_TF32)
+                                        mma2_tf32_ss(dd, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                                    else if constexpr (DT == CLPK_DT_I8)
+                                        mma2_i8_ss(dd, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                                    else if constexpr (!kFp4)
+                                        mma2_f16_ss(dd, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                                }
+                            };
+                            multiply(d, make_smem_desc(blk, 16, 1024, kSwizzle128B));
+                            if (row_blocks == 2)
+                                multiply(d + p.tn, make_smem_desc(blk + kHalfTileBytes, 16, 1024, kSwizzle128B));
                         }
                         tc_commit_pair(&sh->empty[s_now], pair_mask);
                     }
@@ -332,36 +346,42 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
         for (uint32_t tile = cluster_id; tile < n_tiles; tile += n_clusters, tcount++) {
             uint32_t mb, nb;
             dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
-            const uint32_t acc = tcount & 1, use = tcount >> 1;
+            const uint32_t acc = tcount % accs, use = tcount / accs;
             if (!warp_wait(&sh->tmem_full[acc], use & 1)) {
                 if (lane == 0)
                     atomicCAS(p.status, 0u, 0x224u);
                 break;
             }
             tc_fence_after_sync();
-            const uint32_t taddr = tmem + acc * p.tn + ((q * 32) << 16);
-            const uint32_t row = mb * kTilesM + r * 128 + q * 32;
+            // the row blocks' chunks lie one behind another in tensor memory
+            const uint32_t all_chunks = row_blocks * n_chunks;
+            const uint32_t taddr = tmem + acc * row_blocks * p.tn + ((q * 32) << 16);
+            const uint32_t row = mb * row_blocks * kTilesM + r * 128 + q * 32;
+            auto store = [&](uint32_t (&v)[32], uint32_t c) {
+                const uint32_t block = c >= n_chunks ? 1 : 0;
+                tiles_store_chunk<DT>(v, p.alpha, boxes, n_stored, &maps.c, nb * p.tn + (c - block * n_chunks) * kTilesChunk, row + block * kTilesM, lane);
+            };
             auto release = [&]() {
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
                     mbar_arrive_cluster_relaxed(&sh->tmem_empty[acc], leader);
             };
-            if (half >= n_chunks)
+            if (half >= all_chunks)
                 release();
-            for (uint32_t c = half; c < n_chunks; c += 4) {
+            for (uint32_t c = half; c < all_chunks; c += 4) {
                 // two chunks in flight
-                const bool two = c + 2 < n_chunks;
+                const bool two = c + 2 < all_chunks;
                 uint32_t v0[32], v1[32];
                 tmem_ld_32x32b_x32(taddr + c * kTilesChunk, v0);
                 if (two)
                     tmem_ld_32x32b_x32(taddr + (c + 2) * kTilesChunk, v1);
                 tmem_ld_wait();
-                if (c + 4 >= n_chunks)
+                if (c + 4 >= all_chunks)
                     release();
-                tiles_store_chunk<DT>(v0, p.alpha, boxes, n_stored, &maps.c, nb * p.tn + c * kTilesChunk, row, lane);
+                store(v0, c);
                 if (two)
-                    tiles_store_chunk<DT>(v1, p.alpha, boxes, n_stored, &maps.c, nb * p.tn + (c + 2) * kTilesChunk, row, lane);
+                    store(v1, c + 2);
             }
         }
     } else if (!warp_wait(&sh->tmem_full[0], 0)) {

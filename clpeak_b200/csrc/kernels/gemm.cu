@@ -1111,6 +1111,7 @@ static int launch_persistent(Kernel kernel, const char *what, int threads, size_
 // How gemm_tiles_kernel splits a problem; tn = 0: leave it to gemm_kernel or gemm_block_scaled_kernel.
 struct TilesPlan {
     uint32_t tn, splits;
+    uint32_t row_blocks = 1;            // 2: 512 x tn tiles
 };
 
 // The plan is the cheapest by a cost estimate in microseconds, fitted to timed launches of both kernels: 2500 for 120
@@ -1123,6 +1124,11 @@ struct TilesPlan {
 //                             54 TB/s) + 1.1 W of epilogue) and, split, 1 + 4.3 W per exchanged share of the tile
 //   gemm_block_scaled_kernel  4.0 + waves * (K blocks * (0.275 + T at 43 TB/s) + 0.7)
 //   gemm_tiles_kernel, FP4    3.3 + waves * (K blocks * (0.25 + 0.06 W + T at 62 TB/s) + 1.4 W) and the same exchange
+//   gemm_tiles_kernel, 512    4.75 + waves * (K blocks * (0.157 + 0.344 W + T at 106 TB/s) + 1.2 W of epilogue, 3.2 W from
+//                             tn = 160 on, where tensor memory holds one accumulator); from 24000 launches, residual 6 %.
+//                             Asked for only where gemm_kernel would be taken: of 1269 such shapes of up to four waves
+//                             some 570 take it, 1.22 times faster in the geometric mean, one of them 3 % slower; against
+//                             the 256-row tiles the estimate is not sharp enough (228 of 831 more than 2 % slower)
 // Splits of 2 and 4 are clusters of 4 and 8 CTAs, of which the chip holds 33 and 15 at a time.  From the fifth wave of
 // 512 x 256 tiles on (16384 x 16384 x 256: 140 against 142 us) and the third of block-scaled ones the large tiles'
 // smaller operand traffic wins at every K; an FP4 tile 256 wide that is not split is the large kernel's own.  An FP4 A of a few
@@ -1166,6 +1172,19 @@ static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4,
             if (t < best) {
                 best = t;
                 plan = {tn, splits};
+            }
+        }
+    }
+    // Where the 512 x 256 tiles are left over, narrower ones of 512 rows may fill the chip better.
+    if (!fp4 && plan.tn == 0) {
+        for (uint32_t tn = 32; tn < 256; tn += 32) {
+            const uint64_t tiles = (uint64_t)ceil_div(m, kDenseTileM) * ceil_div(n, tn);
+            const float waves = (float)((tiles - 1) / pairs + 1), wide = (float)tn / 256.0f;
+            const float loaded = (float)(tiles < pairs ? tiles : pairs) * ((m < kDenseTileM ? m : kDenseTileM) + (n < tn ? n : tn)) * kRowBytesK;
+            const float t = 4.75f + waves * (k_blocks * (0.157f + 0.344f * wide + loaded / 105.6e6f) + (tn > 128 ? 3.2f : 1.2f) * wide);
+            if (t < best) {
+                best = t;
+                plan = {tn, 1, 2};
             }
         }
     }
@@ -1246,7 +1265,9 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
             return rc;
     }
     TilesParams p;
-    p.tiles_m = (a->m + kTilesM - 1) / kTilesM;
+    p.row_blocks = plan.row_blocks;
+    p.accs = plan.row_blocks * plan.tn > 256 ? 1 : 2;
+    p.tiles_m = (a->m - 1) / (kTilesM * plan.row_blocks) + 1;
     p.tiles_n = (a->n + plan.tn - 1) / plan.tn;
     p.group = tuning(CLPK_TUNE_GEMM_GROUP) > 0 ? (uint32_t)tuning(CLPK_TUNE_GEMM_GROUP) : 8;
     p.k_blocks = k_blocks;
@@ -1260,14 +1281,14 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
     // two K blocks per stage halve the hand-overs (0.195 -> 0.137 us per block at TN = 32), but from TN = 160 on leave
     // too few stages (2048^3 bf16 at TN = 192: 19.3 -> 20.7 us)
     constexpr bool fp4 = TilesKind<DT>::fp4;
-    p.kps = plan.tn <= 128 && !fp4 ? 2 : 1;
-    const uint32_t stage_bytes = p.kps * tiles_block_bytes(plan.tn) + (fp4 ? tiles_sf_bytes(plan.tn) : 0);
+    p.kps = plan.tn <= 128 && plan.row_blocks == 1 && !fp4 ? 2 : 1;
+    const uint32_t stage_bytes = p.kps * tiles_block_bytes(plan.tn, plan.row_blocks) + (fp4 ? tiles_sf_bytes(plan.tn) : 0);
     p.stages = (uint32_t)((kTilesSmemMax - fixed) / stage_bytes);
     const uint32_t most = fp4 ? 256 / tiles_sf_cols(plan.tn) : kTilesMaxStages;      // scale factors: 256 tensor-memory columns
     if (p.stages > most)
         p.stages = most;
     p.tmem_cols = fp4 ? 512 : 32;
-    while (p.tmem_cols < (n_tiles > clusters ? 2 : 1) * plan.tn)
+    while (p.tmem_cols < (n_tiles > clusters ? p.accs : 1) * plan.row_blocks * plan.tn)
         p.tmem_cols *= 2;
     CLPK_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&p.clock), g_gemm_clock));
     const size_t smem = p.stages * stage_bytes + fixed;
@@ -1386,7 +1407,7 @@ int clpk_gemm_plan(int dtype, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile
     *tile_n = plan.tn;
     *splits = plan.splits;
     if (wide)
-        *wide = 0;
+        *wide = plan.row_blocks - 1;
     return CLPK_OK;
 }
 
