@@ -34,8 +34,8 @@
 //
 // Numbers that the split cannot serve are multiplied as they are, with fused multiply-adds in K order: a warp whose sums
 // are not all finite (an infinity, a NaN or an overflow on the way; x - h of an infinity is a NaN, so none goes unseen)
-// does its 32 x TN / 2 outputs again, and so does a tile that has met a magnitude below 2^-100, of which l would leave
-// the range of bf16.
+// does its 32 x TN / 2 outputs again, and so does one with a sum below 2^-100, whose products' pieces are partly below what
+// fp32 resolves, and a tile that has met a magnitude below 2^-100, of which l would leave the range of bf16.
 #pragma once
 
 constexpr uint32_t kF32M = 256;
@@ -550,8 +550,10 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                 bool again = *reinterpret_cast<volatile uint32_t *>(&sh->small[tcount % kF32TileFlags]) == tcount + 1;
                 float probe = 0.0f;                                       // not finite: 0 x = NaN
 #pragma unroll
-                for (uint32_t i = 0; i < T::half_n; i++)
+                for (uint32_t i = 0; i < T::half_n; i++) {
                     probe = fmaf(sum[i], 0.0f, probe);
+                    again |= too_small(sum[i]);
+                }
                 again |= probe != 0.0f;
                 if (__any_sync(0xffffffffu, again)) {
                     float slow[T::half_n];

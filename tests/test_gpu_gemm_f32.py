@@ -94,6 +94,19 @@ def test_small_magnitudes_keep_their_bits(K, cuda, shape, small, large):
     assert bool((c[100] == 0.0).all()) and bool((c[:, 11] == 0.0).all())
 
 
+@pytest.mark.parametrize("exponents", [(-70, -70), (-60, -72), (-63, -75), (-40, -66)])
+def test_results_near_the_end_of_the_range(K, cuda, exponents):
+    """Products that fp32 holds only in part: K roundings to 2^-149 besides the relative ones."""
+    m, n, k = 300, 200, 2044
+    assert gemm_plan(K, N.DT_F32, m, n, k)[2] == 2
+    a, b = operands(K, cuda, m, n, k)
+    a *= 2.0 ** exponents[0]
+    b *= 2.0 ** exponents[1]
+    c = multiply(K, cuda, a, b)
+    want, s_abs = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
+    assert bool(((c.double() - want).abs() <= (k + 2) * (2.0 ** -24 * s_abs + 2.0 ** -150)).all())
+
+
 def test_wide_range_of_magnitudes(K, cuda):
     """Every element of its own binade between 2^-40 and 2^40: the error stays relative to the products."""
     m, n, k = 513, 260, 1000
