@@ -63,8 +63,6 @@ struct TilesParams {
     uint32_t tiles_m, tiles_n, group;
     uint32_t k_blocks;                  // of 128 bytes
     uint32_t tn, splits, stages;
-    uint32_t row_blocks;                // of 256 rows that share a tile's B: 1, or 2 where K is not split (dense kinds)
-    uint32_t accs;                      // accumulators: 2, or 1 where two would not fit
     uint32_t kps;                       // K blocks per stage: 1 or 2
     uint32_t tmem_cols;                 // power of two: one accumulator, or two when a cluster has several tiles
     float alpha;
@@ -141,22 +139,25 @@ __device__ __forceinline__ void tma_load_pair_3d_at(void *smem_dst, const CUtens
         : "memory");
 }
 
-template <int DT>
+// kRowBlocks: of 256 rows that share a tile's B, 1 or 2.  A template parameter, because as one of the launch the small
+// shapes took 1.4 % longer.
+template <int DT, uint32_t kRowBlocks>
 __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_constant__ TilesMapsOf<DT> maps, TilesParams p)
 {
     constexpr bool kFp4 = TilesKind<DT>::fp4;
     constexpr uint32_t kWords = TilesKind<DT>::words;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const uint32_t row_blocks = kFp4 ? 1 : p.row_blocks, b_at = row_blocks * kHalfTileBytes;
-    const uint32_t block_bytes = tiles_block_bytes(p.tn, row_blocks), stage_bytes = p.kps * block_bytes + (kFp4 ? tiles_sf_bytes(p.tn) : 0);
+    constexpr uint32_t b_at = kRowBlocks * kHalfTileBytes;
+    const uint32_t block_bytes = tiles_block_bytes(p.tn, kRowBlocks), stage_bytes = p.kps * block_bytes + (kFp4 ? tiles_sf_bytes(p.tn) : 0);
     uint8_t *staging = smem + (size_t)p.stages * stage_bytes;
     TilesSmem *sh = reinterpret_cast<TilesSmem *>(staging + kEpilogueWarps * kStagingBytes);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank(), r = rank & 1, leader = rank & ~1u, split = rank >> 1;
     const uint32_t cluster_id = blockIdx.x / (2 * p.splits), n_clusters = gridDim.x / (2 * p.splits);
-    const uint32_t n_tiles = p.tiles_m * p.tiles_n, accs = kFp4 ? 2 : p.accs;
+    const uint32_t n_tiles = p.tiles_m * p.tiles_n;
+    const bool two_accs = kRowBlocks == 1 || p.tn <= 128;        // two accumulators where they fit
     const uint32_t kb0 = split * p.k_blocks / p.splits, kb1 = (split + 1) * p.k_blocks / p.splits;
 
     if (threadIdx.x == 0) {
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
         for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters) {
             uint32_t mb, nb;
             dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
-            const int32_t row_a = (int32_t)(mb * row_blocks * kTilesM + r * 128), row_b = (int32_t)(nb * p.tn + r * (p.tn / 2));
+            const int32_t row_a = (int32_t)(mb * kRowBlocks * kTilesM + r * 128), row_b = (int32_t)(nb * p.tn + r * (p.tn / 2));
             for (uint32_t kb = kb0; kb < kb1; kb += p.kps) {
                 if (!warp_wait(&sh->empty[s], parity)) {       // a fresh barrier's preceding phase counts as complete
                     if (lane == 0)
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
                         if (h < nk) {
                             uint8_t *blk = st + h * block_bytes;
                             tma_load_pair_at(blk, &maps.a, x + h * kRowBytesK, row_a, full0 + 8 * s);
-                            if (row_blocks == 2)
+                            if constexpr (kRowBlocks == 2)
                                 tma_load_pair_at(blk + kHalfTileBytes, &maps.a, x + h * kRowBytesK, row_a + (int32_t)kTilesM, full0 + 8 * s);
                             tma_load_pair_at(blk + b_at, &maps.b, x + h * kRowBytesK, row_b, full0 + 8 * s);
                         }
@@ -259,14 +260,14 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
             uint32_t s = 0, parity = 0, tcount = 0;
             bool ok = true;
             for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters, tcount++) {
-                const uint32_t acc = tcount % accs, use = tcount / accs;
+                const uint32_t acc = two_accs ? tcount & 1 : 0, use = two_accs ? tcount >> 1 : tcount;
                 if (use > 0 && !warp_wait(&sh->tmem_empty[acc], (use - 1) & 1)) {
                     if (lane == 0)
                         atomicCAS(p.status, 0u, 0x222u);
                     break;
                 }
                 tc_fence_after_sync();
-                const uint32_t d = tmem + acc * row_blocks * p.tn;
+                const uint32_t d = tmem + acc * kRowBlocks * p.tn;
                 [[maybe_unused]] uint32_t mb, nb = 0;
                 if constexpr (kFp4)
                     dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
                                 }
                             };
                             multiply(d, make_smem_desc(blk, 16, 1024, kSwizzle128B));
-                            if (row_blocks == 2)
+                            if constexpr (kRowBlocks == 2)
                                 multiply(d + p.tn, make_smem_desc(blk + kHalfTileBytes, 16, 1024, kSwizzle128B));
                         }
                         tc_commit_pair(&sh->empty[s_now], pair_mask);
@@ -346,7 +347,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
         for (uint32_t tile = cluster_id; tile < n_tiles; tile += n_clusters, tcount++) {
             uint32_t mb, nb;
             dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
-            const uint32_t acc = tcount % accs, use = tcount / accs;
+            const uint32_t acc = two_accs ? tcount & 1 : 0, use = two_accs ? tcount >> 1 : tcount;
             if (!warp_wait(&sh->tmem_full[acc], use & 1)) {
                 if (lane == 0)
                     atomicCAS(p.status, 0u, 0x224u);
@@ -354,11 +355,11 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
             }
             tc_fence_after_sync();
             // the row blocks' chunks lie one behind another in tensor memory
-            const uint32_t all_chunks = row_blocks * n_chunks;
-            const uint32_t taddr = tmem + acc * row_blocks * p.tn + ((q * 32) << 16);
-            const uint32_t row = mb * row_blocks * kTilesM + r * 128 + q * 32;
+            const uint32_t all_chunks = kRowBlocks * n_chunks;
+            const uint32_t taddr = tmem + acc * kRowBlocks * p.tn + ((q * 32) << 16);
+            const uint32_t row = mb * kRowBlocks * kTilesM + r * 128 + q * 32;
             auto store = [&](uint32_t (&v)[32], uint32_t c) {
-                const uint32_t block = c >= n_chunks ? 1 : 0;
+                const uint32_t block = kRowBlocks == 2 && c >= n_chunks ? 1 : 0;
                 tiles_store_chunk<DT>(v, p.alpha, boxes, n_stored, &maps.c, nb * p.tn + (c - block * n_chunks) * kTilesChunk, row + block * kTilesM, lane);
             };
             auto release = [&]() {

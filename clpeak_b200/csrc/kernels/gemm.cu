@@ -1126,8 +1126,10 @@ struct TilesPlan {
 //   gemm_tiles_kernel, FP4    3.3 + waves * (K blocks * (0.25 + 0.06 W + T at 62 TB/s) + 1.4 W) and the same exchange
 //   gemm_tiles_kernel, 512    4.75 + waves * (K blocks * (0.157 + 0.344 W + T at 106 TB/s) + 1.2 W of epilogue, 3.2 W from
 //                             tn = 160 on, where tensor memory holds one accumulator); from 24000 launches, residual 6 %.
-//                             Asked for only where gemm_kernel would be taken: of 1269 such shapes of up to four waves
-//                             some 570 take it, 1.22 times faster in the geometric mean, one of them 3 % slower; against
+//                             Not used beyond four waves, narrow ones not beyond two (e4m3 13065 x 1248 x 464, four waves
+//                             of tn = 128: 14.6 us in large tiles, 18.6 in these), and only where gemm_kernel would be taken: 5939 random
+//                             shapes that take it are 1.15 times as fast in the geometric mean, 33 of them 2 to 10 %
+//                             slower (long sums in one wave); against
 //                             the 256-row tiles the estimate is not sharp enough (228 of 831 more than 2 % slower)
 // Splits of 2 and 4 are clusters of 4 and 8 CTAs, of which the chip holds 33 and 15 at a time.  From the fifth wave of
 // 512 x 256 tiles on (16384 x 16384 x 256: 140 against 142 us) and the third of block-scaled ones the large tiles'
@@ -1179,6 +1181,8 @@ static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4,
     if (!fp4 && plan.tn == 0) {
         for (uint32_t tn = 32; tn < 256; tn += 32) {
             const uint64_t tiles = (uint64_t)ceil_div(m, kDenseTileM) * ceil_div(n, tn);
+            if (tiles > (tn >= 192 ? 4ull : 2ull) * pairs)
+                continue;
             const float waves = (float)((tiles - 1) / pairs + 1), wide = (float)tn / 256.0f;
             const float loaded = (float)(tiles < pairs ? tiles : pairs) * ((m < kDenseTileM ? m : kDenseTileM) + (n < tn ? n : tn)) * kRowBytesK;
             const float t = 4.75f + waves * (k_blocks * (0.157f + 0.344f * wide + loaded / 105.6e6f) + (tn > 128 ? 3.2f : 1.2f) * wide);
@@ -1243,7 +1247,7 @@ static int launch_clusters(void (*kernel)(Maps, Params), const char *what, uint3
 }
 
 // wsa, wsb: the packed scale factors (block-scaled kinds)
-template <int DT>
+template <int DT, uint32_t kRowBlocks = 1>
 static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64_t row_bytes, uint32_t k_blocks, TilesPlan plan, cudaStream_t s,
                         const uint8_t *wsa = nullptr, const uint8_t *wsb = nullptr)
 {
@@ -1265,9 +1269,7 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
             return rc;
     }
     TilesParams p;
-    p.row_blocks = plan.row_blocks;
-    p.accs = plan.row_blocks * plan.tn > 256 ? 1 : 2;
-    p.tiles_m = (a->m - 1) / (kTilesM * plan.row_blocks) + 1;
+    p.tiles_m = (a->m - 1) / (kTilesM * kRowBlocks) + 1;
     p.tiles_n = (a->n + plan.tn - 1) / plan.tn;
     p.group = tuning(CLPK_TUNE_GEMM_GROUP) > 0 ? (uint32_t)tuning(CLPK_TUNE_GEMM_GROUP) : 8;
     p.k_blocks = k_blocks;
@@ -1281,18 +1283,24 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
     // two K blocks per stage halve the hand-overs (0.195 -> 0.137 us per block at TN = 32), but from TN = 160 on leave
     // too few stages (2048^3 bf16 at TN = 192: 19.3 -> 20.7 us)
     constexpr bool fp4 = TilesKind<DT>::fp4;
-    p.kps = plan.tn <= 128 && plan.row_blocks == 1 && !fp4 ? 2 : 1;
-    const uint32_t stage_bytes = p.kps * tiles_block_bytes(plan.tn, plan.row_blocks) + (fp4 ? tiles_sf_bytes(plan.tn) : 0);
+    p.kps = plan.tn <= 128 && kRowBlocks == 1 && !fp4 ? 2 : 1;
+    const uint32_t stage_bytes = p.kps * tiles_block_bytes(plan.tn, kRowBlocks) + (fp4 ? tiles_sf_bytes(plan.tn) : 0);
     p.stages = (uint32_t)((kTilesSmemMax - fixed) / stage_bytes);
     const uint32_t most = fp4 ? 256 / tiles_sf_cols(plan.tn) : kTilesMaxStages;      // scale factors: 256 tensor-memory columns
     if (p.stages > most)
         p.stages = most;
     p.tmem_cols = fp4 ? 512 : 32;
-    while (p.tmem_cols < (n_tiles > clusters ? p.accs : 1) * plan.row_blocks * plan.tn)
+    while (p.tmem_cols < (n_tiles > clusters && (kRowBlocks == 1 || plan.tn <= 128) ? 2 : 1) * kRowBlocks * plan.tn)
         p.tmem_cols *= 2;
     CLPK_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&p.clock), g_gemm_clock));
     const size_t smem = p.stages * stage_bytes + fixed;
-    return launch_clusters(gemm_tiles_kernel<DT>, "gemm_tiles", clusters * 2 * plan.splits, kGemmThreads, smem, 2 * plan.splits, s, maps, p);
+    return launch_clusters(gemm_tiles_kernel<DT, kRowBlocks>, "gemm_tiles", clusters * 2 * plan.splits, kGemmThreads, smem, 2 * plan.splits, s, maps, p);
+}
+
+template <int DT>
+static int launch_dense_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64_t row_bytes, uint32_t k_blocks, TilesPlan plan, cudaStream_t s)
+{
+    return plan.row_blocks == 2 ? launch_tiles<DT, 2>(a, ta, row_bytes, k_blocks, plan, s) : launch_tiles<DT>(a, ta, row_bytes, k_blocks, plan, s);
 }
 
 template <int DT>
@@ -1632,12 +1640,12 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
     }
     if (const TilesPlan plan = gemm_plan(a->m, a->n, a->k, elem_bits, false); plan.tn) {
         switch (a->dtype) {
-        case CLPK_DT_BF16: return launch_tiles<CLPK_DT_BF16>(a, ta, row_bytes, p.k_blocks, plan, s);
-        case CLPK_DT_F16:  return launch_tiles<CLPK_DT_F16>(a, ta, row_bytes, p.k_blocks, plan, s);
-        case CLPK_DT_TF32: return launch_tiles<CLPK_DT_TF32>(a, ta, row_bytes, p.k_blocks, plan, s);
-        case CLPK_DT_I8:   return launch_tiles<CLPK_DT_I8>(a, ta, row_bytes, p.k_blocks, plan, s);
-        case CLPK_DT_E5M2: return launch_tiles<CLPK_DT_E5M2>(a, ta, row_bytes, p.k_blocks, plan, s);
-        default:           return launch_tiles<CLPK_DT_E4M3>(a, ta, row_bytes, p.k_blocks, plan, s);
+        case CLPK_DT_BF16: return launch_dense_tiles<CLPK_DT_BF16>(a, ta, row_bytes, p.k_blocks, plan, s);
+        case CLPK_DT_F16:  return launch_dense_tiles<CLPK_DT_F16>(a, ta, row_bytes, p.k_blocks, plan, s);
+        case CLPK_DT_TF32: return launch_dense_tiles<CLPK_DT_TF32>(a, ta, row_bytes, p.k_blocks, plan, s);
+        case CLPK_DT_I8:   return launch_dense_tiles<CLPK_DT_I8>(a, ta, row_bytes, p.k_blocks, plan, s);
+        case CLPK_DT_E5M2: return launch_dense_tiles<CLPK_DT_E5M2>(a, ta, row_bytes, p.k_blocks, plan, s);
+        default:           return launch_dense_tiles<CLPK_DT_E4M3>(a, ta, row_bytes, p.k_blocks, plan, s);
         }
     }
     CUtensorMap tc;

@@ -9,8 +9,8 @@ from tests.test_gpu_gemm_tiles import check_every_element, elements_of
 pytestmark = pytest.mark.gpu
 
 # (tile width, several tiles per pair, (m, n, bytes of K))
-PLANS = [(96, True, (15919, 848, 400)), (128, True, (15638, 824, 400)), (160, False, (305, 9928, 2576)), (160, True, (14827, 792, 3216)),
-         (192, False, (326, 11992, 2960)), (192, True, (11357, 1064, 1808)), (224, True, (6150, 3656, 1552))]
+PLANS = [(96, True, (12912, 400, 272)), (160, False, (305, 9928, 2576)), (160, True, (14827, 792, 3216)),
+         (192, False, (326, 11992, 2960)), (192, True, (11357, 1064, 1808)), (224, False, (12317, 392, 5008)), (224, True, (6150, 3656, 1552))]
 
 
 @pytest.mark.parametrize("tile_n,several,shape", PLANS)
