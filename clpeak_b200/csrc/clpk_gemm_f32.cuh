@@ -48,7 +48,7 @@ constexpr int kF32SumWarps = 8;
 constexpr uint32_t kF32LaunchRegs = 96, kF32IssueRegs = 32, kF32ConverterRegs = 72, kF32SumRegs = 152;
 static_assert(128 * kF32IssueRegs + 128 * kF32Groups * kF32ConverterRegs + 32 * kF32SumWarps * kF32SumRegs <= kF32Threads * kF32LaunchRegs, "no share may wait for registers that nobody gives back");
 constexpr uint32_t kF32BoxLd = 20;                       // floats per row of a warp's 32 x 16 staging box
-constexpr uint32_t kF32TileFlags = 16;                   // converters are at most six chunks ahead of the sums
+constexpr uint32_t kF32TileFlags = 16;                   // converters are fewer tiles ahead of the sums: four turns and four chunks
 constexpr float kF32Smallest = 0x1p-100f;
 
 template <uint32_t TN> struct F32Tile {
