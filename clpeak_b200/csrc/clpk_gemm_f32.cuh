@@ -464,9 +464,13 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
 #pragma unroll 1
                     for (uint32_t j = 0; j < 8; j++)
                         in_a |= any_too_small(*reinterpret_cast<const float4 *>(st + row * 128 + ((j ^ (row & 7)) << 4)));
+                    // the rows of B that this warp has converted, which only it looks at
 #pragma unroll 1
-                    for (uint32_t j = cw * 32 + lane; j < T::half_n * 8; j += 128)
-                        in_b |= any_too_small(*reinterpret_cast<const float4 *>(st + T::a_bytes + 16 * j));
+                    for (uint32_t i = 0; cw + 4 * i < kSteps; i++) {
+                        const uint8_t *src = st + T::a_bytes + step_row(i) * 128;
+                        in_b |= any_too_small(*reinterpret_cast<const float4 *>(src + (((2 * g) ^ (step_row(i) & 7)) << 4)));
+                        in_b |= any_too_small(*reinterpret_cast<const float4 *>(src + (((2 * g + 1) ^ (step_row(i) & 7)) << 4)));
+                    }
                     in_a = __any_sync(0xffffffffu, in_a);
                     in_b = __any_sync(0xffffffffu, in_b);
                     const uint32_t flag = tcount % kF32TileFlags;

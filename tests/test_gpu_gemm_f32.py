@@ -94,6 +94,38 @@ def test_small_magnitudes_keep_their_bits(K, cuda, shape, small, large):
     assert bool((c[100] == 0.0).all()) and bool((c[:, 11] == 0.0).all())
 
 
+@pytest.mark.parametrize("plan,shape", PLANS)
+def test_one_small_element_at_every_row_of_a_tile(K, cuda, plan, shape):
+    """One row of a tile holds zeros and one magnitude that bf16 pieces of the element itself could not hold, the others N(0, 0.02);
+    the other operand is near 2^100, so that the small element's products are ordinary numbers: every row of the tile, in the
+    tile's halves that the two CTAs of a pair convert, in the first, a middle and the last chunk, with K split and not."""
+    assert gemm_plan(K, N.DT_F32, *shape) == (*plan, 2)
+    (m, n, k), tn = shape, plan[0]
+    a, b = operands(K, cuda, *shape)
+    smalls, columns = (2.0 ** -120, 1.375 * 2.0 ** -130, 1.25 * 2.0 ** -140), (0, k - 1, k // 2 + 1)
+    failed = []
+    # every row of B at every magnitude, every row of A at one of them
+    for operand, other, tile, runs in ((b, a, tn, [(r, v) for r in range(tn) for v in range(3)]), (a, b, 256, [(r, r % 3) for r in range(256)])):
+        saved = operand.clone()
+        other *= 2.0 ** 100
+        for r, v in runs:
+            if r >= operand.shape[0]:
+                continue
+            rows = cuda.arange(r, operand.shape[0], tile, device="cuda")
+            at, small = columns[(r + v) % 3], smalls[v]
+            operand[rows] = 0.0
+            operand[rows, at] = small
+            c = multiply(K, cuda, a, b)
+            got = (c[:, rows].T if operand is b else c[rows]).double()
+            want = other[:, at].double() * float(cuda.tensor(small, dtype=cuda.float32))
+            # one product, of which at most 2^-24 is left out, and a rounding of it and of alpha
+            if not bool(((got - want).abs() <= 3 * 2.0 ** -24 * want.abs()).all()):
+                failed.append(("B" if operand is b else "A", r, small))
+            operand[rows] = saved[rows]
+        other *= 2.0 ** -100
+    assert not failed, f"{len(failed)} of the single elements are lost, the first: {failed[:5]}"
+
+
 @pytest.mark.parametrize("exponents", [(-70, -70), (-60, -72), (-63, -75), (-40, -66)])
 def test_results_near_the_end_of_the_range(K, cuda, exponents):
     """Products that fp32 holds only in part: K roundings to 2^-149 besides the relative ones."""
