@@ -1,11 +1,20 @@
 // The fp32 GEMM on the tensor cores (included by gemm.cu).
 //
 // An fp32 number is the sum of three bf16 numbers: h is x rounded to bf16, m what is left rounded to bf16, and l what is
-// left then, which has no more than eight significand bits -- h + m + l = x exactly, with |m| <= 2^-9 |x| and
-// |l| <= 2^-18 |x|.  A product of two fp32 numbers is then nine bf16 products, each exact in fp32; the three smallest
-// (m l, l m, l l: at most 2^-26 of the product together, of either sign) are left out, which is a quarter of the rounding
+// left then, which has no more than eight significand bits -- h + m + l = x exactly, with |m| <= 2^-8 |x| and
+// |l| <= 2^-17 |x|.  A product of two fp32 numbers is then nine bf16 products, each exact in fp32; the three smallest
+// (m l, l m, l l: at most 2^-24 of the product together, of either sign) are left out, which is no more than the rounding
 // that one fp32 operation makes.  Six bf16 instructions per K step at the tensor pipe's 16-bit rate are four times what
 // the fp32 pipe does.
+//
+// bf16 ends where fp32 does, so the pieces of a small x would not exist.  The elements are multiplied by 2^16 on the way, after
+// which none has bits below bf16's last one, 2^-133, and 2^8 m and 2^16 l are kept instead of m and l: every finite number up to
+// 2^111, subnormal ones too, is then three bf16 numbers with m and l as far below h as said above.  (Subnormal bf16 operands and
+// sums are not flushed.)  An instruction that takes up products of the next size divides the accumulator by 2^8, and the sums
+// are multiplied by 2^-32 when they leave the registers: results keep their bits down to the end of the fp32 range, with fewer errors
+// there than fused multiply-adds, which round each step to 2^-149 (K = 2044, results near 2^-135: at most 2 units of 2^-149 against 56).
+// With pieces at their own size, tiles with an element or a sum below 2^-100 had to be multiplied again: 40.5 ms for a 4096^3
+// product of that kind against 0.62, and 1.05 for one with zeros, for which the same alarm went off.
 //
 // The tensor cores cut, not round, what they align to the accumulator, so sums are kept short there: a turn of two chunks of 32
 // floats starts from zero, adds the small products first and the h h ones last -- four instructions in which the cut is of
@@ -33,9 +42,8 @@
 // one chunk 658 there, but 953 at TN = 64 against 833.
 //
 // Numbers that the split cannot serve are multiplied as they are, with fused multiply-adds in K order: a warp whose sums
-// are not all finite (an infinity, a NaN or an overflow on the way; x - h of an infinity is a NaN, so none goes unseen)
-// does its 32 x TN / 2 outputs again, and so does one with a sum below 2^-100, whose products' pieces are partly below what
-// fp32 resolves, and a tile that has met a magnitude below 2^-100, of which l would leave the range of bf16.
+// are not all finite (an infinity, a NaN, or an overflow on the way, which the scales bring to about 2^89;
+// x - h of an infinity is a NaN, so none goes unseen) does its 32 x TN / 2 outputs again.
 #pragma once
 
 constexpr uint32_t kF32M = 256;
@@ -48,8 +56,9 @@ constexpr int kF32SumWarps = 8;
 constexpr uint32_t kF32LaunchRegs = 96, kF32IssueRegs = 32, kF32ConverterRegs = 72, kF32SumRegs = 152;
 static_assert(128 * kF32IssueRegs + 128 * kF32Groups * kF32ConverterRegs + 32 * kF32SumWarps * kF32SumRegs <= kF32Threads * kF32LaunchRegs, "no share may wait for registers that nobody gives back");
 constexpr uint32_t kF32BoxLd = 20;                       // floats per row of a warp's 32 x 16 staging box
-constexpr uint32_t kF32TileFlags = 16;                   // converters are fewer tiles ahead of the sums: four turns and four chunks
-constexpr float kF32Smallest = 0x1p-100f;
+constexpr uint32_t kF32PieceShift = 8;                   // bits between the scales of an element's pieces
+constexpr float kF32Scale = 0x1p16f;                     // of the elements of A and of B
+constexpr float kF32Unscale = 0x1p-32f;                  // of the sums, when they leave the registers
 
 template <uint32_t TN> struct F32Tile {
     static constexpr uint32_t half_n = TN / 2;
@@ -70,7 +79,6 @@ struct F32Smem {
     uint64_t raw_full[8], raw_empty[8];
     uint64_t conv_full[4], conv_empty[4];
     uint64_t d_full[4], d_empty[4];
-    uint32_t small[kF32TileFlags];       // one more than the number of the last tile there that met too small a magnitude
     uint32_t tmem_base;
 };
 static_assert(sizeof(F32Smem) <= 512, "the room that F32Tile leaves for it");
@@ -105,33 +113,57 @@ __device__ __forceinline__ void bf16x2_minus(uint32_t h, float x0, float x1, flo
         : "=f"(d0), "=f"(d1)
         : "r"(h), "f"(x0), "f"(x1));
 }
-__device__ __forceinline__ bool too_small(float x) { return fabsf(x) < kF32Smallest && x != 0.0f; }
-
-__device__ __forceinline__ bool any_too_small(float4 x) { return too_small(x.x) || too_small(x.y) || too_small(x.z) || too_small(x.w); }
-
-// Two floats -> their three bf16 pairs, m with the other sign (the instructions that multiply it with an h negate it again).
-// `least` keeps the smallest magnitude met.
-__device__ __forceinline__ void split_bf16x3(float x0, float x1, uint32_t &h, uint32_t &m, uint32_t &l, float &least)
+// two floats times a power of two, of either sign
+__device__ __forceinline__ void scale_pair(float &x0, float &x1, float by)
 {
-    least = fminf(fminf(fabsf(x0), fabsf(x1)), least);
+    asm("{\n\t"
+        ".reg .b64 x, f;\n\t"
+        "mov.b64 x, {%0, %1};\n\t"
+        "mov.b64 f, {%2, %2};\n\t"
+        "mul.rn.f32x2 x, x, f;\n\t"
+        "mov.b64 {%0, %1}, x;\n\t"
+        "}"
+        : "+f"(x0), "+f"(x1)
+        : "f"(by));
+}
+
+// Two floats -> the three bf16 pairs h, 2^8 m and 2^16 l of their products with kF32Scale.
+__device__ __forceinline__ void split_bf16x3(float x0, float x1, uint32_t &h, uint32_t &m, uint32_t &l)
+{
+    constexpr float kBy = -(float)(1u << kF32PieceShift);                // what bf16x2_minus leaves has the other sign
     float r0, r1, s0, s1;
+    scale_pair(x0, x1, kF32Scale);
     h = pack_bf16x2(x0, x1);
     bf16x2_minus(h, x0, x1, r0, r1);
+    scale_pair(r0, r1, kBy);
     m = pack_bf16x2(r0, r1);
     bf16x2_minus(m, r0, r1, s0, s1);
+    scale_pair(s0, s1, kBy);
     l = pack_bf16x2(s0, s1);
 }
 
-__device__ __forceinline__ void mma2_bf16_ts(uint32_t d, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+// D = A B, D + A B, or 2^-kF32PieceShift D + A B
+enum class Into { fresh, sum, shifted };
+__device__ __forceinline__ void mma2_bf16_ts(uint32_t d, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, Into into)
 {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-        "}\n" ::"r"(d),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if (into == Into::shifted)
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            "setp.eq.u32 p, 0, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t"
+            "}\n" ::"r"(d),
+            "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(kF32PieceShift)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            "setp.ne.u32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+            "}\n" ::"r"(d),
+            "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(into == Into::sum ? 1 : 0)
+            : "memory");
 }
 
 template <bool INC, uint32_t N>
@@ -169,7 +201,7 @@ __device__ __forceinline__ void tma_load_own(void *smem_dst, const CUtensorMap *
         : "memory");
 }
 
-// Arrive on a barrier of the pair's leader.  What is handed over lies in this CTA's own tensor and shared memory, complete
+// Arrive on a barrier of the pair's leader.  All that is handed over lies in this CTA's own tensor and shared memory, complete
 // (tcgen05.wait::st) and fenced for the tensor core that reads it, so no wider release than the default is needed: with
 // .release.cluster each arrive held its warp for about 1000 cycles.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar)
@@ -217,11 +249,6 @@ __device__ __forceinline__ bool team_agrees(uint32_t barrier, bool ok)
         : "r"(ok ? 1u : 0u), "r"(barrier), "n"(THREADS)
         : "memory");
     return all != 0;
-}
-
-__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v)
-{
-    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
 // The sums of one thread again, as they are defined: fused multiply-adds over k0 ... k1 in order.  Row and columns beyond
@@ -275,8 +302,6 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
             mbar_init(&sh->d_full[d], 1);
             mbar_init(&sh->d_empty[d], 2 * kF32SumWarps);
         }
-        for (uint32_t t = 0; t < kF32TileFlags; t++)
-            sh->small[t] = 0;
         mbar_fence_init();
         tma_prefetch_desc(&maps.a);
         tma_prefetch_desc(&maps.b);
@@ -330,7 +355,6 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
         // ---------------- MMA issuers (the pair's leader), every other turn each ----------------
         if (r == 0) {
             const uint32_t idesc = make_idesc(256, TN, kFmtBF16, kFmtBF16, kAccF32);
-            constexpr uint32_t kNegateA = 1u << 13;                       // see split_bf16x3
             const uint16_t pair_mask = (uint16_t)(3u << leader);
             uint32_t turn = 0, chunk = 0;
             bool ok = true;
@@ -349,29 +373,33 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                         tc_fence_after_sync();
                         if (elect_one()) {
                             const uint32_t acc = tmem + d * TN;
-                            // product t = (plane of A, plane of B) of the chunk in stage s
-                            auto multiply = [&](uint32_t s, uint32_t t, uint32_t fresh) {
-                                constexpr uint32_t kOrder[6][2] = {{2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}, {0, 0}};
-                                const uint32_t a = tmem + T::accs * TN + s * T::a_cols + 16 * kOrder[t][0];
+                            // plane pa of A times plane pb of B of the chunk in stage s
+                            auto multiply = [&](uint32_t s, uint32_t pa, uint32_t pb, Into into) {
+                                const uint32_t a = tmem + T::accs * TN + s * T::a_cols + 16 * pa;
                                 const uint64_t b = make_smem_desc(smem_u32(planes + (size_t)s * 3 * T::plane_bytes), 16, 512, kSwizzle64B) +
-                                                   kOrder[t][1] * T::plane_bytes / 16;
-                                const uint32_t id = kOrder[t][0] + kOrder[t][1] == 1 ? idesc | kNegateA : idesc;
-                                mma2_bf16_ts(acc, a, b, id, fresh ? 0u : 1u);
-                                mma2_bf16_ts(acc, a + 8, b + 2, id, 1u);
+                                                   pb * T::plane_bytes / 16;
+                                mma2_bf16_ts(acc, a, b, idesc, into);
+                                mma2_bf16_ts(acc, a + 8, b + 2, idesc, Into::sum);
                             };
-                            // the smallest products first, those of full size last
-#pragma unroll
-                            for (uint32_t t = 0; t < 5; t++)
-                                multiply(s0, t, t == 0);
+                            // the smallest products first, at 2^16 times their size, those of full size last
+                            multiply(s0, 2, 0, Into::fresh);
+                            multiply(s0, 0, 2, Into::sum);
+                            multiply(s0, 1, 1, Into::sum);
                             if (two) {
-#pragma unroll
-                                for (uint32_t t = 0; t < 5; t++)
-                                    multiply(s1, t, 0);
+                                multiply(s1, 2, 0, Into::sum);
+                                multiply(s1, 0, 2, Into::sum);
+                                multiply(s1, 1, 1, Into::sum);
                             }
-                            multiply(s0, 5, 0);
+                            multiply(s0, 1, 0, Into::shifted);
+                            multiply(s0, 0, 1, Into::sum);
+                            if (two) {
+                                multiply(s1, 1, 0, Into::sum);
+                                multiply(s1, 0, 1, Into::sum);
+                            }
+                            multiply(s0, 0, 0, Into::shifted);
                             tc_commit_pair(&sh->conv_empty[s0], pair_mask);
                             if (two) {
-                                multiply(s1, 5, 0);
+                                multiply(s1, 0, 0, Into::sum);
                                 tc_commit_pair(&sh->conv_empty[s1], pair_mask);
                             }
                             tc_commit_pair(&sh->d_full[d], pair_mask);
@@ -389,11 +417,9 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
         set_max_registers<false, kF32ConverterRegs>();
         const uint32_t cw = (uint32_t)warp & 3, group = (uint32_t)(warp - 4) >> 2;
         const uint32_t full0 = cluster_addr(&sh->conv_full[0], leader);
-        uint32_t count = 0, tcount = 0;
+        uint32_t count = 0;
         bool ok = true;
-        for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters, tcount++) {
-            uint32_t mb, nb;
-            dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
+        for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters) {
             for (uint32_t c = c0; c < c1; c++, count++) {
                 if (count % kF32Groups != group)
                     continue;
@@ -420,7 +446,6 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                         xb[i][1] = *reinterpret_cast<const float4 *>(src + (((2 * g + 1) ^ (step_row(i) & 7)) << 4));
                     }
                 const uint32_t row = cw * 32 + lane;
-                float least_a = 1.0f, least_b = 1.0f;
 #pragma unroll
                 for (uint32_t kk = 0; kk < 2; kk++) {
                     float4 xa[4];
@@ -428,14 +453,11 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                     for (uint32_t j = 0; j < 4; j++)
                         xa[j] = *reinterpret_cast<const float4 *>(st + row * 128 + (((4 * kk + j) ^ (row & 7)) << 4));
                     if (4 * kk < kSteps && cw + 4 * kk < kSteps) {
-                        float least = 1.0f;
                         uint4 h, m, l;
-                        split_bf16x3(xb[kk][0].x, xb[kk][0].y, h.x, m.x, l.x, least);
-                        split_bf16x3(xb[kk][0].z, xb[kk][0].w, h.y, m.y, l.y, least);
-                        split_bf16x3(xb[kk][1].x, xb[kk][1].y, h.z, m.z, l.z, least);
-                        split_bf16x3(xb[kk][1].z, xb[kk][1].w, h.w, m.w, l.w, least);
-                        if (nb * TN + r * T::half_n + step_row(kk) < p.n)
-                            least_b = fminf(least_b, least);
+                        split_bf16x3(xb[kk][0].x, xb[kk][0].y, h.x, m.x, l.x);
+                        split_bf16x3(xb[kk][0].z, xb[kk][0].w, h.y, m.y, l.y);
+                        split_bf16x3(xb[kk][1].x, xb[kk][1].y, h.z, m.z, l.z);
+                        split_bf16x3(xb[kk][1].z, xb[kk][1].w, h.w, m.w, l.w);
                         uint8_t *at = dst + step_row(kk) * 64 + ((g ^ ((step_row(kk) >> 1) & 3)) << 4);
                         *reinterpret_cast<uint4 *>(at) = h;
                         *reinterpret_cast<uint4 *>(at + T::plane_bytes) = m;
@@ -444,8 +466,8 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                     uint32_t h[8], m[8], l[8];
 #pragma unroll
                     for (uint32_t j = 0; j < 4; j++) {
-                        split_bf16x3(xa[j].x, xa[j].y, h[2 * j], m[2 * j], l[2 * j], least_a);
-                        split_bf16x3(xa[j].z, xa[j].w, h[2 * j + 1], m[2 * j + 1], l[2 * j + 1], least_a);
+                        split_bf16x3(xa[j].x, xa[j].y, h[2 * j], m[2 * j], l[2 * j]);
+                        split_bf16x3(xa[j].z, xa[j].w, h[2 * j + 1], m[2 * j + 1], l[2 * j + 1]);
                     }
                     const uint32_t taddr = tmem + T::accs * TN + s * T::a_cols + 8 * kk + ((cw * 32) << 16);
                     tmem_st_32x32b_x8(taddr, h);
@@ -455,30 +477,6 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                 tmem_st_wait();
                 tc_fence_before_sync();
                 fence_proxy_async_smem();
-                // rows beyond the operands are zeros that say nothing
-                if (mb * kF32M + r * 128 + row >= p.m)
-                    least_a = 1.0f;
-                if (__any_sync(0xffffffffu, fminf(least_a, least_b) < kF32Smallest)) {
-                    // zeros are small and welcome: look again
-                    bool in_a = false, in_b = false;
-#pragma unroll 1
-                    for (uint32_t j = 0; j < 8; j++)
-                        in_a |= any_too_small(*reinterpret_cast<const float4 *>(st + row * 128 + ((j ^ (row & 7)) << 4)));
-                    // the rows of B that this warp has converted, which only it looks at
-#pragma unroll 1
-                    for (uint32_t i = 0; cw + 4 * i < kSteps; i++) {
-                        const uint8_t *src = st + T::a_bytes + step_row(i) * 128;
-                        in_b |= any_too_small(*reinterpret_cast<const float4 *>(src + (((2 * g) ^ (step_row(i) & 7)) << 4)));
-                        in_b |= any_too_small(*reinterpret_cast<const float4 *>(src + (((2 * g + 1) ^ (step_row(i) & 7)) << 4)));
-                    }
-                    in_a = __any_sync(0xffffffffu, in_a);
-                    in_b = __any_sync(0xffffffffu, in_b);
-                    const uint32_t flag = tcount % kF32TileFlags;
-                    if (lane == 0 && (in_a || in_b))
-                        st_cluster_u32(cluster_addr(&sh->small[flag], rank), tcount + 1);
-                    if (lane == 0 && in_b)                                // this half of B is the other CTA's too
-                        st_cluster_u32(cluster_addr(&sh->small[flag], rank ^ 1), tcount + 1);
-                }
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(&sh->raw_empty[raw]);
@@ -501,9 +499,9 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
         float *box = reinterpret_cast<float *>(boxes + (size_t)(warp - kF32FirstSum) * T::box_bytes);
         const uint32_t own4 = T::half_n / 4 / p.splits;                   // groups of four columns that this pair stores
         auto owner_of = [&](uint32_t g) { return g * p.splits / (T::half_n / 4); };
-        uint32_t count = 0, tcount = 0;
+        uint32_t count = 0;
         bool ok = true;
-        for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters, tcount++) {
+        for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters) {
             uint32_t mb, nb;
             dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
             const uint32_t row0 = mb * kF32M + r * 128 + q * 32, col0 = nb * TN + half * T::half_n;
@@ -551,15 +549,13 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                 }
             }
             if (ok) {
-                bool again = *reinterpret_cast<volatile uint32_t *>(&sh->small[tcount % kF32TileFlags]) == tcount + 1;
                 float probe = 0.0f;                                       // not finite: 0 x = NaN
 #pragma unroll
                 for (uint32_t i = 0; i < T::half_n; i++) {
                     probe = fmaf(sum[i], 0.0f, probe);
-                    again |= too_small(sum[i]);
+                    sum[i] *= kF32Unscale;
                 }
-                again |= probe != 0.0f;
-                if (__any_sync(0xffffffffu, again)) {
+                if (__any_sync(0xffffffffu, probe != 0.0f)) {
                     float slow[T::half_n];
                     const uint32_t k1 = c1 * kF32Chunk < p.k ? c1 * kF32Chunk : p.k;
                     f32_sums_as_defined<T::half_n>(slow, p.a, p.b, row0 + lane, col0, p.m, p.n, p.k, c0 * kF32Chunk, k1);

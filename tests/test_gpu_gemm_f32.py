@@ -83,7 +83,7 @@ def test_infinities_nans_and_overflow(K, cuda, shape):
 @pytest.mark.parametrize("shape", [(300, 200, 1024), (2000, 1500, 260)])
 @pytest.mark.parametrize("small,large", [(2.0 ** -96, 2.0 ** 90), (2.0 ** -110, 2.0 ** 100), (2.0 ** -140, 2.0 ** 120)])
 def test_small_magnitudes_keep_their_bits(K, cuda, shape, small, large):
-    """Where the third bf16 piece of an element would leave bf16's range the tile is multiplied as it is; zeros stay zeros."""
+    """Elements whose pieces at their own size would leave bf16's range; zeros stay zeros."""
     a, b = operands(K, cuda, *shape)
     a[5:9] *= small
     a[100] = 0.0
@@ -96,7 +96,7 @@ def test_small_magnitudes_keep_their_bits(K, cuda, shape, small, large):
 
 @pytest.mark.parametrize("plan,shape", PLANS)
 def test_one_small_element_at_every_row_of_a_tile(K, cuda, plan, shape):
-    """One row of a tile holds zeros and one magnitude that bf16 pieces of the element itself could not hold, the others N(0, 0.02);
+    """One row of a tile holds zeros and one magnitude that bf16 pieces at their own size could not hold, the others N(0, 0.02);
     the other operand is near 2^100, so that the small element's products are ordinary numbers: every row of the tile, in the
     tile's halves that the two CTAs of a pair convert, in the first, a middle and the last chunk, with K split and not."""
     assert gemm_plan(K, N.DT_F32, *shape) == (*plan, 2)
@@ -137,6 +137,46 @@ def test_results_near_the_end_of_the_range(K, cuda, exponents):
     c = multiply(K, cuda, a, b)
     want, s_abs = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
     assert bool(((c.double() - want).abs() <= (k + 2) * (2.0 ** -24 * s_abs + 2.0 ** -150)).all())
+
+
+@pytest.mark.parametrize("exponents", [(-64, -64), (-68, -68), (-58, -70), (-100, -28), (-134, 0), (0, -134), (-120, 60), (60, -135)])
+@pytest.mark.parametrize("plan,shape", [((32, 4), (300, 200, 2044)), ((128, 1), (1544, 2051, 176))])
+def test_small_results_keep_their_bits(K, cuda, plan, shape, exponents):
+    """Results and operands down to the last bits of fp32: the error of larger ones, and a rounding to 2^-149 for each K range and
+    for alpha.  Zeros in their place would be hundreds of such units off."""
+    assert gemm_plan(K, N.DT_F32, *shape) == (*plan, 2)
+    a, b = (cuda.randn(rows, shape[2], generator=cuda.Generator(device="cuda").manual_seed(rows), device="cuda") for rows in shape[:2])
+    a, b = (a.double() * 2.0 ** exponents[0]).float(), (b.double() * 2.0 ** exponents[1]).float()
+    c = multiply(K, cuda, a, b, 0.75)
+    want, s_abs = 0.75 * (a.double() @ b.double().T), 0.75 * (a.double().abs() @ b.double().abs().T)
+    room = bound(shape[2]) * 2.0 ** -24 * s_abs + (plan[1] + 1) * 2.0 ** -150
+    assert bool(((c.double() - want).abs() <= room).all()) and float((want.abs() / room).median()) > 20
+
+
+def test_small_numbers_and_zeros_cost_nothing(K, cuda):
+    """A small element in every row of A, small results, half of A zeros: the time of ordinary operands, within a half."""
+    n = 2048
+    a, b = operands(K, cuda, n, n, n)
+
+    def time(a, b):
+        c, status = dev_empty(n * n, cuda.float32), dev_empty(1, cuda.int32)
+        args = N.GemmArgs(dtype=N.DT_F32, m=n, n=n, k=n, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=1.0, d_status=status.data_ptr())
+        times = []
+        for _ in range(7):
+            start, end = (cuda.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            for _ in range(5):
+                K.clpk_gemm(C.byref(args), stream_ptr())
+            end.record()
+            sync()
+            times.append(start.elapsed_time(end))
+        return sorted(times)[3]
+
+    one_small = a.clone()
+    one_small[:, 7] = 2.0 ** -120
+    ordinary = time(a, b)
+    for x, y in ((one_small, b), (a * 2.0 ** -60, b * 2.0 ** -60), (a.clamp(min=0.0), b)):
+        assert time(x, y) <= 1.5 * ordinary
 
 
 def test_wide_range_of_magnitudes(K, cuda):
