@@ -43,7 +43,7 @@
 //
 // Numbers that the split cannot serve are multiplied as they are, with fused multiply-adds in K order: a warp whose sums
 // are not all finite (an infinity, a NaN, or an overflow on the way, which the scales bring to about 2^89;
-// x - h of an infinity is a NaN, so none goes unseen) does its 32 x TN / 2 outputs again.
+// x - h of an infinity is a NaN, so none goes unseen) does its 32 x TN / 2 outputs again, see f32_tile_as_defined.
 #pragma once
 
 constexpr uint32_t kF32M = 256;
@@ -52,9 +52,7 @@ constexpr int kF32Threads = 640;
 constexpr int kF32Groups = 2;                            // of four converter warps
 constexpr int kF32FirstSum = 4 + 4 * kF32Groups;
 constexpr int kF32SumWarps = 8;
-// registers a thread of the issuing, the converting and the adding warps; the block is launched with 640 x 96
-constexpr uint32_t kF32LaunchRegs = 96, kF32IssueRegs = 32, kF32ConverterRegs = 72, kF32SumRegs = 152;
-static_assert(128 * kF32IssueRegs + 128 * kF32Groups * kF32ConverterRegs + 32 * kF32SumWarps * kF32SumRegs <= kF32Threads * kF32LaunchRegs, "no share may wait for registers that nobody gives back");
+constexpr uint32_t kF32LaunchRegs = 96;                  // a thread of the block is launched with
 constexpr uint32_t kF32BoxLd = 20;                       // floats per row of a warp's 32 x 16 staging box
 constexpr uint32_t kF32PieceShift = 8;                   // bits between the scales of an element's pieces
 constexpr float kF32Scale = 0x1p16f;                     // of the elements of A and of B
@@ -72,6 +70,11 @@ template <uint32_t TN> struct F32Tile {
     static constexpr uint32_t tmem_cols = accs * TN + conv_stages * a_cols > 256 ? 512 : 256;
     static_assert(accs * TN + conv_stages * a_cols <= 512, "tensor memory");
     static constexpr uint32_t box_bytes = 32 * kF32BoxLd * 4;
+    // registers a thread of the issuing, the converting and the adding warps.  With 72 and 152 at every width the converters spill
+    // at 32, 96 and 128 (2 to 7 % longer), with 80 and 144 at 64 (2 %).
+    static constexpr uint32_t issue_regs = 32, converter_regs = TN == 64 ? 72 : 80, sum_regs = TN == 64 ? 152 : 144;
+    static_assert(128 * issue_regs + 128 * kF32Groups * converter_regs + 32 * kF32SumWarps * sum_regs <= kF32Threads * kF32LaunchRegs,
+                  "no share may wait for registers that nobody gives back");
     static constexpr size_t smem_bytes = (size_t)raw_stages * raw_bytes + conv_stages * 3 * plane_bytes + kF32SumWarps * box_bytes + 512 + 1024;
 };
 
@@ -209,6 +212,12 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar)
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
 }
 
+template <int THREADS>
+__device__ __forceinline__ void named_barrier(uint32_t barrier)
+{
+    asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(barrier), "n"(THREADS) : "memory");
+}
+
 // Lane 0 waits for one barrier, lane 1 for another, and the warp for both.  (A poll costs the shared-memory pipe as many
 // turns as lanes take part.)
 __device__ __forceinline__ bool warp_wait_two(uint64_t *bar0, uint32_t parity0, uint64_t *bar1, uint32_t parity1)
@@ -251,25 +260,110 @@ __device__ __forceinline__ bool team_agrees(uint32_t barrier, bool ok)
     return all != 0;
 }
 
-// The sums of one thread again, as they are defined: fused multiply-adds over k0 ... k1 in order.  Row and columns beyond
-// C read the last ones; nothing of them is stored.
-template <uint32_t COLS>
-__device__ __forceinline__ void f32_sums_as_defined(float *sum, const float *a, const float *b, uint32_t row, uint32_t col, uint32_t m, uint32_t n, uint32_t k,
-                                                    uint32_t k0, uint32_t k1)
+// The sums of the warps with AGAIN once more, as they are defined: fused multiply-adds over k0 ... k1 in order.  All the warps
+// that hold sums call this at the same time and bring their CTA's rows of A and B, eight k at a time, into their boxes (`room`): [k][row of A], [k][row of B],
+// four floats between.  A lane computes eight rows x pairs of columns 16 apart of its warp's 32 x TN / 2 sums and hands them to the
+// lanes that hold the rows through the warp's box, 16 columns at a time.  A sum that is a NaN stays one, and a tile without
+// others ends early.  Beyond K are zeros on both sides; what lies beyond C is computed and not stored.
+//
+// Bound by latency: two warps per scheduler, the fp32 pipe half busy; 128 x 128 x 4096 take 620 us, 500 where few warps take part.
+// Before, each lane streamed its own row of A, again for every second column: 4096^3 with one NaN in A 5.0 -> 1.1 ms, one in every
+// 128 rows 23.8 -> 4.1, A all NaN 40.4 -> 0.6, results beyond 2^89 throughout 40.4 -> 4.9; the CUDA-core kernel takes 2.3 for each.
+// Fragments loaded one k ahead, steps of 16 k and fewer polls by the waiting warps changed nothing, scalar multiply-adds
+// took 1.3 times as long.
+template <uint32_t TN, bool AGAIN>
+__device__ __forceinline__ void f32_tile_as_defined(float (&sum)[TN / 2], float *room, const F32Params &p, uint32_t row0, uint32_t col0, uint32_t k0, uint32_t k1)
 {
-    const float *pa = a + (uint64_t)(row < m ? row : m - 1) * k;
+    constexpr uint32_t kStep = 8, kLdA = 128 + 4, kLdB = TN + 4, kBuffer = kStep * (kLdA + kLdB), kPairs = TN / 32;
+    static_assert(2 * kBuffer * sizeof(float) <= kF32SumWarps * F32Tile<TN>::box_bytes, "two steps fit the boxes");
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));                       // read here, so that nothing below is kept in registers before
+    t -= 32 * kF32FirstSum;
+    const uint32_t line = t >> 1, part = 4 * (t & 1);
+    const uint32_t warp = t >> 5, lane = t & 31, lane_row = lane >> 3, lane_col = lane & 7;
+    const bool in_a = row0 + line < p.m, in_b = line < TN && col0 + line < p.n;
+    const float *pa = p.a + (uint64_t)(in_a ? row0 + line : 0) * p.k + part, *pb = p.b + (uint64_t)(in_b ? col0 + line : 0) * p.k + part;
+    float4 xa, xb;
+    auto fetch = [&](uint32_t k) {
+        const bool in_k = k + part < k1;                                  // K is a multiple of 4
+        xa = in_a && in_k ? *reinterpret_cast<const float4 *>(pa + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        xb = in_b && in_k ? *reinterpret_cast<const float4 *>(pb + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    unsigned long long acc[8][kPairs];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++)
+#pragma unroll
+        for (uint32_t j = 0; j < kPairs; j++)
+            acc[i][j] = 0ull;
+    fetch(k0);
+    uint32_t buffer = 0;
+    bool settled = !AGAIN;
 #pragma unroll 1
-    for (uint32_t i = 0; i < COLS; i += 2) {
-        const float *p0 = b + (uint64_t)(col + i < n ? col + i : n - 1) * k, *p1 = b + (uint64_t)(col + i + 1 < n ? col + i + 1 : n - 1) * k;
-        float s0 = 0.0f, s1 = 0.0f;
-#pragma unroll 4
-        for (uint32_t j = k0; j < k1; j += 4) {                           // K is a multiple of 4
-            const float4 x = *reinterpret_cast<const float4 *>(pa + j), y = *reinterpret_cast<const float4 *>(p0 + j), z = *reinterpret_cast<const float4 *>(p1 + j);
-            s0 = __fmaf_rn(x.w, y.w, __fmaf_rn(x.z, y.z, __fmaf_rn(x.y, y.y, __fmaf_rn(x.x, y.x, s0))));
-            s1 = __fmaf_rn(x.w, z.w, __fmaf_rn(x.z, z.z, __fmaf_rn(x.y, z.y, __fmaf_rn(x.x, z.x, s1))));
+    for (uint32_t k = k0; k < k1; k += kStep, buffer ^= 1) {
+        if ((k - k0) % (32 * kStep) == kStep) {
+            if constexpr (AGAIN) {
+                bool nan = true;
+#pragma unroll
+                for (uint32_t i = 0; i < 8 * kPairs; i++) {
+                    float2 v;
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(acc[i / kPairs][i % kPairs]));
+                    nan = nan && isnan(v.x) && isnan(v.y);
+                }
+                settled = __all_sync(0xffffffffu, nan);
+            }
+            if (team_agrees<32 * kF32SumWarps>(1, settled))
+                break;
         }
-        sum[i] = s0;
-        sum[i + 1] = s1;
+        float *sa = room + buffer * kBuffer, *sb = sa + kStep * kLdA;
+        float *to = sa + part * kLdA + line;
+        to[0] = xa.x, to[kLdA] = xa.y, to[2 * kLdA] = xa.z, to[3 * kLdA] = xa.w;
+        if (line < TN) {
+            to = sb + part * kLdB + line;
+            to[0] = xb.x, to[kLdB] = xb.y, to[2 * kLdB] = xb.z, to[3 * kLdB] = xb.w;
+        }
+        if (k + kStep < k1)
+            fetch(k + kStep);
+        named_barrier<32 * kF32SumWarps>(1);
+        if constexpr (!AGAIN)
+            continue;
+        const float *fa = sa + 32 * (warp & 3) + 4 * lane_row, *fb = sb + (warp >> 2) * (TN / 2) + 2 * lane_col;
+#pragma unroll
+        for (uint32_t kk = 0; kk < kStep; kk++) {
+            unsigned long long y[kPairs];
+#pragma unroll
+            for (uint32_t j = 0; j < kPairs; j++)
+                y[j] = *reinterpret_cast<const unsigned long long *>(fb + kk * kLdB + 16 * j);
+#pragma unroll
+            for (uint32_t h = 0; h < 2; h++) {
+                const float4 x = *reinterpret_cast<const float4 *>(fa + kk * kLdA + 16 * h);
+                const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (uint32_t i = 0; i < 4; i++) {
+                    unsigned long long xx;
+                    asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(xs[i]));
+#pragma unroll
+                    for (uint32_t j = 0; j < kPairs; j++)
+                        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[4 * h + i][j]) : "l"(xx), "l"(y[j]));
+                }
+            }
+        }
+    }
+    named_barrier<32 * kF32SumWarps>(1);                                  // the boxes are the warps' own again
+    if constexpr (!AGAIN)
+        return;
+    float *box = room + warp * (F32Tile<TN>::box_bytes / 4);
+#pragma unroll
+    for (uint32_t j = 0; j < kPairs; j++) {
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++)
+            *reinterpret_cast<unsigned long long *>(box + (4 * lane_row + 16 * (i >> 2) + (i & 3)) * kF32BoxLd + 2 * lane_col) = acc[i][j];
+        __syncwarp();
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++) {
+            const float4 v = *reinterpret_cast<const float4 *>(box + lane * kF32BoxLd + 4 * i);
+            sum[16 * j + 4 * i] = v.x, sum[16 * j + 4 * i + 1] = v.y, sum[16 * j + 4 * i + 2] = v.z, sum[16 * j + 4 * i + 3] = v.w;
+        }
+        __syncwarp();
     }
 }
 
@@ -323,7 +417,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
     };
 
     if (warp < 4)
-        set_max_registers<false, kF32IssueRegs>();
+        set_max_registers<false, T::issue_regs>();
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         uint32_t s = 0, parity = 1;
@@ -414,7 +508,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
     } else if (warp >= 4 && warp < kF32FirstSum) {
         // ---------------- converters: groups of four warps that take turns at the chunks; a row of A per lane, and eight floats of
         // B per lane and step ----------------
-        set_max_registers<false, kF32ConverterRegs>();
+        set_max_registers<false, T::converter_regs>();
         const uint32_t cw = (uint32_t)warp & 3, group = (uint32_t)(warp - 4) >> 2;
         const uint32_t full0 = cluster_addr(&sh->conv_full[0], leader);
         uint32_t count = 0;
@@ -494,7 +588,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
         }
     } else {
         // ---------------- sums: 32 rows x TN / 2 columns per warp ----------------
-        set_max_registers<true, kF32SumRegs>();
+        set_max_registers<true, T::sum_regs>();
         const uint32_t q = (uint32_t)warp & 3, half = (uint32_t)(warp - kF32FirstSum) >> 2;
         float *box = reinterpret_cast<float *>(boxes + (size_t)(warp - kF32FirstSum) * T::box_bytes);
         const uint32_t own4 = T::half_n / 4 / p.splits;                   // groups of four columns that this pair stores
@@ -555,13 +649,13 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                     probe = fmaf(sum[i], 0.0f, probe);
                     sum[i] *= kF32Unscale;
                 }
-                if (__any_sync(0xffffffffu, probe != 0.0f)) {
-                    float slow[T::half_n];
+                if (!team_agrees<32 * kF32SumWarps>(1, probe == 0.0f)) {
                     const uint32_t k1 = c1 * kF32Chunk < p.k ? c1 * kF32Chunk : p.k;
-                    f32_sums_as_defined<T::half_n>(slow, p.a, p.b, row0 + lane, col0, p.m, p.n, p.k, c0 * kF32Chunk, k1);
-#pragma unroll
-                    for (uint32_t i = 0; i < T::half_n; i++)
-                        sum[i] = slow[i];
+                    const uint32_t first_row = mb * kF32M + r * 128;
+                    if (__any_sync(0xffffffffu, probe != 0.0f))
+                        f32_tile_as_defined<TN, true>(sum, reinterpret_cast<float *>(boxes), p, first_row, nb * TN, c0 * kF32Chunk, k1);
+                    else
+                        f32_tile_as_defined<TN, false>(sum, reinterpret_cast<float *>(boxes), p, first_row, nb * TN, c0 * kF32Chunk, k1);
                 }
             }
             if (p.splits > 1) {

@@ -153,30 +153,63 @@ def test_small_results_keep_their_bits(K, cuda, plan, shape, exponents):
     assert bool(((c.double() - want).abs() <= room).all()) and float((want.abs() / room).median()) > 20
 
 
+def median_time(K, cuda, dtype, a, b, c, status):
+    (m, k), n = a.shape, b.shape[0]
+    args = N.GemmArgs(dtype=dtype, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=1.0, d_status=status.data_ptr())
+    times = []
+    for _ in range(7):
+        start, end = (cuda.cuda.Event(enable_timing=True) for _ in range(2))
+        start.record()
+        for _ in range(3):
+            K.clpk_gemm(C.byref(args), stream_ptr())
+        end.record()
+        sync()
+        times.append(start.elapsed_time(end))
+    return sorted(times)[3]
+
+
 def test_small_numbers_and_zeros_cost_nothing(K, cuda):
     """A small element in every row of A, small results, half of A zeros: the time of ordinary operands, within a half."""
     n = 2048
     a, b = operands(K, cuda, n, n, n)
-
-    def time(a, b):
-        c, status = dev_empty(n * n, cuda.float32), dev_empty(1, cuda.int32)
-        args = N.GemmArgs(dtype=N.DT_F32, m=n, n=n, k=n, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=1.0, d_status=status.data_ptr())
-        times = []
-        for _ in range(7):
-            start, end = (cuda.cuda.Event(enable_timing=True) for _ in range(2))
-            start.record()
-            for _ in range(5):
-                K.clpk_gemm(C.byref(args), stream_ptr())
-            end.record()
-            sync()
-            times.append(start.elapsed_time(end))
-        return sorted(times)[3]
-
+    c, status = dev_empty(n * n, cuda.float32), dev_empty(1, cuda.int32)
     one_small = a.clone()
     one_small[:, 7] = 2.0 ** -120
-    ordinary = time(a, b)
+    ordinary = median_time(K, cuda, N.DT_F32, a, b, c, status)
     for x, y in ((one_small, b), (a * 2.0 ** -60, b * 2.0 ** -60), (a.clamp(min=0.0), b)):
-        assert time(x, y) <= 1.5 * ordinary
+        assert median_time(K, cuda, N.DT_F32, x, y, c, status) <= 1.5 * ordinary
+
+
+def test_a_nan_costs_no_more_than_the_cuda_cores(K, cuda):
+    """One NaN and nothing but NaNs at 4096^3: not the time of the CUDA-core kernel; results too large for the scaled pieces in every
+    tile: within three times that."""
+    n = 4096
+    a, b = operands(K, cuda, n, n, n)
+    c, status = dev_empty(n * n, cuda.float32), dev_empty(1, cuda.int32)
+    cuda_cores = median_time(K, cuda, N.DT_F32_FFMA, a, b, c, status)
+    one_in_a, one_in_b, all_of_a = a.clone(), b.clone(), cuda.full_like(a, float("nan"))
+    one_in_a[77, 7] = one_in_b[1234, 4000] = float("nan")
+    for x, y in ((one_in_a, b), (a, one_in_b), (all_of_a, b)):
+        assert median_time(K, cuda, N.DT_F32, x, y, c, status) <= cuda_cores
+    assert median_time(K, cuda, N.DT_F32, a * 2.0 ** 50, b * 2.0 ** 50, c, status) <= 3 * cuda_cores
+
+
+@pytest.mark.parametrize("plan,shape", PLANS)
+def test_sums_that_are_not_finite_in_every_plan(K, cuda, plan, shape):
+    """Single infinities and NaNs in the first and the last rows and chunks, then results beyond 2^110 throughout: each output that
+    is finite in 64 bits is, within fp32 rounding, and the others are infinite or NaN as there."""
+    (m, n, k), (a, b) = shape, operands(K, cuda, *shape)
+    a[m - 1, k - 1], a[3, 0], b[n - 1, 1], b[5, k - 2] = float("nan"), float("inf"), float("-inf"), float("nan")
+    assert gemm_plan(K, N.DT_F32, m, n, k) == (*plan, 2)
+    large = [t * 2.0 ** 61 for t in operands(K, cuda, *shape)]
+    for x, y in ((a, b), large):
+        c = multiply(K, cuda, x, y)
+        want = x.double() @ y.double().T
+        s_abs = x.double().abs() @ y.double().abs().T
+        assert bool((cuda.isnan(c) == cuda.isnan(want)).all()) and bool((cuda.isinf(c) == cuda.isinf(want)).all())
+        infinite, finite = cuda.isinf(want), cuda.isfinite(want)
+        assert bool((c.double()[infinite] == want[infinite]).all())
+        assert bool(((c.double() - want).abs()[finite] <= (k + 2) * 2.0 ** -24 * s_abs[finite]).all())
 
 
 def test_wide_range_of_magnitudes(K, cuda):
