@@ -1127,9 +1127,13 @@ struct TilesPlan {
 //   gemm_tiles_kernel, 512    4.75 + waves * (K blocks * (0.157 + 0.344 W + T at 106 TB/s) + 1.2 W of epilogue, 3.2 W from
 //                             tn = 160 on, where tensor memory holds one accumulator); from 24000 launches, residual 6 %.
 //                             Not used beyond four waves, narrow ones not beyond two (e4m3 13065 x 1248 x 464, four waves
-//                             of tn = 128: 14.6 us in large tiles, 18.6 in these), and only where gemm_kernel would be taken: 5939 random
-//                             shapes that take it are 1.15 times as fast in the geometric mean, 33 of them 2 to 10 %
-//                             slower (long sums in one wave); against
+//                             of tn = 128: 14.6 us in large tiles, 18.6 in these), and only where gemm_kernel would be taken: 77922
+//                             random shapes that take it are 1.15 times as fast in the geometric mean.  Operand rows that are
+//                             an odd multiple of 16 bytes, where a row's 128 bytes lie in five 32-byte sectors instead of
+//                             four, gain less (1.11 against 1.20 times), and of them tn = 96 was slower from six blocks on
+//                             (e4m3 270 x 13928 x 784: 11.6 us in large tiles, 12.9 in these; 22 of 50, and none of 600 others),
+//                             so narrow tiles are left to short sums there.  77 wider ones, all but one with such rows, were
+//                             timed 2 to 5 % slower once and most of them no slower again.  Against
 //                             the 256-row tiles the estimate is not sharp enough (228 of 831 more than 2 % slower)
 // Splits of 2 and 4 are clusters of 4 and 8 CTAs, of which the chip holds 33 and 15 at a time.  From the fifth wave of
 // 512 x 256 tiles on (16384 x 16384 x 256: 140 against 142 us) and the third of block-scaled ones the large tiles'
@@ -1139,7 +1143,8 @@ struct TilesPlan {
 // than in large tiles, at worst 1.31 times, and with the term 17, at worst 1.10).  Behind the launch that arranges the
 // scales it does not show (nvf4 5 x 5632 x 3840: 11.1 us in 128-wide tiles, 14.0 in large ones), so `arranged`: FP4 whose
 // scales lie in the workspace already.
-static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4, bool arranged)
+// `sectors`: rows of the operands are whole 32-byte sectors.
+static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool sectors, bool fp4, bool arranged)
 {
     const uint32_t pairs = (uint32_t)num_sms() / 2;
     auto ceil_div = [](uint32_t a, uint32_t b) { return (a - 1) / b + 1; };
@@ -1179,9 +1184,9 @@ static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool fp4,
     }
     // Where the 512 x 256 tiles are left over, narrower ones of 512 rows may fill the chip better.
     if (!fp4 && plan.tn == 0) {
-        for (uint32_t tn = 32; tn < 256; tn += 32) {
+        for (uint32_t tn = 64; tn < 256; tn += 32) {                      // 32 was cheapest for none of 40 million shapes
             const uint64_t tiles = (uint64_t)ceil_div(m, kDenseTileM) * ceil_div(n, tn);
-            if (tiles > (tn >= 192 ? 4ull : 2ull) * pairs)
+            if (tiles > (tn >= 192 ? 4ull : 2ull) * pairs || (tn <= 128 && k_blocks > 5 && !sectors))
                 continue;
             const float waves = (float)((tiles - 1) / pairs + 1), wide = (float)tn / 256.0f;
             const float loaded = (float)(tiles < pairs ? tiles : pairs) * ((m < kDenseTileM ? m : kDenseTileM) + (n < tn ? n : tn)) * kRowBytesK;
@@ -1219,7 +1224,7 @@ static TilesPlan gemm_plan(uint32_t m, uint32_t n, uint32_t k, uint32_t elem_bit
     const bool fp4 = elem_bits == 4;
     if (fp4 && tuning(CLPK_TUNE_GEMM_FP4_TILE) > 0)
         return {0, 1};
-    return plan_tiles(m, n, k_blocks_of(k, elem_bits), fp4, arranged);
+    return plan_tiles(m, n, k_blocks_of(k, elem_bits), (uint64_t)k * elem_bits % 256 == 0, fp4, arranged);
 }
 
 // CTAs in clusters of `cluster`, behind the kernel before them
