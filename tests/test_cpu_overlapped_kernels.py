@@ -55,8 +55,8 @@ def test_every_kernel_launched_behind_another_waits():
     launched = set()
     for path in CSRC.rglob("*.cu"):
         text = path.read_text()
-        launched |= set(re.findall(r"\blaunch_(?:behind|simt)\(\s*(?:\w+ \? )?(\w+)[<,]", text))
-    assert len(launched) >= 15 and launched <= set(OVERLAPPED), launched - set(OVERLAPPED)
+        launched |= set(re.findall(r"\blaunch_(?:behind|simt|clusters)\(\s*(?:\w+ \? )?(\w+)[<,]", text))
+    assert len(launched) >= 17 and {"gemm_tiles_kernel", "gemm_f32_kernel"} <= launched and launched <= set(OVERLAPPED), launched - set(OVERLAPPED)
 
 
 @pytest.mark.parametrize("name", OVERLAPPED)

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from clpeak_b200 import native as N
-from tests.gpu_util import dev_empty, stream_ptr, sync, to_np
+from tests.gpu_util import dev_empty, gemm_plan, stream_ptr, sync, to_np
 
 pytestmark = pytest.mark.gpu
 
@@ -381,7 +381,7 @@ def test_gemm_many_waves_small_k(K, orc, cuda):
     check_samples(orc, N.DT_BF16, a, b, c, m, n, k, samples)
 
 
-# ---- fp32 (CUDA cores) and fp64 (DMMA): the rows without a tcgen05 kind --------------------------------
+# ---- fp32 (CUDA cores; DT_F32 takes the tensor cores where they are faster) and fp64 (DMMA): the rows without a tcgen05 kind ----
 
 def run_simt_gemm(K, cuda, dtype, m, n, k, alpha=1.0):
     """A, B ~ N(0, 0.02) generated on the device as fp32; the fp64 operands are those floats widened."""
@@ -409,14 +409,16 @@ def run_simt_gemm(K, cuda, dtype, m, n, k, alpha=1.0):
     return to_np(ops[0]), to_np(ops[1]), c_all[:m * n]
 
 
-@pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F64])
+@pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F32_FFMA, N.DT_F64])
 @pytest.mark.parametrize("m,n,k", [(128, 128, 16), (256, 384, 64), (384, 128, 1040), (2048, 2048, 512), (4096, 4096, 4096),
-                                   (1, 1, 4), (100, 72, 20), (129, 131, 36), (300, 202, 1044), (64, 257, 16), (1000, 1001, 260)])
+                                   (1, 1, 4), (100, 72, 20), (129, 131, 36), (300, 202, 1044), (64, 257, 16), (1000, 1001, 260), (2047, 2050, 516)])
 def test_simt_gemm_against_the_oracle(K, orc, cuda, dtype, m, n, k):
     """Every element of the small cases, samples of the large one, against the oracle's fp64 dot product; whole
     tiles and shapes that are not (M, N not multiples of the tile, K not of the k block, N odd).
     Tolerance: K sequential roundings of the accumulator, K * u * sum|a||b| with u = 2^-23 (fp32; one extra
     bit over the unit roundoff for the host's own accumulation) or 2^-51 (fp64)."""
+    if dtype == N.DT_F32_FFMA and m >= 2047:
+        assert gemm_plan(K, dtype, m, n, k) == (0, 1, 0), "the 128 x 128 tiles, whole and ragged, over several k blocks"
     a, b, c = run_simt_gemm(K, cuda, dtype, m, n, k)
     assert not np.isnan(c).any(), "some of C was never written"
     u = 2.0 ** -51 if dtype == N.DT_F64 else 2.0 ** -23
@@ -428,12 +430,12 @@ def test_simt_gemm_against_the_oracle(K, orc, cuda, dtype, m, n, k):
     samples = list(zip(rng.integers(0, m, 150), rng.integers(0, n, 150))) + [(0, 0), (m - 1, n - 1), (min(127, m - 1), 0), (0, min(127, n - 1))]
     worst = 0.0
     for i, j in samples:
-        want, s_abs = orc.gemm_element(dtype, a, b, k, int(i), int(j))
+        want, s_abs = orc.gemm_element(N.DT_F64 if dtype == N.DT_F64 else N.DT_F32, a, b, k, int(i), int(j))
         worst = max(worst, abs(float(c[i * n + j]) - want) / (k * u * s_abs + 1e-300))
     assert worst <= 1.0, f"worst sampled error is {worst:.3g}x the stated tolerance"
 
 
-@pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F64])
+@pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F32_FFMA, N.DT_F64])
 def test_simt_gemm_alpha_and_argument_checks(K, orc, cuda, dtype):
     a, b, c1 = run_simt_gemm(K, cuda, dtype, 128, 256, 64)
     _, _, c2 = run_simt_gemm(K, cuda, dtype, 128, 256, 64, alpha=0.5)

@@ -19,11 +19,11 @@ def operands(K, cuda, m, n, k):
     return out
 
 
-def multiply(K, cuda, a, b, alpha=1.0):
+def multiply(K, cuda, a, b, alpha=1.0, dtype=N.DT_F32):
     (m, k), n = a.shape, b.shape[0]
     c = cuda.full((m * n + 1024,), 7.0, dtype=cuda.float32, device="cuda")
     status = cuda.full((1,), 7, dtype=cuda.int32, device="cuda")
-    args = N.GemmArgs(dtype=N.DT_F32, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=alpha, d_status=status.data_ptr())
+    args = N.GemmArgs(dtype=dtype, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=alpha, d_status=status.data_ptr())
     K.clpk_gemm(C.byref(args), stream_ptr())
     sync()
     assert int(status.item()) == 0
@@ -38,9 +38,9 @@ def worst(c, a, b, alpha=1.0):
 
 
 def bound(k):
-    """One rounding per chunk of 32, one of alpha, and at most eight units for what an instruction cuts when it aligns its
-    products (two per chunk cut a sum of full size, in a chunk that is a part of the sum)."""
-    return -(-k // 32) + 9
+    """One rounding for each turn of 64 products, one for each of four K ranges that begins a turn of its own, one of alpha, one unit
+    for the products that are left out, and two for each of the four instructions of a turn that cut a sum of full size."""
+    return -(-k // 64) + 3 + 1 + 1 + 8
 
 
 # (tile width, K ranges) and a shape that takes them: ragged rows, columns and chunks, odd N, several tiles per pair
@@ -58,8 +58,14 @@ def test_every_plan(K, cuda, plan, shape):
     assert bool((c == multiply(K, cuda, a, b, 0.75)).all()), "partial sums are added in a fixed order: the same bits every time"
 
 
-@pytest.mark.parametrize("m,n,k", [(256, 128, 256), (257, 129, 260), (255, 127, 252), (128, 1000, 288), (1000, 131, 1028), (300, 202, 2044), (2000, 2001, 512)])
-def test_edges(K, cuda, m, n, k):
+# whole tiles and chunks, one row, column and four k more, and one less, for each tile width
+@pytest.mark.parametrize("tile_n,m,n,k", [(t, m + d, n + d, k + 4 * d) for t, m, n, k in
+                                          [(32, 512, 128, 1024), (64, 512, 256, 1024), (64, 1024, 512, 512), (96, 512, 1536, 1024)]
+                                          for d in (0, 1, -1)] + [(128, 2048, 2048, 96), (96, 2049, 2049, 100), (128, 2047, 2047, 92), (128, 2000, 2001, 64),
+                                                                  (64, 1000, 131, 1028), (32, 300, 202, 2044)])
+def test_edges(K, cuda, tile_n, m, n, k):
+    plan = gemm_plan(K, N.DT_F32, m, n, k)
+    assert (plan[0], plan[2]) == (tile_n, 2)
     a, b = operands(K, cuda, m, n, k)
     assert worst(multiply(K, cuda, a, b), a, b) <= bound(k)
 
@@ -128,15 +134,17 @@ def test_one_small_element_at_every_row_of_a_tile(K, cuda, plan, shape):
 
 @pytest.mark.parametrize("exponents", [(-70, -70), (-60, -72), (-63, -75), (-40, -66)])
 def test_results_near_the_end_of_the_range(K, cuda, exponents):
-    """Products that fp32 holds only in part: K roundings to 2^-149 besides the relative ones."""
+    """Products that fp32 holds only in part: a rounding to 2^-149 for each of the four K ranges and for alpha besides the relative ones,
+    of results of which many are larger by far."""
     m, n, k = 300, 200, 2044
-    assert gemm_plan(K, N.DT_F32, m, n, k)[2] == 2
+    assert gemm_plan(K, N.DT_F32, m, n, k) == (32, 4, 2)
     a, b = operands(K, cuda, m, n, k)
     a *= 2.0 ** exponents[0]
     b *= 2.0 ** exponents[1]
     c = multiply(K, cuda, a, b)
     want, s_abs = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
-    assert bool(((c.double() - want).abs() <= (k + 2) * (2.0 ** -24 * s_abs + 2.0 ** -150)).all())
+    room = bound(k) * 2.0 ** -24 * s_abs + 5 * 2.0 ** -150
+    assert bool(((c.double() - want).abs() <= room).all()) and float((want.abs() / room).max()) > 3, "zeros would pass"
 
 
 @pytest.mark.parametrize("exponents", [(-64, -64), (-68, -68), (-58, -70), (-100, -28), (-134, 0), (0, -134), (-120, 60), (60, -135)])
@@ -212,6 +220,26 @@ def test_sums_that_are_not_finite_in_every_plan(K, cuda, plan, shape):
         assert bool(((c.double() - want).abs()[finite] <= (k + 2) * 2.0 ** -24 * s_abs[finite]).all())
 
 
+@pytest.mark.parametrize("values", ["uniform", "magnitudes", "constant"])
+@pytest.mark.parametrize("shape", [(2048, 2048, k) for k in (64, 96, 128, 256, 512, 1024, 4096)] + [(512, 512, 16384), (1024, 65, 1028)])
+def test_sums_of_one_sign(K, cuda, shape, values):
+    """What the tensor cores cut does not cancel there: sums come out low by 6 to 8.5e-8 of their size (2^-24 is 6e-8), whatever K.  The
+    CUDA cores' error grows with K and is larger, but where they add eight or more short chains (1024 x 65 x 1028: 7.3 to 7.8e-8)."""
+    assert gemm_plan(K, N.DT_F32, *shape)[2] == 2
+    m, n, k = shape
+    g = cuda.Generator(device="cuda").manual_seed(k)
+    draw = {"uniform": lambda rows: cuda.rand(rows, k, generator=g, device="cuda"), "magnitudes": lambda rows: cuda.randn(rows, k, generator=g, device="cuda").abs(),
+            # the largest products that are left out: all of one sign, 2^-24 of each
+            "constant": lambda rows: cuda.full((rows, k), 1 + 2.0 ** -8 - 2.0 ** -17, device="cuda")}[values]
+    a, b = draw(m), draw(n)
+    want = a.double() @ b.double().T
+    error = {dtype: float((multiply(K, cuda, a, b, dtype=dtype).double() - want).norm() / want.norm()) for dtype in (N.DT_F32, N.DT_F32_FFMA)}
+    # roundings of up to 256 turns beside the cut: half a unit of a sum that grows evenly, as a random walk
+    assert error[N.DT_F32] <= 1e-7 + 2.0 ** -25 * (k / 64) ** 0.5 / 3 ** 0.5
+    if shape != (1024, 65, 1028):
+        assert error[N.DT_F32] <= 1.01 * error[N.DT_F32_FFMA]
+
+
 def test_wide_range_of_magnitudes(K, cuda):
     """Every element of its own binade between 2^-40 and 2^40: the error stays relative to the products."""
     m, n, k = 513, 260, 1000
@@ -227,8 +255,4 @@ def test_the_cuda_cores_on_request(K, cuda):
     m, n, k = 300, 202, 2044
     assert gemm_plan(K, N.DT_F32, m, n, k)[2] == 2 and gemm_plan(K, N.DT_F32_FFMA, m, n, k)[2] != 2
     a, b = operands(K, cuda, m, n, k)
-    c, status = dev_empty(m * n, cuda.float32), dev_empty(1, cuda.int32)
-    args = N.GemmArgs(dtype=N.DT_F32_FFMA, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=1.0, d_status=status.data_ptr())
-    K.clpk_gemm(C.byref(args), stream_ptr())
-    sync()
-    assert worst(c.view(m, n), a, b) <= k + 2
+    assert worst(multiply(K, cuda, a, b, dtype=N.DT_F32_FFMA), a, b) <= k + 2

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 def operand(K, cuda, dtype, rows, k, seed):
     f = dev_empty(rows * k, cuda.float32)
     K.clpk_fill_f32(f.data_ptr(), rows * k, seed, N.DIST_NORMAL, 0.0, 0.02, stream_ptr())
-    if dtype == N.DT_F32:
+    if dtype != N.DT_F64:
         return f
     d = dev_empty(rows * k, cuda.float64)
     K.clpk_convert_f32(d.data_ptr(), f.data_ptr(), rows * k, N.DT_F64, stream_ptr())
@@ -25,14 +25,16 @@ def operand(K, cuda, dtype, rows, k, seed):
 @pytest.mark.parametrize("m,n,k", [(1, 1, 4), (33, 65, 20), (64, 64, 16384), (129, 131, 36), (131, 102, 7688), (201, 73, 2828), (863, 251, 2456),
                                    (1315, 363, 956), (440, 434, 520), (64, 868, 1036), (719, 366, 688), (459, 349, 4636), (3720, 110, 596),
                                    (2254, 496, 464), (1024, 1024, 512), (97, 106, 5732), (719, 368, 6380), (64, 64, 4100)])
-@pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F64])
+@pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F32_FFMA, N.DT_F64])
 def test_every_element(K, cuda, dtype, m, n, k):
     check_every_element(K, cuda, dtype, m, n, k)
 
 
 # (tile, K ranges, twice the K groups) and a shape that takes them
-PLANS = [(N.DT_F32, (0, 1, 0), (1135, 1699, 36)), (N.DT_F32, (64, 1, 0), (52, 36, 64)), (N.DT_F32, (64, 2, 0), (42, 58, 128)),
-         (N.DT_F32, (64, 4, 0), (127, 33, 256)), (N.DT_F32, (64, 8, 0), (94, 36, 512)), (N.DT_F32, (64, 8, 1), (64, 64, 16384)),
+PLANS = [(N.DT_F32_FFMA, (0, 1, 0), (1135, 1699, 36)), (N.DT_F32_FFMA, (0, 1, 0), (2048, 2048, 512)), (N.DT_F32_FFMA, (0, 1, 0), (2047, 2050, 516)),
+         (N.DT_F32_FFMA, (64, 1, 0), (52, 36, 64)), (N.DT_F32_FFMA, (64, 1, 0), (4095, 366, 2456)), (N.DT_F32_FFMA, (64, 1, 1), (459, 863, 520)),
+         (N.DT_F32_FFMA, (64, 2, 0), (42, 58, 128)), (N.DT_F32_FFMA, (64, 2, 1), (719, 366, 2456)), (N.DT_F32_FFMA, (64, 4, 0), (127, 33, 256)),
+         (N.DT_F32_FFMA, (64, 4, 1), (64, 2048, 2456)), (N.DT_F32_FFMA, (64, 8, 0), (94, 36, 512)), (N.DT_F32_FFMA, (64, 8, 1), (64, 64, 16384)),
          (N.DT_F64, (32, 1, 0), (47, 70, 64)), (N.DT_F64, (32, 1, 1), (2287, 33, 512)), (N.DT_F64, (32, 4, 0), (68, 61, 512)),
          (N.DT_F64, (32, 8, 1), (64, 64, 16384)), (N.DT_F64, (64, 8, 0), (130, 197, 512))]
 
@@ -70,18 +72,19 @@ def check_every_element(K, cuda, dtype, m, n, k):
     fa, fb = a.double().view(m, k), b.double().view(n, k)
     want, s_abs = alpha * (fa @ fb.T), alpha * (fa.abs() @ fb.abs().T)
     # K roundings of the accumulator and one of alpha; fp64: the reference sum rounds as often
-    u = 2.0 ** -24 if dtype == N.DT_F32 else 2.0 ** -52
+    u = 2.0 ** -52 if dtype == N.DT_F64 else 2.0 ** -24
     worst = float(((results[0].double().view(m, n) - want).abs() / ((k + 2) * u * s_abs + 1e-300)).max())
     assert worst <= 1.0, f"worst error over all of C is {worst:.3g}x the stated tolerance"
 
 
-def test_nan_and_infinity_stay_in_their_rows_and_columns(K, cuda):
+@pytest.mark.parametrize("dtype", [N.DT_F32, N.DT_F32_FFMA])
+def test_nan_and_infinity_stay_in_their_rows_and_columns(K, cuda, dtype):
     """Zero fill beyond K and beyond the operands must not meet them: 0 * inf would spread."""
     m, n, k = 70, 66, 1028
     a, b = operand(K, cuda, N.DT_F32, m, k, 1), operand(K, cuda, N.DT_F32, n, k, 2)
     a[3 * k + 5], b[7 * k + k - 1] = float("inf"), float("nan")
     c, status = dev_empty(m * n, cuda.float32), dev_empty(1, cuda.int32)
-    args = N.GemmArgs(dtype=N.DT_F32, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=1.0, d_status=status.data_ptr())
+    args = N.GemmArgs(dtype=dtype, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), alpha=1.0, d_status=status.data_ptr())
     K.clpk_gemm(C.byref(args), stream_ptr())
     sync()
     bad = ~np.isfinite(c.view(m, n).cpu().numpy())
