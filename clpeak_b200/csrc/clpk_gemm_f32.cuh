@@ -20,7 +20,9 @@
 // floats starts from zero, adds the small products first and the h h ones last -- four instructions in which the cut is of
 // the sum's size -- and the turn's sum is added to registers with ordinary rounded fp32 additions.  Against the sum in
 // 64 bits that is more accurate than a chain of K fused multiply-adds: N(0, 0.02) operands, 2-norm of the error over that
-// of the result, 8e-8 at K = 256, 1.7e-7 at 4096 and 4.2e-7 at 16384, against 1.1e-6 at 4096.
+// of the result, 0.9e-7 at K = 256, 1.7e-7 at 4096 and 3.0e-7 at 16384, against 2.9e-7, 1.1e-6 and 2.3e-6.  Sums of one sign, where the
+// cuts do not cancel, come out low by 6 to 8.5e-8 of their size at every K; only chains as short as the 128 products of
+// eight that the CUDA-core kernels add for 1024 x 65 x 1028 are better there (7.3e-8 against 8.8e-8).
 //
 //  * Tile 256 x TN per CTA pair (cta_group::2, M = 256), CTA r holding 128 rows of A and of C, and TN / 2 rows of B.
 //  * A chunk is 32 floats of K: one 128-byte row per operand row, fetched by TMA as it lies in memory (warp 0).
@@ -34,16 +36,18 @@
 //
 // What bounds it: a chunk's 12 instructions take 430 cycles at TN = 32 and 890 at 128; converting a pair of floats 14 of an SM
 // quarter's cycles (sub.f32.bf16 takes its bf16 operand as it is; each of the three conversions blocks the ALU for two), 250
-// to 400 a chunk; the hand-over of an accumulator 1400, which two turns in flight hide at TN = 128 only just.  Device time
-// against the CUDA-core kernels: 4096^3 2252 -> 680 us (202 TFLOPS), 2317 x 6252 x 516 323 -> 123, 1636 x 116 x 4084 61 -> 25,
-// 459 x 349 x 4636 69 -> 27; 70 shapes with M and N from 64 to 16384 and K from 256 on 0.51 in the geometric mean.  Earlier
-// forms at 4096^3, TN = 128: hand-overs by .release.cluster arrives and a cluster fence 1279; one issuing warp 707; three
-// groups of converters (whose registers the sums then lack) 691; all warps polling for themselves 680, one per team 658; turns of
-// one chunk 658 there, but 953 at TN = 64 against 833.
+// to 400 a chunk; the hand-over of an accumulator 1400, which two turns in flight hide at TN = 128 only just.  The tensor pipe is
+// busy for 72 % of the cycles of a 4096 x 2304 x 4096 product, issue slots 58 %.  Device time against the CUDA-core kernels: 4096^3
+// 2251 -> 620 us back to back (222 TFLOPS), 710 between inputs that change (194); 2317 x 6252 x 516 338 -> 95,
+// 1636 x 116 x 4084 62 -> 24, 459 x 349 x 4636 70 -> 25; 9019 random shapes that take this kernel 0.40 in the geometric mean.
+// Earlier forms at 4096^3, TN = 128, with pieces at their own size (658 in the end): hand-overs by .release.cluster arrives and a
+// cluster fence 1279; one issuing warp 707; three groups of converters (whose registers the sums then lack) 691; all warps polling for
+// themselves 680; turns of one chunk the same, but 953 at TN = 64 against 833.
 //
 // Numbers that the split cannot serve are multiplied as they are, with fused multiply-adds in K order: a warp whose sums
 // are not all finite (an infinity, a NaN, or an overflow on the way, which the scales bring to about 2^89;
-// x - h of an infinity is a NaN, so none goes unseen) does its 32 x TN / 2 outputs again, see f32_tile_as_defined.
+// x - h of an infinity is a NaN, so none goes unseen) does its 32 x TN / 2 outputs again, see f32_tile_as_defined.  Whoever
+// waits for such a tile waits 0.15 us per element of K at most, under 2.5 s where the operands of more tiles than pairs fill 180 GB.
 #pragma once
 
 constexpr uint32_t kF32M = 256;

@@ -26,8 +26,8 @@ __device__ __forceinline__ void join_stream()
 
 // Which way the CTAs of a kernel that reads an array walk it.  What stands in front has just written or read the same array
 // in rising order, and its end is what the L2 (126 MB) still holds: from the end, arrays beyond the cache are read from
-// there as far as it reaches.  14997 x 2432 (146 MB) NVFP4 operands 144 -> 136 us, bf16 123 -> 117, 8192 x 8192 (268 MB) 258 ->
-// 250 and 222 -> 216.  What fits lies there whichever way it is read, and rising is up to 2 % faster (67 MB: to tf32 57.4
+// there as far as it reaches.  14997 x 2432 (146 MB) NVFP4 operands 144 -> 138 us, bf16 123 -> 117, 8192 x 8192 (268 MB) 257 ->
+// 251 and 222 -> 216.  What fits lies there whichever way it is read, and rising is up to 2 % faster (67 MB: to tf32 57.4
 // against 58.6 us).
 constexpr uint64_t kFallingFrom = 100ull << 20;
 static bool falling_order(uint64_t bytes) { return bytes >= kFallingFrom; }

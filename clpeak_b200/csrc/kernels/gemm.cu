@@ -32,7 +32,6 @@
 
 #include "../clpk_internal.h"
 #include "../clpk_ptx.cuh"
-#include "../clpk_rng_fast.cuh"
 
 namespace clpk {
 

@@ -419,8 +419,10 @@ CLPK_API int clpk_dmma_peak(const double *d_a, const double *d_b, uint32_t n_mma
  *   CLPK_DT_MXF4     e2m1 + ue8m0 per 32             fp32         bf16
  *   CLPK_DT_NVF4     e2m1 + ue4m3 per 16             fp32         bf16
  * CLPK_DT_F32: small products and short sums run on the CUDA cores (FFMA); the others multiply three bf16 pieces of each
- * element on the tensor cores, over the whole range of fp32, and add sums of 64 products with fp32 rounding, which leaves a
- * smaller error than K fused multiply-adds.  Infinities, NaNs and magnitudes beyond 2^89 are multiplied by FFMA in either case.
+ * element on the tensor cores, over the whole range of fp32, and add sums of 64 products with fp32 rounding.  That leaves a
+ * smaller error than K fused multiply-adds, but sums of one sign come out low by up to 8.5e-8 of their size, where FFMA in
+ * eight and more short chains leaves 7e-8.  Infinities, NaNs and magnitudes beyond 2^89 are multiplied by FFMA in either
+ * case, at half the speed of CLPK_DT_F32_FFMA where they are everywhere.
  * tcgen05 kinds: any M, N, K > 0 such that a row of A / B and a row of C are multiples of 16
  * bytes (partial tiles are computed whole and clipped; whole 512 x 256 tiles and K a multiple
  * of 128 bytes waste nothing).  FP4 kinds: K a multiple of 256; the workspace holds scale
