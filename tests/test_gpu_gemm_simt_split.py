@@ -31,7 +31,9 @@ def test_every_element(K, cuda, dtype, m, n, k):
 
 
 # (tile, K ranges, twice the K groups) and a shape that takes them
-PLANS = [(N.DT_F32_FFMA, (0, 1, 0), (1135, 1699, 36)), (N.DT_F32_FFMA, (0, 1, 0), (2048, 2048, 512)), (N.DT_F32_FFMA, (0, 1, 0), (2047, 2050, 516)),
+PLANS = [(N.DT_F32, (0, 1, 0), (1135, 1699, 36)), (N.DT_F32, (64, 1, 0), (52, 36, 64)), (N.DT_F32, (64, 2, 0), (42, 58, 128)),
+         (N.DT_F32, (64, 4, 0), (127, 33, 256)), (N.DT_F32, (64, 8, 0), (94, 36, 512)), (N.DT_F32, (64, 8, 1), (64, 64, 16384)),
+         (N.DT_F32_FFMA, (0, 1, 0), (1135, 1699, 36)), (N.DT_F32_FFMA, (0, 1, 0), (2048, 2048, 512)), (N.DT_F32_FFMA, (0, 1, 0), (2047, 2050, 516)),
          (N.DT_F32_FFMA, (64, 1, 0), (52, 36, 64)), (N.DT_F32_FFMA, (64, 1, 0), (4095, 366, 2456)), (N.DT_F32_FFMA, (64, 1, 1), (459, 863, 520)),
          (N.DT_F32_FFMA, (64, 2, 0), (42, 58, 128)), (N.DT_F32_FFMA, (64, 2, 1), (719, 366, 2456)), (N.DT_F32_FFMA, (64, 4, 0), (127, 33, 256)),
          (N.DT_F32_FFMA, (64, 4, 1), (64, 2048, 2456)), (N.DT_F32_FFMA, (64, 8, 0), (94, 36, 512)), (N.DT_F32_FFMA, (64, 8, 1), (64, 64, 16384)),

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 # pairs of shapes that take the same kernel and ask for different amounts of shared memory, because one gives an SM
 # one CTA and the other two: 64 x 64 tiles in fp32, 32 x 32 and 64 x 64 tiles in fp64
-@pytest.mark.parametrize("dtype,one,two", [(N.DT_F32_FFMA, (52, 36, 64), (2479, 194, 64)), (N.DT_F64, (47, 70, 64), (41, 2373, 64)),
+@pytest.mark.parametrize("dtype,one,two", [(N.DT_F32_FFMA, (52, 36, 64), (2479, 194, 64)), (N.DT_F32, (52, 36, 64), (2479, 194, 64)), (N.DT_F64, (47, 70, 64), (41, 2373, 64)),
                                            (N.DT_F64, (130, 197, 512), (1344, 33, 512))])
 def test_gemms_of_different_shapes_from_two_threads(K, cuda, dtype, one, two):
     if dtype == N.DT_F32_FFMA:
