@@ -115,26 +115,25 @@ __device__ __forceinline__ void st_float8(float *p, f32x2 a, f32x2 b, f32x2 c, f
     asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
 }
 
-// Bound by arithmetic: a normal deviate is 63 issued instructions, which keep the issue slots, the integer and the FMA
-// pipe each 70 % busy; a uniform one the two 64-bit multiplications of its random word.  8192 x 8192: normal 246 ->
-// 162 us, uniform 89 -> 66 (the stores alone would take 41).
+// Bound by arithmetic: see clpk_rng_fast.cuh.  Eight elements per thread and step, and two steps where the array is long
+// enough to fill the chip all the same: at 2^28 floats 536 against 548 us (normal) and 191 against 268 (uniform, bound by the
+// start of CTAs with one step), the same at 2^22, and one step is better below (normal, 2^20: 3.4 against 4.3).  8192 x 8192:
+// normal 160 -> 136 us, uniform 62 -> 49 (the stores alone would take 41), int8 55 -> 48.
+constexpr int kFillF32Threads = 128;
+constexpr uint64_t kTwoStepsFrom = 1 << 19;
+
 template <int DIST>
-__global__ void __launch_bounds__(kFillThreads) fill_f32_kernel(float *dst, Split part, uint64_t mixed_seed, float mean, float stdv)
+__global__ void __launch_bounds__(kFillF32Threads, 8) fill_f32_kernel(float *dst, Split part, uint64_t base, uint32_t steps, float mean, float stdv)
 {
     griddep_launch_dependents();                               // the stores wait, the values need no memory
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    // the 2 P values from element i on
-    auto values = [&](uint64_t i, auto &out) {
+    // the 2 P values of the words
+    auto values = [&](const auto &hi, const auto &lo, auto &out) {
         constexpr int P = sizeof(out) / sizeof(f32x2);
-        uint64_t h[2 * P];
-#pragma unroll
-        for (int j = 0; j < 2 * P; j++)
-            h[j] = rand64_at(mixed_seed, i + j);
         if constexpr (DIST == CLPK_DIST_NORMAL)
-            normal01<P>(h, out);
+            normal01<P>(hi, lo, out);
 #pragma unroll
         for (int j = 0; j < P; j++) {
-            const f32x2 u = pk((float)(uint32_t)(h[2 * j] >> 40), (float)(uint32_t)(h[2 * j + 1] >> 40));
+            const f32x2 u = pk((float)(hi[2 * j] >> 8), (float)(hi[2 * j + 1] >> 8));
             if constexpr (DIST == CLPK_DIST_NORMAL)
                 out[j] = fma2(pk(stdv), out[j], pk(mean));
             else if constexpr (DIST == CLPK_DIST_UNIFORM01)
@@ -143,41 +142,57 @@ __global__ void __launch_bounds__(kFillThreads) fill_f32_kernel(float *dst, Spli
                 out[j] = add2(mul2(u, pk(1.1920928955078125e-07f)), pk(-1.0f));
         }
     };
-    for (uint64_t g = first; g < part.whole; g += stride) {
+    uint64_t g = (uint64_t)blockIdx.x * (steps * kFillF32Threads) + threadIdx.x;
+#pragma unroll 1
+    for (uint32_t step = 0; step < steps && g < part.whole; step++, g += kFillF32Threads) {
+        uint32_t hi[8], lo[8];
+        random_words<8>(base + 8 * g, hi, lo);
         f32x2 v[4];
-        values(8 * g, v);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t hi4[4] = {hi[4 * h], hi[4 * h + 1], hi[4 * h + 2], hi[4 * h + 3]}, lo4[4] = {lo[4 * h], lo[4 * h + 1], lo[4 * h + 2], lo[4 * h + 3]};
+            f32x2 o[2];
+            values(hi4, lo4, o);
+            v[2 * h] = o[0];
+            v[2 * h + 1] = o[1];
+        }
         griddep_wait();
         st_float8(dst + 8 * g, v[0], v[1], v[2], v[3]);
     }
     if (part.has_single()) {
         const int64_t i = part.single(8);
+        uint32_t hi[2], lo[2];
+        random_words<2>(base + i, hi, lo);
         f32x2 v[1];
-        values(i, v);
+        values(hi, lo, v);
         griddep_wait();
         dst[i] = lo_of(v[0]);
     }
 }
 
-__global__ void __launch_bounds__(kFillThreads) fill_i8_kernel(int8_t *dst, Split part, uint64_t mixed_seed)
+__global__ void __launch_bounds__(kFillThreads) fill_i8_kernel(int8_t *dst, Split part, uint64_t base)
 {
     griddep_launch_dependents();                               // the stores wait, the values need no memory
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (uint64_t g = first; g < part.whole; g += stride) {
-        uint32_t w[4];
+        uint32_t w[4], hi[16], lo[16];
+        random_words<16>(base + 16 * g, hi, lo);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             w[j] = 0;
 #pragma unroll
             for (int t = 0; t < 4; t++)
-                w[j] |= ((uint32_t)((int)(rand64_at(mixed_seed, 16 * g + 4 * j + t) >> 60) - 8) & 0xFFu) << (8 * t);
+                w[j] |= (((hi[4 * j + t] >> 28) - 8) & 0xFFu) << (8 * t);
         }
         griddep_wait();
         *reinterpret_cast<uint4 *>(dst + 16 * g) = make_uint4(w[0], w[1], w[2], w[3]);
     }
     if (part.has_single()) {
         const int64_t i = part.single(16);
+        uint32_t hi[1], lo[1];
+        random_words<1>(base + i, hi, lo);
         griddep_wait();
-        dst[i] = (int8_t)((int)(rand64_at(mixed_seed, i) >> 60) - 8);
+        dst[i] = (int8_t)((int)(hi[0] >> 28) - 8);
     }
 }
 
@@ -563,15 +578,16 @@ int clpk_fill_f32(float *d_dst, uint64_t n, uint64_t seed, int dist, float mean,
     if (n == 0)
         return CLPK_OK;
     const Split part = split_at(d_dst, 32, 32, 8, n);
-    const uint64_t mixed = clpk_mix64(seed) + part.head;       // the generator's index is added to it
+    const uint64_t base = rand64_base(seed) + part.head;       // the generator's index is added to it
     d_dst += part.head;
-    const unsigned grid = fill_grid(part.whole);
+    const uint32_t steps = part.whole >= kTwoStepsFrom ? 2 : 1;
+    const unsigned grid = (unsigned)((part.whole + steps * kFillF32Threads - 1) / (steps * kFillF32Threads));
     cudaStream_t s = as_stream(stream);
     if (dist == CLPK_DIST_UNIFORM01)
-        return launch_behind(fill_f32_kernel<CLPK_DIST_UNIFORM01>, "launch fill_f32", grid, kFillThreads, 0, s, d_dst, part, mixed, mean, std);
+        return launch_behind(fill_f32_kernel<CLPK_DIST_UNIFORM01>, "launch fill_f32", grid > 0 ? grid : 1, kFillF32Threads, 0, s, d_dst, part, base, steps, mean, std);
     if (dist == CLPK_DIST_UNIFORM_PM1)
-        return launch_behind(fill_f32_kernel<CLPK_DIST_UNIFORM_PM1>, "launch fill_f32", grid, kFillThreads, 0, s, d_dst, part, mixed, mean, std);
-    return launch_behind(fill_f32_kernel<CLPK_DIST_NORMAL>, "launch fill_f32", grid, kFillThreads, 0, s, d_dst, part, mixed, mean, std);
+        return launch_behind(fill_f32_kernel<CLPK_DIST_UNIFORM_PM1>, "launch fill_f32", grid > 0 ? grid : 1, kFillF32Threads, 0, s, d_dst, part, base, steps, mean, std);
+    return launch_behind(fill_f32_kernel<CLPK_DIST_NORMAL>, "launch fill_f32", grid > 0 ? grid : 1, kFillF32Threads, 0, s, d_dst, part, base, steps, mean, std);
 }
 
 int clpk_fill_i8(int8_t *d_dst, uint64_t n, uint64_t seed, void *stream)
@@ -581,7 +597,7 @@ int clpk_fill_i8(int8_t *d_dst, uint64_t n, uint64_t seed, void *stream)
         return CLPK_OK;
     const Split part = split_at(d_dst, 16, 8, 16, n);
     return launch_behind(fill_i8_kernel, "launch fill_i8", fill_grid(part.whole), kFillThreads, 0, as_stream(stream), d_dst + part.head,
-                         part, clpk_mix64(seed) + part.head);
+                         part, rand64_base(seed) + part.head);
 }
 
 int clpk_convert_f32(void *d_dst, const float *d_src, uint64_t n, int dtype, void *stream)

@@ -37,6 +37,41 @@ def test_normal_deviates_over_their_whole_range(K, orc, cuda):
     assert_bits_equal(to_np(d), orc.fill_f32(n, 5, N.DIST_NORMAL), "normal deviates")
 
 
+@pytest.mark.parametrize("seed,at", [(1884646, 641), (7288700, 535), (6692669, 556), (4960922, 3392)])
+@pytest.mark.parametrize("offset", [0, 5])
+def test_fill_where_a_carry_reaches_bit_30(K, orc, cuda, seed, at, offset):
+    """Consecutive elements share what stands above bit 30 of the generator's first step, until element `at` of these seeds:
+    in the middle of a step, its last element, and its first one."""
+    mask = (1 << 64) - 1
+
+    def mix(z):
+        z = (z + 0x9E3779B97F4A7C15) & mask
+        z = ((z ^ (z >> 30)) * 0xBF58476D1CE4E5B9) & mask
+        z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & mask
+        return z ^ (z >> 31)
+    assert (mix(seed) + 0x9E3779B97F4A7C15 + at) % (1 << 30) == 0
+    n = at + 300
+    d, q = dev_empty(n + 8, cuda.float32), dev_empty(n + 8, cuda.int8)
+    for dist in (N.DIST_UNIFORM01, N.DIST_UNIFORM_PM1, N.DIST_NORMAL):
+        K.clpk_fill_f32(d.data_ptr() + 4 * offset, n, seed, dist, 0.25, 2.0, stream_ptr())
+        sync()
+        assert_bits_equal(to_np(d)[offset:offset + n], orc.fill_f32(n, seed, dist, 0.25, 2.0), "fill")
+    K.clpk_fill_i8(q.data_ptr() + offset, n, seed, stream_ptr())
+    sync()
+    assert_bits_equal(to_np(q)[offset:offset + n], orc.fill_i8(n, seed), "fill_i8")
+
+
+@pytest.mark.parametrize("n", [(1 << 22) - 8, 1 << 22, (1 << 22) + 1031, (1 << 22) + 2048])
+def test_fill_with_one_and_two_steps_per_thread(K, orc, cuda, n):
+    d = cuda.full((n + 8,), 77.0, dtype=cuda.float32, device="cuda")
+    for dist in (N.DIST_UNIFORM01, N.DIST_NORMAL):
+        K.clpk_fill_f32(d.data_ptr(), n, 3, dist, 0.0, 1.0, stream_ptr())
+        sync()
+        got = to_np(d)
+        assert_bits_equal(got[:n], orc.fill_f32(n, 3, dist), "fill")
+        assert np.all(got[n:] == 77.0)
+
+
 @pytest.mark.parametrize("n,offset", [(15, 0), (16, 0), (33, 0), (5000, 3)])
 def test_fill_i8_lengths_and_alignment(K, orc, cuda, n, offset):
     buf = cuda.full((n + offset + 8,), 77, dtype=cuda.int8, device="cuda")
