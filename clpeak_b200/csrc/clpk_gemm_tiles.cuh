@@ -23,7 +23,8 @@
 // TN = 64 on), asking the next stage's barrier ahead of the instructions (no effect), clusters of 16 for eight splits
 // (10 % for single tiles of K > 8000, slower elsewhere).
 //
-// Block-scaled kinds: TN = 64, 128 or 256 (split), one K block and its scale factors per stage; a block is 13 (NVFP4,
+// Block-scaled kinds: TN = 64, 128 or 256 (split, or with one accumulator where the scales are arranged on the way), one K block
+// and its scale factors per stage; a block is 13 (NVFP4,
 // TN = 128) issued instructions and costs 0.25 us, so that splitting K pays early: NVFP4 95 x 352 x 8960 14.7 -> 8.0 us,
 // MXFP4 2654 x 120 x 16384 22.4 -> 11.8, NVFP4 458 x 1176 x 6400 12.4 -> 10.2.
 #pragma once
@@ -57,7 +58,55 @@ struct TilesMaps {
 struct TilesScaleMaps {
     CUtensorMap a, b, c, sfa, sfb;
 };
-template <int DT> using TilesMapsOf = std::conditional_t<TilesKind<DT>::fp4, TilesScaleMaps, TilesMaps>;
+// One operand's scale factors on their way from row-major to the order of tensor memory (see pack_scales_kernel).
+struct PackOperand {
+    const uint32_t *in;
+    uint32_t *out;
+    uint32_t rows, row_groups;          // row groups of 128 after padding
+    uint32_t vector;                    // 1: `in` is aligned to a stage's words
+};
+
+// one row's words of a K block of 256 elements; zeros beyond the operand
+template <int WORDS>
+__device__ __forceinline__ void load_scale_words(const PackOperand &op, uint32_t row, uint32_t kb, uint32_t kblocks, uint32_t (&w)[WORDS])
+{
+    const uint32_t *src = op.in + ((uint64_t)row * kblocks + kb) * WORDS;
+#pragma unroll
+    for (int j = 0; j < WORDS; j++)
+        w[j] = 0;
+    if (row >= op.rows)
+        return;
+    if (op.vector) {
+        if constexpr (WORDS == 4) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(src);
+            w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        } else {
+            const uint2 v = *reinterpret_cast<const uint2 *>(src);
+            w[0] = v.x; w[1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < WORDS; j++)
+            w[j] = src[j];
+    }
+}
+
+// which 512-byte block of the arranged operand has word j of a group of 128 rows' K block; `pairs`: two groups' blocks lie together
+template <int WORDS>
+__device__ __forceinline__ uint64_t scale_block(uint32_t group, uint32_t kb, uint32_t j, uint32_t kblocks, bool pairs)
+{
+    return pairs ? (((uint64_t)(group >> 1) * kblocks + kb) * WORDS + j) * 2 + (group & 1) : ((uint64_t)group * kblocks + kb) * WORDS + j;
+}
+
+// Block-scaled operands whose scales are still row-major: `out` is where the workspace has their blocks.
+struct TilesRawMaps {
+    CUtensorMap a, b, c;
+    PackOperand sa, sb;
+};
+template <int DT, bool kRaw> using TilesMapsOf = std::conditional_t<kRaw, TilesRawMaps, std::conditional_t<TilesKind<DT>::fp4, TilesScaleMaps, TilesMaps>>;
+
+constexpr int kTilesScaleWarps = 6;
+constexpr int tiles_threads(bool raw) { return kGemmThreads + (raw ? 32 * kTilesScaleWarps : 0); }
 
 struct TilesParams {
     uint32_t tiles_m, tiles_n, group;
@@ -139,10 +188,96 @@ __device__ __forceinline__ void tma_load_pair_3d_at(void *smem_dst, const CUtens
         : "memory");
 }
 
+// ---------------- scale factors that are still row-major (six warps of each CTA) ----------------
+// A unit is 32 bytes of 128 rows, the words of two K blocks (NVFP4) or four (MXFP4), of A (this CTA's rows) or of B (each CTA
+// needs those of all its tile's columns).  Neighbouring lanes load those K blocks' words of a row, so that a warp's load touches 16 or
+// eight lines and not 32, each of which costs the L1 a cycle and more; a lane then holds the transposes of rows r, r + 32, r + 64,
+// r + 96, and the lanes of a K block write them to its stage as 16-byte pieces of the blocks that pack_scales_kernel makes.  A K
+// block has two or three units, and two or three sets of warps take turns: one loads while others write theirs.  The CTA pairs of the first tile row and column leave the blocks in the workspace as well, where the next call may look for
+// them (d_sfa = d_sfb = NULL).
+template <uint32_t kWords>
+__device__ __forceinline__ void tiles_arrange_scales(const TilesRawMaps &maps, const TilesParams &p, TilesSmem *sh, uint8_t *smem, uint32_t stage_bytes,
+                                                     uint32_t block_bytes, uint32_t w, uint32_t lane, uint32_t kb0, uint32_t kb1)
+{
+    constexpr uint32_t kGroup = 8 / kWords;                     // K blocks per unit
+    // A wait tells the last two phases of a barrier apart, no more.  So a warp may not come to a stage two rounds early: from one
+    // K block that it waits for to the next there are no more than the ring has stages (five with 256 columns, else six or more).
+    constexpr uint32_t kMostSets = kGroup == 4 ? 2 : 3;
+    static_assert((2 - 1) * kGroup + 1 <= 5 && (kMostSets - 1) * kGroup + 1 <= 6, "sets of warps too far apart");
+    const uint32_t rank = cluster_ctarank(), r = rank & 1, leader = rank & ~1u;
+    const uint32_t cluster_id = blockIdx.x / (2 * p.splits), n_clusters = gridDim.x / (2 * p.splits), n_tiles = p.tiles_m * p.tiles_n;
+    const uint32_t b_halves = (p.tn + 127) / 128, per_block = 1 + b_halves;
+    const uint32_t unit = w % per_block, sets = per_block == 3 ? 2 : kMostSets;
+    if (w >= sets * per_block)
+        return;
+    const bool is_b = unit > 0;
+    const PackOperand op = is_b ? maps.sb : maps.sa;
+    const uint32_t full0 = cluster_addr(&sh->full[0], leader);
+    const uint32_t n_kb = kb1 - kb0, groups = (n_kb + kGroup - 1) / kGroup;
+    const uint32_t x = lane / kGroup, mine = lane % kGroup;
+    uint8_t *const sf0 = smem + block_bytes + (is_b ? 2048 + (unit - 1) * 512 : 0) + x * 16;
+    const uint32_t step = is_b ? b_halves * 512 : 512;
+
+    uint32_t at = w / per_block, before = 0;                   // the group of four of this tile; K blocks of the tiles in front
+    for (uint32_t tile = cluster_id; tile < n_tiles; tile += n_clusters, before += n_kb, at -= groups) {
+        uint32_t mb, nb;
+        dense_tile_coords(tile, p.tiles_m, p.tiles_n, p.group, mb, nb);
+        const uint32_t rows = is_b ? nb * p.tn / 128 + unit - 1 : mb * 2 + r;          // which 128
+        const bool keep = is_b ? mb == 0 && r == 0 && nb * p.tn % 128 == 0 : nb == 0;
+        // a last group of B's rows without a tile for the other half of its 256: that half is zeros
+        const bool pad = is_b && rows % 2 == 0 && (rows + 1) * 128 >= p.tiles_n * p.tn;
+        for (; at < groups; at += sets) {
+            const uint32_t kb = kb0 + kGroup * at, here = kb1 - kb < kGroup ? kb1 - kb : kGroup;
+            uint32_t words[4 * kGroup][kWords];
+#pragma unroll
+            for (uint32_t i = 0; i < 4 * kGroup; i++)
+                load_scale_words<kWords>(op, mine < here ? rows * 128 + 32 / kGroup * i + x : ~0u, kb + mine, p.k_blocks, words[i]);
+            auto piece = [&](uint32_t i, uint32_t j) { return make_uint4(words[i][j], words[i + kGroup][j], words[i + 2 * kGroup][j], words[i + 3 * kGroup][j]); };
+            uint32_t s = (before + kGroup * at) % p.stages, round = (before + kGroup * at) / p.stages;
+            for (uint32_t t = 0; t < here; t++) {
+                if (!warp_wait(&sh->empty[s], (round + 1) & 1)) {          // a fresh barrier's preceding phase counts as complete
+                    if (lane == 0)
+                        atomicCAS(p.status, 0u, 0x226u);
+                    return;
+                }
+                if (mine == t) {
+#pragma unroll
+                    for (uint32_t i = 0; i < kGroup; i++)
+#pragma unroll
+                        for (uint32_t j = 0; j < kWords; j++)
+                            *reinterpret_cast<uint4 *>(sf0 + (size_t)s * stage_bytes + j * step + i * (512 / kGroup)) = piece(i, j);
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive_remote(full0 + 8 * s);
+                if (++s == p.stages) {
+                    s = 0;
+                    round++;
+                }
+            }
+            if (keep && mine < here) {
+                uint4 *out = reinterpret_cast<uint4 *>(op.out) + x;
+#pragma unroll
+                for (uint32_t j = 0; j < kWords; j++) {
+                    const uint64_t block = scale_block<kWords>(rows, kb + mine, j, p.k_blocks, is_b);
+#pragma unroll
+                    for (uint32_t i = 0; i < kGroup; i++) {
+                        out[block * 32 + 32 / kGroup * i] = piece(i, j);
+                        if (pad)
+                            out[(block + 1) * 32 + 32 / kGroup * i] = make_uint4(0, 0, 0, 0);
+                    }
+                }
+            }
+        }
+    }
+}
+
 // kRowBlocks: of 256 rows that share a tile's B, 1 or 2.  A template parameter, because as one of the launch the small
 // shapes took 1.4 % longer.
-template <int DT, uint32_t kRowBlocks>
-__global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_constant__ TilesMapsOf<DT> maps, TilesParams p)
+// kRaw: block-scaled operands whose scales lie row-major as their user has them; the last six warps arrange them.
+template <int DT, uint32_t kRowBlocks, bool kRaw>
+__global__ void __launch_bounds__(tiles_threads(kRaw)) gemm_tiles_kernel(const __grid_constant__ TilesMapsOf<DT, kRaw> maps, TilesParams p)
 {
     constexpr bool kFp4 = TilesKind<DT>::fp4;
     constexpr uint32_t kWords = TilesKind<DT>::words;
@@ -157,12 +292,13 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
     const uint32_t rank = cluster_ctarank(), r = rank & 1, leader = rank & ~1u, split = rank >> 1;
     const uint32_t cluster_id = blockIdx.x / (2 * p.splits), n_clusters = gridDim.x / (2 * p.splits);
     const uint32_t n_tiles = p.tiles_m * p.tiles_n;
-    const bool two_accs = kRowBlocks == 1 || p.tn <= 128;        // two accumulators where they fit
+    const bool two_accs = p.tn <= 128 || (kRowBlocks == 1 && !kFp4);        // two accumulators where they fit
+    const uint32_t b_halves = (p.tn + 127) / 128;                // blocks of 128 rows of B that a tile's scale factors come in
     const uint32_t kb0 = split * p.k_blocks / p.splits, kb1 = (split + 1) * p.k_blocks / p.splits;
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < p.stages; s++) {
-            mbar_init(&sh->full[s], 1);
+            mbar_init(&sh->full[s], kRaw ? 1 + 2 * (1 + b_halves) : 1);
             mbar_init(&sh->empty[s], 1);
         }
         for (int acc = 0; acc < 2; acc++) {
@@ -173,7 +309,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
         tma_prefetch_desc(&maps.a);
         tma_prefetch_desc(&maps.b);
         tma_prefetch_desc(&maps.c);
-        if constexpr (kFp4) {
+        if constexpr (kFp4 && !kRaw) {
             tma_prefetch_desc(&maps.sfa);
             tma_prefetch_desc(&maps.sfb);
         }
@@ -199,7 +335,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         const uint32_t full0 = cluster_addr(&sh->full[0], leader);
-        const uint32_t b_blocks = (p.tn + 127) / 128 * kWords;       // scale blocks of B per K block
+        const uint32_t b_blocks = b_halves * kWords;                 // scale blocks of B per K block
         uint32_t s = 0, parity = 1;                            // parity of the empty barrier's previous phase
         bool ok = true;
         for (uint32_t tile = cluster_id; tile < n_tiles && ok; tile += n_clusters) {
@@ -218,7 +354,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
                 const uint32_t nk = kb1 - kb < p.kps ? kb1 - kb : p.kps;
                 if (elect_one()) {
                     if (r == 0)
-                        mbar_expect_tx(&sh->full[s], nk * 2 * block_bytes + (kFp4 ? 2 * (kWords * 512 + b_blocks * 512) : 0));
+                        mbar_expect_tx(&sh->full[s], nk * 2 * block_bytes + (kFp4 && !kRaw ? 2 * (kWords * 512 + b_blocks * 512) : 0));
 #pragma unroll
                     for (uint32_t h = 0; h < 2; h++)
                         if (h < nk) {
@@ -228,7 +364,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
                                 tma_load_pair_at(blk + kHalfTileBytes, &maps.a, x + h * kRowBytesK, row_a + (int32_t)kTilesM, full0 + 8 * s);
                             tma_load_pair_at(blk + b_at, &maps.b, x + h * kRowBytesK, row_b, full0 + 8 * s);
                         }
-                    if constexpr (kFp4) {
+                    if constexpr (kFp4 && !kRaw) {
                         // A's blocks lie [rows / 128][K block][word], B's [rows / 256][K block][word][half of the 256]
                         uint8_t *sf = st + block_bytes;
                         tma_load_pair_at(sf, &maps.sfa, 0, (int32_t)(((mb * 2 + r) * p.k_blocks + kb) * kWords), full0 + 8 * s);
@@ -255,7 +391,6 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
             const uint32_t idesc = kFp4 ? make_idesc_block_scaled(256, p.tn, kFmtE2M1, kFmtE2M1, kMx ? 1u : 0u, 0, 0)
                                         : make_idesc(256, p.tn, kAFmt, kBFmt, DT == CLPK_DT_I8 ? kAccS32 : kAccF32);
             const uint32_t idesc_hi = make_idesc_block_scaled(256, p.tn, kFmtE2M1, kFmtE2M1, 1u, 2, 2);
-            const uint32_t b_halves = (p.tn + 127) / 128;
             const uint16_t pair_mask = (uint16_t)(3u << leader);
             uint32_t s = 0, parity = 0, tcount = 0;
             bool ok = true;
@@ -341,6 +476,9 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
                 __syncwarp();
             }
         }
+    } else if (kRaw && warp >= 2 + kEpilogueWarps) {
+        if constexpr (kRaw)
+            tiles_arrange_scales<kWords>(maps, p, sh, smem, stage_bytes, block_bytes, warp - (2 + kEpilogueWarps), lane, kb0, kb1);
     } else if (p.splits == 1) {
         // ---------------- epilogue, K not split: the two warps of a lane quarter take every other chunk ----------------
         uint32_t tcount = 0;
@@ -400,7 +538,8 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
         tc_fence_after_sync();
         const uint32_t slots = (n_chunks + p.splits - 1) / p.splits;
         const uint32_t taddr = tmem + ((q * 32) << 16), my_row = q * 32 + lane;
-        if (warp >= 2) {
+        const bool epilogue = warp >= 2 && warp < 2 + kEpilogueWarps;
+        if (epilogue) {
             for (uint32_t c = half; c < n_chunks; c += 2) {
                 const uint32_t owner = c % p.splits;
                 if (owner == split)
@@ -417,7 +556,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tiles_kernel(const __grid_c
         }
         __syncwarp();
         cluster_sync();
-        if (warp >= 2) {
+        if (epilogue) {
             uint32_t mb, nb;
             dense_tile_coords(cluster_id, p.tiles_m, p.tiles_n, p.group, mb, nb);
             const uint32_t row = mb * kTilesM + r * 128 + q * 32;

@@ -88,6 +88,14 @@ __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint64_t *bar, uint3
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
 }
 
+// Arrive on a barrier of the pair's leader.  All that is handed over lies in this CTA's own tensor and shared memory, complete
+// (tcgen05.wait::st) and fenced for the tensor core that reads it, so no wider release than the default is needed: with
+// .release.cluster each arrive held its warp for about 1000 cycles.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar)
+{
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 {
     uint32_t ok;

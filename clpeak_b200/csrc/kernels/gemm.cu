@@ -670,13 +670,6 @@ static_assert(sizeof(NvGemmSmem) <= 512, "NvGemmSmem");
 // line is read once.  The kernel is latency: launched with the programmatic attribute like the GEMM behind it, so that
 // both set up under the tail of what precedes.  NVFP4 one-call GEMM, device time at 2048^3 / 4096^3: 20.4 / 55.3 us with
 // one launch per operand through shared memory, 10.9 / 37.5 now, 8.1 / 31.2 with the scales already packed.
-struct PackOperand {
-    const uint32_t *in;
-    uint32_t *out;
-    uint32_t rows, row_groups;          // row groups of 128 after padding
-    uint32_t vector;                    // 1: `in` is aligned to a stage's words
-};
-
 template <int WORDS>
 __global__ void __launch_bounds__(256) pack_scales_kernel(PackOperand oa, PackOperand ob, uint32_t kblocks, uint32_t b_pairs)
 {
@@ -692,35 +685,12 @@ __global__ void __launch_bounds__(256) pack_scales_kernel(PackOperand oa, PackOp
         return;
     uint32_t w[4][WORDS];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const uint32_t row = group * 128 + i * 32 + lane;
-        const uint32_t *src = op.in + ((uint64_t)row * kblocks + kb) * WORDS;
+    for (int i = 0; i < 4; i++)
+        load_scale_words<WORDS>(op, group * 128 + i * 32 + lane, kb, kblocks, w[i]);
 #pragma unroll
-        for (int j = 0; j < WORDS; j++)
-            w[i][j] = 0;
-        if (row < op.rows) {
-            if (op.vector) {
-                if constexpr (WORDS == 4) {
-                    const uint4 v = *reinterpret_cast<const uint4 *>(src);
-                    w[i][0] = v.x; w[i][1] = v.y; w[i][2] = v.z; w[i][3] = v.w;
-                } else {
-                    const uint2 v = *reinterpret_cast<const uint2 *>(src);
-                    w[i][0] = v.x; w[i][1] = v.y;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < WORDS; j++)
-                    w[i][j] = src[j];
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < WORDS; j++) {
-        const uint64_t block = is_b && b_pairs ? (((uint64_t)(group >> 1) * kblocks + kb) * WORDS + j) * 2 + (group & 1)
-                                               : ((uint64_t)group * kblocks + kb) * WORDS + j;
+    for (int j = 0; j < WORDS; j++)
         // block byte (r % 32) * 16 + (r / 32) * 4 of row r
-        reinterpret_cast<uint4 *>(op.out)[block * 32 + lane] = make_uint4(w[0][j], w[1][j], w[2][j], w[3][j]);
-    }
+        reinterpret_cast<uint4 *>(op.out)[scale_block<WORDS>(group, kb, j, kblocks, is_b && b_pairs) * 32 + lane] = make_uint4(w[0][j], w[1][j], w[2][j], w[3][j]);
 }
 
 template <bool MX, int TN>
@@ -1139,9 +1109,9 @@ struct TilesPlan {
 // smaller operand traffic wins at every K; an FP4 tile 256 wide that is not split is the large kernel's own.  An FP4 A of a few
 // rows, whose lines more than half the pairs ask for at once, costs them 0.04 a block more, up to eight rows 0.15 (mxf4
 // 9 x 9336 x 14592: 32 us in 128-wide tiles, 26 in large ones; of 1400 shapes with few rows 87 were more than 3 % slower
-// than in large tiles, at worst 1.31 times, and with the term 17, at worst 1.10).  Behind the launch that arranges the
-// scales it does not show (nvf4 5 x 5632 x 3840: 11.1 us in 128-wide tiles, 14.0 in large ones), so `arranged`: FP4 whose
-// scales lie in the workspace already.
+// than in large tiles, at worst 1.31 times, and with the term 17, at worst 1.10).  Where the scales are arranged on the way it
+// does not show (nvf4 5 x 5632 x 3840: 10.2 us in 128-wide tiles, 11.4 in large ones; 35 shapes with up to 48 rows 0.835 and
+// 0.832 of the time before), so `arranged`: FP4 whose scales lie in the workspace already.
 // `sectors`: rows of the operands are whole 32-byte sectors.
 static TilesPlan plan_tiles(uint32_t m, uint32_t n, uint32_t k_blocks, bool sectors, bool fp4, bool arranged)
 {
@@ -1226,6 +1196,33 @@ static TilesPlan gemm_plan(uint32_t m, uint32_t n, uint32_t k, uint32_t elem_bit
     return plan_tiles(m, n, k_blocks_of(k, elem_bits), (uint64_t)k * elem_bits % 256 == 0, fp4, arranged);
 }
 
+static PackOperand pack_operand(const void *in, uint8_t *out, uint32_t rows, uint32_t words)
+{
+    return {static_cast<const uint32_t *>(in), reinterpret_cast<uint32_t *>(out), rows, padded_rows(rows) / 128,
+            (uintptr_t)in % (words * 4) == 0 ? 1u : 0u};
+}
+
+// FP4 with row-major scales: the tiles in which gemm_tiles_kernel arranges them on the way (kRaw), tn = 0: in a launch of their own.
+// That launch costs about 4 us in front of the product; on the way NVFP4's cost 0.1 us a K block, which their 16 bytes a row
+// have the L1 look up, and MXFP4's nothing that shows.  So: up to four waves of 256 x 256 tiles, beyond the first one NVFP4 sums only as
+// long as those 4 us allow, and where its words are loaded singly in the first one too.  Device time against the launch in front:
+// NVFP4 2048^3 13.4 -> 9.3 us, 1024 x 1024 x 2048 8.5 -> 7.4, 16384 x 256 x 2048 14.5 -> 9.4, 2048 x 2048 x 8192 22.4 -> 20.4, MXFP4 17.2 ->
+// 11.7 at 2048 x 2048 x 4096; random shapes 0.82 below one wave (worst 1.02), 0.88 up to two, 0.93 up to four (beyond: 1.03;
+// NVFP4 with 16 K blocks and more up to four waves 0.95 to 1.06, from unaligned addresses 1.19).
+static TilesPlan raw_scales_plan(const clpk_gemm_args_t *a, const PackOperand &sa, const PackOperand &sb)
+{
+    const uint64_t tiles = (uint64_t)((a->m - 1) / kTileMN + 1) * ((a->n - 1) / kTileMN + 1), pairs = (uint64_t)num_sms() / 2;
+    if (pairs == 0 || tiles > 4 * pairs || tuning(CLPK_TUNE_GEMM_FP4_TILE) > 0)
+        return {0, 1};
+    const uint64_t waves = (tiles - 1) / pairs + 1;
+    if (a->dtype == CLPK_DT_NVF4 && waves * (a->k / 256) > 40 && (waves > 1 || !sa.vector || !sb.vector))
+        return {0, 1};
+    TilesPlan plan = gemm_plan(a->m, a->n, a->k, 4, false);
+    if (plan.tn == 0)
+        plan.tn = kTileMN;              // the large tiles, by gemm_tiles_kernel
+    return plan;
+}
+
 // CTAs in clusters of `cluster`, behind the kernel before them
 template <typename Maps, typename Params>
 static int launch_clusters(void (*kernel)(Maps, Params), const char *what, uint32_t ctas, int threads, size_t smem, uint32_t cluster, cudaStream_t s,
@@ -1250,12 +1247,12 @@ static int launch_clusters(void (*kernel)(Maps, Params), const char *what, uint3
     return e == cudaSuccess ? CLPK_OK : cuda_fail(e, what);
 }
 
-// wsa, wsb: the packed scale factors (block-scaled kinds)
-template <int DT, uint32_t kRowBlocks = 1>
+// sa, sb: where the arranged scale factors lie (block-scaled kinds), and kRaw: where they come from
+template <int DT, uint32_t kRowBlocks = 1, bool kRaw = false>
 static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64_t row_bytes, uint32_t k_blocks, TilesPlan plan, cudaStream_t s,
-                        const uint8_t *wsa = nullptr, const uint8_t *wsb = nullptr)
+                        const PackOperand &sa = {}, const PackOperand &sb = {})
 {
-    TilesMapsOf<DT> maps;
+    TilesMapsOf<DT, kRaw> maps;
     maps.a = ta;
     int rc = make_operand_map(&maps.b, a->d_b, a->n, row_bytes, plan.tn / 2);
     if (rc != CLPK_OK)
@@ -1263,12 +1260,15 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
     rc = make_output_map(&maps.c, a->d_c, a->m, a->n, DT, true);
     if (rc != CLPK_OK)
         return rc;
-    if constexpr (TilesKind<DT>::fp4) {
+    if constexpr (kRaw) {
+        maps.sa = sa;
+        maps.sb = sb;
+    } else if constexpr (TilesKind<DT>::fp4) {
         constexpr uint32_t words = TilesKind<DT>::words;
-        rc = make_scale_map(&maps.sfa, wsa, (uint64_t)padded_rows(a->m) / 128 * k_blocks * words, words);
+        rc = make_scale_map(&maps.sfa, sa.out, (uint64_t)padded_rows(a->m) / 128 * k_blocks * words, words);
         if (rc != CLPK_OK)
             return rc;
-        rc = make_scale_map_b(&maps.sfb, wsb, (uint64_t)padded_rows(a->n) / 128 * k_blocks * words, words, (plan.tn + 127) / 128);
+        rc = make_scale_map_b(&maps.sfb, sb.out, (uint64_t)padded_rows(a->n) / 128 * k_blocks * words, words, (plan.tn + 127) / 128);
         if (rc != CLPK_OK)
             return rc;
     }
@@ -1283,7 +1283,9 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
     p.status = a->d_status;
     const uint32_t n_tiles = p.tiles_m * p.tiles_n, pairs = (uint32_t)num_sms() / 2;
     const uint32_t clusters = plan.splits > 1 ? n_tiles : (n_tiles < pairs ? n_tiles : pairs);
-    const size_t fixed = kEpilogueWarps * kStagingBytes + sizeof(TilesSmem) + 1024;
+    constexpr size_t fixed = kEpilogueWarps * kStagingBytes + sizeof(TilesSmem) + 1024;
+    static_assert(!kRaw || ((kTilesSmemMax - fixed) / (tiles_block_bytes(256) + tiles_sf_bytes(256)) >= 5 &&
+                            (kTilesSmemMax - fixed) / (tiles_block_bytes(128) + tiles_sf_bytes(128)) >= 6), "the stages that tiles_arrange_scales counts on");
     // two K blocks per stage halve the hand-overs (0.195 -> 0.137 us per block at TN = 32), but from TN = 160 on leave
     // too few stages (2048^3 bf16 at TN = 192: 19.3 -> 20.7 us)
     constexpr bool fp4 = TilesKind<DT>::fp4;
@@ -1298,7 +1300,7 @@ static int launch_tiles(const clpk_gemm_args_t *a, const CUtensorMap &ta, uint64
         p.tmem_cols *= 2;
     CLPK_CUDA(cudaGetSymbolAddress(reinterpret_cast<void **>(&p.clock), g_gemm_clock));
     const size_t smem = p.stages * stage_bytes + fixed;
-    return launch_clusters(gemm_tiles_kernel<DT, kRowBlocks>, "gemm_tiles", clusters * 2 * plan.splits, kGemmThreads, smem, 2 * plan.splits, s, maps, p);
+    return launch_clusters(gemm_tiles_kernel<DT, kRowBlocks, kRaw>, "gemm_tiles", clusters * 2 * plan.splits, tiles_threads(kRaw), smem, 2 * plan.splits, s, maps, p);
 }
 
 template <int DT>
@@ -1482,22 +1484,30 @@ static uint32_t fp4_tile_n(uint32_t m, uint32_t n, uint32_t k)
     return 256;
 }
 
+// 32-bit scale words per row per 256 elements of K, and the bytes that all of an operand's take in the workspace
+static uint32_t scale_words(int dtype) { return dtype == CLPK_DT_MXF4 ? 2 : 4; }
+static size_t scale_bytes(const clpk_gemm_args_t *a, uint32_t rows) { return (size_t)padded_rows(rows) * (a->k / 256) * scale_words(a->dtype) * 4; }
+
+// what the arrangement of row-major scale bytes asks for
+static int check_scales(const clpk_gemm_args_t *a)
+{
+    CLPK_REQUIRE(a->d_sfa && a->d_sfb, "block-scaled FP4 needs d_sfa and d_sfb");
+    CLPK_REQUIRE(a->d_workspace && a->workspace_bytes >= scale_bytes(a, a->m) + scale_bytes(a, a->n) && ((uintptr_t)a->d_workspace % 16) == 0,
+                 "block-scaled FP4 needs a 16-byte aligned workspace of clpk_gemm_workspace_bytes() bytes");
+    CLPK_REQUIRE(((uintptr_t)a->d_sfa % 4) == 0 && ((uintptr_t)a->d_sfb % 4) == 0, "scale arrays must be 4-byte aligned");
+    return CLPK_OK;
+}
+
 // Row-major scale bytes of both operands -> tile order in the workspace (A's blocks, then B's).
 static int pack_scales(const clpk_gemm_args_t *a, cudaStream_t s)
 {
-    const uint32_t words = a->dtype == CLPK_DT_MXF4 ? 2 : 4;   // 32-bit scale words per row per 256 elements of K
-    const size_t sfa_bytes = (size_t)padded_rows(a->m) * (a->k / 256) * words * 4, sfb_bytes = (size_t)padded_rows(a->n) * (a->k / 256) * words * 4;
-    CLPK_REQUIRE(a->d_sfa && a->d_sfb, "block-scaled FP4 needs d_sfa and d_sfb");
-    CLPK_REQUIRE(a->d_workspace && a->workspace_bytes >= sfa_bytes + sfb_bytes && ((uintptr_t)a->d_workspace % 16) == 0,
-                 "block-scaled FP4 needs a 16-byte aligned workspace of clpk_gemm_workspace_bytes() bytes");
-    CLPK_REQUIRE(((uintptr_t)a->d_sfa % 4) == 0 && ((uintptr_t)a->d_sfb % 4) == 0, "scale arrays must be 4-byte aligned");
-    uint8_t *wsa = static_cast<uint8_t *>(a->d_workspace), *wsb = wsa + sfa_bytes;
+    const int rc = check_scales(a);
+    if (rc != CLPK_OK)
+        return rc;
+    const uint32_t words = scale_words(a->dtype);
+    uint8_t *wsa = static_cast<uint8_t *>(a->d_workspace), *wsb = wsa + scale_bytes(a, a->m);
     const uint32_t kblocks = a->k / 256;
-    auto operand = [&](const void *in, uint8_t *out, uint32_t rows) {
-        return PackOperand{static_cast<const uint32_t *>(in), reinterpret_cast<uint32_t *>(out), rows, padded_rows(rows) / 128,
-                           (uintptr_t)in % (words * 4) == 0 ? 1u : 0u};
-    };
-    const PackOperand oa = operand(a->d_sfa, wsa, a->m), ob = operand(a->d_sfb, wsb, a->n);
+    const PackOperand oa = pack_operand(a->d_sfa, wsa, a->m, words), ob = pack_operand(a->d_sfb, wsb, a->n, words);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((oa.row_groups + ob.row_groups) * ((kblocks + 7) / 8));
     cfg.blockDim = dim3(256);
@@ -1598,21 +1608,28 @@ int clpk_gemm(const clpk_gemm_args_t *a, void *stream)
 
     if (block_scaled) {
         const bool mx = a->dtype == CLPK_DT_MXF4;
-        const uint32_t words = mx ? 2 : 4;                      // 32-bit scale words per row per 256 elements of K
-        const size_t sfa_bytes = (size_t)padded_rows(a->m) * (a->k / 256) * words * 4, sfb_bytes = (size_t)padded_rows(a->n) * (a->k / 256) * words * 4;
+        const uint32_t words = scale_words(a->dtype);
+        const size_t sfa_bytes = scale_bytes(a, a->m), sfb_bytes = scale_bytes(a, a->n);
         CLPK_REQUIRE((a->d_sfa != nullptr) == (a->d_sfb != nullptr), "d_sfa and d_sfb: give both, or neither when the workspace is already packed");
         CLPK_REQUIRE(a->d_workspace && a->workspace_bytes >= sfa_bytes + sfb_bytes && ((uintptr_t)a->d_workspace % 16) == 0,
                      "block-scaled FP4 needs a 16-byte aligned workspace of clpk_gemm_workspace_bytes() bytes");
         uint8_t *wsa = static_cast<uint8_t *>(a->d_workspace), *wsb = wsa + sfa_bytes;
+        const PackOperand sa = pack_operand(a->d_sfa, wsa, a->m, words), sb = pack_operand(a->d_sfb, wsb, a->n, words);
         if (a->d_sfa) {
+            rc = check_scales(a);
+            if (rc != CLPK_OK)
+                return rc;
+            if (const TilesPlan plan = raw_scales_plan(a, sa, sb); plan.tn)
+                return mx ? launch_tiles<CLPK_DT_MXF4, 1, true>(a, ta, row_bytes, p.k_blocks, plan, s, sa, sb)
+                          : launch_tiles<CLPK_DT_NVF4, 1, true>(a, ta, row_bytes, p.k_blocks, plan, s, sa, sb);
             rc = pack_scales(a, s);
             if (rc != CLPK_OK)
                 return rc;
         }
         const uint32_t tn = fp4_tile_n(a->m, a->n, a->k);
         if (const TilesPlan plan = gemm_plan(a->m, a->n, a->k, elem_bits, a->d_sfa == nullptr); plan.tn)
-            return mx ? launch_tiles<CLPK_DT_MXF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb)
-                      : launch_tiles<CLPK_DT_NVF4>(a, ta, row_bytes, p.k_blocks, plan, s, wsa, wsb);
+            return mx ? launch_tiles<CLPK_DT_MXF4>(a, ta, row_bytes, p.k_blocks, plan, s, sa, sb)
+                      : launch_tiles<CLPK_DT_NVF4>(a, ta, row_bytes, p.k_blocks, plan, s, sa, sb);
         CUtensorMap tsa, tsb;
         rc = make_scale_map(&tsa, wsa, sfa_bytes / 512, words);
         if (rc != CLPK_OK)

@@ -49,6 +49,29 @@ def test_scales_at_any_word_alignment(K, cuda, dtype, m, n, k):
         assert bool((ws == results[0][0]).all()) and bool((c == results[0][1]).all())
 
 
+# Row-major scales are arranged by the multiplication itself up to four waves of 256 x 256 tiles, and by a launch of their own
+# beyond, and for long NVFP4 sums from the second wave on.  One to nine K blocks (units hold two or four); 64- and 128-wide tiles
+# whose last block of rows has no neighbour; 256-wide ones with one accumulator, one to four waves of them; K split.
+@pytest.mark.parametrize("m,n,k", [(64, 64, 256), (130, 72, 768), (520, 328, 1280), (300, 1160, 2304), (2048, 2048, 2048), (2000, 2056, 512),
+                                   (2200, 2304, 1792), (4096, 4096, 1024), (4100, 4616, 256), (600, 7000, 5376), (458, 1176, 6400), (300, 136, 11008)])
+@pytest.mark.parametrize("dtype,offset", [(N.DT_NVF4, 0), (N.DT_NVF4, 4), (N.DT_MXF4, 0), (N.DT_MXF4, 4), (N.DT_MXF4, 8)])
+def test_scales_arranged_on_the_way_and_in_front(K, cuda, dtype, offset, m, n, k):
+    g = cuda.Generator(device="cuda").manual_seed(m + n + k)
+    a, b = (cuda.randint(0, 256, (rows * k // 2,), dtype=cuda.uint8, device="cuda", generator=g) for rows in (m, n))
+    block = 16 if dtype == N.DT_NVF4 else 32
+    base = 0x30 if dtype == N.DT_NVF4 else 0x78                     # 0.5 ... 15, or 2^-7 ... 2^8
+    sfa, sfb = (cuda.randint(base, base + 16 if dtype == N.DT_MXF4 else base + 0x28, (rows * k // block + offset,), dtype=cuda.uint8, device="cuda",
+                             generator=g)[offset:] for rows in (m, n))
+    in_front, on_the_way = workspace(K, cuda, dtype, m, n, k), workspace(K, cuda, dtype, m, n, k)
+    args = N.GemmArgs(dtype=dtype, m=m, n=n, k=k, d_sfa=sfa.data_ptr(), d_sfb=sfb.data_ptr(), d_workspace=in_front.data_ptr(),
+                      workspace_bytes=in_front.numel())
+    K.clpk_gemm_pack_scales(C.byref(args), stream_ptr())
+    want = run(K, cuda, dtype, m, n, k, a, None, b, None, 0.25, in_front)
+    got = run(K, cuda, dtype, m, n, k, a, sfa.data_ptr(), b, sfb.data_ptr(), 0.25, on_the_way)
+    assert bool((got == want).all()), "the same sums in the same order"
+    assert bool((on_the_way == in_front).all()), "the workspace holds the arranged scales afterwards"
+
+
 def decoded(cuda, dtype, q, sf, rows, k):
     """The operand's values in fp64."""
     codes = cuda.stack((q & 15, q >> 4), dim=-1).view(rows, k).long()
