@@ -27,17 +27,22 @@
 // 54.0 (the warps stood at the tile stores waiting for the global loads); the same through
 // the staging buffer, 58.9.
 //
-// fp64 (dgemm_kernel).  128 x 64 x 16 tile per CTA of 128 threads = 4 warps in a 2 x 2
-// grid, two CTAs per SM, 64 x 32 outputs per warp = 8 x 4 m8n8k4 accumulator tiles (128
-// registers of accumulators per thread).  Operands go global -> shared with cp.async (16 bytes), three
-// stages; rows are padded to 20 doubles so that the fragment reads (lane -> row lane/4,
-// k lane%4) fall in 16 distinct 8-byte banks per half warp.  Bound: the DMMA pipe, 64
-// fp64 FMA / clock / SM, the same rate as the scalar DFMA pipe (37.2 TFLOPS at 1.965 GHz).
+// fp64 (dgemm_kernel).  64 x 64 x 16 tile per CTA of 128 threads = 4 warps in a 2 x 2 grid, four CTAs per SM, 32 x 32
+// outputs per warp = 4 x 4 m8n8k4 accumulator tiles, multiplied two at a time (m16n8k4).  Operands go global -> shared with
+// cp.async (16 bytes), three stages; a row's chunks are permuted so that the fragment reads (lane -> row lane/4, k lane%4)
+// fall in 16 distinct 8-byte banks per half warp.  Bound: the DMMA pipe, 64 fp64 FMA / clock / SM, the same rate as the scalar
+// DFMA pipe (37.2 TFLOPS at 1.965 GHz).  Measured 34.6 TFLOPS at 4096^3 and 8192 x 8192 x 512, 32.9 at 2048 x 2048 x 512, where
+// 1024 tiles are 6.9 per SM.  Before, 128 x 64 tiles of four 64 x 32 warps, two CTAs per SM, rows padded to 20 doubles, took
+// 4027 us at 4096^3 (3968 now), 2066 at 8192 x 8192 x 512 (1987), 136 at 10770 x 310 x 410 (97): with half the CTAs per SM a
+// partial round keeps fewer of them busy.  64 x 64 tiles whose result goes through shared memory, in blocks of eight k: 2048 x 2048 x 512
+// 144 us (131 now), 5001 x 5001 x 4 78 (59).  Tried: two warps of 64 x 32 per CTA 155, m16n8k8 and m16n8k16 as m16n8k4 and 4 %
+// slower, 128 x 64 tiles with this layout and four stages 3962 at 4096^3, a last row loaded again in place of the zeros beyond an
+// operand (65 x 10179 x 180 25 -> 33 us), fragments loaded a step ahead (within 1 %).
 //
 // Shapes of which those tiles make too few CTAs take 64 x 64 (fp32, fp64) or 32 x 32 (fp64) tiles with K split over the
 // CTAs of a cluster and over groups of warps inside a CTA (sgemm64_kernel, dgemm_split_kernel; plan_simt has the rule).
 // Device time before -> after: fp32 64 x 64 x 16384 1545 -> 57 us, 459 x 349 x 4636 474 -> 69; fp64
-// 64 x 64 x 16384 1388 -> 26, 863 x 251 x 2456 228 -> 42, 2048 x 2048 x 512 151 -> 143.
+// 64 x 64 x 16384 1388 -> 26, 863 x 251 x 2456 228 -> 42.
 //
 // All take any M, N > 0 and any K that keeps operand rows 16-byte aligned (a multiple of 4
 // floats, 2 doubles): a second instantiation of the large kernels, and the others always, zero-fill the chunks a tile
@@ -46,6 +51,8 @@
 //
 // CTAs walk C in groups of 16 tile rows so that the operand panels a wave of CTAs needs
 // stay in L2.  Work 2*M*N*K flop; minimum HBM bytes (M*K + N*K + M*N) * element.
+#include <algorithm>
+
 #include "../clpk_internal.h"
 #include "../clpk_ptx.cuh"
 
@@ -454,15 +461,11 @@ sgemm64_kernel(const float *A, const float *B, float *C, uint32_t M, uint32_t N,
 // fp64
 // ---------------------------------------------------------------------------------------------
 
-constexpr int kDgemmLd = kSimtBK + 4;                    // doubles per row of a shared tile (160 bytes)
-constexpr int kDgemmStages = 3;
-// CN = columns of C per CTA.  64: four warps and two CTAs per SM, whose barriers and pipeline fills overlap each
-// other; with 128 (eight warps, one CTA per SM) the DMMA pipe idled at every CTA-wide barrier (87 % busy in ncu).
-template <int CN> struct Dgemm {
-    static constexpr int threads = 2 * CN;
-    static constexpr size_t stage_doubles = (size_t)(kSimtTile + CN) * kDgemmLd;
-    static constexpr size_t smem_bytes = kDgemmStages * stage_doubles * sizeof(double);
-};
+constexpr int kDgemmTile = 64, kDgemmThreads = 128, kDgemmStages = 3;
+constexpr int kDgemmPartLd = kDgemmTile + 8;             // doubles per row of a tile of C in shared memory: 16-byte pieces of two rows on all banks
+constexpr size_t kDgemmStageDoubles = 2 * (size_t)kDgemmTile * kSimtBK;
+constexpr size_t kDgemmSmemBytes = kDgemmStages * kDgemmStageDoubles * sizeof(double);
+static_assert(kDgemmTile * kDgemmPartLd * sizeof(double) <= kDgemmSmemBytes, "the tile of C takes the ring's place");
 
 __device__ __forceinline__ void dmma_m8n8k4(double &d0, double &d1, double a, double b)
 {
@@ -471,50 +474,55 @@ __device__ __forceinline__ void dmma_m8n8k4(double &d0, double &d1, double a, do
         : "d"(a), "d"(b));
 }
 
-template <int CN, bool RAGGED>
-__global__ void __launch_bounds__(Dgemm<CN>::threads, 128 / CN)
+// rows g and g + 8 of 16 (g = lane / 4): the same operations as two m8n8k4, in half the instructions
+__device__ __forceinline__ void dmma_m16n8k4(double (&upper)[2], double (&lower)[2], double a_upper, double a_lower, double b)
+{
+    asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+        : "+d"(upper[0]), "+d"(upper[1]), "+d"(lower[0]), "+d"(lower[1])
+        : "d"(a_upper), "d"(a_lower), "d"(b));
+}
+
+// 64 x 64 tile, four warps of 32 x 32, four CTAs per SM.  RAGGED as for sgemm_kernel.  STAGED: N is odd, so that pairs of columns are
+// not aligned; a tile of C goes through shared memory and leaves in whole rows of single doubles.
+template <bool RAGGED, bool STAGED>
+__global__ void __launch_bounds__(kDgemmThreads, 4)
 dgemm_kernel(const double *A, const double *B, double *C, uint32_t M, uint32_t N,
              uint32_t K, double alpha, uint32_t *status)
 {
+    static_assert(RAGGED || !STAGED, "whole tiles have an even N");
     extern __shared__ __align__(16) double dsm[];
-    constexpr int kThreads = Dgemm<CN>::threads;
-    constexpr size_t kDgemmStageDoubles = Dgemm<CN>::stage_doubles;
     uint32_t tm, tn;
-    raster(blockIdx.x, (M + kSimtTile - 1) / kSimtTile, (N + CN - 1) / CN, &tm, &tn);
+    raster(blockIdx.x, (M + kDgemmTile - 1) / kDgemmTile, (N + kDgemmTile - 1) / kDgemmTile, &tm, &tn);
     join_stream(status);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int kWarpsN = CN / 32;
-    const int wm = (warp / kWarpsN) * 64, wn = (warp % kWarpsN) * 32;   // this warp's 64 x 32 corner inside the tile
-    const double *gA = A + (size_t)tm * kSimtTile * K, *gB = B + (size_t)tn * CN * K;
+    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;              // this warp's 32 x 32 corner inside the tile
+    const double *gA = A + (size_t)tm * kDgemmTile * K, *gB = B + (size_t)tn * kDgemmTile * K;
 
-    // one stage = A tile [128][kDgemmLd] then B tile [CN][kDgemmLd]; 16-byte chunks, 8 per row
-    auto load_stage = [&](int stage, uint32_t k0) {
-        double *sa = dsm + (size_t)stage * kDgemmStageDoubles, *sb = sa + (size_t)kSimtTile * kDgemmLd;
-#pragma unroll
-        for (int i = 0; i < kSimtTile * 8 / kThreads; i++) {
-            const int c = tid + kThreads * i, r = c >> 3, kc = (c & 7) * 2;
-            if (RAGGED) {
-                const bool inside = tm * kSimtTile + r < M && k0 + kc < K;
-                cp_async_16_or_zeros(sa + r * kDgemmLd + kc, inside ? gA + (size_t)r * K + k0 + kc : A, inside);
-            } else {
-                cp_async_16(sa + r * kDgemmLd + kc, gA + (size_t)r * K + k0 + kc);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < CN * 8 / kThreads; i++) {
-            const int c = tid + kThreads * i, r = c >> 3, kc = (c & 7) * 2;
-            if (RAGGED) {
-                const bool inside = tn * CN + r < N && k0 + kc < K;
-                cp_async_16_or_zeros(sb + r * kDgemmLd + kc, inside ? gB + (size_t)r * K + k0 + kc : B, inside);
-            } else {
-                cp_async_16(sb + r * kDgemmLd + kc, gB + (size_t)r * K + k0 + kc);
-            }
+    // One stage = A tile [64][16] then B tile [64][16] in 16-byte chunks, eight per row; chunk c of row r lies at c ^ 2 (r % 4), so
+    // that the fragment reads of a half warp (four rows, four k) fall in 16 distinct 8-byte banks.  Piece i of it is 16 rows, the
+    // first four pieces A's.  Ragged: zeros arrive in place of what lies beyond an operand, and of a whole piece without `more`.
+    constexpr int kPieces = 2 * kDgemmTile * 8 / kDgemmThreads;
+    auto load_piece = [&](int stage, uint32_t k0, int i, bool more) {
+        const int c = tid + kDgemmThreads * (i % (kPieces / 2)), r = c >> 3, kc = (c & 7) * 2;
+        const bool is_a = i < kPieces / 2;
+        double *dst = dsm + (size_t)stage * kDgemmStageDoubles + (r + (is_a ? 0 : kDgemmTile)) * kSimtBK + (kc ^ ((r & 3) << 2));
+        const double *src = (is_a ? gA : gB) + (size_t)r * K + k0 + kc;
+        if (RAGGED) {
+            const bool inside = more && (is_a ? tm * kDgemmTile + r < M : tn * kDgemmTile + r < N) && k0 + kc < K;
+            cp_async_16_or_zeros(dst, inside ? src : A, inside);
+        } else {
+            cp_async_16(dst, src);
         }
     };
-
-    double acc[8][4][2];
+    auto load_stage = [&](int stage, uint32_t k0) {
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+        for (int i = 0; i < kPieces; i++)
+            load_piece(stage, k0, i, true);
+    };
+
+    double acc[4][4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++)
             acc[i][j][0] = acc[i][j][1] = 0.0;
@@ -530,51 +538,68 @@ dgemm_kernel(const double *A, const double *B, double *C, uint32_t M, uint32_t N
     for (uint32_t kb = 0; kb < nk; kb++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kDgemmStages - 2) : "memory");
         __syncthreads();                                            // stage kb has landed; stage kb-1 is free for reuse
-        if (kb + kDgemmStages - 1 < nk)
-            load_stage((kb + kDgemmStages - 1) % kDgemmStages, (kb + kDgemmStages - 1) * kSimtBK);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        const double *sa = dsm + (size_t)(kb % kDgemmStages) * kDgemmStageDoubles, *sb = sa + (size_t)kSimtTile * kDgemmLd;
+        // Whole tiles ask for the next block here.  Ragged ones do so a piece at a time under the multiplications: the tests on
+        // each piece would hold up a warp that has its scheduler to itself (109 x 8532 x 4434 345 -> 327 us, 2290 x 1258 x 5472
+        // 1140 -> 999; for whole tiles 1 % slower).
+        const uint32_t next = kb + kDgemmStages - 1;
+        if (!RAGGED && next < nk)
+            load_stage(next % kDgemmStages, next * kSimtBK);
+        const double *sa = dsm + (size_t)(kb % kDgemmStages) * kDgemmStageDoubles + (wm + fr) * kSimtBK;
+        const double *sb = dsm + (size_t)(kb % kDgemmStages) * kDgemmStageDoubles + (kDgemmTile + wn + fr) * kSimtBK;
 #pragma unroll
         for (int k4 = 0; k4 < kSimtBK; k4 += 4) {
-            double a[8], b[4];
+            const int at = (k4 ^ ((fr & 3) << 2)) + fk;
+            double a[4], b[4];
 #pragma unroll
-            for (int i = 0; i < 8; i++)
-                a[i] = sa[(wm + 8 * i + fr) * kDgemmLd + k4 + fk];
+            for (int i = 0; i < 4; i++)
+                a[i] = sa[8 * i * kSimtBK + at];
 #pragma unroll
             for (int j = 0; j < 4; j++)
-                b[j] = sb[(wn + 8 * j + fr) * kDgemmLd + k4 + fk];
+                b[j] = sb[8 * j * kSimtBK + at];
+            if (RAGGED) {
 #pragma unroll
-            for (int i = 0; i < 8; i++)
+                for (int i = 0; i < kPieces / 4; i++)
+                    load_piece(next % kDgemmStages, next * kSimtBK, k4 / 4 * (kPieces / 4) + i, next < nk);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i += 2)
 #pragma unroll
                 for (int j = 0; j < 4; j++)
-                    dmma_m8n8k4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+                    dmma_m16n8k4(acc[i][j], acc[i + 1][j], a[i], a[i + 1], b[j]);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 
     // accumulator tile (i, j): this lane holds row lane/4, columns 2*(lane%4) and the next one
-    double *gC = C + ((size_t)tm * kSimtTile + wm) * N + (size_t)tn * CN + wn;
+    if constexpr (STAGED) {
+        __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                *reinterpret_cast<double2 *>(dsm + (wm + 8 * i + fr) * kDgemmPartLd + wn + 8 * j + 2 * fk) = make_double2(alpha * acc[i][j][0], alpha * acc[i][j][1]);
+        __syncthreads();
+        const uint32_t col = tn * kDgemmTile + lane;
+#pragma unroll
+        for (int i = 0; i < kDgemmTile / 4; i++) {
+            const int r = warp + 4 * i;
+            const uint32_t row = tm * kDgemmTile + r;
+            double *dst = C + (size_t)row * N + col;
+            if (row < M && col < N)
+                dst[0] = dsm[r * kDgemmPartLd + lane];
+            if (row < M && col + 32 < N)
+                dst[32] = dsm[r * kDgemmPartLd + lane + 32];
+        }
+        return;
+    }
+    double *gC = C + ((size_t)tm * kDgemmTile + wm) * N + (size_t)tn * kDgemmTile + wn;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++)
-        {
-            double *dst = gC + (size_t)(8 * i + fr) * N + 8 * j + 2 * fk;
-            const double2 v = make_double2(alpha * acc[i][j][0], alpha * acc[i][j][1]);
-            if (!RAGGED) {
-                *reinterpret_cast<double2 *>(dst) = v;
-            } else if (tm * kSimtTile + wm + 8 * i + fr < M) {
-                const uint32_t col = tn * CN + wn + 8 * j + 2 * fk;
-                if ((N & 1) == 0 && col < N) {
-                    *reinterpret_cast<double2 *>(dst) = v;
-                } else {
-                    if (col < N)
-                        dst[0] = v.x;
-                    if (col + 1 < N)
-                        dst[1] = v.y;
-                }
-            }
-        }
+            if (!RAGGED || (tm * kDgemmTile + wm + 8 * i + fr < M && tn * kDgemmTile + wn + 8 * j + 2 * fk < N))
+                *reinterpret_cast<double2 *>(gC + (size_t)(8 * i + fr) * N + 8 * j + 2 * fk) = make_double2(alpha * acc[i][j][0], alpha * acc[i][j][1]);
 }
 
 // Smaller tiles, K split over the CTAs of a cluster and over WK groups of WM x WN warps inside a CTA; 32 x 32 outputs
@@ -718,28 +743,39 @@ static int launch_simt(void (*kernel)(Params...), const char *what, uint64_t cta
     return CLPK_OK;
 }
 
-// Tile edge (128: the large kernels) and K ranges for a problem: the cheapest by an estimate in microseconds, fitted to
-// 400 timed launches of all kernels on 90 shapes (M and N from 64 to 15000, K to 16000; residuals 5 to 9 %, 13 % for the
-// 32-wide fp64 tile; the chosen plans are 2 to 3 % slower than the fastest in the geometric mean).  With L CTAs on the
-// busiest SM, a block of 16 k costs its CTA  max(alone, L * shared):
+// Tile edge and K ranges for a problem (128: sgemm_kernel, and dgemm_kernel, whose tiles are 64 wide, with an even N): the cheapest
+// by an estimate in microseconds, fitted to 400 timed launches of all kernels on 90 shapes (M and N from 64 to 15000, K to 16000;
+// residuals 5 to 9 %, 13 % for the 32-wide fp64 tile; the chosen plans are 2 to 3 % slower than the fastest in the geometric
+// mean), and dgemm_kernel's to 400 more (4 %).  With L CTAs on the busiest SM, a block of 16 k costs its CTA  max(alone, L * shared):
 //   fp32  128 x 128  max(1.62, 1.43 L)    64 x 64  max(0.51, 0.40 L)    (the pipe's own time: 1.07 and 0.27 L)
-//   fp64  128 x 64   max(1.48, 1.24 L)    64 x 64  max(0.91, 0.62 L)    32 x 32  max(0.22, 0.17 L)    (1.08, 0.54, 0.13 L)
+//   fp64  whole 64 x 64  max(0.75, 0.607 L)    split 64 x 64  max(0.91, 0.62 L)    32 x 32  max(0.22, 0.16 to 0.174 L, the less the
+//   longer)    (0.54, 0.54, 0.13 L)
 // A CTA alone on its SM with a range of 32 blocks (fp32) or 24 (fp64) takes twice the K groups: 0.41 and 0.18 a block,
 // and 1.5 and 0.6 us more for the longer sum at the end (shorter ranges lose up to 20 % by it, long ones gain up to 33 %).
-// The large tiles are kept unless the estimate is 8 % better; a K range has at least four blocks.  Short fp64 sums have an
+// The 128 x 128 tiles are kept unless the estimate is 8 % better; a K range has at least four blocks.  Short fp64 sums have an
 // estimate of their own (plan_short_f64).
 struct SimtPlan {
     uint32_t tile, splits;
     bool wide;                  // twice the K groups
     float us = 0.0f;            // the estimate it was chosen by (fp32 and long fp64 sums)
+    bool whole = false;         // dgemm_kernel
 };
 
+// What clpk_gemm_plan says of dgemm_kernel's tiles: 64 where C goes through shared memory (an odd N), else that they are its own.
+static SimtPlan whole_f64_plan(uint32_t n, float us) { return {n % 2 ? 64u : 128u, 1, false, us, true}; }
+
+// dgemm_kernel is not considered for fewer tiles than two SMs of three have one.  32-wide tiles serve most of those better, up to
+// three times; not all of them (1481 x 215 x 40: 5.9 us, 4.5 in 64-wide ones).
+static uint64_t whole_f64_tiles(uint32_t m, uint32_t n)
+{
+    const uint64_t tiles = (uint64_t)((m - 1) / kDgemmTile + 1) * ((n - 1) / kDgemmTile + 1);
+    return 3 * tiles < 2 * simt_capacity(1) ? 0 : tiles;
+}
+
 // fp64 with fewer than 24 blocks: what a CTA costs besides them -- start, pipeline fill, sum, stores -- is then a good part
-// of its time.  Small tiles pay it once per round of the CTAs that an SM holds (4 of 64 x 64, 3 of 32 x 32), the large
-// kernel, whose odd rows of C are stored in 8-byte pieces, with every CTA.  Fitted to 490 shapes with K from 2 to 368
-// (residuals 10, 6 and 7 %; the chosen plans are 1 % slower than the fastest in the geometric mean, where the estimate
-// above was 10 % slower and 2.7 times at worst: 4153 x 558 x 6 took 23.5 us in 32 x 32 tiles against 9.3 in the large
-// ones, 12879 x 166 x 12 23.9 against 9.9, 963 x 955 x 248 35.9 against 24.3 in 64 x 64 ones).
+// of its time, paid once per round of the CTAs that an SM holds (4 of 64 x 64, 3 of 32 x 32).  Fitted to 490 shapes with K from
+// 2 to 368 (residuals 6 and 7 %; the chosen plans are 1 % slower than the fastest in the geometric mean, where the estimate
+// above was 10 % slower and 2.7 times at worst) and, for dgemm_kernel, to 180 (4 %).
 static SimtPlan plan_short_f64(uint32_t m, uint32_t n, uint32_t blocks)
 {
     auto per_sm = [&](uint32_t rows, uint32_t cols, uint32_t splits) {
@@ -750,11 +786,14 @@ static SimtPlan plan_short_f64(uint32_t m, uint32_t n, uint32_t blocks)
         auto round = [&](uint32_t c) { return c == 0 ? 0.0f : alone > c * shared ? alone : c * shared; };
         return (float)(ctas / held) * round(held) + round(ctas % held);
     };
-    SimtPlan plan = {128, 1, false};
-    const uint32_t large = per_sm(128, 64, 1);
-    float best = (large > 1 ? 0.90f : 0.95f) * (1.2f + (float)large * (1.45f * (float)blocks + 1.57f + (n % 2 ? 1.32f : 0.0f)));
+    SimtPlan plan = {32, 1, false};
+    float best = 1e30f;
+    if (whole_f64_tiles(m, n)) {
+        best = 0.97f * (2.75f + rounds(per_sm(64, 64, 1), 4, 0.785f * (float)blocks - 0.71f, 0.587f * (float)blocks + 0.36f));
+        plan = whole_f64_plan(n, best);
+    }
     for (uint32_t splits = 1; splits <= 4 && (splits == 1 || blocks >= 4 * splits); splits *= 2)
-        for (uint32_t tile = 32; tile <= 64; tile *= 2) {
+        for (uint32_t tile = 32; tile <= (splits == 1 ? 32u : 64u); tile *= 2) {
             const uint32_t ctas = per_sm(tile, tile, splits);
             const float range = (float)((blocks - 1) / splits + 1);
             const float t = tile == 64 ? 3.4f + rounds(ctas, 4, 0.92f * range + 1.54f, 0.60f * range + 1.05f)
@@ -777,9 +816,16 @@ static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
         const float busiest = shared * (float)((ctas(rows, cols, splits) - 1) / simt_capacity(splits) + 1);
         return (float)((blocks - 1) / splits + 1) * (alone > busiest ? alone : busiest);
     };
-    const float large = f64 ? 3.8f + estimate(128, 64, 1, 1.48f, 1.24f) : 2.0f + estimate(128, 128, 1, 1.62f, 1.43f);
-    float best = 0.92f * large;
-    SimtPlan plan = {128, 1, false, large};
+    float best = 1e30f;
+    SimtPlan plan = {32, 1, false};
+    if (!f64) {
+        const float large = 2.0f + estimate(128, 128, 1, 1.62f, 1.43f);
+        best = 0.92f * large;
+        plan = {128, 1, false, large};
+    } else if (whole_f64_tiles(m, n)) {
+        best = 3.2f + estimate(64, 64, 1, 0.75f, 0.607f);
+        plan = whole_f64_plan(n, best);
+    }
     for (uint32_t splits = 1; splits <= 8 && (splits == 1 || blocks >= 4 * splits); splits *= 2)
         for (uint32_t tile = f64 ? 32 : 64; tile <= 64; tile *= 2) {
             const bool wide = !(f64 && tile == 64) && ctas(tile, tile, splits) <= simt_capacity(splits) && blocks >= (f64 ? 24 : 32) * splits;
@@ -790,7 +836,8 @@ static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
             else if (tile == 64)
                 t = 4.56f + estimate(64, 64, splits, 0.907f, 0.616f);
             else
-                t = (wide ? 4.5f + estimate(32, 32, splits, 0.178f, 0.0f) : 3.9f + estimate(32, 32, splits, 0.223f, 0.174f)) +
+                t = (wide ? 4.5f + estimate(32, 32, splits, 0.178f, 0.0f)
+                          : 3.9f + estimate(32, 32, splits, 0.223f, std::min(0.174f, 0.16f + 0.6f * (float)splits / (float)blocks))) +
                     (splits > 1 ? 0.5f * splits : 0.0f);
             if (t < best) {
                 best = t;
@@ -810,10 +857,11 @@ void simt_gemm_plan(bool f64, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile
     *wide = plan.wide ? 1 : 0;
 }
 
-static uint64_t large_tiles(int dtype, uint32_t m, uint32_t n)
+// tiles of sgemm_kernel or dgemm_kernel
+static uint64_t whole_tiles(int dtype, uint32_t m, uint32_t n)
 {
-    const uint32_t tile_n = dtype == CLPK_DT_F32 ? kSimtTile : 64;
-    return (uint64_t)((m + kSimtTile - 1) / kSimtTile) * ((n + tile_n - 1) / tile_n);
+    const uint32_t tile = dtype == CLPK_DT_F32 ? kSimtTile : kDgemmTile;
+    return (uint64_t)((m - 1) / tile + 1) * ((n - 1) / tile + 1);
 }
 
 int check_simt_gemm(int dtype, const void *a, const void *b, const void *c, uint32_t m, uint32_t n, uint32_t k)
@@ -822,17 +870,17 @@ int check_simt_gemm(int dtype, const void *a, const void *b, const void *c, uint
     const uint32_t k_unit = dtype == CLPK_DT_F32 ? 4 : 2;            // elements per 16 bytes: operand rows stay aligned
     CLPK_REQUIRE(k % k_unit == 0, "K = %u: a row of A and B must be a multiple of 16 bytes", k);
     CLPK_REQUIRE(((uintptr_t)a % 16) == 0 && ((uintptr_t)b % 16) == 0 && ((uintptr_t)c % 16) == 0, "operands must be 16-byte aligned");
-    CLPK_REQUIRE(large_tiles(dtype, m, n) <= 0x3FFFFFFFull, "too many tiles");
+    CLPK_REQUIRE((uint64_t)((m - 1) / 128 + 1) * ((n - 1) / (dtype == CLPK_DT_F32 ? 128 : 64) + 1) <= 0x3FFFFFFFull, "too many tiles");
     return CLPK_OK;
 }
 
 int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t m, uint32_t n, uint32_t k, float alpha,
                      uint32_t *status, cudaStream_t s)
 {
-    const uint32_t tile_n = dtype == CLPK_DT_F32 ? kSimtTile : 64;
-    const uint64_t tiles = large_tiles(dtype, m, n);
+    const uint32_t tile = dtype == CLPK_DT_F32 ? kSimtTile : kDgemmTile;
+    const uint64_t tiles = whole_tiles(dtype, m, n);
     // whole tiles and whole k blocks take the kernel without the bounds checks
-    const bool ragged = m % kSimtTile != 0 || n % tile_n != 0 || k % kSimtBK != 0;
+    const bool ragged = m % tile != 0 || n % tile != 0 || k % kSimtBK != 0;
     const SimtPlan plan = plan_simt(dtype == CLPK_DT_F64, m, n, k);
     const uint64_t ctas = (uint64_t)((m - 1) / plan.tile + 1) * ((n - 1) / plan.tile + 1) * plan.splits;
     if (dtype == CLPK_DT_F32) {
@@ -848,18 +896,19 @@ int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t 
     }
     const double *da = static_cast<const double *>(a), *db = static_cast<const double *>(b);
     double *dc = static_cast<double *>(c);
+    if (plan.whole) {
+        const bool odd = n % 2 != 0;
+        return launch_simt(odd ? dgemm_kernel<true, true> : ragged ? dgemm_kernel<true, false> : dgemm_kernel<false, false>, "launch dgemm", tiles, kDgemmThreads,
+                           kDgemmSmemBytes, 1, true, s, da, db, dc, m, n, k, alpha, status);
+    }
     if (plan.tile == 64)
         return launch_simt(dgemm_split_kernel<2, 2, 1>, "launch dgemm 64", ctas, DgemmSplit<2, 2, 1>::threads, DgemmSplit<2, 2, 1>::smem_bytes, plan.splits,
                            true, s, da, db, dc, m, n, k, alpha, plan.splits, status);
     if (plan.tile == 32 && plan.wide)
         return launch_simt(dgemm_split_kernel<1, 1, 8>, "launch dgemm 32", ctas, DgemmSplit<1, 1, 8>::threads, DgemmSplit<1, 1, 8>::smem_bytes, plan.splits,
                            false, s, da, db, dc, m, n, k, alpha, plan.splits, status);
-    if (plan.tile == 32)
-        return launch_simt(dgemm_split_kernel<1, 1, 4>, "launch dgemm 32", ctas, DgemmSplit<1, 1, 4>::threads, DgemmSplit<1, 1, 4>::smem_bytes, plan.splits,
-                           true, s, da, db, dc, m, n, k, alpha, plan.splits, status);
-    // 128 x 64 CTA tiles: 34.2-34.5 TFLOPS at 4096^3 / 8192^3 against 31.9-32.1 with 128 x 128 tiles of 8 warps
-    return launch_simt(ragged ? dgemm_kernel<64, true> : dgemm_kernel<64, false>, "launch dgemm", tiles, Dgemm<64>::threads, Dgemm<64>::smem_bytes, 1, false,
-                       s, da, db, dc, m, n, k, alpha, status);
+    return launch_simt(dgemm_split_kernel<1, 1, 4>, "launch dgemm 32", ctas, DgemmSplit<1, 1, 4>::threads, DgemmSplit<1, 1, 4>::smem_bytes, plan.splits, true, s,
+                       da, db, dc, m, n, k, alpha, plan.splits, status);
 }
 
 } // namespace clpk

@@ -57,6 +57,16 @@ def test_short_fp64_sums(K, cuda, tile, shape):
     check_every_element(K, cuda, N.DT_F64, *shape)
 
 
+# fp64 with K whole in 64 x 64 tiles: whole tiles, ragged ones with an even N and with an odd one (whose C goes through shared memory,
+# and whose plan says so), sums of one block to more than the ring holds and with every remainder of a block's pieces
+@pytest.mark.parametrize("tile,m,n", [(0, 640, 704), (0, 641, 702), (64, 639, 705), (0, 7000, 2), (64, 6401, 1), (0, 63, 6402), (64, 65, 6465)])
+@pytest.mark.parametrize("k", [2, 16, 18, 32, 46, 48, 50, 64, 464])
+def test_whole_fp64_tiles(K, cuda, tile, m, n, k):
+    if k < 384 and gemm_plan(K, N.DT_F64, m, n, k)[0] != 32:
+        assert gemm_plan(K, N.DT_F64, m, n, k) == (tile, 1, 0)
+    check_every_element(K, cuda, N.DT_F64, m, n, k)
+
+
 def check_every_element(K, cuda, dtype, m, n, k):
     a, b = operand(K, cuda, dtype, m, k, 40), operand(K, cuda, dtype, n, k, 41)
     alpha, results = 0.75, []
