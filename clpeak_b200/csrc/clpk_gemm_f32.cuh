@@ -8,13 +8,15 @@
 // the fp32 pipe does.
 //
 // bf16 ends where fp32 does, so the pieces of a small x would not exist.  The elements are multiplied by 2^16 on the way, after
-// which none has bits below bf16's last one, 2^-133, and 2^8 m and 2^16 l are kept instead of m and l: every finite number up to
-// 2^111, subnormal ones too, is then three bf16 numbers with m and l as far below h as said above.  (Subnormal bf16 operands and
-// sums are not flushed.)  An instruction that takes up products of the next size divides the accumulator by 2^8, and the sums
-// are multiplied by 2^-32 when they leave the registers: results keep their bits down to the end of the fp32 range, with fewer errors
-// there than fused multiply-adds, which round each step to 2^-149 (K = 2044, results near 2^-135: at most 2 units of 2^-149 against 56).
-// With pieces at their own size, tiles with an element or a sum below 2^-100 had to be multiplied again: 40.5 ms for a 4096^3
-// product of that kind against 0.62, and 1.05 for one with zeros, for which the same alarm went off.
+// which none has bits below bf16's last one, 2^-133: every finite number up to 2^111, subnormal ones too, is then three bf16
+// numbers with m and l as far below h as said above.  (Subnormal bf16 operands and sums are not flushed.)  The sums are multiplied
+// by 2^-32 when they leave the registers.  A product that a result of 2^-149 could feel is 2^-117 and more in the accumulator, and
+// its last bit 2^-149: results keep their bits down to the end of the fp32 range, with fewer errors there than fused
+// multiply-adds, which round each step to 2^-149 (K = 2044, results near 2^-135: at most 2 units of 2^-149 against 56).
+// With elements at their own size, tiles with an element or a sum below 2^-100 had to be multiplied again: 40.5 ms for a 4096^3
+// product of that kind against 0.62, and 1.05 for one with zeros, for which the same alarm went off.  (m and l at 2^8 and 2^16
+// times their size besides, with the accumulator divided between products of different sizes, took two more multiplications of a
+// pair and gained nothing.)
 //
 // The tensor cores cut, not round, what they align to the accumulator, so sums are kept short there: a turn of two chunks of 32
 // floats starts from zero, adds the small products first and the h h ones last -- four instructions in which the cut is of
@@ -34,12 +36,14 @@
 //  * K over 1, 2 or 4 pairs of a cluster as in gemm_tiles_kernel: partial sums meet in the raw tiles' shared memory and
 //    are added in pair order.
 //
-// What bounds it: a chunk's 12 instructions take 430 cycles at TN = 32 and 890 at 128; converting a pair of floats 14 of an SM
-// quarter's cycles (sub.f32.bf16 takes its bf16 operand as it is; each of the three conversions blocks the ALU for two), 250
-// to 400 a chunk; the hand-over of an accumulator 1400, which two turns in flight hide at TN = 128 only just.  The tensor pipe is
-// busy for 72 % of the cycles of a 4096 x 2304 x 4096 product, issue slots 58 %.  Device time against the CUDA-core kernels: 4096^3
-// 2251 -> 620 us back to back (222 TFLOPS), 710 between inputs that change (194); 2317 x 6252 x 516 338 -> 95,
-// 1636 x 116 x 4084 62 -> 24, 459 x 349 x 4636 70 -> 25; 9019 random shapes that take this kernel 0.40 in the geometric mean.
+// What bounds it: the turns of converters, instructions and sums rather than any one of them.  A chunk's 12 instructions take 430
+// cycles at TN = 32 and 890 at 128, a whole turn of one chunk 1060: without the arithmetic of the conversion (12 issue slots of an
+// SM quarter for a pair of floats) 880, without the additions 1000, with two of the 12 instructions 1000.  The tensor pipe is busy
+// for 71 % of the cycles of a 2304 x 4096 x 2048 product, issue slots 53 %; from about 300 us on the power cap takes the clock down to
+// 1.4 GHz and with it what is left to gain.  Device time against the CUDA-core kernels: 4096^3 2251 -> 599 us back to back (229 TFLOPS),
+// 688 between inputs that change (200); 2317 x 6252 x 516 338 -> 92, 1636 x 116 x 4084 62 -> 23, 459 x 349 x 4636 70 -> 24; 9019
+// random shapes that take this kernel 0.40 in the geometric mean.  Pieces with scales of their own and four conversion stages
+// (14 or more slots a pair): 3 % longer at 128 columns, 4 at 96, 7 at 32.
 // Earlier forms at 4096^3, TN = 128, with pieces at their own size (658 in the end): hand-overs by .release.cluster arrives and a
 // cluster fence 1279; one issuing warp 707; three groups of converters (whose registers the sums then lack) 691; all warps polling for
 // themselves 680; turns of one chunk the same, but 953 at TN = 64 against 833.
@@ -58,7 +62,6 @@ constexpr int kF32FirstSum = 4 + 4 * kF32Groups;
 constexpr int kF32SumWarps = 8;
 constexpr uint32_t kF32LaunchRegs = 96;                  // a thread of the block is launched with
 constexpr uint32_t kF32BoxLd = 20;                       // floats per row of a warp's 32 x 16 staging box
-constexpr uint32_t kF32PieceShift = 8;                   // bits between the scales of an element's pieces
 constexpr float kF32Scale = 0x1p16f;                     // of the elements of A and of B
 constexpr float kF32Unscale = 0x1p-32f;                  // of the sums, when they leave the registers
 
@@ -68,15 +71,14 @@ template <uint32_t TN> struct F32Tile {
     static constexpr uint32_t raw_bytes = a_bytes + half_n * 128;
     static constexpr uint32_t plane_bytes = half_n * 64;
     static constexpr uint32_t a_cols = 48;                               // h, m, l of 32 floats: 16 columns each
-    static constexpr uint32_t conv_stages = 4;
+    static constexpr uint32_t conv_stages = TN == 96 ? 4 : 5;             // what tensor memory has room for
     static constexpr uint32_t accs = TN <= 64 ? 4 : TN == 96 ? 3 : 2;
-    static constexpr uint32_t raw_stages = TN <= 64 ? 8 : TN == 96 ? 7 : 6;
+    static constexpr uint32_t raw_stages = TN <= 64 ? 8 : TN == 96 ? 7 : 5;
     static constexpr uint32_t tmem_cols = accs * TN + conv_stages * a_cols > 256 ? 512 : 256;
     static_assert(accs * TN + conv_stages * a_cols <= 512, "tensor memory");
     static constexpr uint32_t box_bytes = 32 * kF32BoxLd * 4;
-    // registers a thread of the issuing, the converting and the adding warps.  With 72 and 152 at every width the converters spill
-    // at 32, 96 and 128 (2 to 7 % longer), with 80 and 144 at 64 (2 %).
-    static constexpr uint32_t issue_regs = 32, converter_regs = TN == 64 ? 72 : 80, sum_regs = TN == 64 ? 152 : 144;
+    // registers a thread of the issuing, the converting and the adding warps; at 64 columns 72 and 152 take 7 % longer
+    static constexpr uint32_t issue_regs = 32, converter_regs = 80, sum_regs = 144;
     static_assert(128 * issue_regs + 128 * kF32Groups * converter_regs + 32 * kF32SumWarps * sum_regs <= kF32Threads * kF32LaunchRegs,
                   "no share may wait for registers that nobody gives back");
     static constexpr size_t smem_bytes = (size_t)raw_stages * raw_bytes + conv_stages * 3 * plane_bytes + kF32SumWarps * box_bytes + 512 + 1024;
@@ -84,7 +86,7 @@ template <uint32_t TN> struct F32Tile {
 
 struct F32Smem {
     uint64_t raw_full[8], raw_empty[8];
-    uint64_t conv_full[4], conv_empty[4];
+    uint64_t conv_full[5], conv_empty[5];
     uint64_t d_full[4], d_empty[4];
     uint32_t tmem_base;
 };
@@ -134,43 +136,29 @@ __device__ __forceinline__ void scale_pair(float &x0, float &x1, float by)
         : "f"(by));
 }
 
-// Two floats -> the three bf16 pairs h, 2^8 m and 2^16 l of their products with kF32Scale.
-__device__ __forceinline__ void split_bf16x3(float x0, float x1, uint32_t &h, uint32_t &m, uint32_t &l)
+// Two floats -> the three bf16 pairs h, -m and l of their products with kF32Scale (bf16x2_minus leaves the other sign).
+__device__ __forceinline__ void split_bf16x3(float x0, float x1, uint32_t &h, uint32_t &minus_m, uint32_t &l)
 {
-    constexpr float kBy = -(float)(1u << kF32PieceShift);                // what bf16x2_minus leaves has the other sign
     float r0, r1, s0, s1;
     scale_pair(x0, x1, kF32Scale);
     h = pack_bf16x2(x0, x1);
     bf16x2_minus(h, x0, x1, r0, r1);
-    scale_pair(r0, r1, kBy);
-    m = pack_bf16x2(r0, r1);
-    bf16x2_minus(m, r0, r1, s0, s1);
-    scale_pair(s0, s1, kBy);
+    minus_m = pack_bf16x2(r0, r1);
+    bf16x2_minus(minus_m, r0, r1, s0, s1);
     l = pack_bf16x2(s0, s1);
 }
 
-// D = A B, D + A B, or 2^-kF32PieceShift D + A B
-enum class Into { fresh, sum, shifted };
-__device__ __forceinline__ void mma2_bf16_ts(uint32_t d, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, Into into)
+// D = A B or D + A B
+__device__ __forceinline__ void mma2_bf16_ts(uint32_t d, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate)
 {
-    if (into == Into::shifted)
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p;\n\t"
-            "setp.eq.u32 p, 0, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t"
-            "}\n" ::"r"(d),
-            "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(kF32PieceShift)
-            : "memory");
-    else
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p;\n\t"
-            "setp.ne.u32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-            "}\n" ::"r"(d),
-            "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(into == Into::sum ? 1 : 0)
-            : "memory");
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.u32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "}\n" ::"r"(d),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate ? 1 : 0)
+        : "memory");
 }
 
 template <bool INC, uint32_t N>
@@ -444,7 +432,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
     } else if (warp < 3) {
         // ---------------- MMA issuers (the pair's leader), every other turn each ----------------
         if (r == 0) {
-            const uint32_t idesc = make_idesc(256, TN, kFmtBF16, kFmtBF16, kAccF32);
+            const uint32_t idesc = make_idesc(256, TN, kFmtBF16, kFmtBF16, kAccF32), idesc_minus = idesc | kNegateA;
             const uint16_t pair_mask = (uint16_t)(3u << leader);
             uint32_t turn = 0, chunk = 0;
             bool ok = true;
@@ -464,32 +452,33 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                         if (elect_one()) {
                             const uint32_t acc = tmem + d * TN;
                             // plane pa of A times plane pb of B of the chunk in stage s
-                            auto multiply = [&](uint32_t s, uint32_t pa, uint32_t pb, Into into) {
+                            auto multiply = [&](uint32_t s, uint32_t pa, uint32_t pb, bool accumulate = true) {
                                 const uint32_t a = tmem + T::accs * TN + s * T::a_cols + 16 * pa;
                                 const uint64_t b = make_smem_desc(smem_u32(planes + (size_t)s * 3 * T::plane_bytes), 16, 512, kSwizzle64B) +
                                                    pb * T::plane_bytes / 16;
-                                mma2_bf16_ts(acc, a, b, idesc, into);
-                                mma2_bf16_ts(acc, a + 8, b + 2, idesc, Into::sum);
+                                const uint32_t desc = (pa == 1) != (pb == 1) ? idesc_minus : idesc;        // one factor is -m
+                                mma2_bf16_ts(acc, a, b, desc, accumulate);
+                                mma2_bf16_ts(acc, a + 8, b + 2, desc, true);
                             };
-                            // the smallest products first, at 2^16 times their size, those of full size last
-                            multiply(s0, 2, 0, Into::fresh);
-                            multiply(s0, 0, 2, Into::sum);
-                            multiply(s0, 1, 1, Into::sum);
+                            // the smallest products first, those of full size last
+                            multiply(s0, 2, 0, false);
+                            multiply(s0, 0, 2);
+                            multiply(s0, 1, 1);
                             if (two) {
-                                multiply(s1, 2, 0, Into::sum);
-                                multiply(s1, 0, 2, Into::sum);
-                                multiply(s1, 1, 1, Into::sum);
+                                multiply(s1, 2, 0);
+                                multiply(s1, 0, 2);
+                                multiply(s1, 1, 1);
                             }
-                            multiply(s0, 1, 0, Into::shifted);
-                            multiply(s0, 0, 1, Into::sum);
+                            multiply(s0, 1, 0);
+                            multiply(s0, 0, 1);
                             if (two) {
-                                multiply(s1, 1, 0, Into::sum);
-                                multiply(s1, 0, 1, Into::sum);
+                                multiply(s1, 1, 0);
+                                multiply(s1, 0, 1);
                             }
-                            multiply(s0, 0, 0, Into::shifted);
+                            multiply(s0, 0, 0);
                             tc_commit_pair(&sh->conv_empty[s0], pair_mask);
                             if (two) {
-                                multiply(s1, 0, 0, Into::sum);
+                                multiply(s1, 0, 0);
                                 tc_commit_pair(&sh->conv_empty[s1], pair_mask);
                             }
                             tc_commit_pair(&sh->d_full[d], pair_mask);

@@ -403,6 +403,8 @@ __host__ __device__ __forceinline__ uint32_t make_idesc(uint32_t m, uint32_t n, 
     return d;
 }
 
+constexpr uint32_t kNegateA = 1u << 13;         // floating kinds: A's elements with the other sign
+
 // Block-scaled kinds (mxf8f6f4 / mxf4 / mxf4nvf4): same operand fields, plus
 //   [4,6) B scale-factor id   [23] scale format (0 ue4m3, 1 ue8m0)
 //   [29,31) A scale-factor id [31] K size selector (0 = the dense K64 / sparse K128 shape)
