@@ -54,11 +54,22 @@ struct __align__(32) Float8 {
     float v[8];
 };
 
-// 32 bytes, 32-byte aligned: one 256-bit access
-__device__ __forceinline__ Float8 ld_float8(const float *p)
+// 32 bytes, 32-byte aligned: one 256-bit access.  absmax and the quantiser ask for the lines of arrays beyond the cache
+// as the first to leave it (FIRST), so that those which come from DRAM do not push out, before they are read, those that the
+// kernel in front has left: 8192 x 8192 (268 MB) normal fill with NVFP4 229 -> 220 us, with MXFP4 185 -> 180, 4096 x 8192
+// 116 -> 111 and 93 -> 90.  (Conversions gain 1 %, and only through this access.  Letting the fill's first stores go first as well:
+// 223; keeping what absmax reads last for the quantiser: 219 to 222.)
+template <bool FIRST>
+__device__ __forceinline__ Float8 ld_float8x32(const float *p)
 {
     unsigned long long w[4];
-    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]) : "l"(p) : "memory");
+    if constexpr (FIRST)
+        asm volatile("ld.global.L1::no_allocate.L2::evict_first.v4.b64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
+                     : "l"(p)
+                     : "memory");
+    else
+        asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]) : "l"(p) : "memory");
     Float8 r;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -69,11 +80,11 @@ __device__ __forceinline__ Float8 ld_float8(const float *p)
 }
 
 // eight floats from an address that is a multiple of ALIGN bytes
-template <int ALIGN>
+template <int ALIGN, bool FIRST = false>
 __device__ __forceinline__ Float8 ld_float8(const float *p)
 {
     if constexpr (ALIGN == 32) {
-        return ld_float8(p);
+        return ld_float8x32<FIRST>(p);
     } else {
         Float8 r;
         if constexpr (ALIGN == 16) {
@@ -303,17 +314,17 @@ __global__ void __launch_bounds__(kFillThreads) convert_kernel(void *dst, const 
 // writes the result itself; otherwise the CTAs meet in an atomicMax on a word that has been cleared.
 constexpr int kAbsmaxLoads = 4;
 
-template <bool SINGLE>
-__global__ void __launch_bounds__(kFillThreads) absmax_kernel(float *out, const float *src, Split part, bool falling)
+template <bool SINGLE, bool FALLING>
+__global__ void __launch_bounds__(kFillThreads) absmax_kernel(float *out, const float *src, Split part)
 {
     join_stream();
     float m = 0.0f;
     const uint64_t step = (uint64_t)gridDim.x * kFillThreads * kAbsmaxLoads;
-    for (uint64_t g = ordered_cta(falling) * kFillThreads * kAbsmaxLoads + threadIdx.x; g < part.whole; g += step) {
+    for (uint64_t g = ordered_cta(FALLING) * kFillThreads * kAbsmaxLoads + threadIdx.x; g < part.whole; g += step) {
         Float8 x[kAbsmaxLoads];
 #pragma unroll
         for (int u = 0; u < kAbsmaxLoads; u++)
-            x[u] = g + u * kFillThreads < part.whole ? ld_float8(src + 8 * (g + u * kFillThreads)) : Float8{};
+            x[u] = g + u * kFillThreads < part.whole ? ld_float8x32<FALLING>(src + 8 * (g + u * kFillThreads)) : Float8{};
 #pragma unroll
         for (int u = 0; u < kAbsmaxLoads; u++)
 #pragma unroll
@@ -409,7 +420,7 @@ __device__ __forceinline__ void st_codes(uint8_t *p, uint64_t codes)
 // ALIGN: 32 when the source is aligned to that and the codes to 8 bytes, else what the source is aligned to, 16 or 4.  The
 // blocks lie where they lie, so there is no head to cut off: 8192 x 8192 from a source 16 bytes off 45 to 49 us, 4 bytes
 // off 122 (each of 16 loads touches 32 sectors) against 168 to 349 with one thread per block.
-template <int BLOCK, bool UE8M0, int ALIGN>
+template <int BLOCK, bool UE8M0, int ALIGN, bool FIRST>
 __global__ void __launch_bounds__(kFillThreads) quantize_fp4_kernel(uint8_t *packed, uint8_t *scales, const float *src, uint64_t n16, TensorScale ts, bool falling)
 {
     join_stream();
@@ -422,7 +433,7 @@ __global__ void __launch_bounds__(kFillThreads) quantize_fp4_kernel(uint8_t *pac
         const bool inside = g < n16;
         float x[kQuantPerLane] = {};
         if (inside) {
-            const Float8 a = ld_float8<ALIGN>(src + 16 * g), b = ld_float8<ALIGN>(src + 16 * g + 8);
+            const Float8 a = ld_float8<ALIGN, FIRST>(src + 16 * g), b = ld_float8<ALIGN, FIRST>(src + 16 * g + 8);
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 x[i] = a.v[i];
@@ -557,11 +568,14 @@ static int launch_quantize(uint8_t *d_packed, uint8_t *d_scales, const float *d_
     const unsigned grid = fill_grid(n16);
     // an NVFP4 tensor's maximum has been taken in front, in falling order: its beginning was read last
     const bool falling = UE8M0 && falling_order(4 * n);
-    if (aligned(d_src, 32) && aligned(d_packed, 8))
-        return launch_behind(quantize_fp4_kernel<BLOCK, UE8M0, 32>, "launch quantize_fp4", grid, kFillThreads, 0, s, d_packed, d_scales, d_src, n16, ts, falling);
+    if (aligned(d_src, 32) && aligned(d_packed, 8)) {
+        if (falling_order(4 * n))
+            return launch_behind(quantize_fp4_kernel<BLOCK, UE8M0, 32, true>, "launch quantize_fp4", grid, kFillThreads, 0, s, d_packed, d_scales, d_src, n16, ts, falling);
+        return launch_behind(quantize_fp4_kernel<BLOCK, UE8M0, 32, false>, "launch quantize_fp4", grid, kFillThreads, 0, s, d_packed, d_scales, d_src, n16, ts, falling);
+    }
     if (aligned(d_src, 16))
-        return launch_behind(quantize_fp4_kernel<BLOCK, UE8M0, 16>, "launch quantize_fp4", grid, kFillThreads, 0, s, d_packed, d_scales, d_src, n16, ts, falling);
-    return launch_behind(quantize_fp4_kernel<BLOCK, UE8M0, 4>, "launch quantize_fp4", grid, kFillThreads, 0, s, d_packed, d_scales, d_src, n16, ts, falling);
+        return launch_behind(quantize_fp4_kernel<BLOCK, UE8M0, 16, false>, "launch quantize_fp4", grid, kFillThreads, 0, s, d_packed, d_scales, d_src, n16, ts, falling);
+    return launch_behind(quantize_fp4_kernel<BLOCK, UE8M0, 4, false>, "launch quantize_fp4", grid, kFillThreads, 0, s, d_packed, d_scales, d_src, n16, ts, falling);
 }
 
 } // namespace clpk
@@ -630,14 +644,15 @@ int clpk_absmax_f32(float *d_absmax, const float *d_src, uint64_t n, void *strea
     const Split part = split_at(d_src, 32, 32, 8, n);
     // up to 32 Ki floats one CTA reads in the time that clearing the word would take
     if (n > 0 && n <= 32768 && d_src)
-        return launch_behind(absmax_kernel<true>, "launch absmax", 1, kFillThreads, 0, s, d_absmax, d_src + part.head,
-                             part, false);
+        return launch_behind(absmax_kernel<true, false>, "launch absmax", 1, kFillThreads, 0, s, d_absmax, d_src + part.head, part);
     CLPK_CUDA(cudaMemsetAsync(d_absmax, 0, sizeof(float), s));
     if (n == 0)
         return CLPK_OK;
     CLPK_REQUIRE(d_src, "d_src is NULL");
-    return launch_behind(absmax_kernel<false>, "launch absmax", fill_grid(part.whole / kAbsmaxLoads + 1), kFillThreads, 0, s, d_absmax,
-                         d_src + part.head, part, falling_order(4 * n));
+    const unsigned grid = fill_grid(part.whole / kAbsmaxLoads + 1);
+    if (falling_order(4 * n))
+        return launch_behind(absmax_kernel<false, true>, "launch absmax", grid, kFillThreads, 0, s, d_absmax, d_src + part.head, part);
+    return launch_behind(absmax_kernel<false, false>, "launch absmax", grid, kFillThreads, 0, s, d_absmax, d_src + part.head, part);
 }
 
 int clpk_quantize_fp4(uint8_t *d_packed, uint8_t *d_scales, const float *d_src, uint64_t rows,
