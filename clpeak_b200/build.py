@@ -7,6 +7,8 @@ Outputs (all under clpeak_b200/_lib/, which is not tracked):
                              B200 backend) behind the clpeak_ffi C ABI of
                              include/clpeak_ffi.h
   clpeak                     the command-line front end
+  _clpk_calls.so             calls into the kernels from Python without ctypes between
+                             (only where the interpreter's headers are installed)
 
 Only sm_100a code is generated.  Run as `python -m clpeak_b200.build`.
 """
@@ -16,6 +18,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -116,9 +119,22 @@ def build_host(force: bool = False) -> list[Path]:
     return outs
 
 
+def build_calls(force: bool = False) -> Path | None:
+    inc = Path(sysconfig.get_paths()["include"])
+    if not (inc / "Python.h").exists():
+        return None
+    src, header, out = CSRC / "python" / "calls.cpp", ROOT / "include" / "clpeak_b200_kernels.h", LIB / "_clpk_calls.so"
+    LIB.mkdir(parents=True, exist_ok=True)
+    if force or _stale(out, [src, header]):
+        cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
+        _run([cxx, *CXX_FLAGS, "-shared", "-I", str(inc), "-I", str(ROOT / "include"), str(src), "-o", str(out)])
+    return out
+
+
 def build_all(force: bool = False) -> None:
     build_kernels(force)
     build_host(force)
+    build_calls(force)
 
 
 if __name__ == "__main__":

@@ -1,4 +1,4 @@
-"""ctypes bindings for the two native libraries.
+"""Bindings for the two native libraries: ctypes, and an extension for the calls that are made once per launch.
 
 ``kernels()`` loads ``libclpeak_b200_kernels.so`` and declares every symbol of
 ``include/clpeak_b200_kernels.h``; ``ffi()`` loads ``libclpeak_ffi.so``
@@ -8,6 +8,8 @@ built -- nothing here substitutes for it.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 from functools import lru_cache
 from pathlib import Path
 
@@ -163,6 +165,18 @@ FFI_API = {
 EVENT_CALLBACK = C.CFUNCTYPE(None, C.c_void_p, C.c_void_p)
 
 
+@lru_cache(maxsize=None)
+def _calls():
+    """The extension with the calls that are made once per launch (csrc/python/calls.cpp), None where it has not been built."""
+    path = LIB_DIR / "_clpk_calls.so"
+    if not path.exists():
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("_clpk_calls", str(path))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_clpk_calls", loader))
+    loader.exec_module(module)
+    return module
+
+
 class Kernels:
     """Checked calls into libclpeak_b200_kernels.so."""
 
@@ -180,13 +194,18 @@ class Kernels:
             setattr(self, name, self._checked(name, fn))
 
     def _checked(self, name: str, fn):
-        """The call a user makes: the function is looked up once and not with every call (a wrapped call of five arguments
-        4.0 -> 2.6 us, of which 2.6 are ctypes' own)."""
+        """The call a user makes: bound once, and past ctypes where the extension has the function and the arguments are
+        plain."""
+        def failed(rc):
+            raise ClpkError(rc, self.last_error(), name)
+
         def call(*args):
             rc = fn(*args)
             if rc != OK:
-                raise ClpkError(rc, self.last_error(), name)
-        return call
+                failed(rc)
+        if _calls() is None:
+            return call
+        return _calls().bind(name, C.cast(fn, C.c_void_p).value, call, failed, type(C.byref(C.c_int())), GemmArgs) or call
 
     def last_error(self) -> str:
         return (self.lib.clpk_last_error() or b"").decode()

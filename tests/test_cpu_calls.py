@@ -1,0 +1,61 @@
+"""Calls past ctypes answer as the ctypes wrapper does: plain arguments, arguments that only ctypes converts, and those it refuses.
+Nothing is launched: no element, a NULL buffer, or no such type."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+from clpeak_b200 import native as N
+
+FAST = N._calls()
+pytestmark = pytest.mark.skipif(FAST is None, reason="built without the interpreter's headers")
+
+ARRAY = (N.GemmArgs * 2)()
+FILL = "clpk_fill_f32"
+CALLS = [(FILL, (0, 0, 1, 2, 0.0, 1.0, None)), (FILL, (None, 5, 1, 2, 0.0, 1.0, 0)), (FILL, (None, 5, 1, 7, 0.0, 1.0, 0)),
+         (FILL, (0, 0, 2 ** 64 - 1, 2, 0.0, 1.0, 0)), (FILL, (2 ** 64 - 1, 0, 2 ** 63, 2, 0.0, 1.0, 0)), (FILL, (0, 0, 2 ** 70, 2, 0.0, 1.0, 0)),
+         (FILL, (0, 0, -1, 2, 0.0, 1.0, 0)), (FILL, (-1, 0, 1, 2, 0.0, 1.0, 0)), (FILL, (0, 0, 1, 2 ** 31, 0.0, 1.0, 0)),
+         (FILL, (0, 0, 1, -1, 0.0, 1.0, 0)), (FILL, (0, 0, 1, 2 ** 32 + 2, 0.0, 1.0, 0)), (FILL, (0, 0, 1, True, 0.0, 1.0, 0)),
+         (FILL, (0, 0, 1, 2, 0, 1, 0)), (FILL, (0, 0, 1, 2, 1e300, float("nan"), 0)), (FILL, (0, 0, 1, 2.0, 0.0, 1.0, 0)),
+         (FILL, (0, 0.0, 1, 2, 0.0, 1.0, 0)), (FILL, (0, 0, 1, 2, "0", 1.0, 0)), (FILL, (0, np.int64(0), 1, 2, 0.0, 1.0, 0)),
+         (FILL, (0, 0, 1, 2, np.float32(0), 1.0, 0)), (FILL, (C.c_void_p(0), C.c_uint64(0), 1, C.c_int(2), C.c_float(0), 1.0, C.c_void_p(0))),
+         (FILL, (0, 0, 1)), (FILL, ()), (FILL, (b"", 0, 1, 2, 0.0, 1.0, 0)), (FILL, ([], 0, 1, 2, 0.0, 1.0, 0)),
+         ("clpk_fill_i8", (0, 0, 1, 0)), ("clpk_fill_i8", (0, 5, 1, 0)), ("clpk_convert_f32", (0, 0, 0, N.DT_BF16, 0)),
+         ("clpk_convert_f32", (0, 0, 0, 99, 0)), ("clpk_quantize_fp4", (0, 0, 0, 4, 64, N.DT_NVF4, 1.0, 0)),
+         ("clpk_quantize_fp4", (0, 0, 0, 4, 64, N.DT_NVF4, 1, 0)), ("clpk_absmax_f32", (None, None, 0, None)),
+         ("clpk_stream_read", (99, 0, 0, 0, 0)), ("clpk_stream_copy", (99, 0, 0, 0, 0)), ("clpk_stream_triad", (99, 0, 0, 0, 1.5, 0, 0)),
+         ("clpk_gemm", (C.byref(N.GemmArgs()), 0)), ("clpk_gemm", (N.GemmArgs(), 0)), ("clpk_gemm", (None, 0)), ("clpk_gemm", (C.byref(ARRAY), 0)),
+         ("clpk_gemm", (C.byref(ARRAY[1]), None)), ("clpk_gemm", (C.pointer(ARRAY[0]), 0)), ("clpk_gemm", (C.byref(C.c_int()), 0)),
+         ("clpk_gemm", (0, 0)), ("clpk_gemm_pack_scales", (C.byref(N.GemmArgs(dtype=N.DT_BF16)), 0)),
+         ("clpk_gemm_pack_scales", (C.byref(N.GemmArgs(dtype=N.DT_NVF4, m=1, n=1, k=100)), 0))]
+
+
+def outcome(f, args):
+    try:
+        return f(*args)
+    except Exception as e:                                          # noqa: BLE001: whatever either raises
+        return type(e), str(e)
+
+
+@pytest.mark.parametrize("name,args", CALLS)
+def test_the_same_answer_as_through_ctypes(K, name, args):
+    assert type(getattr(K, name)) is not type(outcome)              # not the Python wrapper
+    assert outcome(getattr(K, name), args) == outcome(lambda *a: K.call(name, *a), args)
+
+
+def test_errors_of_several_threads_at_once(K):
+    wrong = []
+
+    def work(what, text):
+        for _ in range(300):
+            got = outcome(getattr(K, what[0]), what[1])
+            if got[0] is not N.ClpkError or text not in got[1]:
+                wrong.append(got)
+    threads = [threading.Thread(target=work, args=a) for a in (((FILL, (None, 5, 1, 2, 0.0, 1.0, 0)), "d_dst is NULL"),
+                                                               ((FILL, (1, 5, 1, 9, 0.0, 1.0, 0)), "unknown distribution 9"))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
