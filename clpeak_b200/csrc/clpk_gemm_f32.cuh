@@ -39,7 +39,7 @@
 // What bounds it: the turns of converters, instructions and sums rather than any one of them.  A chunk's 12 instructions take 430
 // cycles at TN = 32 and 890 at 128, a whole turn of one chunk 1060: without the arithmetic of the conversion (12 issue slots of an
 // SM quarter for a pair of floats) 880, without the additions 1000, with two of the 12 instructions 1000.  The tensor pipe is busy
-// for 71 % of the cycles of a 2304 x 4096 x 2048 product, issue slots 53 %; from about 300 us on the power cap takes the clock down to
+// for 73 % of the cycles of a 2304 x 4096 x 2048 product, issue slots 54 %; from about 300 us on the power cap takes the clock down to
 // 1.4 GHz and with it what is left to gain.  Device time against the CUDA-core kernels: 4096^3 2251 -> 599 us back to back (229 TFLOPS),
 // 688 between inputs that change (200); 2317 x 6252 x 516 338 -> 92, 1636 x 116 x 4084 62 -> 23, 459 x 349 x 4636 70 -> 24; 9019
 // random shapes that take this kernel 0.40 in the geometric mean.  Pieces with scales of their own and four conversion stages
@@ -49,7 +49,7 @@
 // themselves 680; turns of one chunk the same, but 953 at TN = 64 against 833.
 //
 // Numbers that the split cannot serve are multiplied as they are, with fused multiply-adds in K order: a warp whose sums
-// are not all finite (an infinity, a NaN, or an overflow on the way, which the scales bring to about 2^89;
+// are not all finite (an infinity, a NaN, or an overflow on the way, which the scale brings to about 2^96;
 // x - h of an infinity is a NaN, so none goes unseen) does its 32 x TN / 2 outputs again, see f32_tile_as_defined.  Whoever
 // waits for such a tile waits 0.15 us per element of K at most, under 2.5 s where the operands of more tiles than pairs fill 180 GB.
 #pragma once
