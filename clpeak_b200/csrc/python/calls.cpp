@@ -24,7 +24,40 @@ struct Call {
     PyObject *slow;              // the ctypes wrapper
     PyObject *failed;            // raises for a status
     PyTypeObject *byref_type, *gemm_args_type;
+    Py_ssize_t address_at;       // see where_the_address_lies
 };
+
+const void *address_in(PyObject *byref, Py_ssize_t at)
+{
+    const void *p;
+    memcpy(&p, reinterpret_cast<const char *>(byref) + at, sizeof p);
+    return p;
+}
+
+// Where a byref object keeps the address that it carries.  No interface says so, so it is looked for: the one word that is the
+// structure's address plus the offset, for several structures and offsets.  0: no word is, or more than one.
+Py_ssize_t where_the_address_lies(PyObject *byref, PyObject *args_type)
+{
+    Py_ssize_t at = 0;
+    for (int round = 0; round < 4; round++) {
+        PyObject *args = PyObject_CallNoArgs(args_type), *ref = args ? PyObject_CallFunction(byref, "Oi", args, 24 * round) : nullptr;
+        Py_buffer buffer = {};
+        Py_ssize_t found = 0;
+        if (ref && PyObject_GetBuffer(args, &buffer, PyBUF_SIMPLE) == 0) {
+            for (Py_ssize_t i = sizeof(PyObject); i + (Py_ssize_t)sizeof(void *) <= Py_TYPE(ref)->tp_basicsize; i += sizeof(void *))
+                if (address_in(ref, i) == static_cast<const char *>(buffer.buf) + 24 * round)
+                    found = found == 0 ? i : -1;
+            PyBuffer_Release(&buffer);
+        }
+        Py_XDECREF(ref);
+        Py_XDECREF(args);
+        PyErr_Clear();
+        if (found <= 0 || (at != 0 && found != at))
+            return 0;
+        at = found;
+    }
+    return at;
+}
 
 // One argument on its way from Python; false: not plain
 template <typename T, typename = void> struct Arg {
@@ -84,13 +117,14 @@ template <typename P> struct Arg<P *, std::enable_if_t<!std::is_same<P, const cl
     void done() {}
 };
 
-// byref(args): the structure lies in the buffer of the object that it refers to
+// byref(args): the structure lies in the buffer of the object that it refers to, unless byref was given an offset: only where the
+// address that it carries is the buffer's.
 template <> struct Arg<const clpk_gemm_args_t *> {
     const clpk_gemm_args_t *v = nullptr;
     Py_buffer buffer = {};
     bool from(const Call *call, PyObject *o)
     {
-        if (Py_TYPE(o) != call->byref_type)
+        if (Py_TYPE(o) != call->byref_type || call->address_at == 0)
             return false;
         static PyObject *const name = PyUnicode_InternFromString("_obj");
         PyObject *args = PyObject_GetAttr(o, name);
@@ -104,7 +138,7 @@ template <> struct Arg<const clpk_gemm_args_t *> {
             ok = false;
         }
         Py_DECREF(args);                                     // the buffer holds the object
-        if (ok && buffer.len != (Py_ssize_t)sizeof(clpk_gemm_args_t)) {
+        if (ok && (buffer.len != (Py_ssize_t)sizeof(clpk_gemm_args_t) || address_in(o, call->address_at) != buffer.buf)) {
             done();
             ok = false;
         }
@@ -181,13 +215,13 @@ void call_dealloc(PyObject *self)
 
 PyTypeObject CallType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-// bind(name, address, slow, failed, byref type, args type): the call, or None for a name that has none here
+// bind(name, address, slow, failed, byref, its type, args type): the call, or None for a name that has none here
 PyObject *bind(PyObject *, PyObject *args)
 {
     const char *name;
     unsigned long long address;
-    PyObject *slow, *failed, *byref_type, *args_type;
-    if (!PyArg_ParseTuple(args, "sKOOO!O!", &name, &address, &slow, &failed, &PyType_Type, &byref_type, &PyType_Type, &args_type))
+    PyObject *slow, *failed, *byref, *byref_type, *args_type;
+    if (!PyArg_ParseTuple(args, "sKOOOO!O!", &name, &address, &slow, &failed, &byref, &PyType_Type, &byref_type, &PyType_Type, &args_type))
         return nullptr;
     for (const auto &c : kCalls)
         if (strcmp(c.name, name) == 0) {
@@ -200,6 +234,7 @@ PyObject *bind(PyObject *, PyObject *args)
             call->failed = Py_NewRef(failed);
             call->byref_type = reinterpret_cast<PyTypeObject *>(Py_NewRef(byref_type));
             call->gemm_args_type = reinterpret_cast<PyTypeObject *>(Py_NewRef(args_type));
+            call->address_at = where_the_address_lies(byref, args_type);
             PyObject_GC_Track(reinterpret_cast<PyObject *>(call));
             return reinterpret_cast<PyObject *>(call);
         }

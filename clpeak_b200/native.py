@@ -205,7 +205,7 @@ class Kernels:
                 failed(rc)
         if _calls() is None:
             return call
-        return _calls().bind(name, C.cast(fn, C.c_void_p).value, call, failed, type(C.byref(C.c_int())), GemmArgs) or call
+        return _calls().bind(name, C.cast(fn, C.c_void_p).value, call, failed, C.byref, type(C.byref(C.c_int())), GemmArgs) or call
 
     def last_error(self) -> str:
         return (self.lib.clpk_last_error() or b"").decode()

@@ -44,6 +44,28 @@ def test_the_same_answer_as_through_ctypes(K, name, args):
     assert outcome(getattr(K, name), args) == outcome(lambda *a: K.call(name, *a), args)
 
 
+@C.CFUNCTYPE(C.c_int, C.POINTER(N.GemmArgs), C.c_void_p)
+def tells_m(args, stream):
+    return args[0].m if args else -1
+
+
+def test_the_structure_that_a_byref_names(K):
+    """A byref may carry an offset: what it passes then is not the structure that it refers to."""
+    array = (N.GemmArgs * 3)(*(N.GemmArgs(m=m) for m in (5, 6, 7)))
+    inside = N.GemmArgs.from_buffer(array, C.sizeof(N.GemmArgs))
+    named = [(C.byref(array[0]), 5), (C.byref(array[0], 0), 5), (C.byref(array[0], C.sizeof(N.GemmArgs)), 6), (C.byref(array[1]), 6),
+             (C.byref(array[1], C.sizeof(N.GemmArgs)), 7), (C.byref(array[1], -C.sizeof(N.GemmArgs)), 5), (C.byref(array[2], -C.sizeof(N.GemmArgs)), 6),
+             (C.byref(inside), 6), (C.byref(inside, C.sizeof(N.GemmArgs)), 7), (C.pointer(array[2]), 7),
+             (C.byref(N.GemmArgs(m=9)), 9), (N.GemmArgs(m=9), 9), (None, -1)]
+    call = K._checked("clpk_gemm", tells_m)
+    for args, m in named:
+        with pytest.raises(N.ClpkError) as e:
+            call(args, None)
+        assert e.value.code == m
+    with pytest.raises(C.ArgumentError):
+        call(C.byref(array, C.sizeof(N.GemmArgs)), None)
+
+
 def test_errors_of_several_threads_at_once(K):
     wrong = []
 
