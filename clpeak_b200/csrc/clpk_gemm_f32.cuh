@@ -65,6 +65,20 @@ constexpr uint32_t kF32BoxLd = 20;                       // floats per row of a 
 constexpr float kF32Scale = 0x1p16f;                     // of the elements of A and of B
 constexpr float kF32Unscale = 0x1p-32f;                  // of the sums, when they leave the registers
 
+// A wait tells the last two phases of a barrier apart, no more: whoever waits for one has to know that the phase before it is
+// complete, and those who take turns know that only of what they have waited for themselves.
+//  * A group of converters comes to every second chunk: raw stages in an even number, so that a stage is always the same group's.
+//  * Converted stages may be an odd number, since their barriers are not the stage's but come round after kF32Bars chunks.  An issuing
+//    warp, whose turns are of one chunk at the end of a range, has waited for a chunk of either group among the six before.
+//    Nobody arrives for a chunk before the barrier's phase before is complete: a chunk is converted when the one conv_stages in front
+//    has been consumed, whose group had seen the same, and so on back.
+//  * An issuing warp waits for an accumulator at every second turn, and all accumulators are given back in the order of the turns.
+// With a barrier for each of five (or seven) stages a late load or a late converter let the other group's or warp's wait end a round
+// too early.  (160 random shapes: 0.985 of that form's time at 32 and 96 columns, 0.995 at 64, 1.005 at 128; barriers of the raw stages that
+// come round after 16 chunks as well 1.01 at 128 and 1.015 at 96.)
+constexpr uint32_t kF32Bars = 16;
+static_assert(kF32Bars % kF32Groups == 0 && kF32Bars >= 6, "waits that cannot end a round too early");
+
 template <uint32_t TN> struct F32Tile {
     static constexpr uint32_t half_n = TN / 2;
     static constexpr uint32_t a_bytes = 128 * 128;
@@ -73,9 +87,10 @@ template <uint32_t TN> struct F32Tile {
     static constexpr uint32_t a_cols = 48;                               // h, m, l of 32 floats: 16 columns each
     static constexpr uint32_t conv_stages = TN == 96 ? 4 : 5;             // what tensor memory has room for
     static constexpr uint32_t accs = TN <= 64 ? 4 : TN == 96 ? 3 : 2;
-    static constexpr uint32_t raw_stages = TN <= 64 ? 8 : TN == 96 ? 7 : 5;
+    static constexpr uint32_t raw_stages = TN <= 64 ? 8 : 6;
     static constexpr uint32_t tmem_cols = accs * TN + conv_stages * a_cols > 256 ? 512 : 256;
     static_assert(accs * TN + conv_stages * a_cols <= 512, "tensor memory");
+    static_assert(raw_stages % kF32Groups == 0 && 2 * conv_stages <= kF32Bars, "see kF32Bars");
     static constexpr uint32_t box_bytes = 32 * kF32BoxLd * 4;
     // registers a thread of the issuing, the converting and the adding warps; at 64 columns 72 and 152 take 7 % longer
     static constexpr uint32_t issue_regs = 32, converter_regs = 80, sum_regs = 144;
@@ -86,11 +101,14 @@ template <uint32_t TN> struct F32Tile {
 
 struct F32Smem {
     uint64_t raw_full[8], raw_empty[8];
-    uint64_t conv_full[5], conv_empty[5];
+    uint64_t conv_full[kF32Bars], conv_empty[kF32Bars];
     uint64_t d_full[4], d_empty[4];
     uint32_t tmem_base;
 };
 static_assert(sizeof(F32Smem) <= 512, "the room that F32Tile leaves for it");
+
+// Parity of a chunk's phase.  Below zero that is the phase in front of a fresh barrier's, which counts as complete.
+__device__ __forceinline__ uint32_t chunk_parity(uint32_t chunk) { return chunk / kF32Bars & 1; }
 
 struct F32Maps {
     CUtensorMap a, b;
@@ -372,9 +390,9 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
             mbar_init(&sh->raw_full[s], 1);
             mbar_init(&sh->raw_empty[s], 4);
         }
-        for (uint32_t s = 0; s < T::conv_stages; s++) {
-            mbar_init(&sh->conv_full[s], 2 * 4);
-            mbar_init(&sh->conv_empty[s], 1);
+        for (uint32_t i = 0; i < kF32Bars; i++) {
+            mbar_init(&sh->conv_full[i], 2 * 4);
+            mbar_init(&sh->conv_empty[i], 1);
         }
         for (uint32_t d = 0; d < T::accs; d++) {
             mbar_init(&sh->d_full[d], 1);
@@ -441,9 +459,10 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                     const bool two = c + 1 < c1;
                     if ((turn & 1) == (uint32_t)warp - 1) {
                         const uint32_t d = turn % T::accs, s0 = chunk % T::conv_stages, s1 = (chunk + 1) % T::conv_stages;
+                        const uint32_t bar0 = chunk % kF32Bars, bar1 = (chunk + 1) % kF32Bars;
                         // a fresh barrier's preceding phase counts as complete
-                        if (!warp_wait_two(&sh->d_empty[d], (turn / T::accs + 1) & 1, &sh->conv_full[s0], (chunk / T::conv_stages) & 1) ||
-                            (two && !warp_wait_one(&sh->conv_full[s1], ((chunk + 1) / T::conv_stages) & 1))) {
+                        if (!warp_wait_two(&sh->d_empty[d], (turn / T::accs + 1) & 1, &sh->conv_full[bar0], chunk_parity(chunk)) ||
+                            (two && !warp_wait_one(&sh->conv_full[bar1], chunk_parity(chunk + 1)))) {
                             give_up(0x233u);
                             ok = false;
                             break;
@@ -476,10 +495,10 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                                 multiply(s1, 0, 1);
                             }
                             multiply(s0, 0, 0);
-                            tc_commit_pair(&sh->conv_empty[s0], pair_mask);
+                            tc_commit_pair(&sh->conv_empty[bar0], pair_mask);
                             if (two) {
                                 multiply(s1, 0, 0);
-                                tc_commit_pair(&sh->conv_empty[s1], pair_mask);
+                                tc_commit_pair(&sh->conv_empty[bar1], pair_mask);
                             }
                             tc_commit_pair(&sh->d_full[d], pair_mask);
                         }
@@ -503,7 +522,8 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                 if (count % kF32Groups != group)
                     continue;
                 const uint32_t raw = count % T::raw_stages, s = count % T::conv_stages;
-                const bool there = cw != 0 || warp_wait_two(&sh->raw_full[raw], (count / T::raw_stages) & 1, &sh->conv_empty[s], (count / T::conv_stages + 1) & 1);
+                const bool there = cw != 0 || warp_wait_two(&sh->raw_full[raw], (count / T::raw_stages) & 1,
+                                                            &sh->conv_empty[(count - T::conv_stages) % kF32Bars], chunk_parity(count - T::conv_stages));
                 if (!team_agrees<128>(2 + group, there)) {
                     give_up(0x234u);
                     ok = false;
@@ -559,7 +579,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) gemm_f32_kernel(const __grid_c
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(&sh->raw_empty[raw]);
-                    mbar_arrive_remote(full0 + 8 * s);
+                    mbar_arrive_remote(full0 + 8 * (count % kF32Bars));
                 }
             }
         }
