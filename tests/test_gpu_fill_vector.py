@@ -139,6 +139,26 @@ def test_absmax_lengths(K, cuda, orc, n, offset):
     assert float(out.item()) == 9.5
 
 
+@pytest.mark.parametrize("n,offset", [(25 << 20, 0), ((25 << 20) + 1, 0), ((25 << 20) + 4099, 3)])
+def test_absmax_of_arrays_beyond_the_cache(K, cuda, n, offset):
+    """From 100 MiB on the array is read from its end, by a kernel of its own: the largest magnitude is found wherever it lies."""
+    src = cuda.zeros(n + offset, dtype=cuda.float32, device="cuda")
+    K.clpk_fill_f32(src.data_ptr(), n + offset, 8, N.DIST_UNIFORM_PM1, 0.0, 1.0, stream_ptr())
+    out = cuda.empty(1, dtype=cuda.float32, device="cuda")
+    for at in (None, 0, 1, 8, n // 2, n - 8193, n - 9, n - 2, n - 1):
+        if at is not None:
+            src[offset + at] = -2.0 - at / n
+        want = float(src[offset:].abs().max())
+        out.fill_(1e9)
+        K.clpk_absmax_f32(out.data_ptr(), src.data_ptr() + 4 * offset, n, stream_ptr())
+        assert float(out.item()) == want
+        if at is not None:
+            src[offset + at] = float("nan")                         # ignored, as fmaxf does
+            K.clpk_absmax_f32(out.data_ptr(), src.data_ptr() + 4 * offset, n, stream_ptr())
+            assert float(out.item()) < want
+            src[offset + at] = 0.0
+
+
 BLOCK = {N.DT_MXF4: 32, N.DT_MXF4_B64: 64, N.DT_NVF4: 16, N.DT_NVF4_B32: 32}
 
 
@@ -180,6 +200,22 @@ def test_quantize_generated_operands(K, orc, cuda, dtype):
     rows, cols = 2048, 2048
     x = orc.fill_f32(rows * cols, 40, N.DIST_NORMAL, 0.0, 0.02)
     ts = float(np.float32(np.abs(x).max()) / np.float32(6.0 * 448.0)) if dtype == N.DT_NVF4 else 1.0
+    want_packed, want_scales = orc.quantize_fp4(x.reshape(rows, cols), dtype, ts)
+    src = cuda.from_numpy(x).cuda()
+    packed, scales = dev_empty(rows * cols // 2, cuda.uint8), dev_empty(rows * cols // BLOCK[dtype], cuda.uint8)
+    K.clpk_quantize_fp4(packed.data_ptr(), scales.data_ptr(), src.data_ptr(), rows, cols, dtype, ts, stream_ptr())
+    sync()
+    assert_bits_equal(to_np(scales), want_scales.ravel(), "fp4 scales")
+    assert_bits_equal(to_np(packed), want_packed.ravel(), "fp4 codes")
+
+
+@pytest.mark.parametrize("rows,cols", [(25600, 1024), (409, 65600)])
+@pytest.mark.parametrize("dtype", list(BLOCK))
+def test_quantize_operands_beyond_the_cache(K, orc, cuda, dtype, rows, cols):
+    """From 100 MiB on kernels of their own read the source as lines that leave the cache first, the MX kinds from its end."""
+    x = orc.fill_f32(rows * cols, 40, N.DIST_NORMAL, 0.0, 0.02)
+    ts = float(np.float32(np.abs(x).max()) / np.float32(6.0 * 448.0)) if dtype in (N.DT_NVF4, N.DT_NVF4_B32) else 1.0
+    x[rows * cols - 70:rows * cols - 3], x[:64:3], x[4096:4160] = 0.0, -0.0, np.float32(1e-42)
     want_packed, want_scales = orc.quantize_fp4(x.reshape(rows, cols), dtype, ts)
     src = cuda.from_numpy(x).cuda()
     packed, scales = dev_empty(rows * cols // 2, cuda.uint8), dev_empty(rows * cols // BLOCK[dtype], cuda.uint8)
