@@ -7,8 +7,8 @@ Outputs (all under clpeak_b200/_lib/, which is not tracked):
                              B200 backend) behind the clpeak_ffi C ABI of
                              include/clpeak_ffi.h
   clpeak                     the command-line front end
-  _clpk_calls.so             calls into the kernels from Python without ctypes between
-                             (only where the interpreter's headers are installed)
+  _clpk_calls.<abi>.so       calls into the kernels from Python without ctypes between, for the interpreter that
+                             builds (only where its headers are installed)
 
 Only sm_100a code is generated.  Run as `python -m clpeak_b200.build`.
 """
@@ -120,14 +120,18 @@ def build_host(force: bool = False) -> list[Path]:
 
 
 def build_calls(force: bool = False) -> Path | None:
+    src, header = CSRC / "python" / "calls.cpp", ROOT / "include" / "clpeak_b200_kernels.h"
+    out = LIB / ("_clpk_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+    if not force and not _stale(out, [src, header]):
+        return out
+    # what was built from other sources must not stay in use where it cannot be built again
+    out.unlink(missing_ok=True)
     inc = Path(sysconfig.get_paths()["include"])
     if not (inc / "Python.h").exists():
         return None
-    src, header, out = CSRC / "python" / "calls.cpp", ROOT / "include" / "clpeak_b200_kernels.h", LIB / "_clpk_calls.so"
     LIB.mkdir(parents=True, exist_ok=True)
-    if force or _stale(out, [src, header]):
-        cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
-        _run([cxx, *CXX_FLAGS, "-shared", "-I", str(inc), "-I", str(ROOT / "include"), str(src), "-o", str(out)])
+    cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
+    _run([cxx, *CXX_FLAGS, "-shared", "-I", str(inc), "-I", str(ROOT / "include"), str(src), "-o", str(out)])
     return out
 
 

@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes as C
 import importlib.machinery
 import importlib.util
+import sysconfig
 from functools import lru_cache
 from pathlib import Path
 
@@ -167,8 +168,9 @@ EVENT_CALLBACK = C.CFUNCTYPE(None, C.c_void_p, C.c_void_p)
 
 @lru_cache(maxsize=None)
 def _calls():
-    """The extension with the calls that are made once per launch (csrc/python/calls.cpp), None where it has not been built."""
-    path = LIB_DIR / "_clpk_calls.so"
+    """The extension with the calls that are made once per launch (csrc/python/calls.cpp), None where it has not been built for this
+    interpreter."""
+    path = LIB_DIR / ("_clpk_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
     if not path.exists():
         return None
     loader = importlib.machinery.ExtensionFileLoader("_clpk_calls", str(path))

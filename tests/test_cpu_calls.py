@@ -1,11 +1,14 @@
 """Calls past ctypes answer as the ctypes wrapper does: plain arguments, arguments that only ctypes converts, and those it refuses.
 Nothing is launched: no element, a NULL buffer, or no such type."""
 import ctypes as C
+import os
+import sysconfig
 import threading
 
 import numpy as np
 import pytest
 
+from clpeak_b200 import build
 from clpeak_b200 import native as N
 
 FAST = N._calls()
@@ -81,3 +84,25 @@ def test_errors_of_several_threads_at_once(K):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_an_extension_of_another_interpreter_is_not_loaded(tmp_path, monkeypatch):
+    for name in ("_clpk_calls.so", "_clpk_calls.cpython-39-x86_64-linux-gnu.so", "_clpk_calls.abi3.so"):
+        (tmp_path / name).write_bytes(b"not for this one")
+    monkeypatch.setattr(N, "LIB_DIR", tmp_path)
+    assert N._calls.__wrapped__() is None
+
+
+@pytest.mark.parametrize("headers", [False, True])
+def test_an_extension_of_older_sources_does_not_stay(tmp_path, monkeypatch, headers):
+    old = tmp_path / ("_clpk_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+    old.write_bytes(b"older than its sources")
+    os.utime(old, (0, 0))
+    monkeypatch.setattr(build, "LIB", tmp_path)
+    if not headers:
+        monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+        assert build.build_calls() is None and not old.exists()
+    else:
+        assert build.build_calls() == old and old.read_bytes()[:4] == b"\x7fELF"
+        built = old.stat().st_mtime_ns
+        assert build.build_calls() == old and old.stat().st_mtime_ns == built
