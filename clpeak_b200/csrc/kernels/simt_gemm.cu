@@ -743,10 +743,10 @@ static int launch_simt(void (*kernel)(Params...), const char *what, uint64_t cta
     return CLPK_OK;
 }
 
-// Tile edge and K ranges for a problem (128: sgemm_kernel, and dgemm_kernel, whose tiles are 64 wide, with an even N): the cheapest
-// by an estimate in microseconds, fitted to 400 timed launches of all kernels on 90 shapes (M and N from 64 to 15000, K to 16000;
-// residuals 5 to 9 %, 13 % for the 32-wide fp64 tile; the chosen plans are 2 to 3 % slower than the fastest in the geometric
-// mean), and dgemm_kernel's to 400 more (4 %).  With L CTAs on the busiest SM, a block of 16 k costs its CTA  max(alone, L * shared):
+// Kernel, tile edge and K ranges for a problem: the cheapest by an estimate in microseconds, fitted to 400 timed launches of all
+// kernels on 90 shapes (M and N from 64 to 15000, K to 16000; residuals 5 to 9 %, 13 % for the 32-wide fp64 tile; the chosen plans
+// are 2 to 3 % slower than the fastest in the geometric mean), and dgemm_kernel's to 400 more (4 %).  With L CTAs on the busiest
+// SM, a block of 16 k costs its CTA  max(alone, L * shared):
 //   fp32  128 x 128  max(1.62, 1.43 L)    64 x 64  max(0.51, 0.40 L)    (the pipe's own time: 1.07 and 0.27 L)
 //   fp64  whole 64 x 64  max(0.75, 0.607 L)    split 64 x 64  max(0.91, 0.62 L)    32 x 32  max(0.22, 0.16 to 0.174 L, the less the
 //   longer)    (0.54, 0.54, 0.13 L)
@@ -758,11 +758,8 @@ struct SimtPlan {
     uint32_t tile, splits;
     bool wide;                  // twice the K groups
     float us = 0.0f;            // the estimate it was chosen by (fp32 and long fp64 sums)
-    bool whole = false;         // dgemm_kernel
+    bool whole = false;         // sgemm_kernel or dgemm_kernel
 };
-
-// What clpk_gemm_plan says of dgemm_kernel's tiles: 64 where C goes through shared memory (an odd N), else that they are its own.
-static SimtPlan whole_f64_plan(uint32_t n, float us) { return {n % 2 ? 64u : 128u, 1, false, us, true}; }
 
 // dgemm_kernel is not considered for fewer tiles than two SMs of three have one.  32-wide tiles serve most of those better, up to
 // three times; not all of them (1481 x 215 x 40: 5.9 us, 4.5 in 64-wide ones).
@@ -790,7 +787,7 @@ static SimtPlan plan_short_f64(uint32_t m, uint32_t n, uint32_t blocks)
     float best = 1e30f;
     if (whole_f64_tiles(m, n)) {
         best = 0.97f * (2.75f + rounds(per_sm(64, 64, 1), 4, 0.785f * (float)blocks - 0.71f, 0.587f * (float)blocks + 0.36f));
-        plan = whole_f64_plan(n, best);
+        plan = {kDgemmTile, 1, false, best, true};
     }
     for (uint32_t splits = 1; splits <= 4 && (splits == 1 || blocks >= 4 * splits); splits *= 2)
         for (uint32_t tile = 32; tile <= (splits == 1 ? 32u : 64u); tile *= 2) {
@@ -821,13 +818,15 @@ static SimtPlan plan_simt(bool f64, uint32_t m, uint32_t n, uint32_t k)
     if (!f64) {
         const float large = 2.0f + estimate(128, 128, 1, 1.62f, 1.43f);
         best = 0.92f * large;
-        plan = {128, 1, false, large};
+        plan = {kSimtTile, 1, false, large, true};
     } else if (whole_f64_tiles(m, n)) {
         best = 3.2f + estimate(64, 64, 1, 0.75f, 0.607f);
-        plan = whole_f64_plan(n, best);
+        plan = {kDgemmTile, 1, false, best, true};
     }
     for (uint32_t splits = 1; splits <= 8 && (splits == 1 || blocks >= 4 * splits); splits *= 2)
-        for (uint32_t tile = f64 ? 32 : 64; tile <= 64; tile *= 2) {
+        // (fp64 in one range: dgemm_kernel's estimate is below the other 64-wide tiles' wherever it is considered, and where it is
+        // not, an SM has three 32-wide tiles at most, which are cheaper too)
+        for (uint32_t tile = f64 ? 32 : 64; tile <= (f64 && splits == 1 ? 32u : 64u); tile *= 2) {
             const bool wide = !(f64 && tile == 64) && ctas(tile, tile, splits) <= simt_capacity(splits) && blocks >= (f64 ? 24 : 32) * splits;
             float t;
             if (!f64)
@@ -852,7 +851,7 @@ float simt_f32_estimate(uint32_t m, uint32_t n, uint32_t k) { return plan_simt(f
 void simt_gemm_plan(bool f64, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile_n, uint32_t *splits, uint32_t *wide)
 {
     const SimtPlan plan = plan_simt(f64, m, n, k);
-    *tile_n = plan.tile == 128 ? 0 : plan.tile;
+    *tile_n = plan.whole ? 0 : plan.tile;
     *splits = plan.splits;
     *wide = plan.wide ? 1 : 0;
 }
@@ -886,7 +885,7 @@ int launch_simt_gemm(int dtype, const void *a, const void *b, void *c, uint32_t 
     if (dtype == CLPK_DT_F32) {
         const float *fa = static_cast<const float *>(a), *fb = static_cast<const float *>(b);
         float *fc = static_cast<float *>(c);
-        if (plan.tile == 64)
+        if (!plan.whole)
             return plan.wide ? launch_simt(sgemm64_kernel<4>, "launch sgemm64", ctas, 4 * kSgemm64GroupThreads, kSgemm64SmemBytes<4>, plan.splits, false, s, fa, fb,
                                        fc, m, n, k, alpha, plan.splits, status)
                          : launch_simt(sgemm64_kernel<2>, "launch sgemm64", ctas, 2 * kSgemm64GroupThreads, kSgemm64SmemBytes<2>, plan.splits, true, s, fa, fb,

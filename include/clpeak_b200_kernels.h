@@ -454,10 +454,11 @@ CLPK_API int clpk_gemm_workspace_bytes(int dtype, uint32_t m, uint32_t n, uint32
 CLPK_API int clpk_gemm_pack_scales(const clpk_gemm_args_t *args, void *stream);
 CLPK_API int clpk_gemm(const clpk_gemm_args_t *args, void *stream);
 /* How clpk_gemm splits a problem of these sizes on the current device: the tile's width in columns and the number of
- * K ranges.  A width of 0 is the kernel for large shapes, whose tiles are its own.  For CLPK_DT_F32 and CLPK_DT_F64
- * tiles are square; *wide (may be NULL) is 1 where a CTA takes twice the K groups, and 2 where an fp32 product runs on the
- * tensor cores, in tiles of 256 rows.  Tiles of the dense tensor kinds have 256 rows, 512 where *wide is 1.  For the FP4 kinds: of a call without
- * scale pointers.  Lets a benchmark or a test record which kernel it ran; needs no GPU work. */
+ * K ranges.  A width of 0 is the kernel whose tiles are its own: that for large shapes, and for CLPK_DT_F64 that with K
+ * whole (64 x 64 tiles), whatever N.  For CLPK_DT_F32 and CLPK_DT_F64 tiles are square; *wide (may be NULL) is 1 where a CTA
+ * takes twice the K groups, and 2 where an fp32 product runs on the tensor cores, in tiles of 256 rows.  Tiles of the dense
+ * tensor kinds have 256 rows, 512 where *wide is 1.  For the FP4 kinds: of a call without scale pointers.  Lets a benchmark
+ * or a test record which kernel it ran; needs no GPU work. */
 CLPK_API int clpk_gemm_plan(int dtype, uint32_t m, uint32_t n, uint32_t k, uint32_t *tile_n, uint32_t *splits, uint32_t *wide);
 /* 1 if the calling thread's last clpk_gemm launch ran with the per-wave producer meeting, 0 if
  * it ran without (small problem, knob), -1 before any launch.  Lets a benchmark record which schedule it timed. */

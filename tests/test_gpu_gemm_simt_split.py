@@ -47,24 +47,34 @@ def test_every_plan(K, cuda, dtype, plan, shape):
     check_every_element(K, cuda, dtype, *shape)
 
 
-# short fp64 sums: shapes that 32-wide tiles made 1.1 to 2.5 times slower than the large ones take those or 64-wide ones,
-# an odd N also in more CTAs than run at once, and shapes that small tiles serve best keep them
-@pytest.mark.parametrize("tile,shape", [(0, (4153, 558, 6)), (0, (2888, 782, 2)), (0, (12879, 166, 12)), (0, (11657, 120, 14)), (64, (394, 15109, 38)),
-                                        (64, (963, 955, 248)), (0, (12127, 1916, 10)), (64, (1674, 807, 4)), (32, (863, 251, 248)), (32, (64, 64, 128)),
-                                        (64, (661, 6775, 24)), (32, (1481, 215, 40))])
+# short fp64 sums: shapes that 32-wide tiles made 1.1 to 2.5 times slower take the kernel with K whole, an odd N also in more CTAs than
+# run at once, and shapes that small tiles serve best keep them
+@pytest.mark.parametrize("tile,shape", [(0, (4153, 558, 6)), (0, (2888, 782, 2)), (0, (12879, 166, 12)), (0, (11657, 120, 14)), (0, (394, 15109, 38)),
+                                        (0, (963, 955, 248)), (0, (12127, 1916, 10)), (0, (1674, 807, 4)), (32, (863, 251, 248)), (32, (64, 64, 128)),
+                                        (0, (661, 6775, 24)), (32, (1481, 215, 40))])
 def test_short_fp64_sums(K, cuda, tile, shape):
     assert gemm_plan(K, N.DT_F64, *shape)[0] == tile
     check_every_element(K, cuda, N.DT_F64, *shape)
 
 
-# fp64 with K whole in 64 x 64 tiles: whole tiles, ragged ones with an even N and with an odd one (whose C goes through shared memory,
-# and whose plan says so), sums of one block to more than the ring holds and with every remainder of a block's pieces
-@pytest.mark.parametrize("tile,m,n", [(0, 640, 704), (0, 641, 702), (64, 639, 705), (0, 7000, 2), (64, 6401, 1), (0, 63, 6402), (64, 65, 6465)])
-@pytest.mark.parametrize("k", [2, 16, 18, 32, 46, 48, 50, 64, 464])
-def test_whole_fp64_tiles(K, cuda, tile, m, n, k):
-    if k < 384 and gemm_plan(K, N.DT_F64, m, n, k)[0] != 32:
-        assert gemm_plan(K, N.DT_F64, m, n, k) == (tile, 1, 0)
+# fp64 with K whole in 64 x 64 tiles: whole tiles, ragged ones with an even N and with an odd one (whose C goes through shared memory),
+# sums of one block to more than the ring holds and with every remainder of a block's pieces
+WHOLE = [(m, n, k) for m, n in ((640, 704), (641, 702), (639, 705), (7000, 2), (6401, 1), (63, 6402), (65, 6465)) for k in (2, 16, 18, 32, 46, 48, 50, 64)]
+WHOLE += [(641, 702, 368), (639, 705, 368), (2048, 2048, 464), (2047, 2046, 466), (2046, 2047, 1042)]
+
+
+@pytest.mark.parametrize("m,n,k", WHOLE)
+def test_whole_fp64_tiles(K, cuda, m, n, k):
+    assert gemm_plan(K, N.DT_F64, m, n, k) == (0, 1, 0)
     check_every_element(K, cuda, N.DT_F64, m, n, k)
+
+
+# beside them, the same sizes with K split or in 32-wide tiles
+@pytest.mark.parametrize("plan,shape", [((64, 2, 0), (641, 702, 464)), ((64, 2, 0), (639, 705, 464)), ((64, 2, 0), (65, 6465, 368)), ((32, 1, 0), (640, 704, 464)),
+                                        ((32, 1, 0), (7000, 2, 96)), ((32, 2, 0), (6401, 1, 464)), ((32, 1, 0), (63, 6402, 464))])
+def test_fp64_beside_whole_tiles(K, cuda, plan, shape):
+    assert gemm_plan(K, N.DT_F64, *shape) == plan
+    check_every_element(K, cuda, N.DT_F64, *shape)
 
 
 def check_every_element(K, cuda, dtype, m, n, k):
