@@ -72,6 +72,31 @@ def test_scales_arranged_on_the_way_and_in_front(K, cuda, dtype, offset, m, n, k
     assert bool((on_the_way == in_front).all()), "the workspace holds the arranged scales afterwards"
 
 
+# both sides of each line: four waves of 74 tiles of 256 x 256; NVFP4 sums of more than 40 K blocks over all waves, in the first wave only
+# where a scale array is not aligned to a K block's words
+@pytest.mark.parametrize("launches,dtype,offset,m,n,k",
+                         [(1, N.DT_NVF4, 0, 2048, 2048, 2048), (1, N.DT_NVF4, 0, 2048, 2048, 16384), (2, N.DT_NVF4, 4, 2048, 2048, 16384),
+                          (1, N.DT_NVF4, 4, 2048, 2048, 10240), (1, N.DT_NVF4, 0, 2304, 2304, 5120), (2, N.DT_NVF4, 0, 2304, 2304, 5376),
+                          (1, N.DT_NVF4, 0, 4352, 4352, 2560), (2, N.DT_NVF4, 0, 4352, 4352, 2816), (2, N.DT_NVF4, 0, 4352, 4608, 256),
+                          (1, N.DT_NVF4, 0, 64, 64, 256), (1, N.DT_MXF4, 0, 2304, 2304, 5376), (1, N.DT_MXF4, 4, 2048, 2048, 16384),
+                          (1, N.DT_MXF4, 4, 4352, 4352, 16384), (2, N.DT_MXF4, 0, 4352, 4608, 256)])
+def test_launches_of_a_call_with_row_major_scales(K, cuda, launches, dtype, offset, m, n, k):
+    if cuda.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the waves are those of 148 SMs")
+    block = 16 if dtype == N.DT_NVF4 else 32
+    a, b, sfa, sfb = (cuda.zeros(size, dtype=cuda.uint8, device="cuda") for size in (m * k // 2, n * k // 2, m * k // block + offset, n * k // block + offset))
+    c, status, ws = cuda.zeros(m * n, dtype=cuda.int16, device="cuda"), cuda.zeros(1, dtype=cuda.int32, device="cuda"), workspace(K, cuda, dtype, m, n, k)
+    args = N.GemmArgs(dtype=dtype, m=m, n=n, k=k, d_a=a.data_ptr(), d_b=b.data_ptr(), d_c=c.data_ptr(), d_sfa=sfa.data_ptr() + offset,
+                      d_sfb=sfb.data_ptr() + offset, alpha=1.0, d_workspace=ws.data_ptr(), workspace_bytes=ws.numel(), d_status=status.data_ptr())
+    K.clpk_gemm(C.byref(args), stream_ptr())
+    sync()
+    graph, stream, nodes = cuda.cuda.CUDAGraph(keep_graph=True), cuda.cuda.Stream(), C.c_size_t(0)
+    with cuda.cuda.graph(graph, stream=stream):
+        K.clpk_gemm(C.byref(args), stream.cuda_stream)
+    assert C.CDLL("libcuda.so.1").cuGraphGetNodes(C.c_void_p(graph.raw_cuda_graph()), None, C.byref(nodes)) == 0
+    assert nodes.value == launches
+
+
 def decoded(cuda, dtype, q, sf, rows, k):
     """The operand's values in fp64."""
     codes = cuda.stack((q & 15, q >> 4), dim=-1).view(rows, k).long()
