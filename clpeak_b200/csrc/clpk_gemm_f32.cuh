@@ -40,8 +40,8 @@
 // cycles at TN = 32 and 890 at 128, a whole turn of one chunk 1060: without the arithmetic of the conversion (12 issue slots of an
 // SM quarter for a pair of floats) 880, without the additions 1000, with two of the 12 instructions 1000.  The tensor pipe is busy
 // for 73 % of the cycles of a 2304 x 4096 x 2048 product, issue slots 54 %; from about 300 us on the power cap takes the clock down to
-// 1.4 GHz and with it what is left to gain.  Device time against the CUDA-core kernels: 4096^3 2251 -> 599 us back to back (229 TFLOPS),
-// 688 between inputs that change (200); 2317 x 6252 x 516 338 -> 92, 1636 x 116 x 4084 62 -> 23, 459 x 349 x 4636 70 -> 24; 9019
+// 1.4 GHz and with it what is left to gain.  Device time against the CUDA-core kernels: 4096^3 2251 -> 570 to 650 us back to back
+// (210 to 240 TFLOPS, by the clock), 690 between inputs that change (199); 2317 x 6252 x 516 338 -> 92, 1636 x 116 x 4084 62 -> 23, 459 x 349 x 4636 70 -> 24; 9019
 // random shapes that take this kernel 0.40 in the geometric mean.  Pieces with scales of their own and four conversion stages
 // (14 or more slots a pair): 3 % longer at 128 columns, 4 at 96, 7 at 32.
 // Earlier forms at 4096^3, TN = 128, with pieces at their own size (658 in the end): hand-overs by .release.cluster arrives and a
@@ -270,7 +270,7 @@ __device__ __forceinline__ bool team_agrees(uint32_t barrier, bool ok)
 //
 // Bound by latency: two warps per scheduler, the fp32 pipe half busy; 128 x 128 x 4096 take 620 us, 500 where few warps take part.
 // Before, each lane streamed its own row of A, again for every second column: 4096^3 with one NaN in A 5.0 -> 1.1 ms, one in every
-// 128 rows 23.8 -> 4.1, A all NaN 40.4 -> 0.6, results beyond 2^89 throughout 40.4 -> 4.9; the CUDA-core kernel takes 2.3 for each.
+// 128 rows 23.8 -> 4.1, A all NaN 40.4 -> 0.6, results beyond the range (now 2^96) throughout 40.4 -> 4.9; the CUDA-core kernel takes 2.3 for each.
 // Fragments loaded one k ahead, steps of 16 k and fewer polls by the waiting warps changed nothing, scalar multiply-adds
 // took 1.3 times as long.
 template <uint32_t TN, bool AGAIN>

@@ -17,7 +17,7 @@
 // What bounds it: a K block (128 bytes of K) costs the issuing warps about 0.12 us whatever the tile -- barrier wait,
 // four instructions, commit -- against 0.17 us of tensor pipe at TN = 256, so narrow tiles are issue-bound and their
 // width is chosen for parallelism; wide ones come within 10 % of the operand traffic's floor.  Below 2 us per K range
-// the launch is the time: 3.5 us from one launch to the next.  Device time, operands in L2, 512 x 256 tiles -> this
+// the launch is the time: 4 to 5 us from one launch's last CTA to the next one's first full stage.  Device time, operands in L2, 512 x 256 tiles -> this
 // kernel: bf16 512 x 256 x 512 10.2 -> 4.4 us, e4m3 1024 x 1024 x 2048 15.0 -> 6.4, bf16 2048^3 25.1 -> 15.3, e4m3
 // 128 x 8192 x 8192 42.4 -> 18.6, bf16 64 x 64 x 16384 147 -> 13.3.  Tried: four K blocks per stage (slower from
 // TN = 64 on), asking the next stage's barrier ahead of the instructions (no effect), clusters of 16 for eight splits

@@ -129,7 +129,7 @@ __device__ __forceinline__ void st_float8(float *p, f32x2 a, f32x2 b, f32x2 c, f
 // Bound by arithmetic: see clpk_rng_fast.cuh.  Eight elements per thread and step, and two steps where the array is long
 // enough to fill the chip all the same: at 2^28 floats 536 against 548 us (normal) and 191 against 268 (uniform, bound by the
 // start of CTAs with one step), the same at 2^22, and one step is better below (normal, 2^20: 3.4 against 4.3).  8192 x 8192:
-// normal 160 -> 136 us, uniform 62 -> 49 (the stores alone would take 41), int8 55 -> 48.
+// normal 160 -> 136 us, uniform 62 -> 49 (the stores alone would take 41), int8 55 -> 47.
 constexpr int kFillF32Threads = 128;
 constexpr uint64_t kTwoStepsFrom = 1 << 19;
 
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kFillThreads) convert_kernel(void *dst, const 
     }
 }
 
-// Bound by memory (8192 x 8192: 111 -> 42 us, 6.4 TB/s, from any address); a CTA takes four accesses per thread of one
+// Bound by memory (8192 x 8192: 111 -> 40 us, 6.6 TB/s, from any address); a CTA takes four accesses per thread of one
 // contiguous range (8 Ki floats), so that the chip walks the array in address order.  SINGLE: one CTA reads everything and
 // writes the result itself; otherwise the CTAs meet in an atomicMax on a word that has been cleared.
 constexpr int kAbsmaxLoads = 4;
@@ -361,8 +361,8 @@ __global__ void __launch_bounds__(kFillThreads) absmax_kernel(float *out, const 
 // holds while nothing under- or overflows: magnitudes and tensor scales within 2^+-60.  A warp that meets any other
 // block (zeros, NaN, infinities) takes the divisions.  NVFP4 codes come from one product with the reciprocal of both divisors, taken
 // a little too small and a little too large; a warp for which the two disagree anywhere (an element within 2^-20 of a tie)
-// does the quotients.  8192 x 8192: NVFP4 171 -> 44 us, MXFP4 270 -> 40; 4096 x 4096, in the L2, with quotients throughout and two
-// codes converted at a time 11.2 and 9.5, now 9.2 and 7.2.
+// does the quotients.  8192 x 8192: NVFP4 171 -> 44 to 47 us, MXFP4 270 -> 40 to 43; 4096 x 4096, in the L2, with quotients throughout and two
+// codes converted at a time 11.2 and 9.5, now 9.2 and 7.2 to 7.8.
 
 // divisor and reciprocal for the whole tensor; plain: outside the range above
 struct TensorScale {

@@ -421,16 +421,17 @@ CLPK_API int clpk_dmma_peak(const double *d_a, const double *d_b, uint32_t n_mma
  * CLPK_DT_F32: small products and short sums run on the CUDA cores (FFMA); the others multiply three bf16 pieces of each
  * element on the tensor cores, over the whole range of fp32, and add sums of 64 products with fp32 rounding.  That leaves a
  * smaller error than K fused multiply-adds, but sums of one sign come out low by up to 8.5e-8 of their size, where FFMA in
- * eight and more short chains leaves 7e-8.  Infinities, NaNs and magnitudes beyond 2^89 are multiplied by FFMA in either
- * case, at half the speed of CLPK_DT_F32_FFMA where they are everywhere.
+ * eight and more short chains leaves 7e-8.  Infinities, NaNs, elements beyond 2^111 and results beyond about 2^96 are
+ * multiplied by FFMA in either case, at half the speed of CLPK_DT_F32_FFMA where they are everywhere.
  * tcgen05 kinds: any M, N, K > 0 such that a row of A / B and a row of C are multiples of 16
  * bytes (partial tiles are computed whole and clipped; whole 512 x 256 tiles and K a multiple
  * of 128 bytes waste nothing).  FP4 kinds: K a multiple of 256; the workspace holds scale
  * blocks for M and N rounded up to multiples of 256.
  * FP4 kinds: d_a/d_b are packed e2m1 (K/2 bytes per row); d_sfa/d_sfb are the
  * scale bytes row-major [rows][K/16] (NVF4) or [rows][K/32] (MXF4) as written by
- * clpk_quantize_fp4; the call repacks them into the tensor-core tile order in
- * d_workspace (clpk_gemm_workspace_bytes) before the main kernel.  Operands that
+ * clpk_quantize_fp4; the call brings them into the tensor-core tile order, in a launch
+ * in front of the main kernel or in that kernel itself, and once it has completed in its
+ * stream d_workspace (clpk_gemm_workspace_bytes) holds them in that order.  Operands that
  * are multiplied more than once can be repacked once: clpk_gemm_pack_scales does
  * only the repack (same arguments; d_a, d_b, d_c, d_status unused), and a
  * clpk_gemm call with d_sfa = d_sfb = NULL takes the workspace as already packed
