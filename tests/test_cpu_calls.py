@@ -69,6 +69,15 @@ def test_the_structure_that_a_byref_names(K):
         call(C.byref(array, C.sizeof(N.GemmArgs)), None)
 
 
+def test_which_structures_go_past_ctypes():
+    went = []
+    call = FAST.bind("clpk_gemm", C.cast(tells_m, C.c_void_p).value, lambda *a: went.append("ctypes"), went.append, C.byref, type(C.byref(C.c_int())), N.GemmArgs)
+    array = (N.GemmArgs * 2)(N.GemmArgs(m=5), N.GemmArgs(m=6))
+    for args in (C.byref(array[1]), C.byref(N.GemmArgs(m=7)), C.byref(array[0], C.sizeof(N.GemmArgs)), array[0]):
+        call(args, None)
+    assert went == [6, 7, "ctypes", "ctypes"]
+
+
 def test_errors_of_several_threads_at_once(K):
     wrong = []
 
